@@ -1,6 +1,6 @@
-// fp32 NCHW convolution with fp32 FMA accumulate: the exact-precision path (max-relative
-// 1e-5 against a double-accumulating CPU result) used where the graph boundary is fp32 and
-// for cross-checking the tensor-core path.  Not the throughput path: that is conv_tc.cu.
+// fp32 NCHW convolution with fp32 FMA accumulate: the exact-precision path (max-relative 1e-5 against a
+// double-accumulating CPU result).  The tiled kernels of conv_f32.cu serve every geometry within their limits
+// (f32_gemm_ok: 32-bit offsets, at most 63 taps); the one-thread-per-output kernels here take what is left.
 #include "common.cuh"
 
 namespace adk {
@@ -150,12 +150,19 @@ static int geometry(const ad_conv2d_args* a, ConvG& g) {
   return AD_OK;
 }
 
+bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane);
+int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
+int f32_gemm_dgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
+int f32_gemm_wgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
+size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q);
+
 int conv_direct_fprop(const ad_conv2d_args* a, cudaStream_t s) {
   ConvG g;
   int st = geometry(a, g);
   if (st != AD_OK) return st;
   if (!a->x || !a->w || !a->y) return AD_ERR_BAD_ARG;
   if (a->out_row_count) return AD_ERR_UNSUPPORTED;   // row ranges: tensor-core path only
+  if (f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_fprop(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
   const size_t total = (size_t)g.N * g.K * g.P * g.Q;
   conv_fprop_f32<<<grid_for(total, 256, 16), 256, 0, s>>>(g, (const float*)a->x, (const float*)a->w, a->bias, (float*)a->y);
   count_launch();
@@ -168,10 +175,18 @@ int conv_direct_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
   if (st != AD_OK) return st;
   if (!a->y || !a->w || !a->dx) return AD_ERR_BAD_ARG;
   if (a->dx_col_count) return AD_ERR_UNSUPPORTED;   // column ranges: tensor-core path only
+  if (f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_dgrad(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
   const size_t total = (size_t)g.N * g.C * g.H * g.W;
   conv_dgrad_f32<<<grid_for(total, 256, 16), 256, 0, s>>>(g, (const float*)a->y, (const float*)a->w, (float*)a->dx);
   count_launch();
   return launch_status();
+}
+
+// Scratch with which a filter gradient of few outputs and many pixels is split further (optional: less or none is fine)
+size_t conv_direct_scratch_bytes(const ad_conv2d_args* a, int pass) {
+  ConvG g;
+  if (pass != 2 || geometry(a, g) != AD_OK || g.kh * g.kw > 49 || !f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return 0;
+  return f32_wgrad_scratch(a, g.P, g.Q);
 }
 
 int conv_direct_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
@@ -180,6 +195,7 @@ int conv_direct_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
   if (st != AD_OK) return st;
   if (!a->x || !a->y || !a->dw) return AD_ERR_BAD_ARG;
   const uint32_t taps = g.kh * g.kw;
+  if (taps <= 49 && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_wgrad(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
   if (taps <= 9) conv_wgrad_f32<9><<<g.K * g.C, 256, 0, s>>>(g, (const float*)a->x, (const float*)a->y, (float*)a->dw);
   else if (taps <= 49) conv_wgrad_f32<49><<<g.K * g.C, 256, 0, s>>>(g, (const float*)a->x, (const float*)a->y, (float*)a->dw);
   else return AD_ERR_UNSUPPORTED;

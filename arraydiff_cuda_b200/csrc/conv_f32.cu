@@ -1,0 +1,631 @@
+// fp32 NCHW convolution with fp32 FMA accumulate, as tiled implicit GEMMs: forward, data gradient, filter and bias
+// gradient.  Every product and every sum is an fp32 FMA (packed two to an instruction: fma.rn.f32x2 rounds each half as
+// fmaf does), and long sums are kept short in two levels: a running sum of at most a few hundred terms is added to the
+// main accumulator and restarted.
+//
+// The bound is the fp32 FMA pipe (148 SMs x 128 FMA per clock: 74 TFLOP/s on paper, 60-68 in a loop of nothing else)
+// and, just below it, the 128 bytes per clock a shared-memory read brings into registers: an 8 x 8 outputs-per-thread
+// tile needs all of both (58-62 TFLOP/s in a loop of reads and packed FMAs, 8 x 4 outputs 52).  So a thread owns 8 x 8
+// outputs, pairs of which sit in one packed FMA, and what is left goes into cheap gathers: operands come by 4-byte
+// cp.async into a ring of stages, ~6 instructions per element (table entry, test, address, a predicated copy or a
+// predicated store of zero for the implicit padding).
+//
+// A shape with few output tiles splits its reduction over the CTAs of a cluster (up to 8), whose partial tiles meet
+// through distributed shared memory in rank order, and a filter gradient further over slices of the caller's scratch:
+// no atomics, reproducible.
+//
+// Measured on a B200 against one thread per output (the kernels of conv_direct.cu, which remain for geometries outside
+// f32_gemm_ok): figures at the launchers.
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace cg = cooperative_groups;
+
+namespace adk {
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ void ffma2(u64& d, u64 a, u64 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
+__device__ __forceinline__ u64 dup2(float v) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(u64 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+// 4 bytes global -> shared asynchronously where all bits of `need` are in `have`, else a zero (source size 0: not read)
+__device__ __forceinline__ void gather4(uint32_t dst, const float* src, uint32_t have, uint32_t need) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"((have & need) == need ? 4u : 0u) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+constexpr int kF32Group = 128;           // threads that share one tile; a CTA is one or two such groups
+constexpr int kF32MaxK = 15;             // filter rows / columns: one bit each in a 32-bit word (rows 0.., columns 16..)
+constexpr uint32_t kF32Never = 1u << 31; // a bit no pixel has
+
+// A group is 4 warps, WM x WN of them over rows and columns; a warp's lanes are LM x (32 / LM) over rows and columns, a
+// thread owns 8 rows x 8 columns.  A CTA of G = 2 groups (filter gradients) halves every stage's pixels between them: 8
+// warps where the grid leaves an SM one CTA.
+template <int LM, int WM, int WN, int G> struct F32Tile {
+  static constexpr int LN = 32 / LM, BM = 8 * LM * WM, BN = 8 * LN * WN, threads = kF32Group * G;
+  static_assert(WM * WN == 4, "four warps");
+};
+
+// Sum of one element of the tiles of all groups of all CTAs of the cluster, in order; all loads are in flight together
+template <int G>
+__device__ __forceinline__ float cluster_total(cg::cluster_group& cluster, float* sm, uint32_t cs, size_t at, size_t group_stride) {
+  float v[8 * G];
+#pragma unroll
+  for (uint32_t q = 0; q < 8; ++q)
+#pragma unroll
+    for (int g = 0; g < G; ++g) v[q * G + g] = q < cs ? (cs > 1 ? cluster.map_shared_rank(sm, q) : sm)[at + g * group_stride] : 0.f;
+  float t = v[0];
+#pragma unroll
+  for (uint32_t q = 1; q < 8 * G; ++q) if (q < cs * G) t += v[q];
+  return t;
+}
+
+// ---------------------------------------------------------------- forward / data gradient
+// GEMM: rows m = output channels of the pass, columns = output pixels, reduction kd = (channel, tap), tap fastest.
+// A data gradient of a strided layer is one such GEMM per residue class of its pixels (blockIdx.z): the pixels
+// (y mod sh, x mod sw) = (ry, rx) meet only the taps whose distance is a multiple of the stride, so no tap is multiplied
+// that does not contribute.
+struct GemmF32 {
+  const float *in, *w, *bias;
+  float* out;
+  uint32_t M, CR, NI;
+  uint32_t IH, IW;                    // extent of `in`
+  long long in_pitch, in_plane, in_img;
+  uint32_t OH, OW;                    // full output extent
+  long long out_pitch, out_plane, out_img;
+  long long w_m, w_c;                 // filter strides of m and of the reduction channel (taps are contiguous)
+  uint32_t kh, kw, sh, sw, dh, dw;
+  int ph, pw;
+  int relu, accumulate;
+};
+// Shared memory: a ring of stages ([kd][m], pitch BM + 4, and [kd][pixel]; KB reduction indices each) beside the BM x BN
+// tile of main accumulators, to which the running sums of 256 terms go
+template <int LM, int WM, int WN> struct GemmTile : F32Tile<LM, WM, WN, 1> {
+  typedef F32Tile<LM, WM, WN, 1> B;
+  static constexpr int KB = B::BN > 512 ? 8 : 16, flush = 256 / KB;
+  static constexpr int PA = B::BM + 4, stage_floats = KB * (PA + B::BN);
+  static constexpr int stages = B::BN > 256 ? 2 : 3;
+  static constexpr int smem = (stages * stage_floats + B::BM * B::BN) * 4;
+};
+
+template <int LM, int WM, int WN, bool DGRAD>
+__global__ void __launch_bounds__(kF32Group, 3) conv_gemm_f32(const GemmF32 p) {
+  typedef GemmTile<LM, WM, WN> T;
+  constexpr int BM = T::BM, BN = T::BN, LN = T::LN, KB = T::KB, PA = T::PA, STAGES = T::stages;
+  constexpr int NPX = BN / kF32Group;                                          // pixels a thread gathers for
+  extern __shared__ __align__(16) float sm[];
+  float* const tile = sm + STAGES * T::stage_floats;
+  __shared__ int tap_off[64], tap_bits[64], tap_w[64], row_t[16], col_t[16], s_ntaps;
+  __shared__ int4 tab[2][KB];         // per reduction index of a stage: input offset, needed row and column bits, filter offset
+
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t cs = cluster.num_blocks(), rank = cluster.block_rank();
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t m_base = blockIdx.y * BM;
+
+  // the class of pixels and its taps
+  uint32_t ry = 0, rx = 0, my = p.sh, mx = p.sw, OHc = p.OH, OWc = p.OW;
+  if (DGRAD) {
+    ry = blockIdx.z / p.sw; rx = blockIdx.z % p.sw;
+    my = mx = 1;
+    OHc = p.OH > ry ? (p.OH - ry + p.sh - 1) / p.sh : 0;
+    OWc = p.OW > rx ? (p.OW - rx + p.sw - 1) / p.sw : 0;
+  }
+  if (warp == 0) {
+    // row and column offsets of the taps (INT_MIN / 2: the class does not meet that row or column)
+    constexpr int kNone = -(1 << 30);
+    int vy = kNone, vx = kNone;
+    if (lane < p.kh) {
+      const int ay = (int)ry + p.ph - (int)(lane * p.dh);
+      vy = DGRAD ? (ay % (int)p.sh == 0 ? ay / (int)p.sh : kNone) : (int)(lane * p.dh) - p.ph;
+    }
+    if (lane < p.kw) {
+      const int ax = (int)rx + p.pw - (int)(lane * p.dw);
+      vx = DGRAD ? (ax % (int)p.sw == 0 ? ax / (int)p.sw : kNone) : (int)(lane * p.dw) - p.pw;
+    }
+    if (lane < 16) { row_t[lane] = vy; col_t[lane] = vx; }
+    __syncwarp();
+    const int taps = (int)(p.kh * p.kw);
+    int base = 0;
+    for (int t0 = 0; t0 < taps; t0 += 32) {
+      const int t = t0 + (int)lane, i = t / (int)p.kw, j = t - i * (int)p.kw;
+      const int ty = t < taps ? row_t[i] : kNone, tx = t < taps ? col_t[j] : kNone;
+      const bool ok = ty != kNone && tx != kNone;
+      const unsigned b = __ballot_sync(0xffffffffu, ok);
+      if (ok) {
+        const int at = base + __popc(b & ((1u << lane) - 1u));
+        tap_off[at] = (int)(ty * p.in_pitch) + tx;
+        tap_bits[at] = (int)((1u << i) | (1u << (16 + j)));
+        tap_w[at] = t;
+      }
+      base += __popc(b);
+    }
+    if (lane == 0) s_ntaps = base;
+  }
+  __syncthreads();
+  const uint32_t ntaps = (uint32_t)s_ntaps;
+  const uint32_t npx = p.NI * OHc * OWc, n_base = (blockIdx.x / cs) * BN;
+  if (n_base >= npx) return;          // the whole cluster shares the tile
+
+  // this CTA's share of the reduction
+  const uint32_t Kd = p.CR * ntaps;
+  const uint32_t per = ((Kd + cs - 1) / cs + KB - 1) / KB * KB;
+  const uint32_t k_lo = rank * per < Kd ? rank * per : Kd, k_hi = k_lo + per < Kd ? k_lo + per : Kd;
+  const uint32_t steps = (k_hi - k_lo + KB - 1) / KB;
+
+  // the pixels this thread gathers for (and writes): where their windows start, which rows and columns lie inside
+  const float* in_px[NPX];
+  float* out_px[NPX];
+  uint32_t bits[NPX];
+#pragma unroll
+  for (int u = 0; u < NPX; ++u) {
+    const uint32_t pxi = n_base + tid + u * kF32Group;
+    in_px[u] = p.in; out_px[u] = nullptr; bits[u] = 0;
+    if (pxi < npx) {
+      const uint32_t ox = pxi % OWc, r = pxi / OWc, oy = r % OHc, n = r / OHc;
+      const int iy0 = (int)(oy * my), ix0 = (int)(ox * mx);
+      in_px[u] = p.in + (long long)n * p.in_img + (long long)iy0 * p.in_pitch + ix0;
+      for (uint32_t i = 0; i < p.kh; ++i) if ((unsigned)(iy0 + row_t[i]) < p.IH) bits[u] |= 1u << i;
+      for (uint32_t j = 0; j < p.kw; ++j) if ((unsigned)(ix0 + col_t[j]) < p.IW) bits[u] |= 1u << (16 + j);
+      const uint32_t fy = DGRAD ? oy * p.sh + ry : oy, fx = DGRAD ? ox * p.sw + rx : ox;
+      out_px[u] = p.out + (long long)n * p.out_img + (long long)fy * p.out_pitch + fx;
+    }
+  }
+
+  auto make_tab = [&](uint32_t step) {
+    if (tid < KB) {
+      const uint32_t kd = k_lo + step * KB + tid;
+      int4 e = make_int4(0, (int)kF32Never, 0, 0);
+      if (kd < k_hi) {
+        const uint32_t c = kd / ntaps, t = kd - c * ntaps;
+        e = make_int4((int)(c * p.in_plane) + tap_off[t], tap_bits[t], (int)(c * p.w_c) + tap_w[t], 0);
+      }
+      tab[step & 1u][tid] = e;
+    }
+  };
+  auto load = [&](uint32_t step) {
+    const uint32_t a0 = smem_addr(sm + (size_t)(step % STAGES) * T::stage_floats), b0 = a0 + (KB * PA + tid) * 4;
+    const int4* tb = tab[step & 1u];
+#pragma unroll
+    for (int r = 0; r < KB; ++r) {
+      const int2 e = *(const int2*)&tb[r];
+#pragma unroll
+      for (int u = 0; u < NPX; ++u) gather4(b0 + (r * BN + u * kF32Group) * 4, in_px[u] + e.x, bits[u], (uint32_t)e.y);
+    }
+#pragma unroll
+    for (int i = 0; i < (KB * BM + kF32Group - 1) / kF32Group; ++i) {
+      const uint32_t idx = tid + i * kF32Group;
+      if (KB * BM % kF32Group && idx >= KB * BM) break;
+      // filter rows are contiguous along (channel, tap) forward and along m (taps apart) backward
+      const uint32_t r = DGRAD ? idx / BM : idx % KB, m = DGRAD ? idx % BM : idx / KB;
+      const int4 e = tb[r];
+      gather4(a0 + (r * PA + m) * 4, p.w + ((long long)(m_base + m) * p.w_m + e.z), m_base + m < p.M ? 0x7fffffffu : 0u, (uint32_t)e.y);
+    }
+  };
+
+  const uint32_t m0 = (warp % WM) * 8 * LM + lane / LN * 8, n0 = (warp / WM) * 8 * LN + lane % LN * 4;
+  u64 acc[4][8];                      // [pair of rows][column]: columns n0 .. n0 + 3 and n0 + 4 LN .. n0 + 4 LN + 3
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+  auto flush = [&](bool first) {      // running sums -> main accumulators in shared memory (this thread's own elements)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float lo[4], hi[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 v = unpack2(acc[i][h * 4 + j]);
+          lo[j] = v.x; hi[j] = v.y;
+          acc[i][h * 4 + j] = 0ull;
+        }
+        float4* t0 = (float4*)(tile + (size_t)(m0 + 2 * i) * BN + n0 + h * 4 * LN);
+        float4* t1 = t0 + BN / 4;
+        float4 o0 = make_float4(lo[0], lo[1], lo[2], lo[3]), o1 = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        if (!first) {
+          const float4 p0 = *t0, p1 = *t1;
+          o0.x += p0.x; o0.y += p0.y; o0.z += p0.z; o0.w += p0.w;
+          o1.x += p1.x; o1.y += p1.y; o1.z += p1.z; o1.w += p1.w;
+        }
+        *t0 = o0; *t1 = o1;
+      }
+  };
+  if (steps) {
+    for (uint32_t st = 0; st < STAGES - 1; ++st) {
+      make_tab(st);
+      __syncthreads();
+      if (st < steps) load(st);
+      cp_async_commit();
+    }
+    make_tab(STAGES - 1);
+  }
+  for (uint32_t st = 0; st < steps; ++st) {
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    if (st + STAGES - 1 < steps) load(st + STAGES - 1);
+    cp_async_commit();
+    make_tab(st + STAGES);
+    const float* As = sm + (size_t)(st % STAGES) * T::stage_floats;
+    const float* Bs = As + KB * PA + n0;
+    As += m0;
+    ulonglong2 na0 = *(const ulonglong2*)As, na1 = *(const ulonglong2*)(As + 4);
+    float4 nb0 = *(const float4*)Bs, nb1 = *(const float4*)(Bs + 4 * LN);
+#pragma unroll
+    for (int r = 0; r < KB; ++r) {     // the next row's operands are read underneath this row's products
+      const ulonglong2 a0 = na0, a1 = na1;
+      const float4 b0 = nb0, b1 = nb1;
+      if (r + 1 < KB) {
+        na0 = *(const ulonglong2*)(As + (r + 1) * PA); na1 = *(const ulonglong2*)(As + (r + 1) * PA + 4);
+        nb0 = *(const float4*)(Bs + (r + 1) * BN); nb1 = *(const float4*)(Bs + (r + 1) * BN + 4 * LN);
+      }
+      const u64 av[4] = {a0.x, a0.y, a1.x, a1.y};
+      const float bf[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const u64 bb = dup2(bf[j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ffma2(acc[i][j], av[i], bb);
+      }
+    }
+    if (st % T::flush == T::flush - 1) flush(st == T::flush - 1);
+  }
+  if (steps % T::flush || steps == 0) flush(steps < T::flush);
+  if (cs > 1) cluster.sync();
+  else __syncthreads();
+  // each CTA of the cluster finishes BM / cs rows
+  const uint32_t rows = BM / cs;
+  for (uint32_t i = 0; i < rows; ++i) {
+    const uint32_t m = rank * rows + i;
+#pragma unroll
+    for (int u = 0; u < NPX; ++u) {
+      float v = cluster_total<1>(cluster, tile, cs, (size_t)m * BN + tid + u * kF32Group, 0);
+      if (out_px[u] && m_base + m < p.M) {
+        float* o = out_px[u] + (long long)(m_base + m) * p.out_plane;
+        if (!DGRAD) {
+          if (p.bias) v += p.bias[m_base + m];
+          if (p.relu) v = fmaxf(v, 0.f);
+        } else if (p.accumulate) {
+          v += *o;
+        }
+        *o = v;
+      }
+    }
+  }
+  if (cs > 1) cluster.sync();         // nobody leaves while its tile is still read
+}
+
+template <typename Kernel, typename Params>
+static int launch_f32(Kernel k, dim3 grid, int threads, int smem, uint32_t cs, const Params& p, unsigned& attr_done, cudaStream_t s) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(attr_done & (1u << (dev & 31)))) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return AD_ERR_CUDA;
+    }
+    attr_done |= 1u << (dev & 31);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cs > 1 ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, k, p) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
+  count_launch();
+  return launch_status();
+}
+
+// CTAs that share one tile: until the grid holds `want` CTAs, each with at least four stages of reduction
+static uint32_t f32_cluster(unsigned long long tiles, unsigned long long want, uint32_t steps, uint32_t most) {
+  uint32_t cs = 1;
+  while (cs < most && tiles * cs * 2 <= want && steps >= 8 * cs) cs *= 2;
+  return cs;
+}
+
+template <int LM, int WM, int WN, bool DGRAD>
+static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uint32_t Kd, cudaStream_t s) {
+  typedef GemmTile<LM, WM, WN> T;
+  static unsigned attr_done = 0;      // one bit per device
+  const uint32_t tn = (npx + T::BN - 1) / T::BN, tm = (p.M + T::BM - 1) / T::BM;
+  // three CTAs per SM are resident (BM >= 8 rows: a cluster of 8 still has a row per CTA)
+  const uint32_t cs = f32_cluster((unsigned long long)tn * tm * classes, 3ull * kNumSMs, Kd / T::KB, 8);
+  return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, attr_done, s);
+}
+
+// Tile height by the row count: a row of the tile costs the same FMAs whether it holds a channel or not, a column is
+// gathered once per tile row: 64 x 128 for more than 32 channels, 32 x 256, 16 x 512 and 8 x 1024 below.
+template <bool DGRAD>
+static int run_gemm_f32(const GemmF32& p, cudaStream_t s) {
+  const uint32_t classes = DGRAD ? p.sh * p.sw : 1;
+  const uint32_t OHc = DGRAD ? (p.OH + p.sh - 1) / p.sh : p.OH, OWc = DGRAD ? (p.OW + p.sw - 1) / p.sw : p.OW;
+  const uint32_t npx = p.NI * OHc * OWc, Kd = p.CR * ((p.kh * p.kw + classes - 1) / classes);
+  if (p.M <= 8) return launch_gemm_f32<1, 1, 4, DGRAD>(p, npx, classes, Kd, s);
+  if (p.M <= 16) return launch_gemm_f32<2, 1, 4, DGRAD>(p, npx, classes, Kd, s);
+  if (p.M <= 32) return launch_gemm_f32<4, 1, 4, DGRAD>(p, npx, classes, Kd, s);
+  return launch_gemm_f32<4, 2, 2, DGRAD>(p, npx, classes, Kd, s);
+}
+
+// ---------------------------------------------------------------- filter gradient
+// GEMM: rows m = output channels, columns n = (input channel, tap), reduction = output pixels, which is the order both
+// operands have in memory.  The reduction is split over the CTAs of a cluster and over `slices` of the grid; with more
+// than one slice the clusters write partial gradients to scratch and wgrad_f32_finish adds them in order.
+struct WgradF32 {
+  const float *x, *dy;
+  float *dw, *db, *part;
+  uint32_t K, C, N, P, Q, H, W, kh, kw, sh, sw, dh, dw_;
+  int ph, pw;
+  long long dy_pitch, dy_plane;
+  int accumulate;
+  uint32_t slices;
+};
+// Shared memory: a ring of stages ([row][32 pixels], pitch 36: reads and writes free of bank conflicts) beside the BM x BN
+// tile of main accumulators.  One packed FMA multiplies two neighbouring pixels; the halves are added at the end.
+constexpr int kWgKB = 32, kWgPitch = 36, kWgStages = 2, kWgFlush = 8;
+
+template <int LM, int WM, int WN, int G> struct WgTile : F32Tile<LM, WM, WN, G> {
+  typedef F32Tile<LM, WM, WN, G> B;
+  static constexpr int group_floats = (B::BM + B::BN) * kWgPitch, stage_floats = G * group_floats;
+  static constexpr int smem = (kWgStages * stage_floats + G * B::BM * B::BN) * 4;
+};
+
+template <int LM, int WM, int WN, int G>
+__global__ void __launch_bounds__(kF32Group * G, G == 1 ? 2 : 1) conv_wgrad_gemm_f32(const WgradF32 p) {
+  typedef WgTile<LM, WM, WN, G> T;
+  constexpr int BM = T::BM, BN = T::BN, LN = T::LN, STAGES = kWgStages, PITCH = kWgPitch, KB = kWgKB;
+  extern __shared__ __align__(16) float sm[];
+  float* const tile = sm + STAGES * T::stage_floats;
+  __shared__ int2 col[BN];            // per column: input offset of (channel, tap), row and column bits
+  __shared__ int row_t[16], col_t[16];
+  __shared__ float sdb[G * BM];
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t cs = cluster.num_blocks(), rank = cluster.block_rank();
+  const uint32_t group = threadIdx.x / kF32Group, tid = threadIdx.x % kF32Group, warp = tid >> 5, lane = tid & 31;
+  const uint32_t taps = p.kh * p.kw, NC = p.C * taps;
+  const uint32_t n_base = (blockIdx.x / cs) * BN, m_base = blockIdx.y * BM, slice = blockIdx.z;
+  const long long x_img = (long long)p.C * p.H * p.W, dy_img = (long long)p.K * p.dy_plane;
+  if (threadIdx.x < 16) { row_t[tid] = (int)(tid * p.dh) - p.ph; col_t[tid] = (int)(tid * p.dw_) - p.pw; }
+  for (uint32_t i = threadIdx.x; i < BN; i += T::threads) {
+    const uint32_t n = n_base + i;
+    int2 e = make_int2(0, (int)kF32Never);
+    if (n < NC) {
+      const uint32_t c = n / taps, t = n - c * taps, ti = t / p.kw, tj = t - ti * p.kw;
+      e = make_int2((int)(c * p.H * p.W) + ((int)(ti * p.dh) - p.ph) * (int)p.W + (int)(tj * p.dw_) - p.pw, (int)((1u << ti) | (1u << (16 + tj))));
+    }
+    col[i] = e;
+  }
+  __syncthreads();
+  const uint32_t npx = p.N * p.P * p.Q, pq = p.P * p.Q;
+  const uint32_t all = (npx + KB * G - 1) / (KB * G), parts = cs * p.slices, per = (all + parts - 1) / parts, me = slice * cs + rank;
+  const uint32_t s_lo = me * per < all ? me * per : all, steps = (s_lo + per < all ? s_lo + per : all) - s_lo;
+
+  auto load = [&](uint32_t st) {
+    const uint32_t pxi = ((s_lo + st) * G + group) * KB + lane;
+    float* As = sm + (size_t)(st % STAGES) * T::stage_floats + group * T::group_floats;
+    const bool in = pxi < npx;
+    const uint32_t n = in ? pxi / pq : 0, r = in ? pxi - n * pq : 0, oy = r / p.Q, ox = r - oy * p.Q;
+    const float* dp = p.dy + (long long)n * dy_img + (long long)oy * p.dy_pitch + ox + (long long)(m_base + warp) * p.dy_plane;
+    const uint32_t a0 = smem_addr(As + warp * PITCH + lane), b0 = a0 + BM * PITCH * 4;
+#pragma unroll 16
+    for (int i = 0; i < BM / 4; ++i) {
+      gather4(a0 + i * 4 * PITCH * 4, dp, in && m_base + warp + i * 4 < p.K, 1u);
+      dp += 4 * p.dy_plane;
+    }
+    const int iy0 = (int)(oy * p.sh), ix0 = (int)(ox * p.sw);
+    uint32_t bits = 0;
+    if (in) {
+      for (uint32_t i = 0; i < p.kh; ++i) if ((unsigned)(iy0 + row_t[i]) < p.H) bits |= 1u << i;
+      for (uint32_t j = 0; j < p.kw; ++j) if ((unsigned)(ix0 + col_t[j]) < p.W) bits |= 1u << (16 + j);
+    }
+    const float* xp = p.x + (long long)n * x_img + (long long)iy0 * p.W + ix0;
+#pragma unroll 16
+    for (int i = 0; i < BN / 4; ++i) {
+      const int2 e = col[warp + i * 4];
+      gather4(b0 + i * 4 * PITCH * 4, xp + e.x, bits, (uint32_t)e.y);
+    }
+  };
+
+  const uint32_t m0 = (warp % WM) * 8 * LM + lane / LN, n0 = (warp / WM) * 8 * LN + lane % LN;
+  u64 acc[8][8];                      // rows m0 + i LM, columns n0 + j LN
+  float dbs = 0.f;
+  const bool with_db = p.db && n_base == 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+  auto flush = [&](bool first) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 v = unpack2(acc[i][j]);
+        float* t = tile + ((size_t)group * BM + m0 + i * LM) * BN + n0 + j * LN;
+        *t = first ? v.x + v.y : *t + (v.x + v.y);
+        acc[i][j] = 0ull;
+      }
+  };
+  for (uint32_t st = 0; st < STAGES - 1; ++st) {
+    if (st < steps) load(st);
+    cp_async_commit();
+  }
+  for (uint32_t st = 0; st < steps; ++st) {
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    if (st + STAGES - 1 < steps) load(st + STAGES - 1);
+    cp_async_commit();
+    const float* As = sm + (size_t)(st % STAGES) * T::stage_floats + group * T::group_floats;
+    const float* a0 = As + m0 * PITCH;
+    const float* b0 = As + (BM + n0) * PITCH;
+#pragma unroll
+    for (int q = 0; q < KB / 4; ++q) {
+      ulonglong2 b[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[j] = *(const ulonglong2*)(b0 + j * LN * PITCH + q * 4);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const ulonglong2 a = *(const ulonglong2*)(a0 + i * LM * PITCH + q * 4);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { ffma2(acc[i][j], a.x, b[j].x); ffma2(acc[i][j], a.y, b[j].y); }
+      }
+    }
+    if (with_db && tid < BM) {        // the bias gradient: row sums of the same dy tile
+      float d = 0.f;
+#pragma unroll
+      for (int q = 0; q < KB / 4; ++q) {
+        const float4 v = *(const float4*)(As + tid * PITCH + q * 4);
+        d += (v.x + v.y) + (v.z + v.w);
+      }
+      dbs += d;
+    }
+    if (st % kWgFlush == kWgFlush - 1) flush(st == kWgFlush - 1);
+  }
+  if (steps % kWgFlush || steps == 0) flush(steps < kWgFlush);
+  if (with_db && tid < BM) sdb[group * BM + tid] = dbs;
+  if (cs > 1) cluster.sync();
+  else __syncthreads();
+  const uint32_t rows = BM / cs;
+  float* const dw = p.slices > 1 ? p.part + (size_t)slice * ((size_t)p.K * NC + p.K) : p.dw;
+  float* const db = p.slices > 1 ? dw + (size_t)p.K * NC : p.db;
+  const bool acc_out = p.accumulate && p.slices == 1;
+  for (uint32_t e = threadIdx.x; e < rows * BN; e += T::threads) {
+    const uint32_t m = rank * rows + e / BN, n = e % BN;
+    const float v = cluster_total<G>(cluster, tile, cs, (size_t)m * BN + n, (size_t)BM * BN);
+    if (m_base + m < p.K && n_base + n < NC) {
+      float* o = dw + (size_t)(m_base + m) * NC + n_base + n;
+      *o = acc_out ? *o + v : v;
+    }
+  }
+  if (with_db && threadIdx.x < rows && m_base + rank * rows + threadIdx.x < p.K) {
+    const uint32_t m = rank * rows + threadIdx.x;
+    const float v = cluster_total<G>(cluster, sdb, cs, m, BM);
+    float* o = db + m_base + m;
+    *o = acc_out ? *o + v : v;
+  }
+  if (cs > 1) cluster.sync();
+}
+
+// dw (+)= sum of the slices, in order; the bias gradient's K values follow the filter's
+__global__ void __launch_bounds__(256) wgrad_f32_finish(size_t n, uint32_t K, uint32_t slices, const float* __restrict__ part, float* dw,
+                                                        float* db, int accumulate) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x, stride = n + K;
+  if (i >= (db ? stride : n)) return;
+  float v[16], t = 0.f;
+#pragma unroll
+  for (uint32_t s = 0; s < 16; ++s) v[s] = s < slices ? part[s * stride + i] : 0.f;
+#pragma unroll
+  for (uint32_t s = 0; s < 16; ++s) t += v[s];
+  float* o = i < n ? dw + i : db + (i - n);
+  *o = accumulate ? *o + t : t;
+}
+
+static uint32_t wg_rows(uint32_t K) { return K > 32 ? 64u : (K > 16 ? 32u : 16u); }
+static uint32_t wg_cols(uint32_t K) { return 8192u / wg_rows(K); }
+// Slices of the pixel range beyond a cluster of 8: until the grid holds two CTAs per SM, each with at least eight
+// stages of pixels
+static uint32_t wg_slices(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
+  const unsigned long long tiles = (unsigned long long)((a->K + wg_rows(a->K) - 1) / wg_rows(a->K)) *
+                                   ((a->C * a->kh * a->kw + wg_cols(a->K) - 1) / wg_cols(a->K));
+  const unsigned long long steps = ((unsigned long long)a->N * P * Q + kWgKB - 1) / kWgKB;
+  const unsigned long long fit = 2ull * kNumSMs / (tiles * 8), most = steps / (8 * 8);
+  const unsigned long long n = fit < most ? fit : most;
+  return (uint32_t)(n > 16 ? 16 : (n < 1 ? 1 : n));
+}
+
+template <int LM, int WM, int WN, int G>
+static int launch_wgrad_f32(WgradF32& p, cudaStream_t s) {
+  typedef WgTile<LM, WM, WN, G> T;
+  static unsigned attr_done = 0;      // one bit per device
+  const uint32_t tn = (p.C * p.kh * p.kw + T::BN - 1) / T::BN, tm = (p.K + T::BM - 1) / T::BM;
+  const uint32_t cs = f32_cluster((unsigned long long)tn * tm * p.slices, (G == 1 ? 2ull : 1ull) * kNumSMs, p.N * p.P * p.Q / (kWgKB * G) / p.slices, 8);
+  int st = launch_f32(conv_wgrad_gemm_f32<LM, WM, WN, G>, dim3(tn * cs, tm, p.slices), T::threads, T::smem, cs, p, attr_done, s);
+  if (st != AD_OK || p.slices == 1) return st;
+  const size_t n = (size_t)p.K * p.C * p.kh * p.kw;
+  wgrad_f32_finish<<<(unsigned)((n + p.K + 255) / 256), 256, 0, s>>>(n, p.K, p.slices, p.part, p.dw, p.db, p.accumulate);
+  count_launch();
+  return launch_status();
+}
+
+// ---------------------------------------------------------------- entry points (called by conv_direct.cu)
+static bool fits31(long long v) { return v >= 0 && v < (1ll << 31); }
+
+// Limits of the tiled kernels: 32-bit offsets inside one image and one filter, 31-bit pixel counts, a bit per filter row
+// and column.
+bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane) {
+  if (a->kh > kF32MaxK || a->kw > kF32MaxK || a->kh * a->kw > 64) return false;
+  if ((unsigned long long)a->stride_h * a->stride_w > 65535) return false;
+  const long long reach = ((long long)a->dil_h * (a->kh - 1) + a->pad_h + 1) * ((long long)a->W + y_pitch) + (long long)a->dil_w * (a->kw - 1) + a->pad_w;
+  return fits31(reach) && fits31((long long)a->C * a->H * a->W + reach) && fits31((long long)a->K * y_plane + reach) &&
+         fits31((long long)a->N * P * Q) && fits31((long long)a->N * a->H * a->W) && fits31((long long)a->K * a->C * a->kh * a->kw) &&
+         a->K <= 65535u * 8 && a->C <= 65535u * 8 && y_pitch >= 0 && y_plane >= 0;
+}
+
+size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
+  const uint32_t s = wg_slices(a, P, Q);
+  return s > 1 ? (size_t)s * ((size_t)a->K * a->C * a->kh * a->kw + a->K) * 4 : 0;
+}
+
+// Measured (one B200; per call, before -> now): 64 -> 64 channels, 3x3, 64 x 64 pixels, one image: forward 188 -> 19 us, data
+// gradient 158 -> 23, filter and bias gradient 286 -> 29.  4 x 64 x 112 x 112, 64 -> 64 3x3: 1440 -> 127, 1500 -> 125, 2330 ->
+// 222 us (29 / 30 / 17 TFLOP/s).  What is left above the FMA pipe: 12 warps per SM do not hide the latency of the
+// shared-memory reads (issue slots 42 % busy); 4 x 8 outputs per thread or packed pairs along the reduction were slower.
+int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
+  GemmF32 p = {};
+  p.in = (const float*)a->x; p.w = (const float*)a->w; p.bias = a->bias; p.out = (float*)a->y;
+  p.M = a->K; p.CR = a->C; p.NI = a->N; p.IH = a->H; p.IW = a->W;
+  p.in_pitch = a->W; p.in_plane = (long long)a->H * a->W; p.in_img = p.in_plane * a->C;
+  p.OH = P; p.OW = Q; p.out_pitch = y_pitch; p.out_plane = y_plane; p.out_img = y_plane * a->K;
+  p.w_m = (long long)a->C * a->kh * a->kw; p.w_c = (long long)a->kh * a->kw;
+  p.kh = a->kh; p.kw = a->kw; p.sh = a->stride_h; p.sw = a->stride_w; p.dh = a->dil_h; p.dw = a->dil_w;
+  p.ph = (int)a->pad_h; p.pw = (int)a->pad_w; p.relu = a->relu;
+  return run_gemm_f32<false>(p, s);
+}
+
+int f32_gemm_dgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
+  GemmF32 p = {};
+  p.in = (const float*)a->y; p.w = (const float*)a->w; p.out = (float*)a->dx;
+  p.M = a->C; p.CR = a->K; p.NI = a->N; p.IH = P; p.IW = Q;
+  p.in_pitch = y_pitch; p.in_plane = y_plane; p.in_img = y_plane * a->K;
+  p.OH = a->H; p.OW = a->W; p.out_pitch = a->W; p.out_plane = (long long)a->H * a->W; p.out_img = p.out_plane * a->C;
+  p.w_m = (long long)a->kh * a->kw; p.w_c = (long long)a->C * a->kh * a->kw;
+  p.kh = a->kh; p.kw = a->kw; p.sh = a->stride_h; p.sw = a->stride_w; p.dh = a->dil_h; p.dw = a->dil_w;
+  p.ph = (int)a->pad_h; p.pw = (int)a->pad_w; p.accumulate = a->accumulate;
+  return run_gemm_f32<true>(p, s);
+}
+
+int f32_gemm_wgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
+  WgradF32 p = {};
+  p.x = (const float*)a->x; p.dy = (const float*)a->y; p.dw = (float*)a->dw; p.db = a->db;
+  p.K = a->K; p.C = a->C; p.N = a->N; p.P = P; p.Q = Q; p.H = a->H; p.W = a->W;
+  p.kh = a->kh; p.kw = a->kw; p.sh = a->stride_h; p.sw = a->stride_w; p.dh = a->dil_h; p.dw_ = a->dil_w;
+  p.ph = (int)a->pad_h; p.pw = (int)a->pad_w;
+  p.dy_pitch = y_pitch; p.dy_plane = y_plane; p.accumulate = a->accumulate;
+  p.slices = 1;
+  const size_t need = f32_wgrad_scratch(a, P, Q);
+  if (need && a->scratch && a->scratch_bytes >= need) { p.slices = wg_slices(a, P, Q); p.part = (float*)a->scratch; }
+  // clusters of 8 fill at most one CTA per SM: two groups per CTA (9 tiles of 4096 pixels: 31 -> 27 us)
+  const unsigned long long tiles = (unsigned long long)((a->K + 63) / 64) * ((a->C * a->kh * a->kw + 127) / 128) * p.slices;
+  switch (wg_rows(a->K)) {
+    case 64: return tiles * 8 <= kNumSMs ? launch_wgrad_f32<4, 2, 2, 2>(p, s) : launch_wgrad_f32<4, 2, 2, 1>(p, s);
+    case 32: return launch_wgrad_f32<4, 1, 4, 1>(p, s);
+    default: return launch_wgrad_f32<2, 1, 4, 1>(p, s);
+  }
+}
+
+}  // namespace adk

@@ -959,6 +959,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
 int conv_direct_fprop(const ad_conv2d_args* a, cudaStream_t s);
 int conv_direct_dgrad(const ad_conv2d_args* a, cudaStream_t s);
 int conv_direct_wgrad(const ad_conv2d_args* a, cudaStream_t s);
+size_t conv_direct_scratch_bytes(const ad_conv2d_args* a, int pass);
 
 }  // namespace adk
 
@@ -972,8 +973,11 @@ static int path_of(const ad_conv2d_args* a) {
 }
 
 extern "C" size_t ad_conv2d_scratch_bytes(const ad_conv2d_args* a, int32_t pass) {
-  if (path_of(a) != 1) return 0;
-  return tc::conv_tc_scratch_bytes(a, pass);
+  switch (path_of(a)) {
+    case 0: return conv_direct_scratch_bytes(a, pass);
+    case 1: return tc::conv_tc_scratch_bytes(a, pass);
+    default: return 0;
+  }
 }
 
 // ---------------------------------------------------------------- per-call timing (ad_conv2d_profile)

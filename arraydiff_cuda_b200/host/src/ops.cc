@@ -569,6 +569,10 @@ void CudnnConv2DOpF::_backward(TxnId txn) {
     }
     if (f32) {
       a.dw = dw.dptr(); a.db = db; a.accumulate = 1;
+      if (const size_t need = ad_conv2d_scratch_bytes(&a, 2)) {
+        g->reserve_scratch(need);
+        a.scratch = g->get_scratch(); a.scratch_bytes = g->scratch_size();
+      }
       AD_CHECK(ad_conv2d_wgrad(&a, s));
     } else {
       ad_conv2d_args b = a;

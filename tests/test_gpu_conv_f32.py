@@ -1,0 +1,65 @@
+"""Tiled fp32 convolution kernels against the oracle, at the edges of their tiles, splits and tap classes."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from arraydiff_cuda_b200 import abi
+from oracle import orc
+from tests import helpers as H
+from tests.test_gpu_conv import conv_args
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # N, C, H, W, K, k, stride, dil, pad
+    (1, 1, 1, 1, 1, 1, 1, 1, 0),         # one output
+    (1, 3, 23, 29, 33, 3, 1, 1, 1),      # a row past the 32-row tile
+    (2, 65, 9, 13, 65, 3, 1, 2, 2),      # a row past the 64-row tile, reduction split over a cluster
+    (3, 16, 31, 33, 129, 1, 1, 1, 0),    # 1x1, a row past the 128-row tile
+    (1, 8, 97, 131, 24, 3, 2, 1, 1),     # strided: four classes of gradient pixels, unequal tap counts
+    (2, 6, 15, 14, 7, 2, 3, 1, 0),       # stride above the filter: classes without any tap
+    (1, 5, 21, 22, 9, 3, 2, 2, 1),       # strided and dilated: taps of one class only
+    (1, 3, 40, 44, 64, 7, 1, 1, 3),      # 49 taps
+    (4, 40, 120, 118, 48, 3, 1, 1, 0),   # no cluster split forward; filter gradient in slices of the scratch
+    (2, 24, 130, 129, 20, 3, 1, 1, 1),   # 32-row tiles
+    (1, 17, 60, 61, 16, 5, 1, 1, 2),     # 16-row tiles
+    (2, 9, 70, 50, 8, 3, 1, 1, 1),       # 8-row tiles: a row per CTA of a cluster of 8
+    (1, 96, 100, 101, 128, 3, 1, 1, 1),  # two 64-row tiles
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_conv_f32_tiles(case):
+    import torch
+    N, Cc, Hh, W, K, k, s, d, pd = case
+    x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, k, k), float(np.sqrt(2.0 / (k * k * Cc)))), H.normal(3, (K,))
+    y_w = orc.conv2d_fprop(x, w, b, (s, s), (d, d), (pd, pd), omp=True)
+    dy = H.uniform(4, y_w.shape)
+    dx_w = orc.conv2d_dgrad(dy, w, x.shape, (s, s), (d, d), (pd, pd), omp=True)
+    db_w = np.zeros(K, np.float32)
+    dw_w = orc.conv2d_wgrad(x, dy, w.shape, (s, s), (d, d), (pd, pd), db=db_w, omp=True)
+    L = abi.lib()
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, k, s, d, pd)
+    dx_, dw_, db_, ddy = H.dev(x), H.dev(w), H.dev(b), H.dev(dy)
+    P, Q = y_w.shape[2:]
+    # y and dy as views into wider rows, as a strip inside a padded buffer is
+    y, gy = torch.full((N, K, P + 1, Q + 3), 7.0, device="cuda"), torch.full((N, K, P + 1, Q + 3), float("nan"), device="cuda")
+    gy[:, :, :P, :Q] = ddy
+    a.x, a.w, a.bias, a.y, a.relu = dx_.data_ptr(), dw_.data_ptr(), db_.data_ptr(), y.data_ptr(), 1
+    a.y_pitch, a.y_plane = Q + 3, (P + 1) * (Q + 3)
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    gdx, gdw, gdb = torch.ones(x.shape, device="cuda"), torch.full(w.shape, 9.0, device="cuda"), torch.full((K,), 9.0, device="cuda")
+    a.y, a.dx, a.dw, a.db, a.accumulate = gy.data_ptr(), gdx.data_ptr(), gdw.data_ptr(), gdb.data_ptr(), 1
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    a.accumulate = 0
+    scratch = torch.full((max(16, L.ad_conv2d_scratch_bytes(C.byref(a), 2)),), 255, dtype=torch.uint8, device="cuda")
+    a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
+    abi.check(L.ad_conv2d_wgrad(C.byref(a), H.stream()))
+    H.sync()
+    got = H.host(y)
+    assert H.max_rel(got[:, :, :P, :Q], np.maximum(y_w, 0)) < 1e-5
+    assert np.all(got[:, :, P:, :] == 7.0) and np.all(got[:, :, :, Q:] == 7.0)
+    assert H.max_rel(H.host(gdx) - 1, dx_w) < 1e-5
+    assert H.max_rel(H.host(gdw), dw_w) < 2e-5
+    assert H.max_rel(H.host(gdb), db_w) < 2e-5
