@@ -90,10 +90,10 @@ struct GemmF32 {
   int relu, accumulate;
 };
 // Shared memory: a ring of stages ([kd][m], pitch BM + 4, and [kd][pixel]; KB reduction indices each) beside the BM x BN
-// tile of main accumulators, to which the running sums of 256 terms go
+// tile of main accumulators, to which the running sums of 64 terms go
 template <int LM, int WM, int WN> struct GemmTile : F32Tile<LM, WM, WN, 1> {
   typedef F32Tile<LM, WM, WN, 1> B;
-  static constexpr int KB = B::BN > 512 ? 8 : 16, flush = 256 / KB;
+  static constexpr int KB = B::BN > 512 ? 8 : 16, flush = 64 / KB;
   static constexpr int PA = B::BM + 4, stage_floats = KB * (PA + B::BN);
   static constexpr int stages = B::BN > 256 ? 2 : 3;
   static constexpr int smem = (stages * stage_floats + B::BM * B::BN) * 4;
