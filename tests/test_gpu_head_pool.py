@@ -1,0 +1,165 @@
+"""Bilinear row kernels, per-pixel loss forms, global pooling, linear layer, pooling tiles and the bias gradient against
+the oracle, at the edges of their blocks and tiles."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from arraydiff_cuda_b200 import abi
+from oracle import orc
+from tests import helpers as H
+from tests.test_gpu_conv import conv_args
+
+pytestmark = pytest.mark.gpu
+FMT = {"f32": (abi.AD_F32, abi.AD_NCHW, H.view_nchw), "bf16": (abi.AD_BF16, abi.AD_NHWC, H.view_nhwc)}
+
+
+def _dev(a, dtype):
+    return H.dev(a) if dtype == "f32" else H.dev_bf16(orc.nchw_to_nhwc(a))
+
+
+def _host(t, dtype):
+    a = H.host(t)
+    return a if dtype == "f32" else orc.nhwc_to_nchw(a)
+
+
+def _q(a, dtype):
+    return a if dtype == "f32" else orc.round_bf16(a)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape,scale", [
+    ((1, 1, 1, 1), 2), ((2, 3, 1, 5), 3), ((1, 19, 9, 40), 8), ((2, 150, 3, 37), 4),    # wide classes: several chunks per row
+    ((1, 2, 4, 700), 8), ((3, 5, 7, 4), 5), ((1, 64, 5, 33), 1),
+])
+def test_upsample_rows(dtype, shape, scale):
+    import torch
+    N, Cc, Hh, W = shape
+    x = _q(H.normal(1, shape), dtype)
+    dy = _q(H.normal(2, (N, Cc, Hh * scale, W * scale)), dtype)
+    y_w, dx_w = orc.upsample_bilinear_fwd(x, scale), orc.upsample_bilinear_bwd(dy, scale)
+    _, _, view = FMT[dtype]
+    dx_, ddy = _dev(x, dtype), _dev(dy, dtype)
+    y, gx = torch.empty_like(ddy), torch.ones_like(dx_)
+    vx, vy, vdy, vgx = view(dx_), view(y), view(ddy), view(gx)
+    L = abi.lib()
+    abi.check(L.ad_upsample_bilinear_fwd(C.byref(vx), C.byref(vy), scale, 0, Hh, 0, H.stream()))
+    abi.check(L.ad_upsample_bilinear_bwd(C.byref(vdy), C.byref(vgx), scale, 0, Hh, 0, 1, H.stream()))
+    H.sync()
+    tol = 1e-5 if dtype == "f32" else 1e-2
+    assert H.max_rel(_host(y, dtype), y_w) < tol
+    assert H.max_rel(_host(gx, dtype), 1 + dx_w) < tol
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
+@pytest.mark.parametrize("Cc,HW", [(1, 300), (8, 257), (9, 255), (32, 256), (33, 130), (64, 31), (65, 77), (128, 3), (129, 9), (256, 5), (257, 4), (1000, 1)])
+def test_ce_class_counts(dtype, layout, Cc, HW):
+    import torch
+    N = 3
+    logits = _q(H.normal(3, (N, Cc, HW), 2.0), dtype)
+    label = H.rng(4).integers(0, Cc, (N, HW)).astype(np.uint32)
+    dloss = H.uniform(5, (N, HW))
+    loss_w = orc.softmax_ce_pixel_fwd(logits, label)[0]
+    dlog_w = orc.softmax_ce_pixel_bwd(logits, label, dloss)
+    arr = logits if layout == abi.AD_NCHW else np.ascontiguousarray(np.transpose(logits, (0, 2, 1)))
+    d = H.dev(arr) if dtype == "f32" else H.dev_bf16(arr)
+    dl, ddl = torch.from_numpy(label.view(np.int32)).cuda(), H.dev(dloss)
+    loss, dlog = torch.empty((N, HW), device="cuda"), torch.ones_like(d)
+    L, dt = abi.lib(), FMT[dtype][0]
+    abi.check(L.ad_softmax_ce_pixel_fwd(dt, layout, N, Cc, HW, H.ptr(d), H.ptr(dl), H.ptr(loss), None, H.stream()))
+    abi.check(L.ad_softmax_ce_pixel_bwd(dt, layout, N, Cc, HW, H.ptr(d), H.ptr(dl), H.ptr(ddl), H.ptr(dlog), 1, H.stream()))
+    H.sync()
+    got = H.host(dlog) - 1
+    if layout == abi.AD_NHWC:
+        got = np.transpose(got, (0, 2, 1))
+    assert H.max_rel(H.host(loss), loss_w) < 1e-5
+    assert np.max(np.abs(got - dlog_w)) < (2e-6 if dtype == "f32" else 1e-2)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(1, 8, 1, 1), (2, 40, 19, 23), (3, 2048, 7, 7), (5, 264, 5, 4)])
+def test_global_average_pool(dtype, shape):
+    import torch
+    N, Cc, Hh, W = shape
+    x, dy = _q(H.normal(6, shape), dtype), _q(H.normal(7, (N, Cc, 1, 1)), dtype)
+    y_w, dx_w = orc.avgpool2d_fwd(x, (Hh, W), (1, 1)), orc.avgpool2d_bwd(dy, shape, (Hh, W), (1, 1))
+    _, _, view = FMT[dtype]
+    dx_, ddy = _dev(x, dtype), _dev(dy, dtype)
+    y, gx, ga = torch.empty_like(ddy), torch.empty_like(dx_), torch.ones_like(dx_)
+    vx, vy, vdy, vgx, vga = view(dx_), view(y), view(ddy), view(gx), view(ga)
+    L = abi.lib()
+    abi.check(L.ad_avgpool2d_fwd(C.byref(vx), C.byref(vy), Hh, W, 1, 1, H.stream()))
+    abi.check(L.ad_avgpool2d_bwd(C.byref(vdy), C.byref(vgx), Hh, W, 1, 1, 0, H.stream()))
+    abi.check(L.ad_avgpool2d_bwd(C.byref(vdy), C.byref(vga), Hh, W, 1, 1, 1, H.stream()))
+    H.sync()
+    tol = 1e-5 if dtype == "f32" else 1e-2
+    assert H.max_rel(_host(y, dtype), y_w) < tol
+    assert H.max_rel(_host(gx, dtype), dx_w) < tol
+    assert H.max_rel(_host(ga, dtype), 1 + dx_w) < tol
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("B,I,O", [(1, 1, 1), (9, 33, 9), (8, 257, 1000), (17, 512, 7)])
+def test_linear_groups(dtype, B, I, O):
+    import torch
+    x, w, b, dy = _q(H.normal(8, (B, I)), dtype), H.normal(9, (O, I), 0.1), H.normal(10, (O,)), _q(H.normal(11, (B, O)), dtype)
+    y_w = orc.linear_fwd(x, w, b)
+    dx_w, dw_w, db_w = orc.linear_bwd(x, w, dy)
+    mk = H.dev if dtype == "f32" else H.dev_bf16
+    dx_, ddy, dw_, db_ = mk(x), mk(dy), H.dev(w), H.dev(b)
+    y, gx = torch.empty_like(ddy), torch.ones_like(dx_)
+    gw, gb = torch.ones(O, I, device="cuda"), torch.ones(O, device="cuda")
+    L, dt = abi.lib(), FMT[dtype][0]
+    abi.check(L.ad_linear_fwd(dt, B, I, O, H.ptr(dx_), H.ptr(dw_), H.ptr(db_), H.ptr(y), H.stream()))
+    abi.check(L.ad_linear_bwd(dt, B, I, O, H.ptr(dx_), H.ptr(dw_), H.ptr(ddy), H.ptr(gx), H.ptr(gw), H.ptr(gb), 1, 1, H.stream()))
+    H.sync()
+    tol = 2e-5 if dtype == "f32" else 1e-2
+    assert H.max_rel(H.host(y), y_w) < tol
+    assert H.max_rel(H.host(gx), 1 + dx_w) < tol
+    assert H.max_rel(H.host(gw), 1 + dw_w) < 2e-5
+    assert H.max_rel(H.host(gb), 1 + db_w) < 2e-5
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape,k,s", [
+    ((1, 8, 3, 3), (3, 3), (2, 2)), ((2, 16, 33, 35), (3, 3), (2, 2)), ((1, 24, 17, 16), (2, 2), (2, 2)), ((1, 72, 18, 31), (3, 3), (1, 1)),
+    ((1, 40, 20, 21), (2, 5), (1, 3)), ((2, 8, 65, 66), (3, 3), (4, 4)), ((1, 8, 40, 70), (7, 9), (2, 2)), ((1, 8, 37, 37), (17, 2), (1, 1)),
+])
+def test_maxpool_tiles(dtype, shape, k, s):
+    import torch
+    N, Cc, Hh, W = shape
+    x = _q(np.round(H.normal(12, shape) * 2) / 2, dtype)        # many ties
+    y_w = orc.maxpool2d_fwd(x, k, s)
+    dy = _q(H.normal(13, y_w.shape), dtype)
+    dx_w = orc.maxpool2d_bwd(x, dy, k, s)
+    _, _, view = FMT[dtype]
+    dx_, ddy = _dev(x, dtype), _dev(dy, dtype)
+    y, gx, ga = torch.empty_like(ddy), torch.empty_like(dx_), torch.ones_like(dx_)
+    vx, vy, vdy, vgx, vga = view(dx_), view(y), view(ddy), view(gx), view(ga)
+    L = abi.lib()
+    abi.check(L.ad_maxpool2d_fwd(C.byref(vx), C.byref(vy), *k, *s, H.stream()))
+    abi.check(L.ad_maxpool2d_bwd(C.byref(vx), C.byref(vdy), C.byref(vgx), *k, *s, 0, H.stream()))
+    abi.check(L.ad_maxpool2d_bwd(C.byref(vx), C.byref(vdy), C.byref(vga), *k, *s, 1, H.stream()))
+    H.sync()
+    assert np.array_equal(_host(y, dtype), y_w)
+    tol = 1e-6 if dtype == "f32" else 1e-2
+    assert H.max_rel(_host(gx, dtype), dx_w) < tol
+    assert H.max_rel(_host(ga, dtype), 1 + dx_w) < tol
+
+
+@pytest.mark.parametrize("N,Cc,Hh,W,K", [(1, 64, 3, 5, 8), (2, 64, 40, 130, 64), (1, 128, 65, 67, 256), (3, 64, 33, 31, 19), (1, 64, 70, 300, 520)])
+def test_bias_gradient(N, Cc, Hh, W, K):
+    import torch
+    dy = orc.round_bf16(H.uniform(14, (N, K, Hh, W), -0.5, 1.0))
+    L = abi.lib()
+    a = conv_args(abi.AD_BF16, abi.AD_NHWC, (N, Cc, Hh, W), K, 1, 1, 1, 0)
+    x, ddy = torch.zeros(N, Hh, W, Cc, dtype=torch.bfloat16, device="cuda"), H.dev_bf16(orc.nchw_to_nhwc(dy))
+    dw, db = torch.empty(K, 1, 1, Cc, device="cuda"), torch.ones(K, device="cuda")
+    scratch = torch.zeros(L.ad_conv2d_scratch_bytes(C.byref(a), 2), dtype=torch.uint8, device="cuda")
+    a.x, a.y, a.dw, a.db, a.scratch, a.scratch_bytes, a.accumulate = (x.data_ptr(), ddy.data_ptr(), dw.data_ptr(), db.data_ptr(), scratch.data_ptr(),
+                                                                     scratch.numel(), 1)
+    dw.zero_()
+    abi.check(L.ad_conv2d_wgrad(C.byref(a), H.stream()))
+    H.sync()
+    assert H.max_rel(H.host(db), 1 + dy.astype(np.float64).sum(axis=(0, 2, 3))) < 1e-5
