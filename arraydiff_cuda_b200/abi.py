@@ -116,6 +116,7 @@ SIGNATURES = {
     "ad_maxpool2d_fwd": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), u32, u32, u32, u32, vp]),
     "ad_maxpool2d_bwd": (C.c_int, [C.POINTER(Tensor4)] * 3 + [u32, u32, u32, u32, i32, vp]),
     "ad_relu_fwd": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), vp]),
+    "ad_bn_bwd_add": (C.c_int, [C.POINTER(Tensor4)] * 4 + [vp, vp, vp, vp, vp, vp, i32, i32, vp, sz, vp]),
     "ad_relu_bwd": (C.c_int, [C.POINTER(Tensor4)] * 3 + [i32, vp]),
     "ad_add": (C.c_int, [C.POINTER(Tensor4)] * 3 + [vp]),
     "ad_convert": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), i32, vp]),

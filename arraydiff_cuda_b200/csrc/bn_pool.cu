@@ -100,68 +100,74 @@ __global__ void __launch_bounds__(256) bn_reduce_cfast(BnRed p, float* partial) 
   }
 }
 
-// Stage 2 of the statistics, 32 channels per block of 1024 threads: 32 row lanes walk the partial rows
-// (each warp access is one 128-byte line, up to 8 rows in flight per thread), sum in double, and are
-// combined in a fixed order.
+// Stage 2 of the statistics: the partial rows are added in double.
 //   kind 0: mean / invstd / var from (sum x, sum x^2); double arithmetic for the cancellation in E[x^2]-E[x]^2
-//   kind 1: sums[0..2C) = (sum g, sum g*xhat), sums[2C..4C) = those over count; dbeta += sum g, dgamma += sum g*xhat
+//   kind 1: sums[0..2C) = (sum g, sum g*xhat), sums[2C..4C) = those over count; dbeta, dgamma (+)= those sums
 //   kind 2: sums[0..2C) only
-constexpr int kFinishLanes = 32;
-__global__ void __launch_bounds__(32 * kFinishLanes) bn_finish(int kind, uint32_t C, int nsplit, const float* __restrict__ partial,
-                                                               double count, float eps, float* mean, float* invstd,
-                                                               float* var, float* sums, float* dgamma, float* dbeta) {
-  const uint32_t lane = threadIdx.x & 31, rl = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
-  double s = 0.0, ss = 0.0;
-  if (c < C) {
-    for (int k0 = rl; k0 < nsplit; k0 += 8 * kFinishLanes) {
-      float v[8], w[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int k = k0 + u * kFinishLanes;
-        v[u] = w[u] = 0.f;
-        if (k < nsplit) { v[u] = partial[(size_t)k * 2 * C + c]; w[u] = partial[(size_t)k * 2 * C + C + c]; }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) { s += (double)v[u]; ss += (double)w[u]; }
-    }
-  }
-  __shared__ double sh[2][kFinishLanes][33];
-  sh[0][rl][lane] = s;
-  sh[1][rl][lane] = ss;
-  __syncthreads();
-  // warp w < 2 sums statistic w: lane = channel, row lanes in order
-  if (rl >= 2) return;
-  double t = 0.0;
-#pragma unroll 8
-  for (int w = 0; w < kFinishLanes; ++w) t += sh[rl][w][lane];
-  __shared__ double tot[2][32];
-  tot[rl][lane] = t;
-  __syncwarp();
-  // the two warps meet through shared memory: named barrier over these 64 threads
-  asm volatile("bar.sync 1, 64;" ::: "memory");
-  if (rl != 0 || c >= C) return;
-  s = tot[0][lane]; ss = tot[1][lane];
-  if (kind == 0) {
-    double m = s / count, v = ss / count - m * m;
+struct BnFin {
+  int kind;
+  uint32_t C;
+  double count;
+  float eps;
+  float *mean, *invstd, *var, *sums, *dgamma, *dbeta;
+  int accumulate;     // kind 1: add to dgamma / dbeta (else overwrite)
+};
+__device__ __forceinline__ void bn_finish_channel(const BnFin& f, uint32_t c, double s, double ss) {
+  if (f.kind == 0) {
+    double m = s / f.count, v = ss / f.count - m * m;
     if (v < 0.0) v = 0.0;
-    if (mean) mean[c] = (float)m;
-    if (invstd) invstd[c] = (float)(1.0 / sqrt(v + (double)eps));
-    if (var) var[c] = (float)v;
+    if (f.mean) f.mean[c] = (float)m;
+    if (f.invstd) f.invstd[c] = (float)(1.0 / sqrt(v + (double)f.eps));
+    if (f.var) f.var[c] = (float)v;
     return;
   }
   const float fs = (float)s, fss = (float)ss;
-  sums[c] = fs;
-  sums[C + c] = fss;
-  if (kind == 1) {
-    sums[2 * C + c] = (float)((double)fs / count);
-    sums[3 * C + c] = (float)((double)fss / count);
-    if (dbeta) dbeta[c] += fs;
-    if (dgamma) dgamma[c] += fss;
+  f.sums[c] = fs;
+  f.sums[f.C + c] = fss;
+  if (f.kind == 1) {
+    f.sums[2 * f.C + c] = (float)((double)fs / f.count);
+    f.sums[3 * f.C + c] = (float)((double)fss / f.count);
+    if (f.dbeta) f.dbeta[c] = f.accumulate ? f.dbeta[c] + fs : fs;
+    if (f.dgamma) f.dgamma[c] = f.accumulate ? f.dgamma[c] + fss : fss;
   }
+}
+// 8 channels per block (a row's 32-byte sector), 32 row lanes of 16 values: a thread has its rows (10 of the usual 296) in
+// flight at once, so the kernel is one trip to L2 and a short tree.  As 32 channels per block with 8 rows in flight and a
+// serial sum of 32 lanes it took 5.6 us, this form 3.3 us at 256 channels.
+constexpr uint32_t kFinishThreads = 512, kFinishRows = 10;
+__global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit, const float* __restrict__ partial) {
+  const uint32_t v = threadIdx.x & 15, rl = threadIdx.x >> 4, which = v >> 3, c = blockIdx.x * 8 + (v & 7);
+  double t = 0.0;
+  if (c < f.C) {
+    const float* src = partial + which * f.C + c;
+    for (uint32_t k0 = rl; k0 < (uint32_t)nsplit; k0 += 32 * kFinishRows) {
+      float r[kFinishRows];
+#pragma unroll
+      for (uint32_t u = 0; u < kFinishRows; ++u) {
+        const uint32_t k = k0 + u * 32;
+        r[u] = k < (uint32_t)nsplit ? src[(size_t)k * 2 * f.C] : 0.f;
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kFinishRows; ++u) t += (double)r[u];
+    }
+  }
+  t += __shfl_xor_sync(0xffffffffu, t, 16);
+  __shared__ double sh[16][17];
+  if ((threadIdx.x & 31) < 16) sh[threadIdx.x >> 5][v] = t;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  // lane: value v, half of the 16 warps' sums
+  const uint32_t h = threadIdx.x >> 4;
+  t = 0.0;
+#pragma unroll
+  for (uint32_t w = 0; w < 8; ++w) t += sh[h * 8 + w][v];
+  t += __shfl_xor_sync(0xffffffffu, t, 16);
+  const double ss = __shfl_down_sync(0xffffffffu, t, 8);
+  if (threadIdx.x < 8 && c < f.C) bn_finish_channel(f, c, t, ss);
 }
 
 struct BnApply {
-  BView x, dy, out;
+  BView x, dy, out, add;   // add: what the backward form adds to its result (accumulate), of out's dims
   uint32_t N, C, H, W;
   int c_fastest, relu, accumulate;
   const float *gamma, *beta, *mean, *invstd;
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(256) bn_apply(BnApply p) {
       if (p.relu && fmaf(p.gamma[c], xhat, p.beta[c]) <= 0.f) g = 0.f;
       const float m1 = (float)((double)p.partial[c] / p.count), m2 = (float)((double)p.partial[p.C + c] / p.count);
       float v = p.gamma[c] * p.invstd[c] * (g - m1 - xhat * m2);
-      if (p.accumulate) v += ld_f(op);
+      if (p.accumulate) v += ld_f((const T*)p.add.base + (n * p.add.sn + c * p.add.sc + y * p.add.sy + x * p.add.sx));
       st_f(op, v);
     }
   }
@@ -205,7 +211,8 @@ __global__ void __launch_bounds__(256) bn_apply(BnApply p) {
 // ------------------------------------------------------------------ NHWC bf16 fast paths
 // Channel-fastest bf16 views whose strides are multiples of 8 elements: a thread owns 8 adjacent
 // channels (one 16-byte load / store per pixel) of a fixed channel group, so the per-channel
-// constants sit in registers and every warp access is a run of whole 128-byte lines.
+// constants sit in registers and every warp access is a run of whole 128-byte lines.  A block holds
+// 256 / (C / 8) pixel lanes; up to C / 8 - 1 threads are over when C / 8 is no power of two.
 __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
@@ -225,14 +232,17 @@ __device__ __forceinline__ long long pix_off(const BView& v, uint32_t i, uint32_
   const uint32_t r = i / W, x = i - r * W, n = r / H, y = r - n * H;
   return n * v.sn + y * v.sy + x * v.sx;
 }
-__device__ __forceinline__ uint4 ld16(const BView& v, long long off) {
-  return *(const uint4*)((const __nv_bfloat16*)v.base + off);
-}
+__device__ __forceinline__ const void* at16(const BView& v, long long off) { return (const __nv_bfloat16*)v.base + off; }
 
-constexpr int kBnUnroll = 4;  // pixels in flight per thread: all loads of a batch are issued before any use
+constexpr int kBnUnroll = 4;      // pixels per thread below which a smaller grid would do (vec_grid)
+constexpr int kBnDepth = 8;       // loads in flight per thread and stream
 
+// HBM-bound.  131,072 x 512 bf16 inside a net: 34 -> 27 us (MODE 0), 60 -> 53 us (MODE 1) against batches of 4 loads in
+// registers; 16 in flight gained nothing more.
 template <int MODE>
 __global__ void __launch_bounds__(256, 2) bn_reduce_vec(BnRed p, float* partial) {
+  extern __shared__ __align__(128) uint4 ring_smem[];
+  LoadRing<MODE + 1, kBnDepth> ring(ring_smem);
   const uint32_t G = p.C / 8, cg = threadIdx.x % G, pl = threadIdx.x / G, PL = 256 / G;
   const uint32_t per = p.N * p.H * p.W, stride = gridDim.x * PL;
   float a[8], b[8], mean[8], invstd[8], gam[8], bet[8];
@@ -243,36 +253,35 @@ __global__ void __launch_bounds__(256, 2) bn_reduce_vec(BnRed p, float* partial)
   }
   // Pixels are walked from the last to the first: the tensor was just written front to back by its producer, so its
   // tail is what the L2 still holds; the apply pass that follows walks front to back and meets what this pass read last.
-  for (uint32_t i0 = blockIdx.x * PL + pl; i0 < per; i0 += kBnUnroll * stride) {
-    uint4 xr[kBnUnroll], gr[kBnUnroll];
-#pragma unroll
-    for (int u = 0; u < kBnUnroll; ++u) {
-      const uint32_t k = i0 + u * stride;
-      if (k < per) {
-        const uint32_t i = per - 1u - k;
-        xr[u] = ld16(p.x, pix_off(p.x, i, p.H, p.W) + cg * 8);
-        if (MODE == 1) gr[u] = ld16(p.dy, pix_off(p.dy, i, p.H, p.W) + cg * 8);
-      }
+  auto issue = [&](uint32_t k) {
+    if (k < per) {
+      const uint32_t i = per - 1u - k;
+      ring.copy(0, at16(p.x, pix_off(p.x, i, p.H, p.W) + cg * 8));
+      if (MODE == 1) ring.copy(MODE, at16(p.dy, pix_off(p.dy, i, p.H, p.W) + cg * 8));
     }
+    ring.commit();
+  };
+  uint32_t k = pl < PL ? blockIdx.x * PL + pl : per;
 #pragma unroll
-    for (int u = 0; u < kBnUnroll; ++u) {
-      if (i0 + u * stride >= per) break;
-      float xv[8];
-      unpack8(xr[u], xv);
-      if (MODE == 0) {
+  for (int d = 0; d < kBnDepth - 1; ++d) issue(k + d * stride);
+  for (; k < per; k += stride) {
+    ring.wait();
+    float xv[8], g[8];
+    unpack8(ring.get(0), xv);
+    if (MODE == 1) unpack8(ring.get(MODE), g);
+    ring.next();
+    issue(k + (kBnDepth - 1) * stride);
+    if (MODE == 0) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { a[j] += xv[j]; b[j] = fmaf(xv[j], xv[j], b[j]); }
-      } else {
-        float g[8];
-        unpack8(gr[u], g);
+      for (int j = 0; j < 8; ++j) { a[j] += xv[j]; b[j] = fmaf(xv[j], xv[j], b[j]); }
+    } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xhat = (xv[j] - mean[j]) * invstd[j];
-          float gj = g[j];
-          if (p.relu && fmaf(gam[j], xhat, bet[j]) <= 0.f) gj = 0.f;
-          a[j] += gj;
-          b[j] = fmaf(gj, xhat, b[j]);
-        }
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = (xv[j] - mean[j]) * invstd[j];
+        float gj = g[j];
+        if (p.relu && fmaf(gam[j], xhat, bet[j]) <= 0.f) gj = 0.f;
+        a[j] += gj;
+        b[j] = fmaf(gj, xhat, b[j]);
       }
     }
   }
@@ -284,14 +293,18 @@ __global__ void __launch_bounds__(256, 2) bn_reduce_vec(BnRed p, float* partial)
   for (uint32_t t = threadIdx.x; t < 2 * p.C; t += 256) {
     const uint32_t which = t / p.C, c = t - which * p.C, g = c >> 3, j = c & 7;
     float acc = 0.f;
+#pragma unroll 8
     for (uint32_t q = 0; q < PL; ++q) acc += which ? sb[q * G + g][j] : sa[q * G + g][j];
     partial[(size_t)blockIdx.x * 2 * p.C + t] = acc;
   }
 }
 
-// U pixels in flight per thread (the backward form holds three 16-byte values per pixel, so fewer)
-template <int MODE, int U = (MODE == 0 ? kBnUnroll : 2)>
+// ADD: the backward form adds *add to what it writes.  HBM-bound: 131,072 x 512 bf16 50 -> 42 us (MODE 0, 6.4 TB/s) and
+// 78 -> 62 us (MODE 1, 6.5 TB/s) against batches of 3-4 loads in registers.
+template <int MODE, bool ADD>
 __global__ void __launch_bounds__(256, 2) bn_apply_vec(BnApply p) {
+  extern __shared__ __align__(128) uint4 ring_smem[];
+  LoadRing<MODE + 1 + ADD, kBnDepth> ring(ring_smem);
   const uint32_t G = p.C / 8, cg = threadIdx.x % G, pl = threadIdx.x / G, PL = 256 / G;
   const uint32_t per = p.N * p.H * p.W, stride = gridDim.x * PL;
   float sc[8], sh[8], mean[8], invstd[8], m1[8], m2[8];
@@ -302,54 +315,48 @@ __global__ void __launch_bounds__(256, 2) bn_apply_vec(BnApply p) {
     sc[j] = p.gamma[c]; sh[j] = p.beta[c];
     if (MODE == 1) { m1[j] = p.partial[2 * p.C + c]; m2[j] = p.partial[3 * p.C + c]; }
   }
-  for (uint32_t i0 = blockIdx.x * PL + pl; i0 < per; i0 += U * stride) {
-    uint4 xr[U], gr[U], oldr[U];
-    uint4* op[U];
+  auto issue = [&](uint32_t i) {
+    if (i < per) {
+      ring.copy(0, at16(p.x, pix_off(p.x, i, p.H, p.W) + cg * 8));
+      if (MODE == 1) ring.copy(MODE, at16(p.dy, pix_off(p.dy, i, p.H, p.W) + cg * 8));
+      if (ADD) ring.copy(MODE + ADD, at16(p.add, pix_off(p.add, i, p.H, p.W) + cg * 8));
+    }
+    ring.commit();
+  };
+  uint32_t i = pl < PL ? blockIdx.x * PL + pl : per;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t i = i0 + u * stride;
-      if (i < per) {
-        xr[u] = ld16(p.x, pix_off(p.x, i, p.H, p.W) + cg * 8);
-        op[u] = (uint4*)((__nv_bfloat16*)p.out.base + pix_off(p.out, i, p.H, p.W) + cg * 8);
-        if (MODE == 1) {
-          gr[u] = ld16(p.dy, pix_off(p.dy, i, p.H, p.W) + cg * 8);
-          if (p.accumulate) oldr[u] = *op[u];
-        }
+  for (int d = 0; d < kBnDepth - 1; ++d) issue(i + d * stride);
+  for (; i < per; i += stride) {
+    ring.wait();
+    float xv[8], g[8], old[8], o[8];
+    unpack8(ring.get(0), xv);
+    if (MODE == 1) unpack8(ring.get(MODE), g);
+    if (ADD) unpack8(ring.get(MODE + ADD), old);
+    ring.next();
+    issue(i + (kBnDepth - 1) * stride);
+    if (MODE == 0) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = (xv[j] - mean[j]) * invstd[j];
+        float v = fmaf(sc[j], xhat, sh[j]);
+        o[j] = p.relu ? fmaxf(v, 0.f) : v;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = (xv[j] - mean[j]) * invstd[j];
+        float gj = g[j];
+        if (p.relu && fmaf(sc[j], xhat, sh[j]) <= 0.f) gj = 0.f;
+        float v = sc[j] * invstd[j] * (gj - m1[j] - xhat * m2[j]);
+        o[j] = ADD ? v + old[j] : v;
       }
     }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (i0 + u * stride >= per) break;
-      float xv[8], o[8];
-      unpack8(xr[u], xv);
-      if (MODE == 0) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xhat = (xv[j] - mean[j]) * invstd[j];
-          float v = fmaf(sc[j], xhat, sh[j]);
-          o[j] = p.relu ? fmaxf(v, 0.f) : v;
-        }
-      } else {
-        float g[8], old[8];
-        unpack8(gr[u], g);
-        if (p.accumulate) unpack8(oldr[u], old);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xhat = (xv[j] - mean[j]) * invstd[j];
-          float gj = g[j];
-          if (p.relu && fmaf(sc[j], xhat, sh[j]) <= 0.f) gj = 0.f;
-          float v = sc[j] * invstd[j] * (gj - m1[j] - xhat * m2[j]);
-          o[j] = p.accumulate ? v + old[j] : v;
-        }
-      }
-      *op[u] = pack8(o);
-    }
+    *(uint4*)((__nv_bfloat16*)p.out.base + pix_off(p.out, i, p.H, p.W) + cg * 8) = pack8(o);
   }
 }
 
 static bool vec_view_ok(const ad_tensor4* t) {
   if (t->dtype != AD_BF16 || t->sc != 1 || (t->C & 7u) || t->C < 8 || t->C > 2048) return false;
-  if (256 % (t->C / 8)) return false;
   if ((size_t)t->N * t->H * t->W >= (1ull << 31)) return false;
   return !((uintptr_t)t->base & 15u) && !(t->sn & 7) && !(t->sy & 7) && !(t->sx & 7);
 }
@@ -361,6 +368,16 @@ static unsigned vec_grid(const ad_tensor4* t) {
   if (g > (size_t)kNumSMs * 2) g = (size_t)kNumSMs * 2;   // two resident blocks per SM keep ~5 MB of loads in flight
   if (g > (size_t)bn_max_splits(t->C)) g = bn_max_splits(t->C);
   return (unsigned)(g < 1 ? 1 : g);
+}
+
+static int ring_smem_failed() { cudaGetLastError(); return AD_ERR_CUDA; }
+template <int MODE, bool ADD>
+static int launch_apply_vec(const BnApply& a, cudaStream_t s) {
+  constexpr int smem = LoadRing<MODE + 1 + ADD, kBnDepth>::kBytes;
+  if (cudaFuncSetAttribute(bn_apply_vec<MODE, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return ring_smem_failed();
+  const uint32_t PL = 256 / (a.C / 8), per = a.N * a.H * a.W;
+  bn_apply_vec<MODE, ADD><<<grid_for(per, PL * kBnUnroll, 2), 256, smem, s>>>(a);
+  return AD_OK;
 }
 
 static int pick_splits(const ad_tensor4* x, bool cfast) {
@@ -375,24 +392,33 @@ static int pick_splits(const ad_tensor4* x, bool cfast) {
   return (int)want;
 }
 
+static void launch_finish(const BnFin& f, int nsplit, const float* partial, cudaStream_t s) {
+  bn_finish<<<(f.C + 7) / 8, kFinishThreads, 0, s>>>(f, nsplit, partial);
+  count_launch();
+}
+// Both stages of the statistics of x (MODE 0) or of the backward sums (MODE 1) into what `f` names
 template <int MODE>
-static int launch_reduce(const BnRed& p, const ad_tensor4* x, float* partial, int& nsplit, cudaStream_t s) {
+static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, float* partial, cudaStream_t s) {
   const bool cfast = x->sc == 1 && x->C > 1;
+  int nsplit;
   if (vec_view_ok(x) && (MODE == 0 || (p.dy.sc == 1 && !((uintptr_t)p.dy.base & 15u) && !(p.dy.sn & 7) && !(p.dy.sy & 7) && !(p.dy.sx & 7)))) {
     nsplit = (int)vec_grid(x);
-    bn_reduce_vec<MODE><<<nsplit, 256, 0, s>>>(p, partial);
-    count_launch();
-    return launch_status();
-  }
-  nsplit = pick_splits(x, cfast);
-  if (cfast) {
-    dim3 grid((x->C + 31) / 32, nsplit), block(32, 8);
-    AD_DISPATCH_DTYPE(x->dtype, (bn_reduce_cfast<T, MODE><<<grid, block, 0, s>>>(p, partial)));
+    constexpr int smem = LoadRing<MODE + 1, kBnDepth>::kBytes;
+    // the attribute is per function and per device; setting it is cheap enough to do per launch
+    if (cudaFuncSetAttribute(bn_reduce_vec<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return ring_smem_failed();
+    bn_reduce_vec<MODE><<<nsplit, 256, smem, s>>>(p, partial);
   } else {
-    dim3 grid(x->C, nsplit);
-    AD_DISPATCH_DTYPE(x->dtype, (bn_reduce_xfast<T, MODE><<<grid, 256, 0, s>>>(p, partial)));
+    nsplit = pick_splits(x, cfast);
+    if (cfast) {
+      dim3 grid((x->C + 31) / 32, nsplit), block(32, 8);
+      AD_DISPATCH_DTYPE(x->dtype, (bn_reduce_cfast<T, MODE><<<grid, block, 0, s>>>(p, partial)));
+    } else {
+      dim3 grid(x->C, nsplit);
+      AD_DISPATCH_DTYPE(x->dtype, (bn_reduce_xfast<T, MODE><<<grid, 256, 0, s>>>(p, partial)));
+    }
   }
   count_launch();
+  launch_finish(f, nsplit, partial, s);
   return launch_status();
 }
 
@@ -786,18 +812,25 @@ using namespace adk;
 
 extern "C" size_t ad_bn_scratch_bytes(uint32_t C) { return (size_t)(bn_max_splits(C) + 2) * 2 * C * sizeof(float); }
 
+// y = the normalised x with the statistics a.mean / a.invstd, or the backward pass over them
+template <int MODE>
+static int launch_apply(const BnApply& a, const ad_tensor4* x, bool vec, cudaStream_t s) {
+  if (vec) {
+    const int rc = MODE == 1 && a.accumulate ? launch_apply_vec<MODE, MODE == 1>(a, s) : launch_apply_vec<MODE, false>(a, s);
+    if (rc != AD_OK) return rc;
+  } else {
+    const size_t total = (size_t)x->N * x->C * x->H * x->W;
+    AD_DISPATCH_DTYPE(x->dtype, (bn_apply<T, MODE><<<grid_for(total, 256, 16), 256, 0, s>>>(a)));
+  }
+  count_launch();
+  return launch_status();
+}
+
 extern "C" int ad_bn_partial_stats(const ad_tensor4* x, float* sums, void* scratch, size_t scratch_bytes, void* stream) {
   if (!x || !x->base || !sums || !scratch) return AD_ERR_BAD_ARG;
   if (scratch_bytes < ad_bn_scratch_bytes(x->C)) return AD_ERR_SCRATCH;
-  cudaStream_t s = as_stream(stream);
   BnRed p{bview(x), bview(x), x->N, x->C, x->H, x->W, 0, nullptr, nullptr, nullptr, nullptr};
-  int nsplit = 1;
-  int st = launch_reduce<0>(p, x, (float*)scratch, nsplit, s);
-  if (st != AD_OK) return st;
-  bn_finish<<<(x->C + 31) / 32, 32 * kFinishLanes, 0, s>>>(2, x->C, nsplit, (const float*)scratch, 1.0, 0.f, nullptr, nullptr, nullptr, sums,
-                                             nullptr, nullptr);
-  count_launch();
-  return launch_status();
+  return launch_reduce<0>(p, x, BnFin{2, x->C, 1.0, 0.f, nullptr, nullptr, nullptr, sums, nullptr, nullptr, 0}, (float*)scratch, as_stream(stream));
 }
 
 extern "C" int ad_bn_finalize_apply(const ad_tensor4* x, const ad_tensor4* y, const float* sums, double count,
@@ -806,16 +839,10 @@ extern "C" int ad_bn_finalize_apply(const ad_tensor4* x, const ad_tensor4* y, co
   if (!x || !y || !x->base || !y->base || !sums || !gamma || !beta || !save_mean || !save_invstd) return AD_ERR_BAD_ARG;
   if (!dims_eq(x, y) || count <= 0.0) return AD_ERR_BAD_ARG;
   cudaStream_t s = as_stream(stream);
-  bn_finish<<<(x->C + 31) / 32, 32 * kFinishLanes, 0, s>>>(0, x->C, 1, sums, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr,
-                                             nullptr);
-  count_launch();
-  BnApply a{bview(x), bview(x), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
+  launch_finish(BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, 1, sums, s);
+  BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, save_mean, save_invstd, nullptr, 1, count};
-  const size_t total = (size_t)x->N * x->C * x->H * x->W;
-  if (vec_view_ok(x) && vec_view_ok(y)) bn_apply_vec<0><<<kNumSMs * 4, 256, 0, s>>>(a);
-  else AD_DISPATCH_DTYPE(x->dtype, (bn_apply<T, 0><<<grid_for(total, 256, 16), 256, 0, s>>>(a)));
-  count_launch();
-  return launch_status();
+  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), s);
 }
 
 extern "C" int ad_bn_fwd_train(const ad_tensor4* x, const ad_tensor4* y, const float* gamma, const float* beta,
@@ -828,19 +855,12 @@ extern "C" int ad_bn_fwd_train(const ad_tensor4* x, const ad_tensor4* y, const f
   if (total == 0) return AD_OK;
   cudaStream_t s = as_stream(stream);
   BnRed p{bview(x), bview(x), x->N, x->C, x->H, x->W, 0, nullptr, nullptr, nullptr, nullptr};
-  int nsplit = 1;
-  int st = launch_reduce<0>(p, x, (float*)scratch, nsplit, s);
-  if (st != AD_OK) return st;
   const double count = (double)x->N * x->H * x->W;
-  bn_finish<<<(x->C + 31) / 32, 32 * kFinishLanes, 0, s>>>(0, x->C, nsplit, (const float*)scratch, count, eps, save_mean, save_invstd,
-                                             batch_var, nullptr, nullptr, nullptr);
-  count_launch();
-  BnApply a{bview(x), bview(x), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
+  int st = launch_reduce<0>(p, x, BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, (float*)scratch, s);
+  if (st != AD_OK) return st;
+  BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, save_mean, save_invstd, nullptr, 1, count};
-  if (vec_view_ok(x) && vec_view_ok(y)) bn_apply_vec<0><<<kNumSMs * 4, 256, 0, s>>>(a);
-  else AD_DISPATCH_DTYPE(x->dtype, (bn_apply<T, 0><<<grid_for(total, 256, 16), 256, 0, s>>>(a)));
-  count_launch();
-  return launch_status();
+  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), s);
 }
 
 // invstd[c] = 1 / sqrt(var[c] + eps), in double as the training path does
@@ -859,40 +879,40 @@ extern "C" int ad_bn_fwd_inference(const ad_tensor4* x, const ad_tensor4* y, con
   cudaStream_t s = as_stream(stream);
   bn_invstd_kernel<<<(x->C + 255) / 256, 256, 0, s>>>(x->C, var, eps, invstd_out);
   count_launch();
-  BnApply a{bview(x), bview(x), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
+  BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, mean, invstd_out, nullptr, 1, (double)x->N * x->H * x->W};
-  if (vec_view_ok(x) && vec_view_ok(y)) bn_apply_vec<0><<<kNumSMs * 4, 256, 0, s>>>(a);
-  else AD_DISPATCH_DTYPE(x->dtype, (bn_apply<T, 0><<<grid_for(total, 256, 16), 256, 0, s>>>(a)));
-  count_launch();
-  return launch_status();
+  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), s);
+}
+
+extern "C" int ad_bn_bwd_add(const ad_tensor4* x, const ad_tensor4* dy, const ad_tensor4* addend, const ad_tensor4* dx, const float* gamma,
+                             const float* beta, const float* save_mean, const float* save_invstd, float* dgamma,
+                             float* dbeta, int32_t relu, int32_t accumulate_params, void* scratch, size_t scratch_bytes,
+                             void* stream) {
+  if (!x || !dy || !dx || !x->base || !dy->base || !dx->base || !gamma || !beta || !save_mean || !save_invstd || !scratch)
+    return AD_ERR_BAD_ARG;
+  if (addend && !addend->base) return AD_ERR_BAD_ARG;
+  if (!dims_eq(x, dy) || !dims_eq(x, dx) || (addend && !dims_eq(x, addend))) return AD_ERR_BAD_ARG;
+  if (scratch_bytes < ad_bn_scratch_bytes(x->C)) return AD_ERR_SCRATCH;
+  const size_t total = (size_t)x->N * x->C * x->H * x->W;
+  if (total == 0) return AD_OK;
+  cudaStream_t s = as_stream(stream);
+  BnRed p{bview(x), bview(dy), x->N, x->C, x->H, x->W, relu, gamma, beta, save_mean, save_invstd};
+  float* partial = (float*)scratch;
+  float* sums = partial + (size_t)bn_max_splits(x->C) * 2 * x->C;
+  const double count = (double)x->N * x->H * x->W;
+  int st = launch_reduce<1>(p, x, BnFin{1, x->C, count, 0.f, nullptr, nullptr, nullptr, sums, dgamma, dbeta, accumulate_params}, partial, s);
+  if (st != AD_OK) return st;
+  BnApply a{bview(x), bview(dy), bview(dx), bview(addend ? addend : dx), x->N, x->C, x->H, x->W, dx->sc == 1 && dx->C > 1, relu, addend != nullptr,
+            gamma, beta, save_mean, save_invstd, sums, 1, count};
+  return launch_apply<1>(a, x, vec_view_ok(x) && vec_view_ok(dy) && vec_view_ok(dx) && (!addend || vec_view_ok(addend)), s);
 }
 
 extern "C" int ad_bn_bwd(const ad_tensor4* x, const ad_tensor4* dy, const ad_tensor4* dx, const float* gamma,
                          const float* beta, const float* save_mean, const float* save_invstd, float* dgamma,
                          float* dbeta, int32_t relu, int32_t accumulate_dx, void* scratch, size_t scratch_bytes,
                          void* stream) {
-  if (!x || !dy || !dx || !x->base || !dy->base || !dx->base || !gamma || !beta || !save_mean || !save_invstd || !scratch)
-    return AD_ERR_BAD_ARG;
-  if (!dims_eq(x, dy) || !dims_eq(x, dx)) return AD_ERR_BAD_ARG;
-  if (scratch_bytes < ad_bn_scratch_bytes(x->C)) return AD_ERR_SCRATCH;
-  const size_t total = (size_t)x->N * x->C * x->H * x->W;
-  if (total == 0) return AD_OK;
-  cudaStream_t s = as_stream(stream);
-  BnRed p{bview(x), bview(dy), x->N, x->C, x->H, x->W, relu, gamma, beta, save_mean, save_invstd};
-  int nsplit = 1;
-  float* partial = (float*)scratch;
-  int st = launch_reduce<1>(p, x, partial, nsplit, s);
-  if (st != AD_OK) return st;
-  float* sums = partial + (size_t)bn_max_splits(x->C) * 2 * x->C;
-  const double count = (double)x->N * x->H * x->W;
-  bn_finish<<<(x->C + 31) / 32, 32 * kFinishLanes, 0, s>>>(1, x->C, nsplit, partial, count, 0.f, nullptr, nullptr, nullptr, sums, dgamma, dbeta);
-  count_launch();
-  BnApply a{bview(x), bview(dy), bview(dx), x->N, x->C, x->H, x->W, dx->sc == 1 && dx->C > 1, relu, accumulate_dx,
-            gamma, beta, save_mean, save_invstd, sums, 1, count};
-  if (vec_view_ok(x) && vec_view_ok(dy) && vec_view_ok(dx)) bn_apply_vec<1><<<kNumSMs * 4, 256, 0, s>>>(a);
-  else AD_DISPATCH_DTYPE(x->dtype, (bn_apply<T, 1><<<grid_for(total, 256, 16), 256, 0, s>>>(a)));
-  count_launch();
-  return launch_status();
+  return ad_bn_bwd_add(x, dy, accumulate_dx ? dx : nullptr, dx, gamma, beta, save_mean, save_invstd, dgamma, dbeta, relu, 1, scratch, scratch_bytes,
+                       stream);
 }
 
 static int pool_params(const ad_tensor4* x, const ad_tensor4* y, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw,

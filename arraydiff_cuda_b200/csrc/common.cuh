@@ -56,6 +56,32 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
+// A ring of 16-byte loads in flight, D per thread and stream, in shared memory: each thread copies its own next elements
+// (cp.async) and reads only what it copied, so no barrier is needed and the loads in flight cost no registers.  For
+// streaming kernels of 256 threads, two blocks per SM: with 8 x 4 KB per stream the batch normalisation passes measured
+// 5.0-6.5 TB/s where batches of 4 loads in registers reached 4.1-5.4.
+constexpr int kRingThreads = 256;
+template <int S, int D>
+struct LoadRing {
+  static constexpr int kBytes = S * D * kRingThreads * 16;
+  uint4* base;   // this thread's slots
+  int put_at, get_at;
+  __device__ __forceinline__ explicit LoadRing(void* smem) : base((uint4*)smem + threadIdx.x), put_at(0), get_at(0) {}
+  __device__ __forceinline__ void copy(int stream, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(base + (put_at * S + stream) * kRingThreads)),
+                 "l"(src) : "memory");
+  }
+  // after the copies of one element of every stream (or none, past the end)
+  __device__ __forceinline__ void commit() {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (++put_at == D) put_at = 0;
+  }
+  // D - 1 elements are committed ahead of the one that is waited for
+  __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory"); }
+  __device__ __forceinline__ uint4 get(int stream) const { return base[(get_at * S + stream) * kRingThreads]; }
+  __device__ __forceinline__ void next() { if (++get_at == D) get_at = 0; }
+};
+
 // Dispatch a callable templated on the element type.
 #define AD_DISPATCH_DTYPE(dtype, ...)                                   \
   do {                                                                  \

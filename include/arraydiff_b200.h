@@ -278,6 +278,14 @@ int ad_bn_bwd(const ad_tensor4* x, const ad_tensor4* dy, const ad_tensor4* dx, c
               float* dbeta, int32_t relu, int32_t accumulate_dx, void* scratch, size_t scratch_bytes,
               void* stream);
 /*
+ * ad_bn_bwd with its sums spelled out: dx = the gradient of this layer + *addend (NULL: nothing added; a view of dx
+ * itself: ad_bn_bwd with accumulate_dx; any other tensor of the same dims and dtype: the gradient that arrives over a
+ * residual connection, which then needs no copy into dx first).  accumulate_params 0 overwrites dgamma and dbeta.
+ */
+int ad_bn_bwd_add(const ad_tensor4* x, const ad_tensor4* dy, const ad_tensor4* addend, const ad_tensor4* dx, const float* gamma,
+                  const float* beta, const float* save_mean, const float* save_invstd, float* dgamma, float* dbeta,
+                  int32_t relu, int32_t accumulate_params, void* scratch, size_t scratch_bytes, void* stream);
+/*
  * Batch normalisation with FIXED statistics (the running mean / variance an optimizer keeps), optional fused ReLU:
  *   y = relu?(gamma * (x - mean) / sqrt(var + eps) + beta).
  * Replaces cudnnBatchNormalizationForwardInference, src/op.cc:3964-3978 (taken when the net's switch variable is
