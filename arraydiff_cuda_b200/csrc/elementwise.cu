@@ -141,48 +141,50 @@ __device__ __forceinline__ long long ew_pix_off(const View& v, uint32_t i, uint3
   const uint32_t r = i / W, x = i - r * W, n = r / H, y = r - n * H;
   return n * v.sn + y * v.sy + x * v.sx;
 }
-// G = C/8 channel groups; the launcher guarantees N*H*W*G < 2^31.  Two items per thread and pass.
+// G = C/8 channel groups; the launcher guarantees N*H*W*G < 2^31.  HBM-bound: kEwDepth loads per thread and operand in flight.
+constexpr int kEwDepth = 8;
 template <int OP>
-__global__ void __launch_bounds__(256) ew_vec_kernel(Dims d, View a, View b, View yv, int accumulate) {
+__global__ void __launch_bounds__(256, 2) ew_vec_kernel(Dims d, View a, View b, View yv, int accumulate) {
+  constexpr bool kTwo = OP == kAdd2 || OP == kReluBwd;
+  extern __shared__ __align__(128) uint4 ring_smem[];
+  LoadRing<2 + kTwo, kEwDepth> ring(ring_smem);
   const uint32_t G = d.C / 8;
   const uint32_t total = d.N * d.H * d.W * G, nt = gridDim.x * blockDim.x;
-  constexpr int U = 2;
-  for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += U * nt) {
-    uint4 ar[U], br[U], oldr[U];
-    uint4* op[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t i = i0 + u * nt;
-      if (i < total) {
-        const uint32_t pix = i / G, cg = i - pix * G;
-        ar[u] = *(const uint4*)((const __nv_bfloat16*)a.base + ew_pix_off(a, pix, d.H, d.W) + cg * 8);
-        if (OP == kAdd2 || OP == kReluBwd) br[u] = *(const uint4*)((const __nv_bfloat16*)b.base + ew_pix_off(b, pix, d.H, d.W) + cg * 8);
-        op[u] = (uint4*)((__nv_bfloat16*)yv.base + ew_pix_off(yv, pix, d.H, d.W) + cg * 8);
-        if (accumulate) oldr[u] = *op[u];
-      }
+  auto issue = [&](uint32_t i) {
+    if (i < total) {
+      const uint32_t pix = i / G, cg = i - pix * G;
+      ring.copy(0, (const __nv_bfloat16*)a.base + ew_pix_off(a, pix, d.H, d.W) + cg * 8);
+      if (accumulate) ring.copy(1, (const __nv_bfloat16*)yv.base + ew_pix_off(yv, pix, d.H, d.W) + cg * 8);
+      if (kTwo) ring.copy(1 + kTwo, (const __nv_bfloat16*)b.base + ew_pix_off(b, pix, d.H, d.W) + cg * 8);
     }
+    ring.commit();
+  };
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (i0 + u * nt >= total) break;
-      float av[8], bv[8], o[8], old[8];
-      ew_unpack8(ar[u], av);
-      if (OP == kAdd2 || OP == kReluBwd) ew_unpack8(br[u], bv);
-      if (accumulate) ew_unpack8(oldr[u], old);
+  for (int u = 0; u < kEwDepth - 1; ++u) issue(i + u * nt);
+  for (; i < total; i += nt) {
+    ring.wait();
+    float av[8], bv[8], o[8], old[8];
+    ew_unpack8(ring.get(0), av);
+    if (kTwo) ew_unpack8(ring.get(1 + kTwo), bv);
+    if (accumulate) ew_unpack8(ring.get(1), old);
+    ring.next();
+    issue(i + (kEwDepth - 1) * nt);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float v;
-        if (OP == kRelu) v = fmaxf(av[j], 0.f);
-        else if (OP == kConvert) v = av[j];
-        else if (OP == kAdd2) v = av[j] + bv[j];
-        else v = av[j] > 0.f ? bv[j] : 0.f;
-        o[j] = accumulate ? v + old[j] : v;
-      }
-      uint4 pk;
-      __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
-      *op[u] = pk;
+    for (int j = 0; j < 8; ++j) {
+      float v;
+      if (OP == kRelu) v = fmaxf(av[j], 0.f);
+      else if (OP == kConvert) v = av[j];
+      else if (OP == kAdd2) v = av[j] + bv[j];
+      else v = av[j] > 0.f ? bv[j] : 0.f;
+      o[j] = accumulate ? v + old[j] : v;
     }
+    uint4 pk;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&pk);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+    const uint32_t pix = i / G, cg = i - pix * G;
+    *(uint4*)((__nv_bfloat16*)yv.base + ew_pix_off(yv, pix, d.H, d.W) + cg * 8) = pk;
   }
 }
 static bool ew_vec_ok(const ad_tensor4* t) {
@@ -204,7 +206,13 @@ static int ew_launch(const ad_tensor4* a, const ad_tensor4* b, const ad_tensor4*
   View va = view_of(a), vb = b ? view_of(b) : View{nullptr, 0, 0, 0, 0}, vy = view_of(y);
   cudaStream_t s = as_stream(stream);
   if (total / 8 < (1ull << 31) && ew_vec_ok(a) && ew_vec_ok(y) && (!b || ew_vec_ok(b))) {
-    ew_vec_kernel<OP><<<grid_for(total / 16, 256, 16), 256, 0, s>>>(d, va, vb, vy, accumulate);
+    constexpr int smem = LoadRing<2 + (OP == kAdd2 || OP == kReluBwd), kEwDepth>::kBytes;
+    // the attribute is per function and per device; setting it is cheap enough to do per launch
+    if (cudaFuncSetAttribute(ew_vec_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return AD_ERR_CUDA;
+    }
+    ew_vec_kernel<OP><<<grid_for(total / 8, 256, 2), 256, smem, s>>>(d, va, vb, vy, accumulate);
     count_launch();
     return launch_status();
   }
