@@ -65,6 +65,11 @@ class Conv2dArgs(C.Structure):
     ]
 
 
+class FilterItem(C.Structure):
+    _fields_ = [("src", vp), ("krsc", vp), ("crsk", vp), ("krsc_row", i64),
+                ("K", u32), ("C", u32), ("kh", u32), ("kw", u32), ("crsk_k", u32), ("reserved", u32)]
+
+
 class ConvProfileEntry(C.Structure):
     _fields_ = [("pass_", i32), ("kernel", i32), ("status", i32),
                 ("N", u32), ("C", u32), ("H", u32), ("W", u32), ("K", u32), ("kh", u32), ("kw", u32),
@@ -111,12 +116,12 @@ SIGNATURES = {
     "ad_bn_fwd_train_noalloc": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), vp, vp, vp, vp, vp, f32, i32, vp]),
     "ad_bn_fwd_inference": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), vp, vp, vp, vp, vp, f32, i32, vp]),
     "ad_bn_bwd": (C.c_int, [C.POINTER(Tensor4)] * 3 + [vp, vp, vp, vp, vp, vp, i32, i32, vp, sz, vp]),
+    "ad_bn_bwd_add": (C.c_int, [C.POINTER(Tensor4)] * 4 + [vp, vp, vp, vp, vp, vp, i32, i32, vp, sz, vp]),
     "ad_bn_partial_stats": (C.c_int, [C.POINTER(Tensor4), vp, vp, sz, vp]),
     "ad_bn_finalize_apply": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), vp, C.c_double, vp, vp, vp, vp, vp, f32, i32, vp]),
     "ad_maxpool2d_fwd": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), u32, u32, u32, u32, vp]),
     "ad_maxpool2d_bwd": (C.c_int, [C.POINTER(Tensor4)] * 3 + [u32, u32, u32, u32, i32, vp]),
     "ad_relu_fwd": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), vp]),
-    "ad_bn_bwd_add": (C.c_int, [C.POINTER(Tensor4)] * 4 + [vp, vp, vp, vp, vp, vp, i32, i32, vp, sz, vp]),
     "ad_relu_bwd": (C.c_int, [C.POINTER(Tensor4)] * 3 + [i32, vp]),
     "ad_add": (C.c_int, [C.POINTER(Tensor4)] * 3 + [vp]),
     "ad_convert": (C.c_int, [C.POINTER(Tensor4), C.POINTER(Tensor4), i32, vp]),
@@ -131,6 +136,9 @@ SIGNATURES = {
     "ad_conv2d_fprop": (C.c_int, [C.POINTER(Conv2dArgs), vp]),
     "ad_conv2d_dgrad": (C.c_int, [C.POINTER(Conv2dArgs), vp]),
     "ad_conv2d_wgrad": (C.c_int, [C.POINTER(Conv2dArgs), vp]),
+    "ad_conv2d_dgrad_ex": (C.c_int, [C.POINTER(Conv2dArgs), vp, vp, vp]),
+    "ad_conv2d_wgrad_ex": (C.c_int, [C.POINTER(Conv2dArgs), vp, vp]),
+    "ad_filter_prepare": (C.c_int, [u32, C.POINTER(FilterItem), vp]),
     "ad_conv2d_last_kernel": (i32, []),
     "ad_conv2d_profile": (C.c_int, [i32]),
     "ad_conv2d_profile_read": (sz, [C.POINTER(ConvProfileEntry), sz]),

@@ -588,6 +588,74 @@ __global__ void __launch_bounds__(256) filter_transpose_flip_kernel(uint32_t K, 
     wt[i] = k < K ? w[(((size_t)k * kh + (kh - 1 - r)) * kw + (kw - 1 - s)) * C + c] : __float2bfloat16_rn(0.f);
   }
 }
+// Both tensor-core forms of many fp32 KCRS filters in one launch: KRSC bf16 (rows of `row` elements) and, for the data
+// gradient, C,R,S,K bf16 with mirrored taps (Kp entries per row, zero past K).  A block turns KT filters x CT channels x all
+// taps round in shared memory: fp32 rows are read and runs of bf16 pairs written.  The shapes that nearly all filters have
+// (1x1 and 3x3, whole channel tiles) are compiled with constant extents: with divisions by variable ones the kernel was
+// bound by integer arithmetic.  As two launches per layer (one of them in front of every forward and data-gradient
+// kernel) the 23.5 M weights of a 53-layer net took 640 us, in one launch of variable extents 200, so 89.
+constexpr uint32_t kPrepItems = 32, kPrepFloats = 9216;
+struct PrepItem {
+  const float* src;
+  __nv_bfloat16 *krsc, *crsk;
+  uint32_t K, C, taps, Kp, KT, CT, tile0;   // tile0: first tile of this item
+  long long row;
+};
+struct PrepBatch { PrepItem it[kPrepItems]; uint32_t count, tiles; };
+template <uint32_t T, uint32_t CT, uint32_t KT>   // constant taps and tile, even KT; T = 0: those of the item
+__device__ __forceinline__ void filter_prepare_tile(const PrepItem& p, uint32_t k0, uint32_t c0, float* sm) {
+  const uint32_t taps = T ? T : p.taps, ct = T ? CT : p.CT, kt = T ? KT : p.KT;
+  const uint32_t nc = T ? CT : (p.C - c0 < ct ? p.C - c0 : ct), run = nc * taps, pitch = ct * taps + 1;   // odd pitch where ct * taps is even
+  const uint32_t nk = k0 < p.K ? (p.K - k0 < kt ? p.K - k0 : kt) : 0;
+  const float* src = p.src + ((size_t)k0 * p.C + c0) * taps;
+  const size_t krow = (size_t)p.C * taps;
+#pragma unroll 8
+  for (uint32_t i = threadIdx.x; i < nk * run; i += 256) {
+    const uint32_t k = i / run, e = i - k * run;
+    sm[k * pitch + e] = src[k * krow + e];
+  }
+  __syncthreads();
+  if (T) {
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < nk * (run / 2); i += 256) {
+      const uint32_t c = i % (nc / 2) * 2, r = i / (nc / 2), tap = r % taps, k = r / taps;
+      const float* f = sm + k * pitch + c * taps + tap;
+      *(__nv_bfloat162*)(p.krsc + (size_t)(k0 + k) * p.row + (size_t)tap * p.C + c0 + c) = __floats2bfloat162_rn(f[0], f[taps]);
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i < nk * run; i += 256) {
+      const uint32_t c = i % nc, r = i / nc, tap = r % taps, k = r / taps;
+      p.krsc[(size_t)(k0 + k) * p.row + (size_t)tap * p.C + c0 + c] = __float2bfloat16_rn(sm[k * pitch + c * taps + tap]);
+    }
+  }
+  if (p.crsk) {
+    const uint32_t kk = p.Kp - k0 < kt ? p.Kp - k0 : kt, pairs = kt / 2;   // Kp is even
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < pairs * run; i += 256) {
+      const uint32_t k = i % pairs * 2, r = i / pairs, tap = r % taps, c = r / taps;
+      const float* f = sm + k * pitch + c * taps + tap;
+      if (k < kk)
+        *(__nv_bfloat162*)(p.crsk + ((size_t)(c0 + c) * taps + (taps - 1 - tap)) * p.Kp + k0 + k) =
+            __floats2bfloat162_rn(k < nk ? f[0] : 0.f, k + 1 < nk ? f[pitch] : 0.f);
+    }
+  }
+}
+__global__ void __launch_bounds__(256) filter_prepare_kernel(const __grid_constant__ PrepBatch b) {
+  __shared__ float sm[kPrepFloats + 128];
+  for (uint32_t tile = blockIdx.x; tile < b.tiles; tile += gridDim.x) {
+    uint32_t lo = 0, hi = b.count;   // the last item whose tile0 <= tile: one without tiles shares its tile0 with the next
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) / 2;
+      if (b.it[mid].tile0 <= tile) lo = mid; else hi = mid;
+    }
+    const PrepItem& p = b.it[lo];
+    const uint32_t ctiles = (p.C + p.CT - 1) / p.CT, t = tile - p.tile0, k0 = t / ctiles * p.KT, c0 = t % ctiles * p.CT;
+    __syncthreads();
+    if (p.taps == 1 && p.KT == 128) filter_prepare_tile<1, 64, 128>(p, k0, c0, sm);
+    else if (p.taps == 9 && p.C % 32 == 0 && !(p.row & 1) && !((uintptr_t)p.krsc & 3u)) filter_prepare_tile<9, 32, 32>(p, k0, c0, sm);
+    else filter_prepare_tile<0, 0, 0>(p, k0, c0, sm);
+  }
+}
 // dst[pixel][0..Kp) = src[pixel][0..K), zero past K
 __global__ void __launch_bounds__(256) pad_channels_kernel(size_t pixels, uint32_t K, uint32_t Kp,
                                                            const __nv_bfloat16* __restrict__ src, __nv_bfloat16* dst) {
@@ -933,7 +1001,9 @@ int conv_tc_fprop(const ad_conv2d_args* a, cudaStream_t s) {
                       a->relu, 0, status, s);
 }
 
-int conv_tc_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
+// wt: the filter as C,R,S,K with mirrored taps (NULL: made in scratch); status: where waits that run out report (NULL: the
+// first word of scratch)
+int conv_tc_dgrad(const ad_conv2d_args* a, const void* prepared, int32_t* status, cudaStream_t s) {
   Geo g;
   int st = conv_geo(a, g);
   if (st != AD_OK) return st;
@@ -941,13 +1011,16 @@ int conv_tc_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
   if (a->y_pitch || a->y_plane) return AD_ERR_UNSUPPORTED;  // dy must be dense for the TMA view
   if (a->scratch_bytes < conv_tc_scratch_bytes(a, 1)) return AD_ERR_SCRATCH;
   const uint32_t Kp = dgrad_kp(a->K);
-  int32_t* status = (int32_t*)a->scratch;
-  __nv_bfloat16* wt = (__nv_bfloat16*)((char*)a->scratch + 16);
+  if (!status) status = (int32_t*)a->scratch;
+  const void* wt = prepared;
   char* next = (char*)a->scratch + round_1k((size_t)Kp * a->kh * a->kw * a->C * 2 + 16);
   const size_t wcount = (size_t)Kp * a->kh * a->kw * a->C;
-  filter_transpose_flip_kernel<<<grid_for(wcount, 256), 256, 0, s>>>(a->K, Kp, a->kh, a->kw, a->C,
-                                                                     (const __nv_bfloat16*)a->w, wt);
-  count_launch();
+  if (!wt) {
+    __nv_bfloat16* made = (__nv_bfloat16*)((char*)a->scratch + 16);
+    filter_transpose_flip_kernel<<<grid_for(wcount, 256), 256, 0, s>>>(a->K, Kp, a->kh, a->kw, a->C, (const __nv_bfloat16*)a->w, made);
+    count_launch();
+    wt = made;
+  }
   const void* dy = a->y;
   if (Kp != a->K) {
     const size_t pixels = (size_t)a->N * g.P * g.Q;
@@ -983,7 +1056,7 @@ int conv_tc_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
                       nullptr, 0, a->accumulate, status, s);
 }
 
-int conv_tc_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
+int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
   Geo g;
   int st = conv_geo(a, g);
   if (st != AD_OK) return st;
@@ -991,6 +1064,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
   if (a->y_pitch || a->y_plane) return AD_ERR_UNSUPPORTED;
   if (a->C % 64 != 0) return AD_ERR_UNSUPPORTED;
   if (a->scratch_bytes < conv_tc_scratch_bytes(a, 2)) return AD_ERR_SCRATCH;
+  if (!status) status = (int32_t*)a->scratch;
   const uint32_t Kp = wgrad_kp(a->K);
   const void* dy = a->y;
   char* part_base = (char*)a->scratch + 1024;
@@ -1007,7 +1081,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
     // 64-channel layers: one CTA serves all taps from one fetch of x and dy (conv_tc_row.cu)
     st = conv_tc_row_wgrad(a->x, a->N, a->H, a->W, a->C, a->y, a->K, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h,
                            a->dil_w, -(int)a->pad_h, -(int)a->pad_w, g.P, g.Q, (float*)a->dw, a->accumulate, a->dw_kcrs,
-                           part_base, part_bytes, (int32_t*)a->scratch, s);
+                           part_base, part_bytes, status, s);
     if (st == AD_OK && a->db) launch_bias_grad((size_t)a->N * g.P * g.Q, a->K, a->y, a->db, a->accumulate, (float*)part_base, s);
     if (st != AD_ERR_UNSUPPORTED) {
       g_last_conv_kernel = kConvTcRow;
@@ -1029,7 +1103,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
   p.ctiles = (a->C + BN - 1) / BN;
   const uint32_t sp_tiles = p.tiles_b * p.tiles_y * p.tiles_x;
   p.splits = wgrad_splits(sp_tiles, p.kh * p.kw * p.ktiles * p.ctiles);
-  p.status = (int32_t*)a->scratch;
+  p.status = status;
   p.partial = (float*)part_base;
   const size_t wcount_p = (size_t)Kp * a->kh * a->kw * a->C;
   if (part_bytes < (size_t)p.splits * wcount_p * 4) return AD_ERR_SCRATCH;
@@ -1149,21 +1223,66 @@ extern "C" int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream) {
     }
   });
 }
-extern "C" int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream) {
+extern "C" int ad_conv2d_dgrad_ex(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream) {
   return profiled(1, a, stream, [&] {
     switch (path_of(a)) {
       case 0: g_last_conv_kernel = kConvDirectF32; return conv_direct_dgrad(a, as_stream(stream));
-      case 1: return tc::conv_tc_dgrad(a, as_stream(stream));
+      case 1: return tc::conv_tc_dgrad(a, w_crsk, status, as_stream(stream));
       default: return (int)(a ? AD_ERR_UNSUPPORTED : AD_ERR_BAD_ARG);
     }
   });
 }
-extern "C" int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream) {
+extern "C" int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream) { return ad_conv2d_dgrad_ex(a, nullptr, nullptr, stream); }
+extern "C" int ad_conv2d_wgrad_ex(const ad_conv2d_args* a, int32_t* status, void* stream) {
   return profiled(2, a, stream, [&] {
     switch (path_of(a)) {
       case 0: g_last_conv_kernel = kConvDirectF32; return conv_direct_wgrad(a, as_stream(stream));
-      case 1: return tc::conv_tc_wgrad(a, as_stream(stream));
+      case 1: return tc::conv_tc_wgrad(a, status, as_stream(stream));
       default: return (int)(a ? AD_ERR_UNSUPPORTED : AD_ERR_BAD_ARG);
     }
   });
+}
+extern "C" int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream) { return ad_conv2d_wgrad_ex(a, nullptr, stream); }
+
+extern "C" int ad_filter_prepare(uint32_t count, const ad_filter_item* items, void* stream) {
+  if (count && !items) return AD_ERR_BAD_ARG;
+  for (uint32_t i = 0; i < count; ++i) {
+    const ad_filter_item& f = items[i];
+    if (!f.src || !f.krsc || !f.K || !f.C || !f.kh || !f.kw || (f.crsk && (f.crsk_k < f.K || (f.crsk_k & 1) || ((uintptr_t)f.crsk & 3u)))) return AD_ERR_BAD_ARG;
+    if (f.krsc_row < (int64_t)f.kh * f.kw * f.C || (f.crsk && f.krsc_row != (int64_t)f.kh * f.kw * f.C)) return AD_ERR_UNSUPPORTED;
+  }
+  const cudaStream_t s = as_stream(stream);
+  for (uint32_t i0 = 0; i0 < count; i0 += tc::kPrepItems) {
+    tc::PrepBatch b{};
+    b.count = std::min(count - i0, tc::kPrepItems);
+    for (uint32_t i = 0; i < b.count; ++i) {
+      const ad_filter_item& f = items[i0 + i];
+      tc::PrepItem& p = b.it[i];
+      if ((uint64_t)f.kh * f.kw * 32 > tc::kPrepFloats) {   // more taps than the tile holds (over 288): element by element
+        const int64_t taps = (int64_t)f.kh * f.kw;
+        ad_tensor4 src = {(void*)f.src, AD_F32, f.K, f.C, f.kh, f.kw, f.C * taps, taps, f.kw, 1};
+        ad_tensor4 dst = {f.krsc, AD_BF16, f.K, f.C, f.kh, f.kw, f.krsc_row, 1, (int64_t)f.kw * f.C, f.C};
+        if (int rc = ad_convert(&src, &dst, 0, stream)) return rc;
+        if (f.crsk) {
+          tc::filter_transpose_flip_kernel<<<grid_for((size_t)f.C * taps * f.crsk_k, 256), 256, 0, s>>>(
+              f.K, f.crsk_k, f.kh, f.kw, f.C, (const __nv_bfloat16*)f.krsc, (__nv_bfloat16*)f.crsk);
+          count_launch();
+        }
+        p.tile0 = b.tiles;
+        p.K = p.C = p.taps = p.Kp = p.KT = p.CT = 1;
+        continue;
+      }
+      p.src = f.src; p.krsc = (__nv_bfloat16*)f.krsc; p.crsk = (__nv_bfloat16*)f.crsk;
+      p.K = f.K; p.C = f.C; p.taps = f.kh * f.kw; p.Kp = f.crsk ? f.crsk_k : f.K; p.row = f.krsc_row;
+      const bool pairs = !(p.row & 1) && !((uintptr_t)f.krsc & 3u);
+      p.KT = p.taps == 1 && p.C % 64 == 0 && pairs ? 128 : 32;
+      p.CT = p.KT == 128 ? 64 : std::min(32u, tc::kPrepFloats / (32 * p.taps));
+      p.tile0 = b.tiles;
+      b.tiles += (p.Kp + p.KT - 1) / p.KT * ((p.C + p.CT - 1) / p.CT);
+    }
+    if (!b.tiles) continue;
+    tc::filter_prepare_kernel<<<std::min(b.tiles, (uint32_t)kNumSMs * 6), 256, 0, s>>>(b);
+    count_launch();
+  }
+  return launch_status();
 }

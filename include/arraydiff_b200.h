@@ -451,6 +451,24 @@ int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream);
 int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream);
 int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream);
 /*
+ * The gradients with more said by the caller.  w_crsk (tensor-core path): the filter as bf16 C,R,S,K with mirrored taps and
+ * rows of K rounded up to 64 entries, as ad_filter_prepare writes it (NULL: made from a->w on each call, in scratch).
+ * status: the device word that waits which run out report into (NULL: the first word of scratch, which the caller then
+ * keeps zero).
+ */
+int ad_conv2d_dgrad_ex(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream);
+int ad_conv2d_wgrad_ex(const ad_conv2d_args* a, int32_t* status, void* stream);
+/* The tensor-core forms of fp32 KCRS filters, any number in one call: krsc [K] rows of krsc_row elements (kh, kw, C), and
+ * crsk (may be NULL; 4-byte aligned, crsk_k even) [C][kh][kw][crsk_k], taps mirrored, zero past K. */
+typedef struct {
+  const float* src;
+  void* krsc;
+  void* crsk;
+  int64_t krsc_row;
+  uint32_t K, C, kh, kw, crsk_k, reserved;
+} ad_filter_item;
+int ad_filter_prepare(uint32_t count, const ad_filter_item* items /* host */, void* stream);
+/*
  * Which kernel family the calling thread's most recent ad_conv2d_fprop / dgrad / wgrad call launched:
  * 0 none yet, 1 fp32 direct, 2 general tensor-core tiles, 3 row-streaming tensor-core kernels (64-channel
  * layers).  The reference picks its cuDNN algorithm per batch size behind the caller's back

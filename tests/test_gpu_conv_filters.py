@@ -1,0 +1,60 @@
+"""Filter preparation and the KCRS filter-gradient reduction against plain PyTorch forms of the same data."""
+import ctypes as C
+
+import pytest
+
+from arraydiff_cuda_b200 import abi
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shapes", [
+    [(64, 64, 1, 1)], [(19, 64, 1, 1)], [(130, 192, 1, 1)], [(8, 2, 1, 1)],          # 1x1: whole and ragged filter tiles
+    [(64, 64, 3, 3)], [(33, 96, 3, 3)], [(7, 5, 3, 3)],                               # 3x3: constant and variable extents
+    [(64, 3, 7, 7)], [(5, 9, 2, 5)], [(3, 4, 17, 17)],                                # others; more taps than the tile holds
+    [(32 + i, 64, 3, 3) if i % 3 else (3, 2, 17, 18) for i in range(33)],             # more filters than one launch takes
+])
+@pytest.mark.parametrize("pad_row", [0, 45])
+def test_filter_prepare(shapes, pad_row):
+    import torch
+    items, outs = (abi.FilterItem * len(shapes))(), []
+    for n, (K, Cc, kh, kw) in enumerate(shapes):
+        w = torch.randn(K, Cc, kh, kw, device="cuda")
+        row, Kp = kh * kw * Cc + pad_row, (K + 63) // 64 * 64
+        krsc = torch.full((K, row), 3.0, dtype=torch.bfloat16, device="cuda")
+        crsk = None if pad_row else torch.full((Cc, kh, kw, Kp), 3.0, dtype=torch.bfloat16, device="cuda")
+        items[n] = abi.FilterItem(w.data_ptr(), krsc.data_ptr(), crsk.data_ptr() if crsk is not None else None, row, K, Cc, kh, kw, Kp, 0)
+        outs.append((w, krsc, crsk))
+    abi.check(abi.lib().ad_filter_prepare(len(shapes), items, H.stream()))
+    H.sync()
+    for (K, Cc, kh, kw), (w, krsc, crsk) in zip(shapes, outs):
+        n = kh * kw * Cc
+        assert torch.equal(krsc[:, :n], w.permute(0, 2, 3, 1).reshape(K, n).bfloat16()) and torch.all(krsc[:, n:] == 3.0)
+        if crsk is not None:
+            assert torch.equal(crsk[..., :K], w.flip(2, 3).permute(1, 2, 3, 0).bfloat16()) and torch.all(crsk[..., K:] == 0)
+
+
+@pytest.mark.parametrize("K,Cc,k", [(64, 64, 2), (40, 128, 3), (19, 64, 9), (8, 64, 10)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_filter_gradient_order(K, Cc, k, accumulate):
+    """The KCRS form is the KRSC form, turned round, to the bit."""
+    import torch
+    N, Hh = 2, 24
+    L = abi.lib()
+    a = abi.Conv2dArgs()
+    a.dtype, a.layout = abi.AD_BF16, abi.AD_NHWC
+    a.N, a.C, a.H, a.W, a.K, a.kh, a.kw = N, Cc, Hh, Hh, K, k, k
+    a.stride_h = a.stride_w = a.dil_h = a.dil_w = 1
+    P = Hh - k + 1
+    x, dy = (torch.randn(N, n, n, c, device="cuda").bfloat16() for n, c in ((Hh, Cc), (P, K)))
+    sb = L.ad_conv2d_scratch_bytes(C.byref(a), 2)
+    scratch, status = torch.zeros(sb, dtype=torch.uint8, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    a.x, a.y, a.scratch, a.scratch_bytes, a.accumulate = x.data_ptr(), dy.data_ptr(), scratch.data_ptr(), sb, accumulate
+    old = torch.randn(K, k, k, Cc, device="cuda")
+    krsc, kcrs = old.clone(), old.permute(0, 3, 1, 2).contiguous()
+    for out, order in ((krsc, 0), (kcrs, 1)):
+        a.dw, a.dw_kcrs = out.data_ptr(), order
+        abi.check(L.ad_conv2d_wgrad_ex(C.byref(a), H.ptr(status), H.stream()))
+    H.sync()
+    assert int(status[0]) == 0 and torch.equal(kcrs, krsc.permute(0, 3, 1, 2)) and not torch.equal(krsc, old)
