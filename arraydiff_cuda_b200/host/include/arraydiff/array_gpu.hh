@@ -34,6 +34,8 @@ public:
     AD_CHECK(ad_fill_zero(dptr_, size * sizeof(T), conn.stream()));
   }
   static GPUMemory<T> Zeros(size_t size, GPUContext* ctx) { return GPUMemory<T>(size, ctx); }
+  // a view of memory that something else owns
+  static GPUMemory<T> Wrap(T* p, size_t size) { GPUMemory<T> m; m.dptr_ = p; m.size_ = size; return m; }
   T* dptr() const { return dptr_; }
   size_t size() const { return size_; }
   void set_constant(float c, GPUConn& conn);  // float only
@@ -70,6 +72,8 @@ public:
   size_t flat_size() const { return dim_.flat_size() ? dim_.flat_size() : 1; }
   T* dptr() const { return mem_.dptr(); }
   GPUMemory<T>& mem() { return mem_; }
+  // Moves the array into memory that holds its values already (its place in a flat parameter buffer)
+  void rebind(T* p) { mem_ = GPUMemory<T>::Wrap(p, flat_size()); }
 private:
   ShapeT dim_;
   GPUMemory<T> mem_;

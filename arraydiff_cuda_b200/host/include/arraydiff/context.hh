@@ -107,6 +107,14 @@ public:
   void join_side();
   static void JoinAllSides();
   void reserve_side_scratch(size_t min_size);
+  // Tensor-core layers register how to describe their filter (fp32 variable -> bf16 forms); the first of them that runs in a
+  // transaction has all of them made, in one launch per 32 filters.  A describer returns false when its variable has no
+  // value in the transaction (another net on this context); one that gets its value, or a new one, later in the
+  // transaction has another version and is made when its layer asks.
+  typedef std::function<bool(uint64_t txn, ad_filter_item*, uint64_t* version)> FilterItemFn;
+  size_t add_filter(FilterItemFn f);
+  void remove_filter(size_t id);
+  void prepare_filters(size_t id, uint64_t txn, cudaStream_t s);
   void* side_scratch() { return side_scratch_; }
   size_t side_scratch_size() const { return side_scratch_size_; }
 private:
@@ -123,6 +131,8 @@ private:
   size_t scratch_size_;
   int32_t* status_;
   std::function<void(cudaStream_t)> pending_;
+  struct Filter { FilterItemFn describe; uint64_t txn = ~0ull, version = 0; };
+  std::vector<Filter> filters_;
 };
 
 class MultiGPUContext : public virtual Context {

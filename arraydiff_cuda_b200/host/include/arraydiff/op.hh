@@ -81,11 +81,14 @@ private:
 template <typename V>
 struct TxnVarBuf {
   std::optional<uint64_t> curr_txn;
+  uint64_t version = 0;   // counts begin()s
   bool rollover = false;
   std::unordered_set<uint64_t> writers;
   std::optional<V> buffer;
   function<V()> alloc;
   VarId id;
+  V* deferred = nullptr;
+  uint64_t deferred_txn = 0;
 };
 
 template <typename V>
@@ -99,7 +102,7 @@ public:
   bool overwrite(TxnId txn, NodeId node) {
     ensure();
     if (!buf_->curr_txn || *buf_->curr_txn != txn.raw_id()) {
-      buf_->curr_txn = txn.raw_id(); buf_->rollover = false; buf_->writers.clear();
+      begin(txn, false);
       buf_->writers.insert(node.raw_id());
       return true;
     }
@@ -111,7 +114,7 @@ public:
   bool accumulate(TxnId txn, NodeId node, function<void(V*)> init) {
     ensure();
     if (!buf_->curr_txn || *buf_->curr_txn != txn.raw_id()) {
-      buf_->curr_txn = txn.raw_id(); buf_->rollover = false; buf_->writers.clear();
+      begin(txn, false);
       if (init) init(&*buf_->buffer);
     }
     return buf_->writers.insert(node.raw_id()).second;
@@ -122,7 +125,7 @@ public:
   int accumulate_full(TxnId txn, NodeId node, function<bool(V&)> covers, function<void(V*)> init) {
     ensure();
     if (!buf_->curr_txn || *buf_->curr_txn != txn.raw_id()) {
-      buf_->curr_txn = txn.raw_id(); buf_->rollover = false; buf_->writers.clear();
+      begin(txn, false);
       buf_->writers.insert(node.raw_id());
       if (covers && covers(*buf_->buffer)) return 2;
       if (init) init(&*buf_->buffer);
@@ -134,14 +137,25 @@ public:
   V& get_excl(TxnId txn, NodeId n) { return get(txn, n); }
   V& get_mut(TxnId txn, NodeId n) { return get(txn, n); }
   V& raw() { ensure(); return *buf_->buffer; }   // no transaction check (optimizer / tests)
-  bool written_in(TxnId txn) const { return buf_->curr_txn && *buf_->curr_txn == txn.raw_id(); }
+  // A gradient that is to be added by the one contributor that knows how (kJoinDefer): set by the join in its backward
+  // pass, taken by that contributor in the same transaction.
+  void defer(TxnId txn, V* addend) { buf_->deferred = addend; buf_->deferred_txn = txn.raw_id(); }
+  V* take_deferred(TxnId txn) {
+    V* a = buf_->deferred_txn == txn.raw_id() ? buf_->deferred : nullptr;
+    buf_->deferred = nullptr;
+    return a;
+  }
+  bool written_in(TxnId txn) const { return written_in(txn.raw_id()); }
+  bool written_in(uint64_t txn) const { return buf_->curr_txn && *buf_->curr_txn == txn; }
   void rollover(TxnId txn, VarIdSet& vars) {
     if (!vars.contains(buf_->id)) return;
     ensure();
-    buf_->curr_txn = txn.raw_id(); buf_->rollover = true; buf_->writers.clear();
+    begin(txn, true);
   }
-  void stamp(TxnId txn) { ensure(); buf_->curr_txn = txn.raw_id(); buf_->rollover = true; buf_->writers.clear(); }
+  void stamp(TxnId txn) { ensure(); begin(txn, true); }
+  uint64_t version() const { return buf_->version; }
 private:
+  void begin(TxnId txn, bool rollover) { buf_->curr_txn = txn.raw_id(); buf_->rollover = rollover; buf_->writers.clear(); ++buf_->version; }
   void ensure() { if (!buf_->buffer) buf_->buffer = buf_->alloc(); }
   shared_ptr<TxnVarBuf<V>> buf_;
 };
@@ -290,6 +304,11 @@ private:
   VarData<A> data_;
 };
 template <typename A> using SrcOp = IOOp<A>;
+// A reader that moves no data: every parameter-like variable of the walk becomes a view of its place in a flat device
+// buffer (which holds the values already, or will be written through the variables).  Loads from and stores to that
+// buffer then find source and destination to be one and the same and copy nothing: an optimizer that keeps its
+// parameters and gradients flat needs no gather and scatter of hundreds of small arrays per step.
+struct BindFlat { float* base; };
 // A reader for activations that lets every rank take only its rows of a full host image (packed NCHW fp32).
 struct HostRows { const float* base; size_t full_h, row0; };
 
@@ -302,6 +321,8 @@ public:
   VarData<Act> data() override { return y_; }
   size_t rank() const override { return rank_; }
   void _persist(TxnId, VarIdSet&) override {}
+  // The only consumer's gradient is this operator's gradient (kJoinShare): one variable, one buffer
+  void share_grad(const TxnVar<Act>& grad) { y_.grad = grad; }
   // Any activation can be read back, and its gradient set or read, as packed NCHW fp32 of the
   // interior: that is how a caller supplies an upstream gradient or inspects a result.
   size_t _load_grad(TxnId txn, VarIdSet& vars, size_t offset, any* reader) override;
@@ -419,22 +440,23 @@ public:
                  shared_ptr<Context> ctx);
   void _forward(TxnId txn) override;
   void _backward(TxnId txn) override;
+  ~CudnnConv2DOpF() override;
   string _debug_op_label() override { return "CudnnConv2DOp"; }
 private:
   void fill_args(ad_conv2d_args& a, Act& x);
-  void refresh_filter(TxnId txn, cudaStream_t s);
   Conv2DShape shape_;
   ActVar x_;
   shared_ptr<Var<Kernel>> kernel_;
   shared_ptr<Var<Bias>> bias_;
   Shape3D in_dim_;
-  // tensor-core path: bf16 KRSC copy of the filter, fp32 KRSC gradient staging, im2col matrix (stem)
-  void* w_bf16_ = nullptr;
+  // tensor-core path: bf16 KRSC copy of the filter and the C,R,S,K form of the data gradient (made for all layers at once:
+  // GPUContext::prepare_filters), fp32 KRSC gradient staging, im2col matrix (stem)
+  void *w_bf16_ = nullptr, *w_crsk_ = nullptr;
+  size_t filter_id_ = (size_t)-1;
   float* dw_krsc_ = nullptr;
   void* im2col_ = nullptr;
   size_t ck_ = 0;       // channels the tensor-core kernel reduces over per tap (padded)
   bool use_im2col_ = false;
-  std::optional<uint64_t> filter_txn_;
 };
 
 class CudnnPool2DOpF : public ActOp {
@@ -460,8 +482,10 @@ public:
     shared_ptr<CudnnBatchNorm2DOpF> op;
     shared_ptr<IOOp<Stat>> scale, shift, batch_mean, batch_variance, fixed_mean, fixed_variance;
   };
-  static Parts Make(size_t channels, shared_ptr<bool> switch_var, ActVar x, shared_ptr<Context> ctx);
-  CudnnBatchNorm2DOpF(shared_ptr<bool> switch_var, ActVar x, Parts* parts, shared_ptr<Context> ctx);
+  // out_pad: the output is the interior of a zero halo-padded buffer, ready for HaloExch2DOp / a convolution or pool that
+  // reads halo-padded input (what a HaloPad2DOp behind it would copy it into)
+  static Parts Make(size_t channels, shared_ptr<bool> switch_var, ActVar x, shared_ptr<Context> ctx, size_t out_pad = 0);
+  CudnnBatchNorm2DOpF(shared_ptr<bool> switch_var, ActVar x, Parts* parts, shared_ptr<Context> ctx, size_t out_pad = 0);
   void _forward(TxnId txn) override;
   void _backward(TxnId txn) override;
   void fuse_relu() { relu_ = true; }
@@ -470,7 +494,7 @@ private:
   shared_ptr<bool> switch_var_;
   ActVar x_;
   shared_ptr<IOOp<Stat>> scale_, shift_, batch_mean_, batch_variance_, fixed_mean_, fixed_variance_;
-  float *save_mean_ = nullptr, *save_invstd_ = nullptr;
+  float* save_invstd_ = nullptr;   // the batch mean is kept in batch_mean_
   bool relu_ = false;
 };
 
@@ -487,14 +511,21 @@ private:
 
 class SumJoin {};
 // y = sum_i x_i ; dx_i += dy  (reference src/op.cc:630-867)
+// How an input's gradient takes dy is the builder's choice, who knows its other consumers:
+//   kJoinCopy    dx_i += dy in a buffer of its own (any graph);
+//   kJoinShare   the join is the input's only consumer: the input's gradient IS dy, no copy;
+//   kJoinDefer   the input's other consumer is a batch norm whose backward pass runs after this one (it feeds a branch of
+//                this join): that pass adds dy to what it writes, no copy.
+enum JoinGrad { kJoinCopy, kJoinShare, kJoinDefer };
 class SumJoinOpF : public ActOp {
 public:
-  static ActVar Make(vector<ActVar> xs, shared_ptr<Context> ctx);
-  SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx);
+  static ActVar Make(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGrad> grads = {});
+  SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGrad> grads);
   void _forward(TxnId txn) override;
   void _backward(TxnId txn) override;
 private:
   vector<ActVar> xs_;
+  vector<JoinGrad> grads_;
 };
 
 // Re-assembly of the strips on every rank: y_r = concat_q x_q along H.  The reference builds it from

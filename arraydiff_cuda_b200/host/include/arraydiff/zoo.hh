@@ -30,9 +30,11 @@ template <typename V> ParallelParamOp<V> parallel_conv2d(Conv2DShape shape, vect
 template <typename V> ParamOp<V> linear(size_t filters, shared_ptr<Var<V>> input, KernelInitFn kernel_init, shared_ptr<Context> ctx);
 template <typename V> ParallelParamOp<V> parallel_linear(size_t filters, vector<shared_ptr<Var<V>>> inputs, KernelInitFn kernel_init, shared_ptr<Context> ctx);
 template <typename V> vector<shared_ptr<Var<V>>> parallel_relu(vector<shared_ptr<Var<V>>> inputs, shared_ptr<Context> ctx);
-template <typename V> vector<shared_ptr<Var<V>>> parallel_sum(vector<vector<shared_ptr<Var<V>>>> inputs, shared_ptr<Context> ctx);
+// grads: how each branch's gradient takes the sum's (JoinGrad; empty: copies)
+template <typename V> vector<shared_ptr<Var<V>>> parallel_sum(vector<vector<shared_ptr<Var<V>>>> inputs, shared_ptr<Context> ctx, vector<JoinGrad> grads = {});
 // batch norm per rank, optionally with the following ReLU folded in
-template <typename V> ParallelBatchNormParamOp<V> parallel_batch_norm(size_t channels, shared_ptr<bool> switch_var, vector<shared_ptr<Var<V>>> inputs, bool fuse_relu, shared_ptr<Context> ctx);
+// and the output written into a halo-padded buffer (CudnnBatchNorm2DOp::Make)
+template <typename V> ParallelBatchNormParamOp<V> parallel_batch_norm(size_t channels, shared_ptr<bool> switch_var, vector<shared_ptr<Var<V>>> inputs, bool fuse_relu, shared_ptr<Context> ctx, size_t out_pad = 0);
 
 template <typename V> ParallelBatchNormParamOp<V> spatial_parallel_residual_v2_conv2d(Conv2DShape shape, shared_ptr<bool> switch_var, vector<shared_ptr<Var<V>>> inputs, shared_ptr<Context> ctx);
 template <typename V> ParallelBatchNormParamOp<V> spatial_parallel_proj_residual_v2_conv2d(Conv2DShape shape, size_t stride, shared_ptr<bool> switch_var, vector<shared_ptr<Var<V>>> inputs, shared_ptr<Context> ctx);

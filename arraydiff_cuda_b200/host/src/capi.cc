@@ -132,7 +132,11 @@ void* adh_net_create(void* c, const char* kind, int H, int W, int C, int batch, 
   n->opt->reset(n->ctx, &n->rng);
   return n;
 }
-void adh_net_destroy(void* h) { delete (Net*)h; }
+void adh_net_destroy(void* h) {
+  auto* n = (Net*)h;
+  if (n->gexec) cudaGraphExecDestroy(n->gexec);
+  delete n;
+}
 // flat-parameter checkpoint of the net's optimizer state (parameters, momentum, running statistics, iteration)
 int adh_net_save_checkpoint(void* h, const char* path) { return ((Net*)h)->opt->save_checkpoint(path) ? AD_OK : AD_ERR_BAD_ARG; }
 int adh_net_load_checkpoint(void* h, const char* path) {
@@ -153,6 +157,7 @@ int adh_net_configure_sgd(void* h, double step_size, double momentum, double l2,
   vector<float> keep(n->opt->param_dim());
   size_t first = n->ctx->distributed() ? n->ctx->my_rank() : 0;
   n->opt->store_params(first, keep.data());
+  if (n->gexec) { cudaGraphExecDestroy(n->gexec); n->gexec = nullptr; }   // a recorded step works on the old optimizer's buffers
   n->opt.reset(new ParallelSGDOptimizer<float>(sc, n->net.sink, n->net.dev_params, n->net.dev_grads));
   std::mt19937_64 rng(1);
   n->opt->reset(n->ctx, &rng);

@@ -104,6 +104,27 @@ void GPUContext::reserve_side_scratch(size_t min_size) {
   side_scratch_ = arena_.alloc(want);
   side_scratch_size_ = want;
 }
+size_t GPUContext::add_filter(FilterItemFn f) {
+  for (size_t i = 0; i < filters_.size(); ++i)
+    if (!filters_[i].describe) { filters_[i] = Filter{f}; return i; }
+  filters_.push_back(Filter{f});
+  return filters_.size() - 1;
+}
+void GPUContext::remove_filter(size_t id) { filters_.at(id) = Filter(); }
+void GPUContext::prepare_filters(size_t id, uint64_t txn, cudaStream_t s) {
+  std::vector<ad_filter_item> items;
+  auto visit = [&](Filter& f) {
+    ad_filter_item it = {};
+    uint64_t v = 0;
+    if (!f.describe || !f.describe(txn, &it, &v) || (f.txn == txn && f.version == v)) return false;
+    f.txn = txn; f.version = v;
+    items.push_back(it);
+    return true;
+  };
+  if (!visit(filters_.at(id))) return;
+  for (auto& f : filters_) visit(f);
+  AD_CHECK(ad_filter_prepare((uint32_t)items.size(), items.data(), s));
+}
 void GPUContext::sync() { join_side(); GPUConn c = conn(); c.sync(); }
 GPUConn GPUContext::conn() {
   GPUConn c(device_, stream_);

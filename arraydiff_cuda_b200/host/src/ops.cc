@@ -168,12 +168,16 @@ static void io_move(A& a, any* flat, size_t offset, bool to_device, GPUContext* 
       else CUDA_CHECK(cudaMemcpyAsync(host, d, n * 4, cudaMemcpyDeviceToHost, conn.stream()));
       conn.sync();
     }
+  } else if (auto bind = std::any_cast<BindFlat>(flat)) {
+    if constexpr (std::is_same<A, Act>::value) assert(0 && "activations do not live in a flat buffer");
+    else a.rebind(bind->base + offset);
   } else if (auto dp = std::any_cast<GPUMemory<float>>(flat)) {
     if constexpr (std::is_same<A, Act>::value) {
       assert(0 && "activations move through host buffers");
     } else {
       float* d = IOTraits<A>::dptr(a);
       float* f = dp->dptr() + offset;
+      if (d == f) return;   // the variable lives in this buffer (BindFlat)
       if (to_device) CUDA_CHECK(cudaMemcpyAsync(d, f, n * 4, cudaMemcpyDeviceToDevice, conn.stream()));
       else CUDA_CHECK(cudaMemcpyAsync(f, d, n * 4, cudaMemcpyDeviceToDevice, conn.stream()));
     }
@@ -447,9 +451,18 @@ CudnnConv2DOpF::CudnnConv2DOpF(Conv2DShape shape, ActVar x, shared_ptr<Var<Kerne
     GPUContext* g = gpu();
     GPUConn conn = g->conn();
     w_bf16_ = g->arena().alloc(wcount * 2);
-    dw_krsc_ = (float*)g->arena().alloc(wcount * 4);
     AD_CHECK(ad_fill_zero(w_bf16_, wcount * 2, conn.stream()));
+    const uint32_t K = (uint32_t)shape.filters, kh = (uint32_t)shape.kernel[1], kw = (uint32_t)shape.kernel[0], Kp = (K + 63) / 64 * 64;
+    if (!use_im2col_) w_crsk_ = g->arena().alloc((size_t)Kp * taps * C * 2);   // a patch-matrix layer has no data gradient
+    filter_id_ = g->add_filter([this, K, C, kh, kw, Kp](uint64_t txn, ad_filter_item* it, uint64_t* version) {
+      auto w = kernel_->data().val;
+      if (!w.written_in(txn)) return false;
+      *version = w.version();
+      *it = {w.raw().dptr(), w_bf16_, w_crsk_, (int64_t)(use_im2col_ ? ck_ : kh * kw * C), K, (uint32_t)C, kh, kw, Kp, 0};
+      return true;
+    });
     if (use_im2col_) {
+      dw_krsc_ = (float*)g->arena().alloc(wcount * 4);
       const size_t pix = dim_.shape[0] * dim_.shape[1] * batch_;
       im2col_ = g->arena().alloc(pix * ck_ * 2);
       AD_CHECK(ad_fill_zero(im2col_, pix * ck_ * 2, conn.stream()));
@@ -482,14 +495,8 @@ void CudnnConv2DOpF::fill_args(ad_conv2d_args& a, Act& x) {
   }
 }
 
-// bf16 KRSC copy of the fp32 KCRS master filter (columns padded to ck_ for the patch-matrix layer)
-void CudnnConv2DOpF::refresh_filter(TxnId txn, cudaStream_t s) {
-  Kernel& w = kernel_->data().val.get(txn, id());
-  const long long K = (long long)shape_.filters, C = (long long)in_dim_.shape[2], kh = (long long)shape_.kernel[1], kw = (long long)shape_.kernel[0];
-  ad_tensor4 src = {w.dptr(), AD_F32, (uint32_t)K, (uint32_t)C, (uint32_t)kh, (uint32_t)kw, C * kh * kw, kh * kw, kw, 1};
-  const long long row = use_im2col_ ? (long long)ck_ : kh * kw * C;
-  ad_tensor4 dst = {w_bf16_, AD_BF16, (uint32_t)K, (uint32_t)C, (uint32_t)kh, (uint32_t)kw, row, 1, kw * C, C};
-  AD_CHECK(ad_convert(&src, &dst, 0, s));
+CudnnConv2DOpF::~CudnnConv2DOpF() {
+  if (filter_id_ != (size_t)-1) gpu()->remove_filter(filter_id_);
 }
 
 void CudnnConv2DOpF::_forward(TxnId txn) {
@@ -522,7 +529,7 @@ void CudnnConv2DOpF::_forward(TxnId txn) {
     AD_CHECK(ad_conv2d_fprop(&a, conn.stream()));
     return;
   }
-  refresh_filter(txn, conn.stream());
+  g->prepare_filters(filter_id_, txn.raw_id(), conn.stream());
   a.w = w_bf16_;
   if (use_im2col_) {
     ad_tensor4 xv = shape_.halo_padded_input ? x.view_base() : x.view_interior();
@@ -557,18 +564,27 @@ void CudnnConv2DOpF::_backward(TxnId txn) {
   fill_args(a, x);
   a.y = dy.base_dptr();
   const bool f32 = x.storage() == COMPUTE_F32_NCHW;
+  bool bias_adds = false;
   auto kd = kernel_->data();
   // filter (and bias) gradient: += after a once-per-transaction zero fill (reference src/op.cc:1651-1683)
-  if (kd.grad.accumulate(txn, id(), [g](Kernel* k) { GPUConn c = g->conn(); AD_CHECK(ad_fill_zero(k->dptr(), k->flat_size() * 4, c.stream())); })) {
+  // (the first contributor overwrites instead: this operator, in every net the builders make)
+  auto zero_k = [g](Kernel* k) { GPUConn c = g->conn(); AD_CHECK(ad_fill_zero(k->dptr(), k->flat_size() * 4, c.stream())); };
+  auto zero_b = [g](Bias* b) { GPUConn c = g->conn(); AD_CHECK(ad_fill_zero(b->dptr(), b->flat_size() * 4, c.stream())); };
+  if (const int wmode = kd.grad.accumulate_full(txn, id(), [](Kernel&) { return true; }, zero_k)) {
     Kernel& dw = kd.grad.get_mut(txn, id());
+    const int add = wmode == 1 ? 1 : 0;
     float* db = nullptr;
     if (bias_) {
       auto bd = bias_->data();
-      bd.grad.accumulate(txn, id(), [g](Bias* b) { GPUConn c = g->conn(); AD_CHECK(ad_fill_zero(b->dptr(), b->flat_size() * 4, c.stream())); });
+      // one flag serves filter and bias: when the filter adds, so does the bias, into zeros if it is the first
+      const int bmode = bd.grad.accumulate_full(txn, id(), [add](Bias&) { return !add; }, zero_b);
       db = bd.grad.get_mut(txn, id()).dptr();
+      if (!add && bmode == 1) { GPUConn c = g->conn(); AD_CHECK(ad_fill_zero(dw.dptr(), dw.flat_size() * 4, c.stream())); }
+      bias_adds = bmode == 1;
     }
+    const int acc = add || bias_adds;
     if (f32) {
-      a.dw = dw.dptr(); a.db = db; a.accumulate = 1;
+      a.dw = dw.dptr(); a.db = db; a.accumulate = acc;
       if (const size_t need = ad_conv2d_scratch_bytes(&a, 2)) {
         g->reserve_scratch(need);
         a.scratch = g->get_scratch(); a.scratch_bytes = g->scratch_size();
@@ -596,23 +612,21 @@ void CudnnConv2DOpF::_backward(TxnId txn) {
           g->reserve_scratch(need);
           b.scratch = g->get_scratch(); b.scratch_bytes = g->scratch_size();
         }
-        AD_CHECK(ad_fill_zero(b.scratch, 16, ws));
-        b.dw = dw.dptr(); b.db = db; b.accumulate = 1; b.dw_kcrs = 1;
-        AD_CHECK(ad_conv2d_wgrad(&b, ws));
+        b.dw = dw.dptr(); b.db = db; b.accumulate = acc; b.dw_kcrs = 1;
+        AD_CHECK(ad_conv2d_wgrad_ex(&b, g->status_word(), ws));
       } else {
       g->reserve_scratch(need);
       b.scratch = g->get_scratch(); b.scratch_bytes = g->scratch_size();
-      AD_CHECK(ad_fill_zero(b.scratch, 16, s));
-      // patch-matrix layer: the filter gradient is produced with padded rows and then added into the KCRS
+      // patch-matrix layer: the filter gradient is produced with padded rows and then moved into the KCRS
       // variable; the bias gradient is written straight into its variable (this op is the bias's only
       // consumer, so = equals +=)
       b.dw = dw_krsc_; b.db = db; b.accumulate = 0;
-      AD_CHECK(ad_conv2d_wgrad(&b, s));
+      AD_CHECK(ad_conv2d_wgrad_ex(&b, g->status_word(), s));
       const long long K = (long long)shape_.filters, C = (long long)in_dim_.shape[2], kh = (long long)shape_.kernel[1], kw = (long long)shape_.kernel[0];
       const long long row = use_im2col_ ? (long long)ck_ : kh * kw * C;
       ad_tensor4 src = {dw_krsc_, AD_F32, (uint32_t)K, (uint32_t)C, (uint32_t)kh, (uint32_t)kw, row, 1, kw * C, C};
       ad_tensor4 dst = {dw.dptr(), AD_F32, (uint32_t)K, (uint32_t)C, (uint32_t)kh, (uint32_t)kw, C * kh * kw, kh * kw, kw, 1};
-      AD_CHECK(ad_convert(&src, &dst, 1, s));
+      AD_CHECK(ad_convert(&src, &dst, acc, s));
       }
     }
   }
@@ -637,8 +651,7 @@ void CudnnConv2DOpF::_backward(TxnId txn) {
       const size_t need = ad_conv2d_scratch_bytes(&a, 1);
       g->reserve_scratch(need);
       a.scratch = g->get_scratch(); a.scratch_bytes = g->scratch_size();
-      AD_CHECK(ad_fill_zero(a.scratch, 16, s));
-      AD_CHECK(ad_conv2d_dgrad(&a, s));
+      AD_CHECK(ad_conv2d_dgrad_ex(&a, w_crsk_, g->status_word(), s));
     }
   }
 }
@@ -701,7 +714,8 @@ static IOOp<GPUArray1D<float>>::InitFn const_init(float v) {
     cudaDeviceSynchronize();
   };
 }
-CudnnBatchNorm2DOpF::Parts CudnnBatchNorm2DOpF::Make(size_t channels, shared_ptr<bool> switch_var, ActVar x, shared_ptr<Context> ctx) {
+CudnnBatchNorm2DOpF::Parts CudnnBatchNorm2DOpF::Make(size_t channels, shared_ptr<bool> switch_var, ActVar x, shared_ptr<Context> ctx,
+                                                     size_t out_pad) {
   Parts p;
   typedef IOOp<Stat> S;
   const size_t r = x->rank();
@@ -713,10 +727,10 @@ CudnnBatchNorm2DOpF::Parts CudnnBatchNorm2DOpF::Make(size_t channels, shared_ptr
   p.batch_variance = S::Make(Shape1D(channels), 1, nullptr, r, ctx);
   p.fixed_mean = S::Make(Shape1D(channels), 1, const_init(0.f), r, ctx);
   p.fixed_variance = S::Make(Shape1D(channels), 1, const_init(1.f), r, ctx);
-  p.op = make_shared<CudnnBatchNorm2DOpF>(switch_var, x, &p, ctx);
+  p.op = make_shared<CudnnBatchNorm2DOpF>(switch_var, x, &p, ctx, out_pad);
   return p;
 }
-CudnnBatchNorm2DOpF::CudnnBatchNorm2DOpF(shared_ptr<bool> switch_var, ActVar x, Parts* parts, shared_ptr<Context> ctx)
+CudnnBatchNorm2DOpF::CudnnBatchNorm2DOpF(shared_ptr<bool> switch_var, ActVar x, Parts* parts, shared_ptr<Context> ctx, size_t out_pad)
     : ActOp(x->rank(), ctx), switch_var_(switch_var), x_(x), scale_(parts->scale), shift_(parts->shift),
       batch_mean_(parts->batch_mean), batch_variance_(parts->batch_variance), fixed_mean_(parts->fixed_mean),
       fixed_variance_(parts->fixed_variance) {
@@ -728,10 +742,8 @@ CudnnBatchNorm2DOpF::CudnnBatchNorm2DOpF(shared_ptr<bool> switch_var, ActVar x, 
   inputs_.push_back(batch_variance_);
   inputs_.push_back(fixed_mean_);
   inputs_.push_back(fixed_variance_);
-  alloc_output(x->shape(), 0, 0, x->batch_shape());
-  const size_t C = x->shape().shape[2];
-  save_mean_ = (float*)gpu()->arena().alloc(C * 4);
-  save_invstd_ = (float*)gpu()->arena().alloc(C * 4);
+  alloc_output(x->shape(), out_pad, out_pad, x->batch_shape());
+  save_invstd_ = (float*)gpu()->arena().alloc(x->shape().shape[2] * 4);
 }
 void CudnnBatchNorm2DOpF::_forward(TxnId txn) {
   if (!y_.val.overwrite(txn, id())) return;
@@ -751,11 +763,10 @@ void CudnnBatchNorm2DOpF::_forward(TxnId txn) {
   }
   batch_mean_->data().val.stamp(txn);
   batch_variance_->data().val.stamp(txn);
-  AD_CHECK(ad_bn_fwd_train(&xv, &yv, scale_->data().val.get(txn, id()).dptr(), shift_->data().val.get(txn, id()).dptr(), save_mean_,
-                           save_invstd_, batch_variance_->data().val.raw().dptr(), 1.0e-5f, relu_ ? 1 : 0, g->get_scratch(),
-                           g->scratch_size(), conn.stream()));
-  // batch_mean mirrors the saved mean (what the optimizer's running-average step consumes)
-  CUDA_CHECK(cudaMemcpyAsync(batch_mean_->data().val.raw().dptr(), save_mean_, C * 4, cudaMemcpyDeviceToDevice, conn.stream()));
+  // the batch mean the optimizer's running-average step consumes is the mean the backward pass needs
+  AD_CHECK(ad_bn_fwd_train(&xv, &yv, scale_->data().val.get(txn, id()).dptr(), shift_->data().val.get(txn, id()).dptr(),
+                           batch_mean_->data().val.raw().dptr(), save_invstd_, batch_variance_->data().val.raw().dptr(), 1.0e-5f,
+                           relu_ ? 1 : 0, g->get_scratch(), g->scratch_size(), conn.stream()));
 }
 void CudnnBatchNorm2DOpF::_backward(TxnId txn) {
   assert(!(switch_var_ && *switch_var_) && "no backward pass with fixed statistics (reference src/op.cc:4078-4080)");
@@ -765,16 +776,28 @@ void CudnnBatchNorm2DOpF::_backward(TxnId txn) {
   auto sd = scale_->data(), hd = shift_->data();
   const int mode = xd.grad.accumulate_full(txn, id(), unpadded, zero_init(g));
   if (!mode) return;
-  sd.grad.accumulate(txn, id(), zero1);
-  hd.grad.accumulate(txn, id(), zero1);
+  // the first contributor to both parameter gradients overwrites them
+  auto whole = [](Stat&) { return true; };
+  const int smode = sd.grad.accumulate_full(txn, id(), whole, zero1), hmode = hd.grad.accumulate_full(txn, id(), whole, zero1);
+  const int add_params = smode == 1 || hmode == 1;
   GPUConn conn = g->conn();
+  if (add_params && smode == 2) zero1(&sd.grad.get_mut(txn, id()));
+  if (add_params && hmode == 2) zero1(&hd.grad.get_mut(txn, id()));
   const uint32_t C = (uint32_t)dim_.shape[2];
   g->reserve_scratch(ad_bn_scratch_bytes(C));
   ad_tensor4 xv = xd.val.get(txn, id()).view_interior(), dyv = y_.grad.get(txn, id()).view_interior(),
              dxv = xd.grad.get_mut(txn, id()).view_interior();
-  AD_CHECK(ad_bn_bwd(&xv, &dyv, &dxv, sd.val.get(txn, id()).dptr(), hd.val.get(txn, id()).dptr(), save_mean_, save_invstd_,
-                     sd.grad.get_mut(txn, id()).dptr(), hd.grad.get_mut(txn, id()).dptr(), relu_ ? 1 : 0, mode == 1 ? 1 : 0, g->get_scratch(),
-                     g->scratch_size(), conn.stream()));
+  // what is added to the gradient this pass writes: nothing, what its buffer holds, or the gradient a join left to it
+  const ad_tensor4* addend = mode == 1 ? &dxv : nullptr;
+  ad_tensor4 later;
+  if (Act* d = xd.grad.take_deferred(txn)) {
+    later = d->view_interior();
+    if (mode == 1) AD_CHECK(ad_convert(&later, &dxv, 1, conn.stream()));
+    else addend = &later;
+  }
+  AD_CHECK(ad_bn_bwd_add(&xv, &dyv, addend, &dxv, sd.val.get(txn, id()).dptr(), hd.val.get(txn, id()).dptr(),
+                         batch_mean_->data().val.raw().dptr(), save_invstd_, sd.grad.get_mut(txn, id()).dptr(),
+                         hd.grad.get_mut(txn, id()).dptr(), relu_ ? 1 : 0, add_params, g->get_scratch(), g->scratch_size(), conn.stream()));
 }
 
 // ------------------------------------------------------------------ ReLU, residual sum
@@ -801,11 +824,21 @@ void CudnnActivationOpF::_backward(TxnId txn) {
   AD_CHECK(ad_relu_bwd(&xv, &dyv, &dxv, mode == 1 ? 1 : 0, conn.stream()));
 }
 
-ActVar SumJoinOpF::Make(vector<ActVar> xs, shared_ptr<Context> ctx) { return make_shared<SumJoinOpF>(xs, ctx); }
-SumJoinOpF::SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx) : ActOp(xs.at(0)->rank(), ctx), xs_(xs) {
+ActVar SumJoinOpF::Make(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGrad> grads) {
+  return make_shared<SumJoinOpF>(xs, ctx, grads);
+}
+SumJoinOpF::SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGrad> grads)
+    : ActOp(xs.at(0)->rank(), ctx), xs_(xs), grads_(grads) {
   assert(xs.size() >= 2);
   for (auto& x : xs) { inputs_.push_back(x); assert(x->shape() == xs[0]->shape()); }
   alloc_output(xs[0]->shape(), 0, 0, xs[0]->batch_shape());
+  grads_.resize(xs.size(), kJoinCopy);
+  for (size_t i = 0; i < xs.size(); ++i) {
+    if (grads_[i] != kJoinShare) continue;
+    auto* op = dynamic_cast<ActOp*>(xs[i].get());
+    if (op) op->share_grad(y_.grad);
+    else grads_[i] = kJoinCopy;
+  }
 }
 void SumJoinOpF::_forward(TxnId txn) {
   if (!y_.val.overwrite(txn, id())) return;
@@ -821,8 +854,10 @@ void SumJoinOpF::_forward(TxnId txn) {
 void SumJoinOpF::_backward(TxnId txn) {
   GPUConn conn = gpu()->conn();
   ad_tensor4 dyv = y_.grad.get(txn, id()).view_interior();
-  for (auto& x : xs_) {
-    auto xd = x->data();
+  for (size_t i = 0; i < xs_.size(); ++i) {
+    if (grads_[i] == kJoinShare) continue;
+    auto xd = xs_[i]->data();
+    if (grads_[i] == kJoinDefer) { xd.grad.defer(txn, &y_.grad.get(txn, id())); continue; }
     const int mode = xd.grad.accumulate_full(txn, id(), unpadded, zero_init(gpu()));
     if (!mode) continue;
     ad_tensor4 dxv = xd.grad.get_mut(txn, id()).view_interior();

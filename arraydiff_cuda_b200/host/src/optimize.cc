@@ -53,6 +53,13 @@ void ParallelSGDOptimizer<float>::reset(shared_ptr<Context> ctx, std::mt19937_64
     any rd = param_[r];
     sink_->load_val(load_txn, params_[r], 0, &rd);
   }
+  // from here on the parameters and their gradients are places in the flat buffers
+  for (size_t r = 0; r < R; ++r) {
+    if (!mgpu_->is_local(r)) continue;
+    any bp = BindFlat{param_[r].dptr()}, bg = BindFlat{sum_grad_[r].dptr()};
+    sink_->load_val(load_txn, params_[r], 0, &bp);
+    sink_->load_grad(load_txn, grads_[r], 0, &bg);
+  }
   iter_count_ = 0;
   mgpu_->sync();
 }
@@ -148,6 +155,10 @@ void ParallelSGDOptimizer<float>::reset(shared_ptr<Context> parallel_ctx) {
     sink_->load_val(load_txn, params_[r], 0, &rd);
     any rs = running_stat_[r];
     if (stat_dim_) sink_->load_val(load_txn, fixed_stats_[r], 0, &rs);
+    // from here on the parameters are places in the flat buffer; their gradients are not: micro-batches write them anew
+    // while sum_grad_ holds the sum
+    any bp = BindFlat{param_[r].dptr()};
+    sink_->load_val(load_txn, params_[r], 0, &bp);
   }
   iter_count_ = 0;
   mgpu_->sync();

@@ -120,21 +120,21 @@ vector<ActVar> parallel_relu(vector<ActVar> inputs, shared_ptr<Context> ctx) {
   return out;
 }
 template <>
-vector<ActVar> parallel_sum(vector<vector<ActVar>> inputs, shared_ptr<Context> ctx) {
+vector<ActVar> parallel_sum(vector<vector<ActVar>> inputs, shared_ptr<Context> ctx, vector<JoinGrad> grads) {
   vector<ActVar> out;
   for (size_t r = 0; r < inputs.at(0).size(); ++r) {
     vector<ActVar> xs;
     for (auto& branch : inputs) xs.push_back(branch.at(r));
-    out.push_back(SumJoinOpF::Make(xs, ctx));
+    out.push_back(SumJoinOpF::Make(xs, ctx, grads));
   }
   return out;
 }
 template <>
 ParallelBatchNormParamOp<Act> parallel_batch_norm(size_t channels, shared_ptr<bool> switch_var, vector<ActVar> inputs, bool fuse_relu,
-                                                  shared_ptr<Context> ctx) {
+                                                  shared_ptr<Context> ctx, size_t out_pad) {
   ParallelBatchNormParamOp<Act> out;
   for (auto& x : inputs) {
-    auto parts = CudnnBatchNorm2DOpF::Make(channels, switch_var, x, ctx);
+    auto parts = CudnnBatchNorm2DOpF::Make(channels, switch_var, x, ctx, out_pad);
     if (fuse_relu) parts.op->fuse_relu();
     out.ops.push_back(parts.op);
     VarIdSet p, g, bs, fs;
@@ -163,19 +163,20 @@ struct BlockVars {
   vector<VarIdSet> params, grads, batch_stats, fixed_stats;
 };
 
-// BN -> ReLU, fused into one kernel
-static vector<ActVar> bn_relu(const char* name, size_t channels, shared_ptr<bool> sw, vector<ActVar> in, BlockVars& vars, shared_ptr<Context> ctx) {
+// BN -> ReLU, fused into one kernel; pad: written into the halo-padded buffer of its one consumer
+static vector<ActVar> bn_relu(const char* name, size_t channels, shared_ptr<bool> sw, vector<ActVar> in, BlockVars& vars, shared_ptr<Context> ctx,
+                              size_t pad = 0) {
   NameScope scope(name);
-  auto bn = parallel_batch_norm<Act>(channels, sw, in, true, ctx);
+  auto bn = parallel_batch_norm<Act>(channels, sw, in, true, ctx, pad);
   vars.add(bn);
   return bn.ops;
 }
-// halo pad -> halo exchange -> conv on the halo-padded strip
-static vector<ActVar> halo_conv(const char* name, Conv2DShape shape, vector<ActVar> in, BlockVars& vars, shared_ptr<Context> ctx) {
+// halo pad (unless `in` was written halo-padded) -> halo exchange -> conv on the halo-padded strip
+static vector<ActVar> halo_conv(const char* name, Conv2DShape shape, vector<ActVar> in, BlockVars& vars, shared_ptr<Context> ctx, bool padded = false) {
   NameScope scope(name);
   assert(shape.pad[0] == shape.pad[1]);
   shape.halo_padded_input = true;
-  auto pad = HaloPad2DOpF::MakeParallel(shape.pad[0], in, ctx);
+  auto pad = padded ? in : HaloPad2DOpF::MakeParallel(shape.pad[0], in, ctx);
   auto exch = HaloExch2DOpF::MakeParallel(shape.pad[0], pad, ctx);
   const size_t cin = in.at(0)->shape().shape[2];
   auto conv = parallel_conv2d<Act>(shape, exch, kaiming_init_gen<GPUArray4D<float>>(cin * shape.kernel[0] * shape.kernel[1], shape.filters), false, ctx);
@@ -196,11 +197,11 @@ template <>
 ParallelBatchNormParamOp<Act> spatial_parallel_residual_v2_conv2d(Conv2DShape shape, shared_ptr<bool> sw, vector<ActVar> inputs, shared_ptr<Context> ctx) {
   BlockVars vars(inputs.size());
   shape.stride = {1, 1};
-  auto a0 = bn_relu("bn0", inputs.at(0)->shape().shape[2], sw, inputs, vars, ctx);
-  auto c1 = halo_conv("conv1", shape, a0, vars, ctx);
-  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx);
-  auto c2 = halo_conv("conv2", shape, a1, vars, ctx);
-  return vars.finish(parallel_sum<Act>({inputs, c2}, ctx));
+  auto a0 = bn_relu("bn0", inputs.at(0)->shape().shape[2], sw, inputs, vars, ctx, shape.pad[0]);
+  auto c1 = halo_conv("conv1", shape, a0, vars, ctx, true);
+  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx, shape.pad[0]);
+  auto c2 = halo_conv("conv2", shape, a1, vars, ctx, true);
+  return vars.finish(parallel_sum<Act>({inputs, c2}, ctx, {kJoinDefer, kJoinShare}));
 }
 // same with a strided 1x1 projection shortcut taken after the first BN-ReLU   (reference src/zoo.cc:654-738)
 template <>
@@ -211,11 +212,11 @@ ParallelBatchNormParamOp<Act> spatial_parallel_proj_residual_v2_conv2d(Conv2DSha
   Conv2DShape s1 = shape;
   s1.stride = {stride, stride};
   auto c1 = halo_conv("conv1", s1, a0, vars, ctx);
-  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx);
+  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx, shape.pad[0]);
   Conv2DShape s2 = shape;
   s2.stride = {1, 1};
-  auto c2 = halo_conv("conv2", s2, a1, vars, ctx);
-  return vars.finish(parallel_sum<Act>({proj, c2}, ctx));
+  auto c2 = halo_conv("conv2", s2, a1, vars, ctx, true);
+  return vars.finish(parallel_sum<Act>({proj, c2}, ctx, {kJoinShare, kJoinShare}));
 }
 // BN-ReLU-1x1, BN-ReLU-[pad-exch-3x3], BN-ReLU-1x1 (x bottleneck), identity shortcut   (reference src/zoo.cc:740-837)
 template <>
@@ -225,11 +226,11 @@ ParallelBatchNormParamOp<Act> spatial_parallel_bottleneck_residual_v2_conv2d(Con
   shape.stride = {1, 1};
   auto a0 = bn_relu("bn0", inputs.at(0)->shape().shape[2], sw, inputs, vars, ctx);
   auto c1 = conv1x1("conv1", shape.filters, 1, a0, vars, ctx);
-  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx);
-  auto c2 = halo_conv("conv2", shape, a1, vars, ctx);
+  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx, shape.pad[0]);
+  auto c2 = halo_conv("conv2", shape, a1, vars, ctx, true);
   auto a2 = bn_relu("bn2", shape.filters, sw, c2, vars, ctx);
   auto c3 = conv1x1("conv3", bottleneck * shape.filters, 1, a2, vars, ctx);
-  return vars.finish(parallel_sum<Act>({inputs, c3}, ctx));
+  return vars.finish(parallel_sum<Act>({inputs, c3}, ctx, {kJoinDefer, kJoinShare}));
 }
 // bottleneck with a strided 1x1 projection shortcut; the 3x3 carries the stride   (reference src/zoo.cc:839-946,
 // which strides only the projection: the single-GPU twin at :541-542 strides the 3x3 as done here)
@@ -239,13 +240,13 @@ ParallelBatchNormParamOp<Act> spatial_parallel_proj_bottleneck_residual_v2_conv2
   auto a0 = bn_relu("bn0", inputs.at(0)->shape().shape[2], sw, inputs, vars, ctx);
   auto proj = conv1x1("proj", bottleneck * shape.filters, stride, a0, vars, ctx);
   auto c1 = conv1x1("conv1", shape.filters, 1, a0, vars, ctx);
-  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx);
+  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx, shape.pad[0]);
   Conv2DShape s2 = shape;
   s2.stride = {stride, stride};
-  auto c2 = halo_conv("conv2", s2, a1, vars, ctx);
+  auto c2 = halo_conv("conv2", s2, a1, vars, ctx, true);
   auto a2 = bn_relu("bn2", shape.filters, sw, c2, vars, ctx);
   auto c3 = conv1x1("conv3", bottleneck * shape.filters, 1, a2, vars, ctx);
-  return vars.finish(parallel_sum<Act>({proj, c3}, ctx));
+  return vars.finish(parallel_sum<Act>({proj, c3}, ctx, {kJoinShare, kJoinShare}));
 }
 
 // scatter_on_load: every rank's input variable is its strip, filled straight from the host image (HostRows);
@@ -352,12 +353,11 @@ static vector<ActVar> stem(SpatialParallelNet& net, const ConvNetConfig& cfg, si
   { NameScope scope("stem.conv"); conv1 = parallel_conv2d<Act>(c1, exch1, kaiming_init_gen<GPUArray4D<float>>(cfg.input_c * 49, width), false, ctx); }
   absorb(net, conv1.ops, conv1.params, conv1.grads);
   ParallelBatchNormParamOp<Act> bn1;
-  { NameScope scope("stem.bn"); bn1 = parallel_batch_norm<Act>(width, sw, conv1.ops, true, ctx); }
+  { NameScope scope("stem.bn"); bn1 = parallel_batch_norm<Act>(width, sw, conv1.ops, true, ctx, 1); }
   absorb(net, bn1.ops, bn1.params, bn1.grads, &bn1.batch_stats, &bn1.fixed_stats);
   Pool2DShape pool;
   pool.window = {3, 3}; pool.stride = {2, 2}; pool.pad = {1, 1}; pool.halo_padded_input = true;
-  auto pad2 = HaloPad2DOpF::MakeParallel(1, bn1.ops, ctx);
-  auto exch2 = HaloExch2DOpF::MakeParallel(1, pad2, ctx);
+  auto exch2 = HaloExch2DOpF::MakeParallel(1, bn1.ops, ctx);
   return CudnnPool2DOpF::MakeParallel(pool, exch2, ctx);
 }
 
@@ -488,10 +488,9 @@ SpatialParallelNet SpatialParallelResNet<float>::MakeParallelResNet18(const Conv
 // single-rank twins of the halo_conv / bottleneck helpers for the replicated tail of a net: ordinary zero padding
 static vector<ActVar> plain_conv3x3(const char* name, Conv2DShape shape, vector<ActVar> in, BlockVars& vars, shared_ptr<Context> ctx) {
   NameScope scope(name);
-  shape.halo_padded_input = true;   // pad -> conv on the padded buffer, without an exchange: every rank holds all rows
-  auto pad = HaloPad2DOpF::MakeParallel(shape.pad[0], in, ctx);
+  shape.halo_padded_input = true;   // on the padded buffer `in`, without an exchange: every rank holds all rows
   const size_t cin = in.at(0)->shape().shape[2];
-  auto conv = parallel_conv2d<Act>(shape, pad, kaiming_init_gen<GPUArray4D<float>>(cin * shape.kernel[0] * shape.kernel[1], shape.filters), false, ctx);
+  auto conv = parallel_conv2d<Act>(shape, in, kaiming_init_gen<GPUArray4D<float>>(cin * shape.kernel[0] * shape.kernel[1], shape.filters), false, ctx);
   vars.add(conv);
   return conv.ops;
 }
@@ -502,13 +501,13 @@ static ParallelBatchNormParamOp<Act> replicated_bottleneck(Conv2DShape shape, si
   vector<ActVar> shortcut = inputs;
   if (proj) shortcut = conv1x1("proj", bottleneck * shape.filters, stride, a0, vars, ctx);
   auto c1 = conv1x1("conv1", shape.filters, 1, a0, vars, ctx);
-  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx);
+  auto a1 = bn_relu("bn1", shape.filters, sw, c1, vars, ctx, shape.pad[0]);
   Conv2DShape s2 = shape;
   s2.stride = {stride, stride};
   auto c2 = plain_conv3x3("conv2", s2, a1, vars, ctx);
   auto a2 = bn_relu("bn2", shape.filters, sw, c2, vars, ctx);
   auto c3 = conv1x1("conv3", bottleneck * shape.filters, 1, a2, vars, ctx);
-  return vars.finish(parallel_sum<Act>({shortcut, c3}, ctx));
+  return vars.finish(parallel_sum<Act>({shortcut, c3}, ctx, {proj ? kJoinShare : kJoinDefer, kJoinShare}));
 }
 
 template <>
