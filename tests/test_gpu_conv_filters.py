@@ -58,3 +58,45 @@ def test_filter_gradient_order(K, Cc, k, accumulate):
         abi.check(L.ad_conv2d_wgrad_ex(C.byref(a), H.ptr(status), H.stream()))
     H.sync()
     assert int(status[0]) == 0 and torch.equal(kcrs, krsc.permute(0, 3, 1, 2)) and not torch.equal(krsc, old)
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, K, k, stride, dil, pad, columns
+    (2, 64, 15, 21, 64, 3, 2, 1, 1, None), (1, 256, 9, 140, 64, 1, 2, 1, 0, None), (3, 128, 8, 8, 64, 3, 2, 1, 0, (1, 6)),
+    (1, 64, 22, 19, 128, 3, 2, 2, 2, None),      # dilation and stride share a factor: half of the classes have no taps
+    (1, 64, 20, 23, 64, 3, 3, 1, 1, None),       # nine classes: three launches
+    (2, 64, 17, 16, 64, 2, 3, 1, 0, (2, 9)),     # a kernel smaller than the stride
+    (1, 64, 23, 26, 64, 5, 4, 3, 4, None), (1, 19, 12, 12, 64, 3, 2, 1, 1, None), (2, 32, 14, 14, 19, 4, 2, 1, 1, None),
+    (1, 64, 31, 33, 64, 7, 2, 1, 3, None),
+])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_strided_data_gradient(case, accumulate):
+    import numpy as np
+    import torch
+    from oracle import orc
+    N, Cc, Hh, W, K, k, s, d, pd, cols = case
+    P, Q = ((n + 2 * pd - d * (k - 1) - 1) // s + 1 for n in (Hh, W))
+    w = orc.round_bf16(H.normal(1, (K, Cc, k, k), float(np.sqrt(2.0 / (k * k * Cc)))))
+    dy = orc.round_bf16(H.uniform(2, (N, K, P, Q)))
+    want = orc.conv2d_dgrad(dy, w, (N, Cc, Hh, W), (s, s), (d, d), (pd, pd), omp=True)
+    L = abi.lib()
+    a = abi.Conv2dArgs()
+    a.dtype, a.layout = abi.AD_BF16, abi.AD_NHWC
+    a.N, a.C, a.H, a.W, a.K, a.kh, a.kw = N, Cc, Hh, W, K, k, k
+    a.stride_h = a.stride_w = s
+    a.dil_h = a.dil_w = d
+    a.pad_h = a.pad_w = pd
+    if cols:
+        a.dx_col_begin, a.dx_col_count = cols
+    tw, tdy = H.dev_bf16(np.ascontiguousarray(np.transpose(w, (0, 2, 3, 1)))), H.dev_bf16(orc.nchw_to_nhwc(dy))
+    dx = torch.full((N, Hh, W, Cc), 3.0, dtype=torch.bfloat16, device="cuda")
+    sb = L.ad_conv2d_scratch_bytes(C.byref(a), 1)
+    scratch = torch.zeros(sb, dtype=torch.uint8, device="cuda")
+    a.w, a.y, a.dx, a.scratch, a.scratch_bytes, a.accumulate = tw.data_ptr(), tdy.data_ptr(), dx.data_ptr(), scratch.data_ptr(), sb, accumulate
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    H.sync()
+    assert scratch[:4].view(torch.int32).item() == 0
+    lo, n = cols or (0, W)
+    got = orc.nhwc_to_nchw(H.host(dx))
+    assert H.max_rel(got[..., lo:lo + n] - 3.0 * accumulate, want[..., lo:lo + n]) < 2e-2
+    assert np.all(got[..., :lo] == 3.0) and np.all(got[..., lo + n:] == 3.0)
