@@ -406,43 +406,63 @@ struct WgParams {
   int32_t* status;
 };
 
-template <int BN, int STAGES>
+// A work item is one [128 dy channels][BN x channels] block of one tap, summed over the pixel tiles of one split.  The kernel
+// is persistent, one CTA per SM: the copies of the next item start while the last one is still multiplied, and two
+// accumulators let the epilogue drain one item under the next.  With a CTA per item, layers of a few pixel tiles per item
+// (small feature maps) spent most of the time in set-up, pipeline fill and drain.
+// PAIR: two CTAs work on one item of 256 dy channels and load half of the x tile each: 48 KB instead of 64 per 128 pixels
+// and SM; the operand tiles come out of the L2, whose rate (~16 TB/s) is the bound of the plain form: 512 -> 512 channels,
+// 3x3, 65,536 pixels 306 -> 269 us, 1024 -> 256, 1x1 93 -> 67.
+// Items of one split come one after another, so that the blocks at work at any time read the same pixels.
+template <int BN, int STAGES, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_x,
                      const WgParams p) {
   extern __shared__ uint8_t smem_raw[];
-  constexpr uint32_t kABytes = 2 * kSlabBytes, kBBytes = (BN / 64) * kSlabBytes, kStageBytes = kABytes + kBBytes;
+  constexpr int kCtas = PAIR ? 2 : 1;
+  constexpr uint32_t kABytes = 2 * kSlabBytes, kBSlabs = BN / 64 / kCtas, kStageBytes = kABytes + kBSlabs * kSlabBytes;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   SmemCtl* ctl = (SmemCtl*)(smem + (size_t)STAGES * kStageBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr uint32_t kTmemCols = BN < 32 ? 32 : BN;
-
-  // blockIdx.y -> (tap, k tile, c tile); blockIdx.x -> split of the pixel tiles
-  const uint32_t split = blockIdx.x;
-  uint32_t rem = blockIdx.y;
-  const uint32_t ct = rem % p.ctiles; rem /= p.ctiles;
-  const uint32_t kt = rem % p.ktiles; rem /= p.ktiles;
-  const uint32_t tap = rem, r = tap / p.kw, s = tap % p.kw;
+  constexpr uint32_t kTmemCols = 2 * BN;   // 128 or 256
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
   const uint32_t sp_tiles = p.tiles_b * p.tiles_y * p.tiles_x;
-  const uint32_t my_tiles = split < sp_tiles ? (sp_tiles - split + p.splits - 1) / p.splits : 0;
+  const uint32_t outer = p.kh * p.kw * (p.ktiles / kCtas) * p.ctiles, items = outer * p.splits;
+  const uint32_t first = blockIdx.x / kCtas, step = gridDim.x / kCtas;
+
+  struct Item { uint32_t split, tap, kt, ct, tiles; };
+  auto item_at = [&](uint32_t i) {
+    Item t;
+    t.split = i / outer;
+    uint32_t rem = i - t.split * outer;
+    t.ct = rem % p.ctiles; rem /= p.ctiles;
+    t.kt = rem % (p.ktiles / kCtas) * kCtas + rank;
+    t.tap = rem / (p.ktiles / kCtas);
+    t.tiles = t.split < sp_tiles ? (sp_tiles - t.split + p.splits - 1) / p.splits : 0;
+    return t;
+  };
 
   if (threadIdx.x == 0) {
     for (int st = 0; st < STAGES; ++st) {
       mbar_init(smem_u32(&ctl->full[st]), 1);
       mbar_init(smem_u32(&ctl->empty[st]), 1);
     }
-    mbar_init(smem_u32(&ctl->tfull[0]), 1);
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&ctl->tfull[a]), 1);
+      mbar_init(smem_u32(&ctl->tempty[a]), 4 * kCtas);
+    }
     ctl->abort_flag = 0;
     mbar_init_fence();
     tma_prefetch_desc(&map_dy);
     tma_prefetch_desc(&map_x);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
-    tmem_relinquish();
+    if (PAIR) { tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish_pair(); }
+    else { tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish(); }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();   // the other CTA's barriers are initialised
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
@@ -450,67 +470,96 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
   if (warp == 0) {
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
-      for (uint32_t j = 0; j < my_tiles; ++j) {
-        const uint32_t tm = split + j * p.splits;
-        const uint32_t tx = tm % p.tiles_x, ty = (tm / p.tiles_x) % p.tiles_y, n = tm / (p.tiles_x * p.tiles_y) * p.TN;
-        if (!mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1u, abortf)) break;
-        const uint32_t full = smem_u32(&ctl->full[stage]);
-        uint8_t* st = smem + (size_t)stage * kStageBytes;
-        mbar_expect_tx(full, kStageBytes);
-        const int qx = (int)(tx * p.TW), qy = (int)(ty * p.TH);
-        tma_load_4d(smem_u32(st), &map_dy, full, (int)(kt * 128), qx, qy, (int)n);
-        tma_load_4d(smem_u32(st + kSlabBytes), &map_dy, full, (int)(kt * 128 + 64), qx, qy, (int)n);
-        const int ix = qx * (int)p.sw + (int)(s * p.dw) + p.offx, iy = qy * (int)p.sh + (int)(r * p.dh) + p.offy;
+      bool ok = true;
+      for (uint32_t i = first; i < items && ok; i += step) {
+        const Item t = item_at(i);
+        const uint32_t r = t.tap / p.kw, s = t.tap % p.kw;
+        for (uint32_t j = 0; j < t.tiles; ++j) {
+          const uint32_t tm = t.split + j * p.splits;
+          const uint32_t tx = tm % p.tiles_x, ty = (tm / p.tiles_x) % p.tiles_y, n = tm / (p.tiles_x * p.tiles_y) * p.TN;
+          if (!mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1u, abortf)) { ok = false; break; }
+          uint32_t full = smem_u32(&ctl->full[stage]);
+          uint8_t* st = smem + (size_t)stage * kStageBytes;
+          if (rank == 0) mbar_expect_tx(full, kStageBytes * kCtas);
+          if (PAIR) full = cluster_first(full);
+          const int qx = (int)(tx * p.TW), qy = (int)(ty * p.TH), c0 = (int)(t.ct * BN + rank * (BN / kCtas));
+          const int ix = qx * (int)p.sw + (int)(s * p.dw) + p.offx, iy = qy * (int)p.sh + (int)(r * p.dh) + p.offy;
+          auto load = [&](uint32_t dst, const CUtensorMap* map, int c, int x, int y) {
+            if (PAIR) tma_load_4d_pair(dst, map, full, c, x, y, (int)n);
+            else tma_load_4d(dst, map, full, c, x, y, (int)n);
+          };
+          load(smem_u32(st), &map_dy, (int)(t.kt * 128), qx, qy);
+          load(smem_u32(st + kSlabBytes), &map_dy, (int)(t.kt * 128 + 64), qx, qy);
 #pragma unroll
-        for (int b = 0; b < BN / 64; ++b)
-          tma_load_4d(smem_u32(st + kABytes + b * kSlabBytes), &map_x, full, (int)(ct * BN + b * 64), ix, iy, (int)n);
-        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+          for (uint32_t b = 0; b < kBSlabs; ++b) load(smem_u32(st + kABytes + b * kSlabBytes), &map_x, c0 + (int)b * 64, ix, iy);
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(BN, 1, 1);
-      uint32_t stage = 0, phase = 0;
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = idesc_bf16(BN, 1, 1, 128 * kCtas);
+      uint32_t stage = 0, phase = 0, it = 0;
       bool ok = true;
-      for (uint32_t j = 0; j < my_tiles; ++j) {
-        if (!mbar_wait(smem_u32(&ctl->full[stage]), phase, abortf)) { ok = false; break; }
+      for (uint32_t i = first; i < items && ok; i += step, ++it) {
+        const uint32_t tiles = item_at(i).tiles, acc = it & 1u;
+        if (!mbar_wait(smem_u32(&ctl->tempty[acc]), ((it >> 1) & 1u) ^ 1u, abortf)) break;
         tc_fence_after();
-        const uint32_t sa = smem_u32(smem + (size_t)stage * kStageBytes);
+        const uint32_t d = tmem_base + acc * BN;
+        for (uint32_t j = 0; j < tiles; ++j) {
+          if (!mbar_wait(smem_u32(&ctl->full[stage]), phase, abortf)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + (size_t)stage * kStageBytes);
 #pragma unroll
-        for (uint32_t ks = 0; ks < 8; ++ks) {  // 8 x (K = 16 pixels = 16 rows of 128 B)
-          const uint64_t da = smem_desc_sw128(sa + ks * 2048, kSlabBytes, 1024);
-          const uint64_t db = smem_desc_sw128(sa + kABytes + ks * 2048, kSlabBytes, 1024);
-          umma_bf16(tmem_base, da, db, idesc, (j | ks) != 0u);
+          for (uint32_t ks = 0; ks < 8; ++ks) {  // 8 x (K = 16 pixels = 16 rows of 128 B)
+            const uint64_t da = smem_desc_sw128(sa + ks * 2048, kSlabBytes, 1024);
+            const uint64_t db = smem_desc_sw128(sa + kABytes + ks * 2048, kSlabBytes, 1024);
+            if (PAIR) umma_bf16_pair(d, da, db, idesc, (j | ks) != 0u);
+            else umma_bf16(d, da, db, idesc, (j | ks) != 0u);
+          }
+          if (PAIR) umma_commit_pair(smem_u32(&ctl->empty[stage]));
+          else umma_commit(smem_u32(&ctl->empty[stage]));
+          if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        umma_commit(smem_u32(&ctl->empty[stage]));
-        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        if (!ok) break;
+        if (PAIR) umma_commit_pair(smem_u32(&ctl->tfull[acc]));
+        else umma_commit(smem_u32(&ctl->tfull[acc]));
       }
-      if (ok) umma_commit(smem_u32(&ctl->tfull[0]));
     }
   } else {
     const uint32_t q = (uint32_t)warp & 3u;
     const uint32_t taps = p.kh * p.kw;
-    const uint32_t k = kt * 128 + q * 32 + lane;
-    float* orow = p.partial + (((size_t)split * p.KO + k) * taps + tap) * p.CI + (size_t)ct * BN;
-    if (my_tiles == 0) {
-      if (k < p.KO)
-        for (uint32_t c = 0; c < BN && ct * BN + c < p.CI; ++c) orow[c] = 0.f;
-    } else if (mbar_wait(smem_u32(&ctl->tfull[0]), 0, abortf)) {
+    uint32_t it = 0;
+    for (uint32_t i = first; i < items; i += step, ++it) {
+      const Item t = item_at(i);
+      const uint32_t acc = it & 1u, k = t.kt * 128 + q * 32 + lane;
+      float* orow = p.partial + (((size_t)t.split * p.KO + k) * taps + t.tap) * p.CI + (size_t)t.ct * BN;
+      if (!mbar_wait(smem_u32(&ctl->tfull[acc]), (it >> 1) & 1u, abortf)) break;
       tc_fence_after();
 #pragma unroll 1
       for (uint32_t ch = 0; ch < BN / 32; ++ch) {
         uint32_t v[32];
-        tmem_ld32(tmem_base + ((q * 32u) << 16) + ch * 32, v);
+        tmem_ld32(tmem_base + ((q * 32u) << 16) + acc * BN + ch * 32, v);
         tmem_ld_wait();
+        if (t.tiles == 0) {   // more splits than pixel tiles: nothing was accumulated
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0u;
+        }
         if (k < p.KO) {
 #pragma unroll
           for (int g = 0; g < 8; ++g) {
-            const uint32_t c = ct * BN + ch * 32 + g * 4;
+            const uint32_t c = t.ct * BN + ch * 32 + g * 4;
             if (c + 4 <= p.CI)
               *(float4*)(orow + ch * 32 + g * 4) = make_float4(__uint_as_float(v[g * 4]), __uint_as_float(v[g * 4 + 1]),
                                                                __uint_as_float(v[g * 4 + 2]), __uint_as_float(v[g * 4 + 3]));
           }
         }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(cluster_first(smem_u32(&ctl->tempty[acc])));
+        else mbar_arrive(smem_u32(&ctl->tempty[acc]));
       }
     }
   }
@@ -522,10 +571,12 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
     if (threadIdx.x == 0 && p.status) *p.status = AD_ERR_TIMEOUT;
   }
   __syncthreads();
+  if (PAIR) cluster_sync();   // neither CTA leaves while the other's copies, arrivals or MMAs may reach it
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    if (PAIR) tmem_dealloc_pair(tmem_base, kTmemCols);
+    else tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
@@ -939,24 +990,39 @@ static int run_fwd_gemm(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, 
   return run_fwd_tiles<1>(act, IH, IW, filt, kh * kw, p, FwdClasses{}, s);
 }
 
-template <int BN>
+template <int BN, bool PAIR>
 static int launch_wgrad(const CUtensorMap& mdy, const CUtensorMap& mx, const WgParams& p, cudaStream_t s) {
-  constexpr int kStageBytes = 2 * kSlabBytes + (BN / 64) * kSlabBytes;
+  constexpr int kCtas = PAIR ? 2 : 1;
+  constexpr int kStageBytes = 2 * kSlabBytes + (BN / 64 / kCtas) * kSlabBytes;
   constexpr int STAGES = (200 * 1024) / kStageBytes;
   constexpr int smem = STAGES * kStageBytes + 1024 + (int)sizeof(SmemCtl);
+  auto kern = conv_tc_wgrad_kernel<BN, STAGES, PAIR>;
   static unsigned attr_done = 0;  // one bit per device: the attribute is per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(conv_tc_wgrad_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
       cudaGetLastError();
       return AD_ERR_CUDA;
     }
     attr_done |= 1u << (dev & 31);
   }
-  dim3 grid(p.splits, p.kh * p.kw * p.ktiles * p.ctiles);
-  conv_tc_wgrad_kernel<BN, STAGES><<<grid, kThreads, smem, s>>>(mdy, mx, p);
+  const uint32_t items = p.splits * p.kh * p.kw * (p.ktiles / kCtas) * p.ctiles;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::min(items, (uint32_t)kNumSMs / kCtas) * kCtas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kCtas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = PAIR ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, kern, mdy, mx, p) != cudaSuccess) {
+    cudaGetLastError();
+    return AD_ERR_CUDA;
+  }
   count_launch();
   return launch_status();
 }
@@ -1207,7 +1273,9 @@ int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
     st = make_tmap_bf16(&mx, a->x, 4, dims, str, box, es);
     if (st != AD_OK) return st;
   }
-  st = BN == 128 ? launch_wgrad<128>(mdy, mx, p, s) : launch_wgrad<64>(mdy, mx, p, s);
+  // pairs need an even number of 128-channel tiles of dy, and 64 channels of x per CTA
+  st = BN == 128 ? (p.ktiles % 2 == 0 ? launch_wgrad<128, true>(mdy, mx, p, s) : launch_wgrad<128, false>(mdy, mx, p, s))
+                 : launch_wgrad<64, false>(mdy, mx, p, s);
   if (st != AD_OK) return st;
   launch_wgrad_reduce(a->K, a->kh * a->kw, a->C, wcount_p, p.splits, p.partial, (float*)a->dw, a->accumulate, a->dw_kcrs, s);
   if (a->db) launch_bias_grad((size_t)a->N * g.P * g.Q, a->K, a->y, a->db, a->accumulate, p.partial, s);

@@ -35,10 +35,12 @@ def test_filter_prepare(shapes, pad_row):
             assert torch.equal(crsk[..., :K], w.flip(2, 3).permute(1, 2, 3, 0).bfloat16()) and torch.all(crsk[..., K:] == 0)
 
 
-@pytest.mark.parametrize("K,Cc,k", [(64, 64, 2), (40, 128, 3), (19, 64, 9), (8, 64, 10)])
+@pytest.mark.parametrize("K,Cc,k", [
+    (64, 64, 2), (40, 128, 3), (19, 64, 9), (8, 64, 10),
+    (256, 128, 3), (200, 192, 1), (520, 128, 2), (384, 256, 1)])   # CTA pairs: whole, ragged; an odd number of filter tiles
 @pytest.mark.parametrize("accumulate", [0, 1])
 def test_filter_gradient_order(K, Cc, k, accumulate):
-    """The KCRS form is the KRSC form, turned round, to the bit."""
+    """The KRSC form against a double-precision sum; the KCRS form is the KRSC form, turned round, to the bit."""
     import torch
     N, Hh = 2, 24
     L = abi.lib()
@@ -57,7 +59,11 @@ def test_filter_gradient_order(K, Cc, k, accumulate):
         a.dw, a.dw_kcrs = out.data_ptr(), order
         abi.check(L.ad_conv2d_wgrad_ex(C.byref(a), H.ptr(status), H.stream()))
     H.sync()
-    assert int(status[0]) == 0 and torch.equal(kcrs, krsc.permute(0, 3, 1, 2)) and not torch.equal(krsc, old)
+    assert int(status[0]) == 0 and torch.equal(kcrs, krsc.permute(0, 3, 1, 2))
+    d = dy.double().reshape(-1, K).T
+    want = torch.stack([torch.stack([d @ x[:, r:r + P, s:s + P].double().reshape(-1, Cc) for s in range(k)], 1) for r in range(k)], 1)
+    want += accumulate * old.double()
+    assert (krsc - want).abs().max() < 1e-4 * want.abs().max()
 
 
 @pytest.mark.parametrize("case", [
