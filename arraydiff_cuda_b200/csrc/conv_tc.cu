@@ -77,6 +77,11 @@ constexpr int kSlabBytes = 16384;   // one [128 rows][64 bf16] swizzled operand 
 constexpr int kThreads = 192;       // filter-gradient kernel: warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
 constexpr int kFwdThreads = 320;    // forward kernel: warp 0 TMA, warp 1 MMA, two groups of 4 epilogue warps
 
+// The forward kernel is persistent, one CTA per SM, with two accumulators.  What bounds it where the contraction is long is the
+// rate at which an SM gets operand tiles from the L2 (64 bytes per clock): a [128 pixels][256 channels] tile takes 48 KB per 64 of
+// depth.  PAIR: two CTAs make [256][256] together (cta_group::2), each loading its own pixels and half of the filter
+// rows, 32 KB.  512 -> 512 channels, 3x3, 65,536 pixels: 198 -> 180 us, 1024 -> 2048
+// 1x1 261 -> 179.
 // The outputs that a launch computes fall into classes of one tap list each: one class, except for the data gradient of a
 // strided layer (conv_tc_dgrad), where a pixel's taps depend on its row and column modulo the stride.
 struct FwdClass {
@@ -105,13 +110,17 @@ struct FwdParams {
 };
 struct FwdClasses { FwdClass c[kFwdClasses]; uint32_t n; };
 template <int NC> struct FwdOut { CUtensorMap map[NC]; };
-// Where tile number `tile` of the launch lies: channel tile tn, pixel tile (n, ty, tx) of class cls
+// Where tile number `tile` of the launch lies: channel tile tn, pixel tile (n, ty, tx) of class cls (n >= NI: none, a CTA
+// pair has an odd tile too many).  The channel tiles of one pixel tile (of the two of a pair) follow one another, so that
+// they read it together: with all pixel tiles of one channel tile first, wide inputs came from DRAM once per channel tile
+// (1024 -> 2048, 1x1, 65,536 pixels: 291 -> 231 us without pairs).
 struct FwdTile { uint32_t tn, tx, ty, n, cls; };
-template <int NC>
-__device__ __forceinline__ FwdTile fwd_tile(const FwdParams& p, const FwdClasses& k, uint32_t tiles_m, uint32_t tile) {
+template <int NC, bool PAIR>
+__device__ __forceinline__ FwdTile fwd_tile(const FwdParams& p, const FwdClasses& k, uint32_t rank, uint32_t tile) {
   FwdTile t;
-  t.tn = tile / tiles_m;
-  uint32_t tm = tile % tiles_m, tx = p.tiles_x, ty = p.tiles_y;
+  t.tn = tile % p.tiles_n;
+  uint32_t tm = tile / p.tiles_n * (PAIR ? 2 : 1) + rank;
+  uint32_t tx = p.tiles_x, ty = p.tiles_y;
   t.cls = 0;
   if (NC > 1) {
     while (t.cls + 1 < k.n && tm >= k.c[t.cls + 1].tile0) ++t.cls;
@@ -122,10 +131,10 @@ __device__ __forceinline__ FwdTile fwd_tile(const FwdParams& p, const FwdClasses
   return t;
 }
 
-constexpr int kStagingBytes = 2 * 16384;
+constexpr int kStagingBytes = 4 * 16384;   // two 64-channel chunks for each of the two epilogue groups
 
 struct SmemCtl {
-  unsigned long long full[8], empty[8], tfull[2], tempty[2], stg_full[2], stg_free[2];
+  unsigned long long full[8], empty[8], tfull[2], tempty[2], stg_full[4], stg_free[4];
   uint32_t tmem_base;
   volatile int abort_flag;
 };
@@ -136,18 +145,20 @@ __device__ __forceinline__ uint32_t pow2_cols(uint32_t c) {
   return p;
 }
 
-template <int BN, int STAGES, int NC>
+template <int BN, int STAGES, int NC, bool PAIR>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                    const __grid_constant__ FwdOut<NC> out, const FwdParams p, const __grid_constant__ FwdClasses cl) {
   extern __shared__ uint8_t smem_raw[];
-  constexpr uint32_t kStageBytes = kSlabBytes + BN * 128;
+  constexpr int kCtas = PAIR ? 2 : 1;
+  constexpr uint32_t kStageBytes = kSlabBytes + BN / kCtas * 128;
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* osm = smem + (size_t)STAGES * kStageBytes;
   SmemCtl* ctl = (SmemCtl*)(osm + kStagingBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t tiles_m = NC > 1 ? p.tiles_x : p.tiles_b * p.tiles_y * p.tiles_x;   // classes: the host has summed them up
-  const uint32_t total_tiles = tiles_m * p.tiles_n;
+  const uint32_t total_tiles = (tiles_m + kCtas - 1) / kCtas * p.tiles_n;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u, first = blockIdx.x / kCtas, step = gridDim.x / kCtas;
   const uint32_t slabs = p.CK / 64;
   constexpr uint32_t kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;  // BN in {32,64,128,256} -> power of two
 
@@ -159,9 +170,11 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&ctl->tfull[a]), 1);
       // an accumulator is drained by both epilogue groups when a tile has several 64-channel chunks
-      mbar_init(smem_u32(&ctl->tempty[a]), (p.tma_store && BN >= 128) ? 8 : 4);
-      mbar_init(smem_u32(&ctl->stg_full[a]), 4);
-      mbar_init(smem_u32(&ctl->stg_free[a]), 1);
+      mbar_init(smem_u32(&ctl->tempty[a]), ((p.tma_store && BN >= 128) ? 8 : 4) * kCtas);
+    }
+    for (int b = 0; b < 4; ++b) {
+      mbar_init(smem_u32(&ctl->stg_full[b]), 4);
+      mbar_init(smem_u32(&ctl->stg_free[b]), 1);
     }
     ctl->abort_flag = 0;
     mbar_init_fence();
@@ -171,11 +184,12 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       for (uint32_t c = 0; c < (NC > 1 ? cl.n : 1u); ++c) tma_prefetch_desc(&out.map[c]);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols);
-    tmem_relinquish();
+    if (PAIR) { tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish_pair(); }
+    else { tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish(); }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();   // the other CTA's barriers are initialised
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
@@ -183,8 +197,8 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   if (warp == 0) {
     if (lane == 0) {
       uint32_t stage = 0, phase = 0;
-      for (uint32_t tile = blockIdx.x; tile < total_tiles && !*abortf; tile += gridDim.x) {
-        const FwdTile t = fwd_tile<NC>(p, cl, tiles_m, tile);
+      for (uint32_t tile = first; tile < total_tiles && !*abortf; tile += step) {
+        const FwdTile t = fwd_tile<NC, PAIR>(p, cl, rank, tile);
         const FwdClass& k = cl.c[NC > 1 ? t.cls : 0];
         const int x0 = (int)(t.tx * p.TW * p.sw) + (NC > 1 ? k.offx : p.offx), y0 = (int)(t.ty * p.TH * p.sh) + (NC > 1 ? k.offy : p.offy);
         const uint32_t nr = NC > 1 ? k.nr : p.kh, ns = NC > 1 ? k.ns : p.kw;
@@ -195,25 +209,33 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               if (!mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1u, abortf)) { ok = false; break; }
               const uint32_t full = smem_u32(&ctl->full[stage]);
               uint8_t* st = smem + (size_t)stage * kStageBytes;
-              mbar_expect_tx(full, kStageBytes);
-              tma_load_4d(smem_u32(st), &map_a, full, (int)(cb * 64), x0 + (int)(s * p.dw), y0 + (int)(r * p.dh), (int)t.n);
+              if (rank == 0) mbar_expect_tx(full, kStageBytes * kCtas);
               const uint32_t tap = NC > 1 ? k.tap0 + r * k.tap_r + s * k.tap_s : r * p.kw + s;
-              tma_load_2d(smem_u32(st + kSlabBytes), &map_b, full, (int)(tap * p.CK + cb * 64), (int)(t.tn * BN));
+              const int ac = (int)(cb * 64), ax = x0 + (int)(s * p.dw), ay = y0 + (int)(r * p.dh);
+              const int bk = (int)(tap * p.CK + cb * 64), bn = (int)(t.tn * BN + rank * (BN / kCtas));
+              if (PAIR) {
+                const uint32_t bar = cluster_first(full);
+                tma_load_4d_pair(smem_u32(st), &map_a, bar, ac, ax, ay, (int)t.n);
+                tma_load_2d_pair(smem_u32(st + kSlabBytes), &map_b, bar, bk, bn);
+              } else {
+                tma_load_4d(smem_u32(st), &map_a, full, ac, ax, ay, (int)t.n);
+                tma_load_2d(smem_u32(st + kSlabBytes), &map_b, full, bk, bn);
+              }
               if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             }
         if (!ok) break;
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(BN, 0, 0);
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = idesc_bf16(BN, 0, 0, 128 * kCtas);
       uint32_t stage = 0, phase = 0, it = 0;
-      for (uint32_t tile = blockIdx.x; tile < total_tiles && !*abortf; tile += gridDim.x, ++it) {
+      for (uint32_t tile = first; tile < total_tiles && !*abortf; tile += step, ++it) {
         const uint32_t acc = it & 1u, acc_phase = (it >> 1) & 1u;
         if (!mbar_wait(smem_u32(&ctl->tempty[acc]), acc_phase ^ 1u, abortf)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + acc * BN;
-        const FwdClass& c = cl.c[NC > 1 ? fwd_tile<NC>(p, cl, tiles_m, tile).cls : 0];
+        const FwdClass& c = cl.c[NC > 1 ? fwd_tile<NC, PAIR>(p, cl, rank, tile).cls : 0];
         const uint32_t kiters = (NC > 1 ? c.nr * c.ns : p.kh * p.kw) * slabs;
         bool ok = true;
         for (uint32_t k = 0; k < kiters; ++k) {
@@ -222,23 +244,35 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           const uint32_t sa = smem_u32(smem + (size_t)stage * kStageBytes);
           const uint64_t da = smem_desc_sw128(sa, 16, 1024), db = smem_desc_sw128(sa + kSlabBytes, 16, 1024);
 #pragma unroll
-          for (uint32_t kk = 0; kk < 4; ++kk)  // 4 x (K = 16 bf16 = 32 bytes) inside the 128-byte row
-            umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, (k | kk) != 0u);
-          umma_commit(smem_u32(&ctl->empty[stage]));
+          for (uint32_t kk = 0; kk < 4; ++kk) {  // 4 x (K = 16 bf16 = 32 bytes) inside the 128-byte row
+            if (PAIR) umma_bf16_pair(d, da + 2 * kk, db + 2 * kk, idesc, (k | kk) != 0u);
+            else umma_bf16(d, da + 2 * kk, db + 2 * kk, idesc, (k | kk) != 0u);
+          }
+          if (PAIR) umma_commit_pair(smem_u32(&ctl->empty[stage]));
+          else umma_commit(smem_u32(&ctl->empty[stage]));
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        umma_commit(smem_u32(&ctl->tfull[acc]));
+        if (PAIR) umma_commit_pair(smem_u32(&ctl->tfull[acc]));
+        else umma_commit(smem_u32(&ctl->tfull[acc]));
       }
     }
   } else {
     const uint32_t q = (uint32_t)warp & 3u;  // TMEM lane quarter this warp may read
     const uint32_t grp = ((uint32_t)warp - 2u) >> 2;   // epilogue warps 2..5 = group 0, 6..9 = group 1
     const bool leader = (((uint32_t)warp - 2u) & 3u) == 0u;
+    auto drained = [&](uint32_t acc) {   // this warp has read its part of the accumulator
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(cluster_first(smem_u32(&ctl->tempty[acc])));
+        else mbar_arrive(smem_u32(&ctl->tempty[acc]));
+      }
+    };
     uint32_t it = 0, gk = 0;   // gk: chunks this group has staged so far
-    for (uint32_t tile = blockIdx.x; tile < total_tiles && !*abortf; tile += gridDim.x, ++it) {
+    for (uint32_t tile = first; tile < total_tiles && !*abortf; tile += step, ++it) {
       const uint32_t acc = it & 1u, acc_phase = (it >> 1) & 1u;
-      const FwdTile t = fwd_tile<NC>(p, cl, tiles_m, tile);
+      const FwdTile t = fwd_tile<NC, PAIR>(p, cl, rank, tile);
       const uint32_t tn = t.tn, tx = t.tx, ty = t.ty, n = t.n;
       const FwdClass& kc = cl.c[NC > 1 ? t.cls : 0];
       const bool none = NC > 1 && kc.nr * kc.ns == 0;   // no taps: nothing was accumulated
@@ -246,14 +280,13 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       if (BN >= 64 && p.tma_store) {
         // 64-channel chunks of the tile go through a swizzled [128 px][64 ch] staging buffer and one TMA
         // tile store each: coalesced, clipped to the tensor, no per-thread scattered 16-byte stores.  The
-        // two warp groups take alternate chunks (alternate tiles when a tile is one chunk), each with its
-        // own staging buffer, so one group converts while the other group's store drains.
+        // two warp groups take alternate chunks (alternate tiles when a tile is one chunk), each with two
+        // staging buffers of its own: a group converts a chunk while its last one is still being read
+        // (64 -> 256 channels, 262,144 pixels, bound by these stores: 44 -> 35 us).
         constexpr uint32_t kChunks = BN / 64;
         if (kChunks == 1 && (it & 1u) != grp) continue;
         if (!mbar_wait(smem_u32(&ctl->tfull[acc]), acc_phase, abortf)) break;
         tc_fence_after();
-        uint8_t* stg = osm + (size_t)grp * 16384;
-        uint8_t* srow = stg + m * 128u;
         const uint32_t m7 = m & 7u;
         bool live = true;
 #pragma unroll 1
@@ -267,16 +300,21 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
             for (int j = 0; j < 64; ++j) v[j] = 0u;
           }
-          if (c64 + 2 >= kChunks) {   // this warp's last read of the accumulator
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&ctl->tempty[acc]));
-          }
+          if (c64 + 2 >= kChunks) drained(acc);
+          const uint32_t sb = grp * 2 + (gk & 1u);
+          uint8_t *stg = osm + (size_t)sb * 16384, *srow = stg + m * 128u;
           bool ok = true;
-          if (gk >= 1) ok = mbar_wait(smem_u32(&ctl->stg_free[grp]), (gk - 1u) & 1u, abortf);
+          if (gk >= 2) ok = mbar_wait(smem_u32(&ctl->stg_free[sb]), ((gk >> 1) - 1u) & 1u, abortf);
           if (!__all_sync(0xffffffffu, ok)) { live = false; break; }
           const uint32_t cbase = tn * BN + c64 * 64;
-          if (p.bias) {
+          if (p.bias && cbase + 64 <= p.OC && !((uintptr_t)p.bias & 15u)) {
+#pragma unroll
+            for (int j = 0; j < 64; j += 4) {
+              const float4 b = *(const float4*)(p.bias + cbase + j);
+              v[j] = __float_as_uint(__uint_as_float(v[j]) + b.x); v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + b.y);
+              v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + b.z); v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + b.w);
+            }
+          } else if (p.bias) {
 #pragma unroll
             for (int j = 0; j < 64; ++j)
               if (cbase + j < p.OC) v[j] = __float_as_uint(__uint_as_float(v[j]) + p.bias[cbase + j]);
@@ -296,16 +334,16 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&ctl->stg_full[grp]));
+          if (lane == 0) mbar_arrive(smem_u32(&ctl->stg_full[sb]));
           if (leader && lane == 0) {
-            if (mbar_wait(smem_u32(&ctl->stg_full[grp]), gk & 1u, abortf)) {
-              if (cbase < p.OC)
+            if (mbar_wait(smem_u32(&ctl->stg_full[sb]), (gk >> 1) & 1u, abortf)) {
+              if (cbase < p.OC && n < p.NI)
                 asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(&out.map[NC > 1 ? t.cls : 0]),
                              "r"(smem_u32(stg)), "r"((int)cbase), "r"((int)(tx * p.TW)), "r"((int)(ty * p.TH)), "r"((int)n)
                              : "memory");
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-              mbar_arrive(smem_u32(&ctl->stg_free[grp]));
+              asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+              if (gk >= 1) mbar_arrive(smem_u32(&ctl->stg_free[sb ^ 1u]));   // the chunk before has been read
             }
           }
           __syncwarp();
@@ -371,9 +409,7 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&ctl->tempty[acc]));
+      drained(acc);
     }
     if (p.tma_store && leader && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
@@ -386,10 +422,12 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (threadIdx.x == 0 && p.status) *p.status = AD_ERR_TIMEOUT;
   }
   __syncthreads();
+  if (PAIR) cluster_sync();   // neither CTA leaves while the other's copies, arrivals or MMAs may reach it
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    if (PAIR) tmem_dealloc_pair(tmem_base, kTmemCols);
+    else tmem_dealloc(tmem_base, kTmemCols);
   }
 }
 
@@ -876,27 +914,48 @@ static void pick_tile3(uint32_t NI, uint32_t OP, uint32_t OQ, uint32_t sh, uint3
     }
 }
 
-template <int BN, int NC>
-static int launch_fwd(const CUtensorMap& ma, const CUtensorMap& mb, const FwdOut<NC>& mo, const FwdParams& p, const FwdClasses& cl, cudaStream_t s) {
-  constexpr int kStageBytes = kSlabBytes + BN * 128;
-  constexpr int STAGES = (192 * 1024) / kStageBytes > 8 ? 8 : (192 * 1024) / kStageBytes;
-  constexpr int smem = STAGES * kStageBytes + kStagingBytes + 1024 + (int)sizeof(SmemCtl);
-  static unsigned attr_done = 0;  // one bit per device: the attribute is per device
+// A persistent kernel over `items` tiles: one CTA per SM, or a pair of CTAs per two SMs.  attr_done: the caller's record of
+// the devices (a bit each) on which the kernel's shared-memory limit is raised.
+template <typename... KArgs, typename... Args>
+static int launch_tc(void (*kern)(KArgs...), uint32_t ctas, uint32_t items, int threads, int smem, unsigned& attr_done, cudaStream_t s,
+                     const Args&... args) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(conv_tc_fwd_kernel<BN, STAGES, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
       cudaGetLastError();
       return AD_ERR_CUDA;
     }
     attr_done |= 1u << (dev & 31);
   }
-  const uint32_t total = (NC > 1 ? p.tiles_x : p.tiles_b * p.tiles_y * p.tiles_x) * p.tiles_n;
-  const unsigned grid = total < (uint32_t)kNumSMs ? total : kNumSMs;
-  conv_tc_fwd_kernel<BN, STAGES, NC><<<grid, kFwdThreads, smem, s>>>(ma, mb, mo, p, cl);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(std::min(items, (uint32_t)kNumSMs / ctas) * ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = ctas > 1 ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, kern, KArgs(args)...) != cudaSuccess) {
+    cudaGetLastError();
+    return AD_ERR_CUDA;
+  }
   count_launch();
   return launch_status();
+}
+template <int BN, int NC, bool PAIR>
+static int launch_fwd(const CUtensorMap& ma, const CUtensorMap& mb, const FwdOut<NC>& mo, const FwdParams& p, const FwdClasses& cl, cudaStream_t s) {
+  constexpr int kCtas = PAIR ? 2 : 1;
+  constexpr int kStageBytes = kSlabBytes + BN / kCtas * 128;
+  constexpr int STAGES = (160 * 1024) / kStageBytes > 8 ? 8 : (160 * 1024) / kStageBytes;
+  constexpr int smem = STAGES * kStageBytes + kStagingBytes + 1024 + (int)sizeof(SmemCtl);
+  const uint32_t tiles_m = NC > 1 ? p.tiles_x : p.tiles_b * p.tiles_y * p.tiles_x;
+  static unsigned attr_done = 0;
+  return launch_tc(conv_tc_fwd_kernel<BN, STAGES, NC, PAIR>, kCtas, (tiles_m + kCtas - 1) / kCtas * p.tiles_n, kFwdThreads, smem, attr_done, s,
+                   ma, mb, mo, p, cl);
 }
 
 int conv_tc_row_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CK, const void* filt, uint32_t OC,
@@ -917,11 +976,16 @@ template <int NC>
 static int run_fwd_tiles(const void* act, uint32_t IH, uint32_t IW, const void* filt, uint32_t all_taps, FwdParams p, const FwdClasses& cl,
                          cudaStream_t s) {
   g_last_conv_kernel = kConvTcGeneral;
+  const uint32_t tiles_m = NC > 1 ? p.tiles_x : p.tiles_b * p.tiles_y * p.tiles_x;
   const int BN = p.OC > 128 ? 256 : (p.OC > 64 ? 128 : (p.OC > 32 ? 64 : 32));
   p.tiles_n = (p.OC + BN - 1) / BN;
   const bool aligned = !((uintptr_t)p.out & 15u) && p.out_pitch % 8 == 0 && p.out_plane % 8 == 0;
   if (!aligned && (p.OC & 7u) == 0) return AD_ERR_ALIGN;
 
+  // Pairs save operand traffic where there is a second pixel tile to share the filter rows with and the contraction is long
+  // enough to be bound by it; short ones are bound by their stores, which single CTAs spread better in time (65,536
+  // pixels, in a net: 256 -> 1024 channels 50 us against 54 as pairs, 512 -> 2048 118 against 144 the other way round).
+  const bool pair = BN == 256 && tiles_m > 1 && all_taps * (p.CK / 64) >= 8;
   CUtensorMap ma, mb;
   {
     uint64_t dims[4] = {p.CK, IW, IH, p.NI};
@@ -934,7 +998,7 @@ static int run_fwd_tiles(const void* act, uint32_t IH, uint32_t IW, const void* 
   {
     uint64_t dims[2] = {(uint64_t)all_taps * p.CK, p.OC};
     uint64_t str[2] = {0, (uint64_t)all_taps * p.CK * 2};
-    uint32_t box[2] = {64, (uint32_t)BN};
+    uint32_t box[2] = {64, (uint32_t)BN / (pair ? 2 : 1)};
     uint32_t es[2] = {1, 1};
     int st = make_tmap_bf16(&mb, filt, 2, dims, str, box, es);
     if (st != AD_OK) return st;
@@ -952,10 +1016,10 @@ static int run_fwd_tiles(const void* act, uint32_t IH, uint32_t IW, const void* 
       if (st != AD_OK) return st;
     }
   switch (BN) {
-    case 256: return launch_fwd<256>(ma, mb, mo, p, cl, s);
-    case 128: return launch_fwd<128>(ma, mb, mo, p, cl, s);
-    case 64: return launch_fwd<64>(ma, mb, mo, p, cl, s);
-    default: return launch_fwd<32>(ma, mb, mo, p, cl, s);
+    case 256: return pair ? launch_fwd<256, NC, true>(ma, mb, mo, p, cl, s) : launch_fwd<256, NC, false>(ma, mb, mo, p, cl, s);
+    case 128: return launch_fwd<128, NC, false>(ma, mb, mo, p, cl, s);
+    case 64: return launch_fwd<64, NC, false>(ma, mb, mo, p, cl, s);
+    default: return launch_fwd<32, NC, false>(ma, mb, mo, p, cl, s);
   }
 }
 
@@ -996,35 +1060,9 @@ static int launch_wgrad(const CUtensorMap& mdy, const CUtensorMap& mx, const WgP
   constexpr int kStageBytes = 2 * kSlabBytes + (BN / 64 / kCtas) * kSlabBytes;
   constexpr int STAGES = (200 * 1024) / kStageBytes;
   constexpr int smem = STAGES * kStageBytes + 1024 + (int)sizeof(SmemCtl);
-  auto kern = conv_tc_wgrad_kernel<BN, STAGES, PAIR>;
-  static unsigned attr_done = 0;  // one bit per device: the attribute is per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(attr_done & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-      cudaGetLastError();
-      return AD_ERR_CUDA;
-    }
-    attr_done |= 1u << (dev & 31);
-  }
-  const uint32_t items = p.splits * p.kh * p.kw * (p.ktiles / kCtas) * p.ctiles;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(std::min(items, (uint32_t)kNumSMs / kCtas) * kCtas);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = kCtas;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = PAIR ? 1 : 0;
-  if (cudaLaunchKernelEx(&cfg, kern, mdy, mx, p) != cudaSuccess) {
-    cudaGetLastError();
-    return AD_ERR_CUDA;
-  }
-  count_launch();
-  return launch_status();
+  static unsigned attr_done = 0;
+  return launch_tc(conv_tc_wgrad_kernel<BN, STAGES, PAIR>, kCtas, p.splits * p.kh * p.kw * (p.ktiles / kCtas) * p.ctiles, kThreads, smem,
+                   attr_done, s, mdy, mx, p);
 }
 
 // Input channels per CTA of the general filter-gradient kernel.  (A 256-wide tile halves the L2 fetches of the dy
@@ -1152,7 +1190,7 @@ static int conv_tc_dgrad_strided(const ad_conv2d_args* a, const Geo& g, const vo
       FwdClass& k = cl.c[c] = all[i + c];
       k.tiles_y = (k.OP + p.TH - 1) / p.TH; k.tiles_x = (k.OQ + p.TW - 1) / p.TW;
       k.tile0 = p.tiles_x;
-      p.tiles_x += (a->N + p.TN - 1) / p.TN * k.tiles_y * k.tiles_x;
+      p.tiles_x += ((a->N + p.TN - 1) / p.TN * k.tiles_y * k.tiles_x + 1) & ~1u;   // both tiles of a pair are of one class
     }
     const int st = run_fwd_tiles<kFwdClasses>(dy, g.P, g.Q, wt, a->kh * a->kw, p, cl, s);
     if (st != AD_OK) return st;

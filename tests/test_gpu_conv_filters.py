@@ -54,16 +54,16 @@ def test_filter_gradient_order(K, Cc, k, accumulate):
     scratch, status = torch.zeros(sb, dtype=torch.uint8, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
     a.x, a.y, a.scratch, a.scratch_bytes, a.accumulate = x.data_ptr(), dy.data_ptr(), scratch.data_ptr(), sb, accumulate
     old = torch.randn(K, k, k, Cc, device="cuda")
-    krsc, kcrs = old.clone(), old.permute(0, 3, 1, 2).contiguous()
+    krsc, kcrs = old.clone(), old.permute(0, 3, 1, 2).clone(memory_format=torch.contiguous_format)
     for out, order in ((krsc, 0), (kcrs, 1)):
         a.dw, a.dw_kcrs = out.data_ptr(), order
         abi.check(L.ad_conv2d_wgrad_ex(C.byref(a), H.ptr(status), H.stream()))
     H.sync()
     assert int(status[0]) == 0 and torch.equal(kcrs, krsc.permute(0, 3, 1, 2))
-    d = dy.double().reshape(-1, K).T
-    want = torch.stack([torch.stack([d @ x[:, r:r + P, s:s + P].double().reshape(-1, Cc) for s in range(k)], 1) for r in range(k)], 1)
-    want += accumulate * old.double()
-    assert (krsc - want).abs().max() < 1e-4 * want.abs().max()
+    x, d = x.cpu().double(), dy.cpu().double().reshape(-1, K).T
+    want = torch.stack([torch.stack([d @ x[:, r:r + P, s:s + P].reshape(-1, Cc) for s in range(k)], 1) for r in range(k)], 1)
+    want += accumulate * old.cpu().double()
+    assert (krsc.cpu() - want).abs().max() < 1e-4 * want.abs().max()
 
 
 @pytest.mark.parametrize("case", [
@@ -106,3 +106,30 @@ def test_strided_data_gradient(case, accumulate):
     got = orc.nhwc_to_nchw(H.host(dx))
     assert H.max_rel(got[..., lo:lo + n] - 3.0 * accumulate, want[..., lo:lo + n]) < 2e-2
     assert np.all(got[..., :lo] == 3.0) and np.all(got[..., lo + n:] == 3.0)
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, K, k: long contractions and more than 128 output channels run as CTA pairs
+    (1, 512, 9, 29, 256, 1), (3, 512, 11, 13, 200, 1),     # an odd number of pixel tiles; ragged channels (scattered stores)
+    (2, 128, 21, 20, 264, 3), (1, 1024, 16, 16, 520, 1),   # several channel tiles, the last one ragged
+    (1, 512, 8, 16, 256, 1),                               # a single pixel tile: no pair
+])
+@pytest.mark.parametrize("bias", [0, 1])
+def test_forward_pairs(case, bias):
+    import torch
+    N, Cc, Hh, W, K, k = case
+    L = abi.lib()
+    a = abi.Conv2dArgs()
+    a.dtype, a.layout = abi.AD_BF16, abi.AD_NHWC
+    a.N, a.C, a.H, a.W, a.K, a.kh, a.kw = N, Cc, Hh, W, K, k, k
+    a.stride_h = a.stride_w = a.dil_h = a.dil_w = 1
+    x, w, b = (torch.randn(*n, device="cuda") for n in ((N, Hh, W, Cc), (K, k, k, Cc), (K,)))
+    x, w = x.bfloat16(), w.bfloat16()
+    y = torch.full((N, Hh - k + 1, W - k + 1, K), 3.0, dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    a.x, a.w, a.y, a.bias = x.data_ptr(), w.data_ptr(), y.data_ptr(), b.data_ptr() if bias else None
+    a.scratch, a.scratch_bytes = status.data_ptr(), 16
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    H.sync()
+    want = torch.nn.functional.conv2d(x.cpu().float().permute(0, 3, 1, 2), w.cpu().float().permute(0, 3, 1, 2), b.cpu() if bias else None)
+    assert int(status[0]) == 0 and (y.cpu().float() - want.permute(0, 2, 3, 1)).abs().max() < 8e-3 * want.abs().max()
