@@ -139,6 +139,16 @@ struct SmemCtl {
   volatile int abort_flag;
 };
 
+// End of a CTA pair's producer: every stage has been given back.  The arrivals come from the other CTA, so a CTA must not
+// leave (and its shared memory must not go to another one) before they are there.
+template <int STAGES>
+__device__ __forceinline__ void await_stages(SmemCtl* ctl, uint32_t stage, uint32_t phase, volatile int* abortf) {
+  for (int i = 0; i < STAGES; ++i) {
+    if (!mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1u, abortf)) return;
+    if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+  }
+}
+
 __device__ __forceinline__ uint32_t pow2_cols(uint32_t c) {
   uint32_t p = 32;
   while (p < c) p <<= 1;
@@ -183,13 +193,14 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (p.tma_store)
       for (uint32_t c = 0; c < (NC > 1 ? cl.n : 1u); ++c) tma_prefetch_desc(&out.map[c]);
   }
+  if (PAIR) cluster_sync();   // the other CTA runs and its barriers are initialised
   if (warp == 1) {
     if (PAIR) { tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish(); }
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync();   // the other CTA's barriers are initialised
+  if (PAIR) cluster_sync();   // both have their tensor memory
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
@@ -226,6 +237,7 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         if (!ok) break;
       }
     }
+      if (PAIR) await_stages<STAGES>(ctl, stage, phase, abortf);
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
       constexpr uint32_t idesc = idesc_bf16(BN, 0, 0, 128 * kCtas);
@@ -430,6 +442,7 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     else tmem_dealloc(tmem_base, kTmemCols);
   }
 }
+  if (PAIR) cluster_sync();   // the release concerns both CTAs
 
 // ---------------------------------------------------------------- filter gradient
 struct WgParams {
@@ -495,12 +508,13 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
     tma_prefetch_desc(&map_x);
   }
   if (warp == 1) {
+  if (PAIR) cluster_sync();   // the other CTA runs and its barriers are initialised
     if (PAIR) { tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish(); }
   }
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync();   // the other CTA's barriers are initialised
+  if (PAIR) cluster_sync();   // both have their tensor memory
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
@@ -535,6 +549,7 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
       }
     }
   } else if (warp == 1) {
+      if (PAIR) await_stages<STAGES>(ctl, stage, phase, abortf);
     if (lane == 0 && rank == 0) {
       constexpr uint32_t idesc = idesc_bf16(BN, 1, 1, 128 * kCtas);
       uint32_t stage = 0, phase = 0, it = 0;
@@ -618,6 +633,7 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
   }
 }
 
+  if (PAIR) cluster_sync();   // the release concerns both CTAs
 // dw (+)= sum over splits of partial[s][k][tap][c], fixed order: lane l of four sums splits l, l+4, ... (8 loads of 16 bytes in
 // flight), the lanes are combined in order.  The partials were written by the kernel before, so this is bound by L2 latency.
 __device__ __forceinline__ float4 wgrad_lane_sum(const float* src, size_t part_stride, uint32_t splits, uint32_t lane) {
