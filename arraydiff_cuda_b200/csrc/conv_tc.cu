@@ -236,8 +236,8 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
         if (!ok) break;
       }
-    }
       if (PAIR) await_stages<STAGES>(ctl, stage, phase, abortf);
+    }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
       constexpr uint32_t idesc = idesc_bf16(BN, 0, 0, 128 * kCtas);
@@ -441,8 +441,8 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     if (PAIR) tmem_dealloc_pair(tmem_base, kTmemCols);
     else tmem_dealloc(tmem_base, kTmemCols);
   }
-}
   if (PAIR) cluster_sync();   // the release concerns both CTAs
+}
 
 // ---------------------------------------------------------------- filter gradient
 struct WgParams {
@@ -507,8 +507,8 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
     tma_prefetch_desc(&map_dy);
     tma_prefetch_desc(&map_x);
   }
-  if (warp == 1) {
   if (PAIR) cluster_sync();   // the other CTA runs and its barriers are initialised
+  if (warp == 1) {
     if (PAIR) { tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish_pair(); }
     else { tmem_alloc(smem_u32(&ctl->tmem_base), kTmemCols); tmem_relinquish(); }
   }
@@ -547,9 +547,9 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
+      if (PAIR) await_stages<STAGES>(ctl, stage, phase, abortf);
     }
   } else if (warp == 1) {
-      if (PAIR) await_stages<STAGES>(ctl, stage, phase, abortf);
     if (lane == 0 && rank == 0) {
       constexpr uint32_t idesc = idesc_bf16(BN, 1, 1, 128 * kCtas);
       uint32_t stage = 0, phase = 0, it = 0;
@@ -631,9 +631,9 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
     if (PAIR) tmem_dealloc_pair(tmem_base, kTmemCols);
     else tmem_dealloc(tmem_base, kTmemCols);
   }
+  if (PAIR) cluster_sync();   // the release concerns both CTAs
 }
 
-  if (PAIR) cluster_sync();   // the release concerns both CTAs
 // dw (+)= sum over splits of partial[s][k][tap][c], fixed order: lane l of four sums splits l, l+4, ... (8 loads of 16 bytes in
 // flight), the lanes are combined in order.  The partials were written by the kernel before, so this is bound by L2 latency.
 __device__ __forceinline__ float4 wgrad_lane_sum(const float* src, size_t part_stride, uint32_t splits, uint32_t lane) {
