@@ -54,6 +54,7 @@ __device__ __forceinline__ void bn_term(const BnRed& p, uint32_t n, uint32_t c, 
 // NCHW-like: block (256) per (channel, split); threads stride over (n, y, x).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) bn_reduce_xfast(BnRed p, float* partial) {
+  grid_dependency();
   const uint32_t c = blockIdx.x, split = blockIdx.y, nsplit = gridDim.y;
   const size_t per = (size_t)p.N * p.H * p.W;
   float a = 0.f, b = 0.f;
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(256) bn_reduce_xfast(BnRed p, float* partial) 
 // NHWC-like: block (32 channels x 8 pixel lanes) per (channel group, split).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) bn_reduce_cfast(BnRed p, float* partial) {
+  grid_dependency();
   const uint32_t c = blockIdx.x * 32 + threadIdx.x, split = blockIdx.y, nsplit = gridDim.y;
   const size_t per = (size_t)p.N * p.H * p.W;
   float a = 0.f, b = 0.f;
@@ -136,6 +138,7 @@ __device__ __forceinline__ void bn_finish_channel(const BnFin& f, uint32_t c, do
 // serial sum of 32 lanes it took 5.6 us, this form 3.3 us at 256 channels.
 constexpr uint32_t kFinishThreads = 512, kFinishRows = 10;
 __global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit, const float* __restrict__ partial) {
+  grid_dependency();
   const uint32_t v = threadIdx.x & 15, rl = threadIdx.x >> 4, which = v >> 3, c = blockIdx.x * 8 + (v & 7);
   double t = 0.0;
   if (c < f.C) {
@@ -180,6 +183,7 @@ struct BnApply {
 // MODE 1: dx (+)= gamma*invstd*(g - mean(g) - xhat*mean(g*xhat))
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) bn_apply(BnApply p) {
+  grid_dependency();
   const size_t total = (size_t)p.N * p.C * p.H * p.W, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
     uint32_t n, c, y, x;
@@ -241,6 +245,7 @@ constexpr int kBnDepth = 8;       // loads in flight per thread and stream
 // registers; 16 in flight gained nothing more.
 template <int MODE>
 __global__ void __launch_bounds__(256, 2) bn_reduce_vec(BnRed p, float* partial) {
+  grid_dependency();
   extern __shared__ __align__(128) uint4 ring_smem[];
   LoadRing<MODE + 1, kBnDepth> ring(ring_smem);
   const uint32_t G = p.C / 8, cg = threadIdx.x % G, pl = threadIdx.x / G, PL = 256 / G;
@@ -303,6 +308,7 @@ __global__ void __launch_bounds__(256, 2) bn_reduce_vec(BnRed p, float* partial)
 // 78 -> 62 us (MODE 1, 6.5 TB/s) against batches of 3-4 loads in registers.
 template <int MODE, bool ADD>
 __global__ void __launch_bounds__(256, 2) bn_apply_vec(BnApply p) {
+  grid_dependency();
   extern __shared__ __align__(128) uint4 ring_smem[];
   LoadRing<MODE + 1 + ADD, kBnDepth> ring(ring_smem);
   const uint32_t G = p.C / 8, cg = threadIdx.x % G, pl = threadIdx.x / G, PL = 256 / G;
@@ -373,10 +379,10 @@ static unsigned vec_grid(const ad_tensor4* t) {
 static int ring_smem_failed() { cudaGetLastError(); return AD_ERR_CUDA; }
 template <int MODE, bool ADD>
 static int launch_apply_vec(const BnApply& a, cudaStream_t s) {
-  constexpr int smem = LoadRing<MODE + 1 + ADD, kBnDepth>::kBytes;
+  constexpr int smem = LoadRing<MODE + 1 + ADD, kBnDepth>::kSmem;
   if (cudaFuncSetAttribute(bn_apply_vec<MODE, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return ring_smem_failed();
   const uint32_t PL = 256 / (a.C / 8), per = a.N * a.H * a.W;
-  bn_apply_vec<MODE, ADD><<<grid_for(per, PL * kBnUnroll, 2), 256, smem, s>>>(a);
+  launch(bn_apply_vec<MODE, ADD>, grid_for(per, PL * kBnUnroll, 2), 256, smem, s, a);
   return AD_OK;
 }
 
@@ -393,7 +399,7 @@ static int pick_splits(const ad_tensor4* x, bool cfast) {
 }
 
 static void launch_finish(const BnFin& f, int nsplit, const float* partial, cudaStream_t s) {
-  bn_finish<<<(f.C + 7) / 8, kFinishThreads, 0, s>>>(f, nsplit, partial);
+  launch(bn_finish, (f.C + 7) / 8, kFinishThreads, 0, s, f, nsplit, partial);
   count_launch();
 }
 // Both stages of the statistics of x (MODE 0) or of the backward sums (MODE 1) into what `f` names
@@ -403,18 +409,18 @@ static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, fl
   int nsplit;
   if (vec_view_ok(x) && (MODE == 0 || (p.dy.sc == 1 && !((uintptr_t)p.dy.base & 15u) && !(p.dy.sn & 7) && !(p.dy.sy & 7) && !(p.dy.sx & 7)))) {
     nsplit = (int)vec_grid(x);
-    constexpr int smem = LoadRing<MODE + 1, kBnDepth>::kBytes;
+    constexpr int smem = LoadRing<MODE + 1, kBnDepth>::kSmem;
     // the attribute is per function and per device; setting it is cheap enough to do per launch
     if (cudaFuncSetAttribute(bn_reduce_vec<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return ring_smem_failed();
-    bn_reduce_vec<MODE><<<nsplit, 256, smem, s>>>(p, partial);
+    launch(bn_reduce_vec<MODE>, nsplit, 256, smem, s, p, partial);
   } else {
     nsplit = pick_splits(x, cfast);
     if (cfast) {
       dim3 grid((x->C + 31) / 32, nsplit), block(32, 8);
-      AD_DISPATCH_DTYPE(x->dtype, (bn_reduce_cfast<T, MODE><<<grid, block, 0, s>>>(p, partial)));
+      AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_cfast<T, MODE>, grid, block, 0, s, p, partial)));
     } else {
       dim3 grid(x->C, nsplit);
-      AD_DISPATCH_DTYPE(x->dtype, (bn_reduce_xfast<T, MODE><<<grid, 256, 0, s>>>(p, partial)));
+      AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_xfast<T, MODE>, grid, 256, 0, s, p, partial)));
     }
   }
   count_launch();
@@ -448,6 +454,7 @@ __device__ __forceinline__ uint32_t window_argmax(const PoolP& p, uint32_t n, ui
 
 template <typename T>
 __global__ void __launch_bounds__(256) maxpool_fwd_kernel(PoolP p) {
+  grid_dependency();
   const size_t total = (size_t)p.N * p.C * p.P * p.Q, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
     uint32_t n, c, q, s;
@@ -467,6 +474,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_kernel(PoolP p) {
 // contributes iff its first maximum is this element.  No atomics -> reproducible.
 template <typename T>
 __global__ void __launch_bounds__(256) maxpool_bwd_kernel(PoolP p) {
+  grid_dependency();
   const size_t total = (size_t)p.N * p.C * p.H * p.W, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
     uint32_t n, c, y, x;
@@ -518,6 +526,7 @@ __device__ __forceinline__ void argmax8(uint4& best, uint4& pos, const uint4& v,
 // K x K windows, or any extents (K = 0)
 template <int K>
 __global__ void __launch_bounds__(256) maxpool_fwd_vec(PoolP p) {
+  grid_dependency();
   const uint32_t G = p.C / 8, kh = K ? K : p.kh, kw = K ? K : p.kw;
   const size_t total = (size_t)p.N * p.P * p.Q * G, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -551,6 +560,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_vec(PoolP p) {
 }
 // one thread per input pixel x 8 channels; gathers from the (at most ceil(kh/sh) x ceil(kw/sw)) windows over it
 __global__ void __launch_bounds__(256) maxpool_bwd_vec(PoolP p) {
+  grid_dependency();
   const uint32_t G = p.C / 8;
   const size_t total = (size_t)p.N * p.H * p.W * G, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -606,6 +616,7 @@ constexpr uint32_t kPoolTile = 16, kPoolMaxWin = 400;
 // K x K windows of stride S, or any extents (K = 0)
 template <int K, int S>
 __global__ void __launch_bounds__(256) maxpool_bwd_tile(PoolP p, uint32_t gchunks) {
+  grid_dependency();
   extern __shared__ uint4 win[];       // [window][8 groups][position, gradient]
   __shared__ uint32_t codes[256];      // position t < kh * kw as a bf16 in both halves
   const uint32_t kh = K ? K : p.kh, kw = K ? K : p.kw, sh = K ? S : p.sh, sw = K ? S : p.sw;
@@ -707,7 +718,7 @@ static int launch_pool_bwd_tile(const PoolP& p, cudaStream_t s) {
     }
     attr_done |= 1u << (dev & 31);
   }
-  maxpool_bwd_tile<K, S><<<grid, 256, pool_windows(p, kPoolTile, kPoolTile) * 256, s>>>(p, gchunks);
+  launch(maxpool_bwd_tile<K, S>, grid, 256, pool_windows(p, kPoolTile, kPoolTile) * 256, s, p, gchunks);
   count_launch();
   return launch_status();
 }
@@ -718,6 +729,7 @@ static int launch_pool_bwd_tile(const PoolP& p, cudaStream_t s) {
 constexpr uint32_t kPlaneTile = 32, kPlaneMaxWin = 2400;
 template <typename T>
 __global__ void __launch_bounds__(256) maxpool_fwd_plane(PoolP p) {
+  grid_dependency();
   const uint32_t tq = (p.P + 7) / 8, ts = (p.Q + 31) / 32;
   uint32_t r = blockIdx.x;
   const uint32_t s = r % ts * 32 + (threadIdx.x & 31); r /= ts;
@@ -735,6 +747,7 @@ __global__ void __launch_bounds__(256) maxpool_fwd_plane(PoolP p) {
 }
 template <typename T, int K, int S>
 __global__ void __launch_bounds__(256) maxpool_bwd_plane(PoolP p) {
+  grid_dependency();
   extern __shared__ float2 wpl[];      // per window: position (whole number), gradient
   const uint32_t kh = K ? K : p.kh, kw = K ? K : p.kw, sh = K ? S : p.sh, sw = K ? S : p.sw;
   const uint32_t ty = (p.H + kPlaneTile - 1) / kPlaneTile, tx = (p.W + kPlaneTile - 1) / kPlaneTile;
@@ -820,7 +833,7 @@ static int launch_apply(const BnApply& a, const ad_tensor4* x, bool vec, cudaStr
     if (rc != AD_OK) return rc;
   } else {
     const size_t total = (size_t)x->N * x->C * x->H * x->W;
-    AD_DISPATCH_DTYPE(x->dtype, (bn_apply<T, MODE><<<grid_for(total, 256, 16), 256, 0, s>>>(a)));
+    AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply<T, MODE>, grid_for(total, 256, 16), 256, 0, s, a)));
   }
   count_launch();
   return launch_status();
@@ -865,6 +878,7 @@ extern "C" int ad_bn_fwd_train(const ad_tensor4* x, const ad_tensor4* y, const f
 
 // invstd[c] = 1 / sqrt(var[c] + eps), in double as the training path does
 __global__ void bn_invstd_kernel(uint32_t C, const float* __restrict__ var, float eps, float* __restrict__ invstd) {
+  grid_dependency();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < C) invstd[c] = (float)(1.0 / sqrt((double)var[c] + (double)eps));
 }
@@ -877,7 +891,7 @@ extern "C" int ad_bn_fwd_inference(const ad_tensor4* x, const ad_tensor4* y, con
   const size_t total = (size_t)x->N * x->C * x->H * x->W;
   if (total == 0) return AD_OK;
   cudaStream_t s = as_stream(stream);
-  bn_invstd_kernel<<<(x->C + 255) / 256, 256, 0, s>>>(x->C, var, eps, invstd_out);
+  launch(bn_invstd_kernel, (x->C + 255) / 256, 256, 0, s, x->C, var, eps, invstd_out);
   count_launch();
   BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, mean, invstd_out, nullptr, 1, (double)x->N * x->H * x->W};
@@ -938,13 +952,13 @@ extern "C" int ad_maxpool2d_fwd(const ad_tensor4* x, const ad_tensor4* y, uint32
   if (total == 0) return AD_OK;
   cudaStream_t cs = as_stream(stream);
   if (pool_vec_ok(x) && pool_vec_ok(y)) {
-    if (kh == 3 && kw == 3) maxpool_fwd_vec<3><<<grid_for(total / 8, 256, 16), 256, 0, cs>>>(p);
-    else if (kh == 2 && kw == 2) maxpool_fwd_vec<2><<<grid_for(total / 8, 256, 16), 256, 0, cs>>>(p);
-    else maxpool_fwd_vec<0><<<grid_for(total / 8, 256, 16), 256, 0, cs>>>(p);
+    if (kh == 3 && kw == 3) launch(maxpool_fwd_vec<3>, grid_for(total / 8, 256, 16), 256, 0, cs, p);
+    else if (kh == 2 && kw == 2) launch(maxpool_fwd_vec<2>, grid_for(total / 8, 256, 16), 256, 0, cs, p);
+    else launch(maxpool_fwd_vec<0>, grid_for(total / 8, 256, 16), 256, 0, cs, p);
   } else if (pool_plane_ok(p, x, y, nullptr, false)) {
     const unsigned grid = (unsigned)((size_t)p.N * p.C * ((p.P + 7) / 8) * ((p.Q + 31) / 32));
-    AD_DISPATCH_DTYPE(x->dtype, (maxpool_fwd_plane<T><<<grid, 256, 0, cs>>>(p)));
-  } else AD_DISPATCH_DTYPE(x->dtype, (maxpool_fwd_kernel<T><<<grid_for(total, 256, 16), 256, 0, as_stream(stream)>>>(p)));
+    AD_DISPATCH_DTYPE(x->dtype, (launch(maxpool_fwd_plane<T>, grid, 256, 0, cs, p)));
+  } else AD_DISPATCH_DTYPE(x->dtype, (launch(maxpool_fwd_kernel<T>, grid_for(total, 256, 16), 256, 0, as_stream(stream), p)));
   count_launch();
   return launch_status();
 }
@@ -970,14 +984,14 @@ extern "C" int ad_maxpool2d_bwd(const ad_tensor4* x, const ad_tensor4* dy, const
     if (kh == 2 && kw == 2 && sh == 2 && sw == 2) return launch_pool_bwd_tile<2, 2>(p, cs);
     return launch_pool_bwd_tile<0, 0>(p, cs);
   }
-  if (vec) maxpool_bwd_vec<<<grid_for(total / 8, 256, 16), 256, 0, cs>>>(p);
+  if (vec) launch(maxpool_bwd_vec, grid_for(total / 8, 256, 16), 256, 0, cs, p);
   else if (pool_plane_ok(p, x, dy, dx, true)) {
     const unsigned grid = (unsigned)((size_t)p.N * p.C * ((p.H + kPlaneTile - 1) / kPlaneTile) * ((p.W + kPlaneTile - 1) / kPlaneTile));
     const size_t smem = pool_windows(p, kPlaneTile, kPlaneTile) * sizeof(float2);
-    if (kh == 3 && kw == 3 && sh == 2 && sw == 2) AD_DISPATCH_DTYPE(x->dtype, (maxpool_bwd_plane<T, 3, 2><<<grid, 256, smem, cs>>>(p)));
-    else AD_DISPATCH_DTYPE(x->dtype, (maxpool_bwd_plane<T, 0, 0><<<grid, 256, smem, cs>>>(p)));
+    if (kh == 3 && kw == 3 && sh == 2 && sw == 2) AD_DISPATCH_DTYPE(x->dtype, (launch(maxpool_bwd_plane<T, 3, 2>, grid, 256, smem, cs, p)));
+    else AD_DISPATCH_DTYPE(x->dtype, (launch(maxpool_bwd_plane<T, 0, 0>, grid, 256, smem, cs, p)));
   }
-  else AD_DISPATCH_DTYPE(x->dtype, (maxpool_bwd_kernel<T><<<grid_for(total, 256, 16), 256, 0, cs>>>(p)));
+  else AD_DISPATCH_DTYPE(x->dtype, (launch(maxpool_bwd_kernel<T>, grid_for(total, 256, 16), 256, 0, cs, p)));
   count_launch();
   return launch_status();
 }

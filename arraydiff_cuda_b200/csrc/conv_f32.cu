@@ -101,6 +101,7 @@ template <int LM, int WM, int WN> struct GemmTile : F32Tile<LM, WM, WN, 1> {
 
 template <int LM, int WM, int WN, bool DGRAD>
 __global__ void __launch_bounds__(kF32Group, 3) conv_gemm_f32(const GemmF32 p) {
+  grid_dependency();
   typedef GemmTile<LM, WM, WN> T;
   constexpr int BM = T::BM, BN = T::BN, LN = T::LN, KB = T::KB, PA = T::PA, STAGES = T::stages;
   constexpr int NPX = BN / kF32Group;                                          // pixels a thread gathers for
@@ -326,8 +327,8 @@ static int launch_f32(Kernel k, dim3 grid, int threads, int smem, uint32_t cs, c
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
   cfg.numAttrs = cs > 1 ? 1 : 0;
+  cfg.attrs = at;
   if (cudaLaunchKernelEx(&cfg, k, p) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
   count_launch();
   return launch_status();
@@ -388,6 +389,7 @@ template <int LM, int WM, int WN, int G> struct WgTile : F32Tile<LM, WM, WN, G> 
 
 template <int LM, int WM, int WN, int G>
 __global__ void __launch_bounds__(kF32Group * G, G == 1 ? 2 : 1) conv_wgrad_gemm_f32(const WgradF32 p) {
+  grid_dependency();
   typedef WgTile<LM, WM, WN, G> T;
   constexpr int BM = T::BM, BN = T::BN, LN = T::LN, STAGES = kWgStages, PITCH = kWgPitch, KB = kWgKB;
   extern __shared__ __align__(16) float sm[];
@@ -524,6 +526,7 @@ __global__ void __launch_bounds__(kF32Group * G, G == 1 ? 2 : 1) conv_wgrad_gemm
 // dw (+)= sum of the slices, in order; the bias gradient's K values follow the filter's
 __global__ void __launch_bounds__(256) wgrad_f32_finish(size_t n, uint32_t K, uint32_t slices, const float* __restrict__ part, float* dw,
                                                         float* db, int accumulate) {
+  grid_dependency();
   const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x, stride = n + K;
   if (i >= (db ? stride : n)) return;
   float v[16], t = 0.f;
@@ -557,7 +560,7 @@ static int launch_wgrad_f32(WgradF32& p, cudaStream_t s) {
   int st = launch_f32(conv_wgrad_gemm_f32<LM, WM, WN, G>, dim3(tn * cs, tm, p.slices), T::threads, T::smem, cs, p, attr_done, s);
   if (st != AD_OK || p.slices == 1) return st;
   const size_t n = (size_t)p.K * p.C * p.kh * p.kw;
-  wgrad_f32_finish<<<(unsigned)((n + p.K + 255) / 256), 256, 0, s>>>(n, p.K, p.slices, p.part, p.dw, p.db, p.accumulate);
+  launch(wgrad_f32_finish, (unsigned)((n + p.K + 255) / 256), 256, 0, s, n, p.K, p.slices, p.part, p.dw, p.db, p.accumulate);
   count_launch();
   return launch_status();
 }

@@ -202,6 +202,7 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   __syncthreads();
   if (PAIR) cluster_sync();   // both have their tensor memory
   tc_fence_after();
+  grid_dependency();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -516,6 +517,7 @@ conv_tc_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_co
   __syncthreads();
   if (PAIR) cluster_sync();   // both have their tensor memory
   tc_fence_after();
+  grid_dependency();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -654,6 +656,7 @@ __device__ __forceinline__ float4 wgrad_lane_sum(const float* src, size_t part_s
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(size_t n, size_t part_stride, uint32_t splits,
                                                            const float* __restrict__ partial, float* dw, int accumulate,
                                                            uint32_t taps, uint32_t C, int kcrs) {
+  grid_dependency();
   const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6;
   const size_t i = ((size_t)blockIdx.x * 64 + tx) * 4;
   __shared__ float4 sh[4][64];
@@ -678,6 +681,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(size_t n, size_t part
 constexpr uint32_t kWgRedPitch = 36;
 __global__ void wgrad_reduce_kcrs_kernel(size_t part_stride, uint32_t splits, const float* __restrict__ partial, float* dw,
                                          int accumulate, uint32_t taps, uint32_t C) {
+  grid_dependency();
   extern __shared__ float wr[];   // [4][taps][kWgRedPitch]
   const uint32_t ctiles = C / 32, k = blockIdx.x / ctiles, c0 = blockIdx.x % ctiles * 32, items = taps * 8;
   for (uint32_t w = threadIdx.x; w < items * 4; w += blockDim.x) {
@@ -700,9 +704,9 @@ static void launch_wgrad_reduce(uint32_t K, uint32_t taps, uint32_t C, size_t pa
   const size_t n = (size_t)K * taps * C, smem = (size_t)4 * taps * kWgRedPitch * 4;
   if (kcrs && taps > 1 && smem <= 48 * 1024) {   // more taps than shared memory holds (over 85) take the form below
     const uint32_t threads = std::min((taps * 32 + 31) / 32 * 32, 512u);
-    wgrad_reduce_kcrs_kernel<<<K * (C / 32), threads, smem, s>>>(part_stride, splits, partial, dw, accumulate, taps, C);
+    launch(wgrad_reduce_kcrs_kernel, K * (C / 32), threads, smem, s, part_stride, splits, partial, dw, accumulate, taps, C);
   } else {
-    wgrad_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, part_stride, splits, partial, dw, accumulate, taps, C, kcrs && taps > 1);
+    launch(wgrad_reduce_kernel, (unsigned)((n + 255) / 256), 256, 0, s, n, part_stride, splits, partial, dw, accumulate, taps, C, kcrs && taps > 1);
   }
   count_launch();
 }
@@ -712,6 +716,7 @@ static void launch_wgrad_reduce(uint32_t K, uint32_t taps, uint32_t C, size_t pa
 __global__ void __launch_bounds__(256) filter_transpose_flip_kernel(uint32_t K, uint32_t Kp, uint32_t kh, uint32_t kw,
                                                                     uint32_t C, const __nv_bfloat16* __restrict__ w,
                                                                     __nv_bfloat16* wt) {
+  grid_dependency();
   const size_t total = (size_t)Kp * kh * kw * C, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
     uint32_t k = (uint32_t)(i % Kp);
@@ -775,6 +780,7 @@ __device__ __forceinline__ void filter_prepare_tile(const PrepItem& p, uint32_t 
   }
 }
 __global__ void __launch_bounds__(256) filter_prepare_kernel(const __grid_constant__ PrepBatch b) {
+  grid_dependency();
   __shared__ float sm[kPrepFloats + 128];
   for (uint32_t tile = blockIdx.x; tile < b.tiles; tile += gridDim.x) {
     uint32_t lo = 0, hi = b.count;   // the last item whose tile0 <= tile: one without tiles shares its tile0 with the next
@@ -793,6 +799,7 @@ __global__ void __launch_bounds__(256) filter_prepare_kernel(const __grid_consta
 // dst[pixel][0..Kp) = src[pixel][0..K), zero past K
 __global__ void __launch_bounds__(256) pad_channels_kernel(size_t pixels, uint32_t K, uint32_t Kp,
                                                            const __nv_bfloat16* __restrict__ src, __nv_bfloat16* dst) {
+  grid_dependency();
   const size_t total = pixels * Kp, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
     const uint32_t k = (uint32_t)(i % Kp);
@@ -814,6 +821,7 @@ __device__ __forceinline__ void bias_add8(float (&acc)[8], const uint4& v) {
   }
 }
 __global__ void __launch_bounds__(256) bias_grad_vec_kernel(size_t pixels, uint32_t K, uint32_t gb, const __nv_bfloat16* __restrict__ dy, float* part) {
+  grid_dependency();
   __shared__ float red[256][9];
   const uint32_t G = K / 8, gl = threadIdx.x % gb, pl = threadIdx.x / gb, PL = 256 / gb, g = blockIdx.y * gb + gl;
   float acc[8];
@@ -846,6 +854,7 @@ __global__ void __launch_bounds__(256) bias_grad_vec_kernel(size_t pixels, uint3
 // other channel counts (a 19-class head): a thread per channel and pixel lane
 __global__ void __launch_bounds__(256) bias_grad_nhwc_kernel(size_t pixels, uint32_t K, const __nv_bfloat16* __restrict__ dy,
                                                              float* part) {
+  grid_dependency();
   const uint32_t k = blockIdx.y * 32 + threadIdx.x, split = blockIdx.x, nsplit = gridDim.x;
   const size_t chunk = (pixels + nsplit - 1) / nsplit, lo = (size_t)split * chunk, hi = lo + chunk < pixels ? lo + chunk : pixels;
   float acc = 0.f;
@@ -864,6 +873,7 @@ __global__ void __launch_bounds__(256) bias_grad_nhwc_kernel(size_t pixels, uint
 }
 // a block per 32 channels: 8 lanes of blocks' rows, combined in order
 __global__ void __launch_bounds__(256) bias_grad_finish(uint32_t K, uint32_t nsplit, const float* __restrict__ part, float* db, int accumulate) {
+  grid_dependency();
   __shared__ float red[8][33];
   const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5, k = blockIdx.x * 32 + tx;
   float t = 0.f;
@@ -891,11 +901,11 @@ static void launch_bias_grad(size_t pixels, uint32_t K, const void* dy, float* d
   const uint32_t nsplit = bias_grad_blocks(pixels, K);
   if (K % 8 == 0 && ((uintptr_t)dy & 15u) == 0) {
     const uint32_t gb = K / 8 < 256 ? K / 8 : 256;
-    bias_grad_vec_kernel<<<dim3(nsplit, (K / 8 + gb - 1) / gb), 256, 0, s>>>(pixels, K, gb, (const __nv_bfloat16*)dy, part);
+    launch(bias_grad_vec_kernel, dim3(nsplit, (K / 8 + gb - 1) / gb), 256, 0, s, pixels, K, gb, (const __nv_bfloat16*)dy, part);
   } else {
-    bias_grad_nhwc_kernel<<<dim3(nsplit, (K + 31) / 32), dim3(32, 8), 0, s>>>(pixels, K, (const __nv_bfloat16*)dy, part);
+    launch(bias_grad_nhwc_kernel, dim3(nsplit, (K + 31) / 32), dim3(32, 8), 0, s, pixels, K, (const __nv_bfloat16*)dy, part);
   }
-  bias_grad_finish<<<(K + 31) / 32, 256, 0, s>>>(K, nsplit, part, db, accumulate);
+  launch(bias_grad_finish, (K + 31) / 32, 256, 0, s, K, nsplit, part, db, accumulate);
   count_launch(2);
 }
 
@@ -949,12 +959,12 @@ static int launch_tc(void (*kern)(KArgs...), uint32_t ctas, uint32_t items, int 
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = ctas;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
   cfg.numAttrs = ctas > 1 ? 1 : 0;
+  launch_attr(cfg, at);
   if (cudaLaunchKernelEx(&cfg, kern, KArgs(args)...) != cudaSuccess) {
     cudaGetLastError();
     return AD_ERR_CUDA;
@@ -1230,14 +1240,14 @@ int conv_tc_dgrad(const ad_conv2d_args* a, const void* prepared, int32_t* status
   const size_t wcount = (size_t)Kp * a->kh * a->kw * a->C;
   if (!wt) {
     __nv_bfloat16* made = (__nv_bfloat16*)((char*)a->scratch + 16);
-    filter_transpose_flip_kernel<<<grid_for(wcount, 256), 256, 0, s>>>(a->K, Kp, a->kh, a->kw, a->C, (const __nv_bfloat16*)a->w, made);
+    launch(filter_transpose_flip_kernel, grid_for(wcount, 256), 256, 0, s, a->K, Kp, a->kh, a->kw, a->C, (const __nv_bfloat16*)a->w, made);
     count_launch();
     wt = made;
   }
   const void* dy = a->y;
   if (Kp != a->K) {
     const size_t pixels = (size_t)a->N * g.P * g.Q;
-    pad_channels_kernel<<<grid_for(pixels * Kp, 256, 16), 256, 0, s>>>(pixels, a->K, Kp, (const __nv_bfloat16*)a->y,
+    launch(pad_channels_kernel, grid_for(pixels * Kp, 256, 16), 256, 0, s, pixels, a->K, Kp, (const __nv_bfloat16*)a->y,
                                                                         (__nv_bfloat16*)next);
     count_launch();
     dy = next;
@@ -1272,7 +1282,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
   char* part_base = (char*)a->scratch + 1024;
   if (Kp != a->K) {
     const size_t pixels = (size_t)a->N * g.P * g.Q;
-    pad_channels_kernel<<<grid_for(pixels * Kp, 256, 16), 256, 0, s>>>(pixels, a->K, Kp, (const __nv_bfloat16*)a->y,
+    launch(pad_channels_kernel, grid_for(pixels * Kp, 256, 16), 256, 0, s, pixels, a->K, Kp, (const __nv_bfloat16*)a->y,
                                                                         (__nv_bfloat16*)part_base);
     count_launch();
     dy = part_base;
@@ -1425,7 +1435,7 @@ extern "C" int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream) {
     }
   });
 }
-extern "C" int ad_conv2d_dgrad_ex(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream) {
+static int dgrad_call(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream) {
   return profiled(1, a, stream, [&] {
     switch (path_of(a)) {
       case 0: g_last_conv_kernel = kConvDirectF32; return conv_direct_dgrad(a, as_stream(stream));
@@ -1434,8 +1444,11 @@ extern "C" int ad_conv2d_dgrad_ex(const ad_conv2d_args* a, const void* w_crsk, i
     }
   });
 }
-extern "C" int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream) { return ad_conv2d_dgrad_ex(a, nullptr, nullptr, stream); }
-extern "C" int ad_conv2d_wgrad_ex(const ad_conv2d_args* a, int32_t* status, void* stream) {
+extern "C" int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream) { return dgrad_call(a, nullptr, nullptr, stream); }
+extern "C" int ad_conv2d_dgrad_ex(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream) {
+  return dgrad_call(a, w_crsk, status, stream);
+}
+static int wgrad_call(const ad_conv2d_args* a, int32_t* status, void* stream) {
   return profiled(2, a, stream, [&] {
     switch (path_of(a)) {
       case 0: g_last_conv_kernel = kConvDirectF32; return conv_direct_wgrad(a, as_stream(stream));
@@ -1444,7 +1457,11 @@ extern "C" int ad_conv2d_wgrad_ex(const ad_conv2d_args* a, int32_t* status, void
     }
   });
 }
-extern "C" int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream) { return ad_conv2d_wgrad_ex(a, nullptr, stream); }
+extern "C" int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream) { return wgrad_call(a, nullptr, stream); }
+extern "C" int ad_conv2d_wgrad_ex(const ad_conv2d_args* a, int32_t* status, void* stream) {
+  LateLaunch late;
+  return wgrad_call(a, status, stream);
+}
 
 extern "C" int ad_filter_prepare(uint32_t count, const ad_filter_item* items, void* stream) {
   if (count && !items) return AD_ERR_BAD_ARG;
@@ -1466,8 +1483,7 @@ extern "C" int ad_filter_prepare(uint32_t count, const ad_filter_item* items, vo
         ad_tensor4 dst = {f.krsc, AD_BF16, f.K, f.C, f.kh, f.kw, f.krsc_row, 1, (int64_t)f.kw * f.C, f.C};
         if (int rc = ad_convert(&src, &dst, 0, stream)) return rc;
         if (f.crsk) {
-          tc::filter_transpose_flip_kernel<<<grid_for((size_t)f.C * taps * f.crsk_k, 256), 256, 0, s>>>(
-              f.K, f.crsk_k, f.kh, f.kw, f.C, (const __nv_bfloat16*)f.krsc, (__nv_bfloat16*)f.crsk);
+          launch(tc::filter_transpose_flip_kernel, grid_for((size_t)f.C * taps * f.crsk_k, 256), 256, 0, s, f.K, f.crsk_k, f.kh, f.kw, f.C, (const __nv_bfloat16*)f.krsc, (__nv_bfloat16*)f.crsk);
           count_launch();
         }
         p.tile0 = b.tiles;
@@ -1483,7 +1499,7 @@ extern "C" int ad_filter_prepare(uint32_t count, const ad_filter_item* items, vo
       b.tiles += (p.Kp + p.KT - 1) / p.KT * ((p.C + p.CT - 1) / p.CT);
     }
     if (!b.tiles) continue;
-    tc::filter_prepare_kernel<<<std::min(b.tiles, (uint32_t)kNumSMs * 6), 256, 0, s>>>(b);
+    launch(tc::filter_prepare_kernel, std::min(b.tiles, (uint32_t)kNumSMs * 6), 256, 0, s, b);
     count_launch();
   }
   return launch_status();

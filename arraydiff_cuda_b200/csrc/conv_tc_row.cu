@@ -100,6 +100,7 @@ conv_tc_row_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -376,7 +377,7 @@ int conv_tc_row_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  kern<<<grid, kRowThreads, smem, s>>>(ma, mb, mo, p);
+  launch(kern, grid, kRowThreads, smem, s, ma, mb, mo, p);
   count_launch();
   return launch_status();
 }
@@ -496,6 +497,7 @@ conv_tc_stream_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -888,7 +890,7 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  kern<<<grid, kRowThreads, smem, s>>>(ma, mb, mo, p);
+  launch(kern, grid, kRowThreads, smem, s, ma, mb, mo, p);
   count_launch();
   return launch_status();
 }
@@ -940,6 +942,7 @@ conv_tc_row_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gri
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -1088,6 +1091,7 @@ conv_tc_rows_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gr
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_dependency();
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -1189,6 +1193,7 @@ conv_tc_rows_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gr
 __global__ void __launch_bounds__(256) wgrad_rows_reduce_kernel(uint32_t nparts, uint32_t naccs, uint32_t KO, uint32_t kh,
                                                                 uint32_t kw, const float* __restrict__ partial, float* dw,
                                                                 int accumulate, int kcrs) {
+  grid_dependency();
   const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6;
   const uint32_t cols4 = 16 * kh, item = blockIdx.x * 64 + tx, nitems = naccs * 128 * cols4;
   float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1231,6 +1236,7 @@ __global__ void __launch_bounds__(256) wgrad_rows_reduce_kernel(uint32_t nparts,
 __global__ void __launch_bounds__(256) wgrad_row_reduce_kernel(uint32_t nparts, uint32_t naccs, uint32_t KO, uint32_t kh,
                                                                uint32_t kw, const float* __restrict__ partial, float* dw,
                                                                int accumulate, int kcrs) {
+  grid_dependency();
   const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6;
   const uint32_t item = blockIdx.x * 64 + tx, nitems = naccs * 128 * 16;
   float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1337,9 +1343,9 @@ static int conv_tc_rows_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t 
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  conv_tc_rows_wgrad_kernel<3, 3><<<grid, kRowThreads, smem, s>>>(mdy, mx, p);
+  launch(conv_tc_rows_wgrad_kernel<3, 3>, grid, kRowThreads, smem, s, mdy, mx, p);
   count_launch();
-  wgrad_rows_reduce_kernel<<<(p.naccs * 128 * 16 * kh + 63) / 64, 256, 0, s>>>(grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs);
+  launch(wgrad_rows_reduce_kernel, (p.naccs * 128 * 16 * kh + 63) / 64, 256, 0, s, grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs);
   count_launch();
   return launch_status();
 }
@@ -1395,10 +1401,10 @@ int conv_tc_row_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t IW, uint
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  kern<<<grid, kRowThreads, smem, s>>>(mdy, mx, p);
+  launch(kern, grid, kRowThreads, smem, s, mdy, mx, p);
   count_launch();
   const size_t wcount = (size_t)KO * kh * kw * 64;
-  wgrad_row_reduce_kernel<<<(p.naccs * 128 * 16 + 63) / 64, 256, 0, s>>>(grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs);
+  launch(wgrad_row_reduce_kernel, (p.naccs * 128 * 16 + 63) / 64, 256, 0, s, grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs);
   count_launch();
   return launch_status();
 }

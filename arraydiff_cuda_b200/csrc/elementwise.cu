@@ -6,6 +6,7 @@
 namespace adk {
 
 unsigned long long g_launch_count = 0;
+thread_local bool g_early_launch = true;
 thread_local int g_last_conv_kernel = kConvNone;
 
 // ---------------------------------------------------------------- packed fp32 arrays
@@ -28,6 +29,7 @@ __device__ __forceinline__ float arr_apply(float a, float b, float x, float y) {
 
 template <int OP>
 __global__ void __launch_bounds__(256) arr_kernel(size_t n, float a, float b, const float* __restrict__ x, float* y) {
+  grid_dependency();
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
   const bool vec = (((uintptr_t)y | (uintptr_t)(OP == kSet ? (const float*)y : x)) & 15u) == 0;
   if (vec) {
@@ -51,7 +53,7 @@ template <int OP>
 static int arr_launch(size_t n, float a, float b, const float* x, float* y, void* stream) {
   if (n == 0) return AD_OK;
   if (!y || (OP != kSet && !x)) return AD_ERR_BAD_ARG;
-  arr_kernel<OP><<<grid_for((n + 3) / 4, 256), 256, 0, as_stream(stream)>>>(n, a, b, x, y);
+  launch(arr_kernel<OP>, grid_for((n + 3) / 4, 256), 256, 0, as_stream(stream), n, a, b, x, y);
   count_launch();
   return launch_status();
 }
@@ -60,6 +62,7 @@ static int arr_launch(size_t n, float a, float b, const float* x, float* y, void
 __global__ void __launch_bounds__(256) sgd_kernel(size_t n, float* theta, float* g, float* m, float l2, float mu,
                                                   float alpha, float alpha_next, int nesterov,
                                                   __nv_bfloat16* shadow, const int32_t* guard) {
+  grid_dependency();
   // a step whose bounded waits ran out worked on stale halo rows or gradients: leave the parameters alone
   if (guard && *guard != 0) return;
   const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
@@ -109,6 +112,7 @@ enum EwOp { kRelu, kReluBwd, kAdd2, kConvert };
 
 template <int OP, typename TA, typename TB, typename TY>
 __global__ void __launch_bounds__(256) ew_kernel(Dims d, View a, View b, View yv, int accumulate) {
+  grid_dependency();
   const size_t total = (size_t)d.N * d.C * d.H * d.W;
   const size_t nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -145,6 +149,7 @@ __device__ __forceinline__ long long ew_pix_off(const View& v, uint32_t i, uint3
 constexpr int kEwDepth = 8;
 template <int OP>
 __global__ void __launch_bounds__(256, 2) ew_vec_kernel(Dims d, View a, View b, View yv, int accumulate) {
+  grid_dependency();
   constexpr bool kTwo = OP == kAdd2 || OP == kReluBwd;
   extern __shared__ __align__(128) uint4 ring_smem[];
   LoadRing<2 + kTwo, kEwDepth> ring(ring_smem);
@@ -206,19 +211,19 @@ static int ew_launch(const ad_tensor4* a, const ad_tensor4* b, const ad_tensor4*
   View va = view_of(a), vb = b ? view_of(b) : View{nullptr, 0, 0, 0, 0}, vy = view_of(y);
   cudaStream_t s = as_stream(stream);
   if (total / 8 < (1ull << 31) && ew_vec_ok(a) && ew_vec_ok(y) && (!b || ew_vec_ok(b))) {
-    constexpr int smem = LoadRing<2 + (OP == kAdd2 || OP == kReluBwd), kEwDepth>::kBytes;
+    constexpr int smem = LoadRing<2 + (OP == kAdd2 || OP == kReluBwd), kEwDepth>::kSmem;
     // the attribute is per function and per device; setting it is cheap enough to do per launch
     if (cudaFuncSetAttribute(ew_vec_kernel<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
       cudaGetLastError();
       return AD_ERR_CUDA;
     }
-    ew_vec_kernel<OP><<<grid_for(total / 8, 256, 2), 256, smem, s>>>(d, va, vb, vy, accumulate);
+    launch(ew_vec_kernel<OP>, grid_for(total / 8, 256, 2), 256, smem, s, d, va, vb, vy, accumulate);
     count_launch();
     return launch_status();
   }
   const unsigned grid = grid_for(total, 256, 16);
   const int da = a->dtype, db = b ? b->dtype : a->dtype, dy = y->dtype;
-#define EW_CASE(TA_, TB_, TY_) ew_kernel<OP, TA_, TB_, TY_><<<grid, 256, 0, s>>>(d, va, vb, vy, accumulate)
+#define EW_CASE(TA_, TB_, TY_) launch(ew_kernel<OP, TA_, TB_, TY_>, grid, 256, 0, s, d, va, vb, vy, accumulate)
   using bf = __nv_bfloat16;
   if (da == AD_F32 && db == AD_F32 && dy == AD_F32) EW_CASE(float, float, float);
   else if (da == AD_BF16 && db == AD_BF16 && dy == AD_BF16) EW_CASE(bf, bf, bf);
@@ -281,7 +286,7 @@ extern "C" int ad_sgd_step(size_t n, float* theta, float* g, float* m, float l2,
                            float alpha_next, int32_t nesterov, void* bf16_shadow, void* stream) {
   if (n == 0) return AD_OK;
   if (!theta || !g || !m) return AD_ERR_BAD_ARG;
-  sgd_kernel<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(n, theta, g, m, l2, mu, alpha, alpha_next, nesterov,
+  launch(sgd_kernel, grid_for(n, 256), 256, 0, as_stream(stream), n, theta, g, m, l2, mu, alpha, alpha_next, nesterov,
                                                                (__nv_bfloat16*)bf16_shadow, nullptr);
   count_launch();
   return launch_status();
@@ -291,7 +296,7 @@ extern "C" int ad_sgd_step_guarded(size_t n, float* theta, float* g, float* m, f
                                    void* stream) {
   if (n == 0) return AD_OK;
   if (!theta || !g || !m) return AD_ERR_BAD_ARG;
-  sgd_kernel<<<grid_for(n, 256), 256, 0, as_stream(stream)>>>(n, theta, g, m, l2, mu, alpha, alpha_next, nesterov,
+  launch(sgd_kernel, grid_for(n, 256), 256, 0, as_stream(stream), n, theta, g, m, l2, mu, alpha, alpha_next, nesterov,
                                                                (__nv_bfloat16*)bf16_shadow, status_word);
   count_launch();
   return launch_status();
@@ -317,6 +322,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) im2col_kernel(View x, uint32_t N, uint32_t C, uint32_t H, uint32_t W, uint32_t kh,
                                                      uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw,
                                                      uint32_t P, uint32_t Q, __nv_bfloat16* out, uint32_t ldo) {
+  grid_dependency();
   const uint32_t cols = kh * kw * C;
   const size_t total = (size_t)N * P * Q * cols, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -337,6 +343,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) im2col_vec_kernel(View x, uint32_t N, uint32_t C, uint32_t H, uint32_t W, uint32_t kh,
                                                          uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw,
                                                          uint32_t P, uint32_t Q, __nv_bfloat16* out, uint32_t ldo) {
+  grid_dependency();
   const uint32_t cols = kh * kw * C, groups = ldo / 8;
   const size_t total = (size_t)N * P * Q * groups, nt = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -372,6 +379,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) im2col_row_kernel(View x, uint32_t C, uint32_t H, uint32_t W, uint32_t kh, uint32_t kw,
                                                          uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, uint32_t P,
                                                          uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen) {
+  grid_dependency();
   extern __shared__ __align__(16) unsigned char im2col_smem[];
   __nv_bfloat16* rows = (__nv_bfloat16*)im2col_smem;                                    // [kh][rowlen]
   uint32_t* tab = (uint32_t*)(im2col_smem + (((size_t)kh * rowlen * 2 + 15) & ~(size_t)15));  // [ldo]
@@ -419,7 +427,7 @@ static int launch_im2col_row(const View& v, const ad_tensor4* x, uint32_t kh, ui
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  kern<<<x->N * P, 256, smem, s>>>(v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, out, ldo, rowlen);
+  launch(kern, x->N * P, 256, smem, s, v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, out, ldo, rowlen);
   return AD_OK;
 }
 }  // namespace adk
@@ -444,13 +452,11 @@ extern "C" int ad_im2col(const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t
       return adk::launch_status();
     }
     const size_t tv = (size_t)x->N * P * Q * (ldo / 8);
-    AD_DISPATCH_DTYPE(x->dtype, (adk::im2col_vec_kernel<T><<<adk::grid_for(tv, 256, 16), 256, 0, adk::as_stream(stream)>>>(
-                                    v, x->N, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo)));
+    AD_DISPATCH_DTYPE(x->dtype, (launch(adk::im2col_vec_kernel<T>, adk::grid_for(tv, 256, 16), 256, 0, adk::as_stream(stream), v, x->N, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo)));
     adk::count_launch();
     return adk::launch_status();
   }
-  AD_DISPATCH_DTYPE(x->dtype, (adk::im2col_kernel<T><<<adk::grid_for(total, 256, 16), 256, 0, adk::as_stream(stream)>>>(
-                                  v, x->N, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo)));
+  AD_DISPATCH_DTYPE(x->dtype, (launch(adk::im2col_kernel<T>, adk::grid_for(total, 256, 16), 256, 0, adk::as_stream(stream), v, x->N, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo)));
   adk::count_launch();
   return adk::launch_status();
 }

@@ -18,6 +18,7 @@ struct AvgP {
 // one thread per output element; the window mean is accumulated in row-major order
 template <typename T>
 __global__ void __launch_bounds__(256) avgpool_fwd_kernel(AvgP p) {
+  grid_dependency();
   const uint32_t total = p.N * p.C * p.P * p.Q, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)(p.kh * p.kw);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(256) avgpool_fwd_kernel(AvgP p) {
 // one thread per input element gathers from the windows over it
 template <typename T>
 __global__ void __launch_bounds__(256) avgpool_bwd_kernel(AvgP p) {
+  grid_dependency();
   const uint32_t total = p.N * p.C * p.H * p.W, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)(p.kh * p.kw);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -59,6 +61,7 @@ __global__ void __launch_bounds__(256) avgpool_bwd_kernel(AvgP p) {
 // 32 x 2048 channels of 7 x 7: forward 16 us, gradient 54 -> 5 us.
 template <typename T>
 __global__ void __launch_bounds__(256) avgpool_global_plane_fwd(AvgP p) {
+  grid_dependency();
   const uint32_t planes = p.N * p.C, lane = threadIdx.x & 31, hw = p.H * p.W;
   const uint32_t plane = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (plane >= planes) return;
@@ -75,6 +78,7 @@ __global__ void __launch_bounds__(256) avgpool_global_plane_fwd(AvgP p) {
 }
 template <typename T>
 __global__ void __launch_bounds__(256) avgpool_global_plane_bwd(AvgP p) {
+  grid_dependency();
   const uint32_t planes = p.N * p.C, lane = threadIdx.x & 31, hw = p.H * p.W;
   const uint32_t plane = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (plane >= planes) return;
@@ -100,6 +104,7 @@ __device__ __forceinline__ uint4 pk8(const float (&f)[8]) {
   return v;
 }
 __global__ void __launch_bounds__(64) avgpool_global_nhwc_seq(AvgP p) {
+  grid_dependency();
   const uint32_t g = blockIdx.x * 64 + threadIdx.x, n = blockIdx.y;
   if (g >= p.C / 8) return;
   const __nv_bfloat16* X = (const __nv_bfloat16*)p.x.base + n * p.x.sn + g * 8;
@@ -121,6 +126,7 @@ __global__ void __launch_bounds__(64) avgpool_global_nhwc_seq(AvgP p) {
 }
 // gb: groups of 8 channels per block (a power of two up to 32)
 __global__ void __launch_bounds__(256) avgpool_global_nhwc_fwd(AvgP p, uint32_t gb) {
+  grid_dependency();
   __shared__ float sm[256][9];
   const uint32_t G = p.C / 8, gl = threadIdx.x % gb, pl = threadIdx.x / gb, PL = 256 / gb, g = blockIdx.x * gb + gl, n = blockIdx.y;
   const uint32_t hw = p.H * p.W;
@@ -151,6 +157,7 @@ __global__ void __launch_bounds__(256) avgpool_global_nhwc_fwd(AvgP p, uint32_t 
   }
 }
 __global__ void __launch_bounds__(256) avgpool_global_nhwc_bwd(AvgP p, uint32_t gb) {
+  grid_dependency();
   const uint32_t G = p.C / 8, gl = threadIdx.x % gb, pl = threadIdx.x / gb, PL = 256 / gb, g = blockIdx.x * gb + gl, n = blockIdx.y;
   if (g >= G) return;
   const uint32_t hw = p.H * p.W;
@@ -189,13 +196,13 @@ static int launch_global(const AvgP& p, const ad_tensor4* x, const ad_tensor4* y
     while (gb > 1 && (unsigned long long)((p.C / 8 + gb - 1) / gb) * p.N < 2ull * kNumSMs && 256 / gb < p.H * p.W) gb >>= 1;
     while (gb > 1 && gb / 2 >= p.C / 8) gb >>= 1;
     const dim3 grid((p.C / 8 + gb - 1) / gb, p.N);
-    if (bwd) avgpool_global_nhwc_bwd<<<grid, 256, 0, s>>>(p, gb);
-    else if (p.H * p.W <= 256) avgpool_global_nhwc_seq<<<dim3((p.C / 8 + 63) / 64, p.N), 64, 0, s>>>(p);
-    else avgpool_global_nhwc_fwd<<<grid, 256, 0, s>>>(p, gb);
+    if (bwd) launch(avgpool_global_nhwc_bwd, grid, 256, 0, s, p, gb);
+    else if (p.H * p.W <= 256) launch(avgpool_global_nhwc_seq, dim3((p.C / 8 + 63) / 64, p.N), 64, 0, s, p);
+    else launch(avgpool_global_nhwc_fwd, grid, 256, 0, s, p, gb);
   } else if (x->sc != 1 || x->C == 1) {
     const unsigned grid = (unsigned)(((size_t)p.N * p.C + 7) / 8);
-    if (bwd) AD_DISPATCH_DTYPE(x->dtype, (avgpool_global_plane_bwd<T><<<grid, 256, 0, s>>>(p)));
-    else AD_DISPATCH_DTYPE(x->dtype, (avgpool_global_plane_fwd<T><<<grid, 256, 0, s>>>(p)));
+    if (bwd) AD_DISPATCH_DTYPE(x->dtype, (launch(avgpool_global_plane_bwd<T>, grid, 256, 0, s, p)));
+    else AD_DISPATCH_DTYPE(x->dtype, (launch(avgpool_global_plane_fwd<T>, grid, 256, 0, s, p)));
   } else {
     launched = false;
     return AD_OK;
@@ -226,6 +233,7 @@ constexpr uint32_t kFwdI = 1024;
 template <typename T>
 __global__ void __launch_bounds__(256) linear_fwd_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
                                                          const float* __restrict__ w, const float* __restrict__ bias, T* y) {
+  grid_dependency();
   __shared__ float xs[kLinB][kFwdI];
   const uint32_t o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   for (uint32_t b0 = blockIdx.y * kLinB; b0 < B; b0 += gridDim.y * kLinB) {
@@ -273,6 +281,7 @@ constexpr uint32_t kDxCols = 128, kDxRows = 32, kDxStages = 4, kDxMaxO = 1024;
 template <typename T>
 __global__ void __launch_bounds__(kDxCols) linear_dx_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ dy,
                                                             const float* __restrict__ w, T* dx, int accumulate) {
+  grid_dependency();
   extern __shared__ __align__(16) float lin_sm[];
   float* const ring = lin_sm;                                      // [stage][row][column]
   float* const g = lin_sm + kDxStages * kDxRows * kDxCols;         // [row][image]
@@ -338,6 +347,7 @@ constexpr int kDxSmem = (kDxStages * kDxRows * kDxCols + kDxMaxO * kLinB) * 4;
 template <typename T>
 __global__ void __launch_bounds__(256) linear_dw_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
                                                         const T* __restrict__ dy, float* dw, float* db, int accumulate) {
+  grid_dependency();
   __shared__ __align__(16) float g[64][8];
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   for (uint32_t o0 = blockIdx.y * 8; o0 < O; o0 += gridDim.y * 8) {
@@ -390,7 +400,7 @@ extern "C" int ad_avgpool2d_fwd(const ad_tensor4* x, const ad_tensor4* y, uint32
   st = launch_global(p, x, y, false, launched, as_stream(stream));
   if (launched || st != AD_OK) return st;
   p.c_fastest = y->sc == 1 && y->C > 1;
-  AD_DISPATCH_DTYPE(x->dtype, (avgpool_fwd_kernel<T><<<grid_for(total, 256, 16), 256, 0, as_stream(stream)>>>(p)));
+  AD_DISPATCH_DTYPE(x->dtype, (launch(avgpool_fwd_kernel<T>, grid_for(total, 256, 16), 256, 0, as_stream(stream), p)));
   count_launch();
   return launch_status();
 }
@@ -407,7 +417,7 @@ extern "C" int ad_avgpool2d_bwd(const ad_tensor4* dy, const ad_tensor4* dx, uint
   bool launched = false;
   st = launch_global(p, dx, dy, true, launched, as_stream(stream));
   if (launched || st != AD_OK) return st;
-  AD_DISPATCH_DTYPE(dx->dtype, (avgpool_bwd_kernel<T><<<grid_for(total, 256, 16), 256, 0, as_stream(stream)>>>(p)));
+  AD_DISPATCH_DTYPE(dx->dtype, (launch(avgpool_bwd_kernel<T>, grid_for(total, 256, 16), 256, 0, as_stream(stream), p)));
   count_launch();
   return launch_status();
 }
@@ -418,7 +428,7 @@ extern "C" int ad_linear_fwd(int32_t dtype, uint32_t batch, uint32_t in_features
   if ((size_t)batch * out_features >= (1ull << 31) || (size_t)batch * in_features >= (1ull << 31)) return AD_ERR_LIMIT;
   if (batch == 0 || out_features == 0) return AD_OK;
   const dim3 grid((unsigned)(((size_t)out_features + 7) / 8), lin_groups(batch, kLinB));
-  AD_DISPATCH_DTYPE(dtype, (linear_fwd_kernel<T><<<grid, 256, 0, as_stream(stream)>>>(batch, in_features, out_features, (const T*)x, w, bias, (T*)y)));
+  AD_DISPATCH_DTYPE(dtype, (launch(linear_fwd_kernel<T>, grid, 256, 0, as_stream(stream), batch, in_features, out_features, (const T*)x, w, bias, (T*)y)));
   count_launch();
   return launch_status();
 }
@@ -435,7 +445,7 @@ static int launch_linear_dx(uint32_t B, uint32_t I, uint32_t O, const T* dy, con
     }
     attr_done |= 1u << (dev & 31);
   }
-  linear_dx_kernel<T><<<dim3((I + kDxCols - 1) / kDxCols, lin_groups(B, kLinB)), kDxCols, kDxSmem, s>>>(B, I, O, dy, w, dx, accumulate);
+  launch(linear_dx_kernel<T>, dim3((I + kDxCols - 1) / kDxCols, lin_groups(B, kLinB)), kDxCols, kDxSmem, s, B, I, O, dy, w, dx, accumulate);
   return AD_OK;
 }
 
@@ -454,7 +464,7 @@ extern "C" int ad_linear_bwd(int32_t dtype, uint32_t batch, uint32_t in_features
   }
   if (dw && in_features && out_features) {
     const dim3 grid((in_features + 255) / 256, lin_groups(out_features, 8));
-    AD_DISPATCH_DTYPE(dtype, (linear_dw_kernel<T><<<grid, 256, 0, s>>>(batch, in_features, out_features, (const T*)x, (const T*)dy, dw, db, accumulate_dw)));
+    AD_DISPATCH_DTYPE(dtype, (launch(linear_dw_kernel<T>, grid, 256, 0, s, batch, in_features, out_features, (const T*)x, (const T*)dy, dw, db, accumulate_dw)));
     count_launch();
   }
   return launch_status();

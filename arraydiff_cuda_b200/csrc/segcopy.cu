@@ -158,6 +158,7 @@ __device__ __forceinline__ void warp_move(const char* __restrict__ s, char* __re
 
 template <int ELEM, bool ACC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) seg_move_kernel(const SegParams prm) {
+  grid_dependency();
   __shared__ __align__(16) char stage_all[kWarpsPerBlock][kStage];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   char* stage = stage_all[warp];
@@ -219,11 +220,11 @@ static int launch_seg(SegParams& prm, cudaStream_t stream) {
   const unsigned grid = grid_for((size_t)total, kWarpsPerBlock, 8);
   dim3 block(kWarpsPerBlock * 32);
   if (prm.elem == 4) {
-    if (prm.accumulate) seg_move_kernel<4, true><<<grid, block, 0, stream>>>(prm);
-    else seg_move_kernel<4, false><<<grid, block, 0, stream>>>(prm);
+    if (prm.accumulate) launch(seg_move_kernel<4, true>, grid, block, 0, stream, prm);
+    else launch(seg_move_kernel<4, false>, grid, block, 0, stream, prm);
   } else {
-    if (prm.accumulate) seg_move_kernel<2, true><<<grid, block, 0, stream>>>(prm);
-    else seg_move_kernel<2, false><<<grid, block, 0, stream>>>(prm);
+    if (prm.accumulate) launch(seg_move_kernel<2, true>, grid, block, 0, stream, prm);
+    else launch(seg_move_kernel<2, false>, grid, block, 0, stream, prm);
   }
   count_launch();
   return launch_status();

@@ -10,12 +10,14 @@ namespace adk {
 
 __global__ void nll_fwd_kernel(uint32_t C, uint32_t B, const float* __restrict__ y, const uint32_t* __restrict__ label,
                                float* loss) {
+  grid_dependency();
   uint32_t b = threadIdx.x + blockDim.x * blockIdx.x;
   if (b < B) loss[b] = -logf(y[label[b] + (size_t)C * b]);
 }
 
 __global__ void nll_bwd_kernel(uint32_t C, uint32_t B, const float* __restrict__ y, const uint32_t* __restrict__ label,
                                const float* __restrict__ dloss, float* dx) {
+  grid_dependency();
   size_t idx = threadIdx.x + (size_t)blockDim.x * blockIdx.x;
   if (idx >= (size_t)C * B) return;
   uint32_t c = (uint32_t)(idx % C), b = (uint32_t)(idx / C);
@@ -30,6 +32,7 @@ __global__ void nll_bwd_kernel(uint32_t C, uint32_t B, const float* __restrict__
 template <typename T, int CM, bool BWD>
 __global__ void __launch_bounds__(256) ce_nchw_reg(uint32_t N, uint32_t C, uint32_t HW, const T* __restrict__ x, const uint32_t* __restrict__ label,
                                                    float* loss, unsigned long long* picked, const float* __restrict__ dloss, T* dx, int accumulate) {
+  grid_dependency();
   const size_t total = (size_t)N * HW;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t n = i / HW, t = i - n * HW;
@@ -70,6 +73,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) ce_fwd_nchw(uint32_t N, uint32_t C, uint32_t HW, const T* __restrict__ x,
                                                     const uint32_t* __restrict__ label, float* loss,
                                                     unsigned long long* picked) {
+  grid_dependency();
   const size_t total = (size_t)N * HW;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t n = i / HW, t = i % HW;
@@ -89,6 +93,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) ce_bwd_nchw(uint32_t N, uint32_t C, uint32_t HW, const T* __restrict__ x,
                                                     const uint32_t* __restrict__ label,
                                                     const float* __restrict__ dloss, T* dx, int accumulate) {
+  grid_dependency();
   const size_t total = (size_t)N * HW;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const size_t n = i / HW, t = i % HW;
@@ -114,6 +119,7 @@ __global__ void __launch_bounds__(256) ce_nhwc(uint32_t C, size_t pixels, const 
                                                 const uint32_t* __restrict__ label, float* loss,
                                                 unsigned long long* picked, const float* __restrict__ dloss, T* dx,
                                                 int accumulate) {
+  grid_dependency();
   const int lane = threadIdx.x & 31;
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((size_t)gridDim.x * blockDim.x) >> 5;
   for (size_t i = warp; i < pixels; i += nw) {
@@ -145,6 +151,7 @@ __global__ void __launch_bounds__(256) ce_nhwc(uint32_t C, size_t pixels, const 
 template <typename T, int K, bool BWD>
 __global__ void __launch_bounds__(256) ce_nhwc_reg(uint32_t C, size_t pixels, const T* __restrict__ x, const uint32_t* __restrict__ label,
                                                    float* loss, unsigned long long* picked, const float* __restrict__ dloss, T* dx, int accumulate) {
+  grid_dependency();
   constexpr int PX = K <= 2 ? 4 : 2;
   const int lane = threadIdx.x & 31;
   const size_t warp = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((size_t)gridDim.x * blockDim.x) >> 5;
@@ -211,6 +218,7 @@ __global__ void __launch_bounds__(256) ce_nhwc_small(uint32_t C, size_t pixels, 
                                                       const uint32_t* __restrict__ label, float* loss,
                                                       unsigned long long* picked, const float* __restrict__ dloss, T* dx,
                                                       int accumulate) {
+  grid_dependency();
   extern __shared__ __align__(16) uint8_t ce_raw[];   // [256][C]
   T* sm = (T*)ce_raw;
   constexpr uint32_t V = 16 / sizeof(T);
@@ -268,14 +276,14 @@ static int launch_ce(int32_t layout, uint32_t N, uint32_t C, uint32_t HW, const 
   const size_t pixels = (size_t)N * HW;
   if (layout != AD_NCHW && layout != AD_NHWC) return AD_ERR_UNSUPPORTED;
   if (layout == AD_NCHW && HW > 1) {
-    if (C <= 8) ce_nchw_reg<T, 8, BWD><<<grid_for(pixels, 256), 256, 0, s>>>(N, C, HW, x, label, loss, picked, dloss, dx, accumulate);
-    else if (C <= 32) ce_nchw_reg<T, 32, BWD><<<grid_for(pixels, 256), 256, 0, s>>>(N, C, HW, x, label, loss, picked, dloss, dx, accumulate);
-    else if (BWD) ce_bwd_nchw<T><<<grid_for(pixels, 256), 256, 0, s>>>(N, C, HW, x, label, dloss, dx, accumulate);
-    else ce_fwd_nchw<T><<<grid_for(pixels, 256), 256, 0, s>>>(N, C, HW, x, label, loss, picked);
+    if (C <= 8) launch(ce_nchw_reg<T, 8, BWD>, grid_for(pixels, 256), 256, 0, s, N, C, HW, x, label, loss, picked, dloss, dx, accumulate);
+    else if (C <= 32) launch(ce_nchw_reg<T, 32, BWD>, grid_for(pixels, 256), 256, 0, s, N, C, HW, x, label, loss, picked, dloss, dx, accumulate);
+    else if (BWD) launch(ce_bwd_nchw<T>, grid_for(pixels, 256), 256, 0, s, N, C, HW, x, label, dloss, dx, accumulate);
+    else launch(ce_fwd_nchw<T>, grid_for(pixels, 256), 256, 0, s, N, C, HW, x, label, loss, picked);
   } else if (C <= 32 && pixels <= (1ull << 31) * 256 - 256) {
     const int vec = ((uintptr_t)x & 15u) == 0 && (!BWD || ((uintptr_t)dx & 15u) == 0);
     auto go = [&](auto kernel) {
-      kernel<<<(unsigned)((pixels + 255) / 256), 256, 256 * C * sizeof(T), s>>>(C, pixels, vec, x, label, loss, picked, dloss, dx, accumulate);
+      launch(kernel, (unsigned)((pixels + 255) / 256), 256, 256 * C * sizeof(T), s, C, pixels, vec, x, label, loss, picked, dloss, dx, accumulate);
     };
     switch ((C + 3) / 4) {
       case 1: go(ce_nhwc_small<T, 4, BWD>); break;
@@ -288,13 +296,13 @@ static int launch_ce(int32_t layout, uint32_t N, uint32_t C, uint32_t HW, const 
       default: go(ce_nhwc_small<T, 32, BWD>); break;
     }
   } else if (C <= 64) {
-    ce_nhwc_reg<T, 2, BWD><<<grid_for(pixels, 32), 256, 0, s>>>(C, pixels, x, label, loss, picked, dloss, dx, accumulate);
+    launch(ce_nhwc_reg<T, 2, BWD>, grid_for(pixels, 32), 256, 0, s, C, pixels, x, label, loss, picked, dloss, dx, accumulate);
   } else if (C <= 128) {
-    ce_nhwc_reg<T, 4, BWD><<<grid_for(pixels, 16), 256, 0, s>>>(C, pixels, x, label, loss, picked, dloss, dx, accumulate);
+    launch(ce_nhwc_reg<T, 4, BWD>, grid_for(pixels, 16), 256, 0, s, C, pixels, x, label, loss, picked, dloss, dx, accumulate);
   } else if (C <= 256) {
-    ce_nhwc_reg<T, 8, BWD><<<grid_for(pixels, 16), 256, 0, s>>>(C, pixels, x, label, loss, picked, dloss, dx, accumulate);
+    launch(ce_nhwc_reg<T, 8, BWD>, grid_for(pixels, 16), 256, 0, s, C, pixels, x, label, loss, picked, dloss, dx, accumulate);
   } else {
-    ce_nhwc<T, BWD><<<grid_for(pixels, 8), 256, 0, s>>>(C, pixels, x, label, loss, picked, dloss, dx, accumulate);
+    launch(ce_nhwc<T, BWD>, grid_for(pixels, 8), 256, 0, s, C, pixels, x, label, loss, picked, dloss, dx, accumulate);
   }
   count_launch();
   return launch_status();
@@ -308,7 +316,7 @@ extern "C" int ad_softmax_nll_loss_fwd(uint32_t C, uint32_t B, const float* y, c
                                        void* stream) {
   if (B == 0) return AD_OK;
   if (!y || !label || !loss || C == 0) return AD_ERR_BAD_ARG;
-  nll_fwd_kernel<<<(B + 255) / 256, 256, 0, as_stream(stream)>>>(C, B, y, label, loss);
+  launch(nll_fwd_kernel, (B + 255) / 256, 256, 0, as_stream(stream), C, B, y, label, loss);
   count_launch();
   return launch_status();
 }
@@ -318,7 +326,7 @@ extern "C" int ad_softmax_nll_loss_bwd(uint32_t C, uint32_t B, const float* y, c
   if (B == 0 || C == 0) return AD_OK;
   if (!y || !label || !dloss || !dx) return AD_ERR_BAD_ARG;
   size_t total = (size_t)C * B;
-  nll_bwd_kernel<<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>(C, B, y, label, dloss, dx);
+  launch(nll_bwd_kernel, (unsigned)((total + 255) / 256), 256, 0, as_stream(stream), C, B, y, label, dloss, dx);
   count_launch();
   return launch_status();
 }

@@ -34,6 +34,7 @@ __device__ __forceinline__ void bilin_src(uint32_t o, float inv_scale, uint32_t 
 
 template <typename T>
 __global__ void __launch_bounds__(256) upsample_fwd_kernel(UpP p) {
+  grid_dependency();
   const uint32_t total = p.N * p.C * p.YH * p.YW, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)p.scale;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(256) upsample_fwd_kernel(UpP p) {
 // high-resolution gradients whose source pair contains it -- no atomics, reproducible.
 template <typename T>
 __global__ void __launch_bounds__(256) upsample_bwd_kernel(UpP p) {
+  grid_dependency();
   const uint32_t total = p.N * p.C * p.XH * p.XW, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)p.scale;
   const int s = (int)p.scale;
@@ -141,6 +143,7 @@ __device__ __forceinline__ long long plane_off(const UpView& v, uint32_t plane, 
 
 template <typename T>
 __global__ void __launch_bounds__(kUpThreads) upsample_fwd_rows(UpRowP p) {
+  grid_dependency();
   extern __shared__ __align__(16) float L[];   // [rb][XC + 2 low-resolution columns, clamped to the image][Ci]
   const UpP& u = p.u;
   const float inv = 1.0f / (float)u.scale;
@@ -198,6 +201,7 @@ __global__ void __launch_bounds__(kUpThreads) upsample_fwd_rows(UpRowP p) {
 
 template <typename T>
 __global__ void __launch_bounds__(kUpThreads) upsample_bwd_rows(UpRowP p) {
+  grid_dependency();
   extern __shared__ __align__(16) float S[];   // column sums of the chunk's output columns (and one low-resolution column either side)
   constexpr uint32_t V = 16 / sizeof(T);
   const UpP& u = p.u;
@@ -368,9 +372,9 @@ extern "C" int ad_upsample_bilinear_fwd(const ad_tensor4* x, const ad_tensor4* y
   r.u = p;
   if (up_rows(x, y, false, r)) {
     const unsigned grid = (unsigned)((((size_t)r.planes * p.YH + r.rb - 1) / r.rb) * r.chunks);
-    AD_DISPATCH_DTYPE(x->dtype, (upsample_fwd_rows<T><<<grid, kUpThreads, r.smem, as_stream(stream)>>>(r)));
+    AD_DISPATCH_DTYPE(x->dtype, (launch(upsample_fwd_rows<T>, grid, kUpThreads, r.smem, as_stream(stream), r)));
   } else
-    AD_DISPATCH_DTYPE(x->dtype, (upsample_fwd_kernel<T><<<grid_for(total, 256, 16), 256, 0, as_stream(stream)>>>(p)));
+    AD_DISPATCH_DTYPE(x->dtype, (launch(upsample_fwd_kernel<T>, grid_for(total, 256, 16), 256, 0, as_stream(stream), p)));
   count_launch();
   return launch_status();
 }
@@ -388,9 +392,9 @@ extern "C" int ad_upsample_bilinear_bwd(const ad_tensor4* dy, const ad_tensor4* 
   r.u = p;
   if (up_rows(dx, dy, true, r)) {
     const unsigned grid = (unsigned)((size_t)r.planes * p.XH * r.chunks);
-    AD_DISPATCH_DTYPE(dx->dtype, (upsample_bwd_rows<T><<<grid, kUpThreads, r.smem, as_stream(stream)>>>(r)));
+    AD_DISPATCH_DTYPE(dx->dtype, (launch(upsample_bwd_rows<T>, grid, kUpThreads, r.smem, as_stream(stream), r)));
   } else
-    AD_DISPATCH_DTYPE(dx->dtype, (upsample_bwd_kernel<T><<<grid_for(total, 256, 16), 256, 0, as_stream(stream)>>>(p)));
+    AD_DISPATCH_DTYPE(dx->dtype, (launch(upsample_bwd_kernel<T>, grid_for(total, 256, 16), 256, 0, as_stream(stream), p)));
   count_launch();
   return launch_status();
 }

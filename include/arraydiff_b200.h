@@ -454,7 +454,8 @@ int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream);
  * The gradients with more said by the caller.  w_crsk (tensor-core path): the filter as bf16 C,R,S,K with mirrored taps and
  * rows of K rounded up to 64 entries, as ad_filter_prepare writes it (NULL: made from a->w on each call, in scratch).
  * status: the device word that waits which run out report into (NULL: the first word of scratch, which the caller then
- * keeps zero).
+ * keeps zero).  ad_conv2d_wgrad_ex is for a stream beside the critical one: its kernels do not become resident before the
+ * kernel in front of them has ended.
  */
 int ad_conv2d_dgrad_ex(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream);
 int ad_conv2d_wgrad_ex(const ad_conv2d_args* a, int32_t* status, void* stream);
