@@ -136,6 +136,7 @@ SIGNATURES = {
     "ad_conv2d_fprop": (C.c_int, [C.POINTER(Conv2dArgs), vp]),
     "ad_conv2d_dgrad": (C.c_int, [C.POINTER(Conv2dArgs), vp]),
     "ad_conv2d_wgrad": (C.c_int, [C.POINTER(Conv2dArgs), vp]),
+    "ad_conv2d_fprop_add": (C.c_int, [C.POINTER(Conv2dArgs), C.POINTER(Tensor4), vp]),
     "ad_conv2d_dgrad_ex": (C.c_int, [C.POINTER(Conv2dArgs), vp, vp, vp]),
     "ad_conv2d_wgrad_ex": (C.c_int, [C.POINTER(Conv2dArgs), vp, vp]),
     "ad_filter_prepare": (C.c_int, [u32, C.POINTER(FilterItem), vp]),

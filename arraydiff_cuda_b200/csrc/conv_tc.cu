@@ -107,6 +107,8 @@ struct FwdParams {
   int32_t* status;
   int32_t tma_store;   // epilogue: stage 64-channel chunks in shared memory, one TMA tile store each
   long long out_px;    // elements between output pixels of a row
+  const __nv_bfloat16* add;   // tma_store, one class: added to the rounded outputs (a residual sum); pixels OC apart
+  long long add_pitch, add_plane;
 };
 struct FwdClasses { FwdClass c[kFwdClasses]; uint32_t n; };
 template <int NC> struct FwdOut { CUtensorMap map[NC]; };
@@ -298,6 +300,19 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
         // (64 -> 256 channels, 262,144 pixels, bound by these stores: 44 -> 35 us).
         constexpr uint32_t kChunks = BN / 64;
         if (kChunks == 1 && (it & 1u) != grp) continue;
+        // the addend's 128 bytes per pixel and chunk are on their way while the accumulator is awaited
+        uint4 ad[8];
+        const __nv_bfloat16* arow = nullptr;
+        if (NC == 1 && p.add) {
+          const uint32_t mi = m / (p.TW * p.TH), mr = m - mi * (p.TW * p.TH);
+          const uint32_t oy = ty * p.TH + mr / p.TW, ox = tx * p.TW + mr % p.TW, on = n + mi;
+          if (oy < p.OP && ox < p.OQ && on < p.NI) arow = p.add + (long long)on * p.add_plane + (long long)oy * p.add_pitch + (long long)ox * p.OC;
+        }
+        auto load_add = [&](uint32_t cb) {
+#pragma unroll
+          for (uint32_t g8 = 0; g8 < 8; ++g8) ad[g8] = arow && cb + g8 * 8 < p.OC ? *(const uint4*)(arow + cb + g8 * 8) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        if (NC == 1 && p.add) load_add(tn * BN + (kChunks == 1 ? 0u : grp) * 64);
         if (!mbar_wait(smem_u32(&ctl->tfull[acc]), acc_phase, abortf)) break;
         tc_fence_after();
         const uint32_t m7 = m & 7u;
@@ -343,8 +358,17 @@ conv_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               p2[j] = __floats2bfloat162_rn(__uint_as_float(v[g8 * 8 + 2 * j]), __uint_as_float(v[g8 * 8 + 2 * j + 1]));
+            if (NC == 1 && p.add) {
+              const __nv_bfloat162* a2 = (const __nv_bfloat162*)&ad[g8];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 r = __bfloat1622float2(p2[j]), e = __bfloat1622float2(a2[j]);
+                p2[j] = __floats2bfloat162_rn(r.x + e.x, r.y + e.y);
+              }
+            }
             *(uint4*)(srow + ((g8 ^ m7) * 16u)) = pk;
           }
+          if (NC == 1 && p.add && c64 + 2 < kChunks) load_add(cbase + 128);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&ctl->stg_full[sb]));
@@ -1049,12 +1073,20 @@ static int run_fwd_tiles(const void* act, uint32_t IH, uint32_t IW, const void* 
   }
 }
 
+// out += add, dims of add: for the forms whose epilogue does not
+static int add_to_output(const ad_tensor4* add, void* out, long long pitch, long long plane, cudaStream_t s) {
+  ad_tensor4 y = *add;
+  y.base = out;
+  y.sc = 1; y.sx = add->C; y.sy = pitch; y.sn = plane;
+  return ad_add(&y, add, &y, s);
+}
+
 // Generic forward-style implicit GEMM launch (fprop, or dgrad expressed as fprop).
 static int run_fwd_gemm(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CK, const void* filt,
                         uint32_t OC, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw,
                         int offy, int offx, uint32_t OP, uint32_t OQ, void* out, long long out_pitch,
                         long long out_plane, const float* bias, int relu, int accumulate, int32_t* status,
-                        cudaStream_t s) {
+                        cudaStream_t s, const ad_tensor4* add = nullptr) {
   if (CK % 64 != 0) return AD_ERR_UNSUPPORTED;
   if (!getenv("ARRAYDIFF_B200_NO_ROW_KERNEL")) {
     // 64-channel layers: the row-tile kernel fetches each activation patch once (conv_tc_row.cu)
@@ -1062,7 +1094,7 @@ static int run_fwd_gemm(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, 
                              out_plane, bias, relu, accumulate, status, s);
     if (st != AD_ERR_UNSUPPORTED) {
       g_last_conv_kernel = kConvTcRow;
-      return st;
+      return st == AD_OK && add ? add_to_output(add, out, out_pitch, out_plane, s) : st;
     }
   }
   FwdParams p{};
@@ -1077,7 +1109,12 @@ static int run_fwd_gemm(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, 
   p.out_plane = out_plane ? out_plane : (long long)OP * OQ * OC;
   p.out = (__nv_bfloat16*)out;
   p.bias = bias; p.relu = relu; p.accumulate = accumulate; p.status = status;
-  return run_fwd_tiles<1>(act, IH, IW, filt, kh * kw, p, FwdClasses{}, s);
+  // In the epilogue where it stores by TMA and the addend's pixels are as dense as the output's
+  const bool in_epilogue = add && OC > 32 && OC % 8 == 0 && add->sc == 1 && add->sx == (int64_t)OC && !(add->sy & 7) && !(add->sn & 7) &&
+                           !((uintptr_t)add->base & 15u) && !((uintptr_t)out & 15u) && p.out_pitch % 8 == 0 && p.out_plane % 8 == 0;
+  if (in_epilogue) { p.add = (const __nv_bfloat16*)add->base; p.add_pitch = add->sy; p.add_plane = add->sn; }
+  const int st = run_fwd_tiles<1>(act, IH, IW, filt, kh * kw, p, FwdClasses{}, s);
+  return st == AD_OK && add && !in_epilogue ? add_to_output(add, out, p.out_pitch, p.out_plane, s) : st;
 }
 
 template <int BN, bool PAIR>
@@ -1142,7 +1179,7 @@ size_t conv_tc_scratch_bytes(const ad_conv2d_args* a, int pass) {
   return 16;
 }
 
-int conv_tc_fprop(const ad_conv2d_args* a, cudaStream_t s) {
+int conv_tc_fprop(const ad_conv2d_args* a, const ad_tensor4* addend, cudaStream_t s) {
   Geo g;
   int st = conv_geo(a, g);
   if (st != AD_OK) return st;
@@ -1161,9 +1198,16 @@ int conv_tc_fprop(const ad_conv2d_args* a, cudaStream_t s) {
   const long long pitch = a->y_pitch ? a->y_pitch : (long long)g.Q * a->K;
   const long long plane = a->y_plane ? a->y_plane : (long long)g.P * g.Q * a->K;
   __nv_bfloat16* out = (__nv_bfloat16*)a->y + (long long)q0 * pitch;
+  ad_tensor4 add;
+  if (addend) {
+    if (!addend->base || addend->dtype != AD_BF16 || addend->N != a->N || addend->C != a->K || addend->H != g.P || addend->W != g.Q) return AD_ERR_BAD_ARG;
+    add = *addend;
+    add.H = nq;
+    add.base = (__nv_bfloat16*)addend->base + (long long)q0 * addend->sy;
+  }
   return run_fwd_gemm(a->x, a->N, a->H, a->W, a->C, a->w, a->K, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h,
                       a->dil_w, -(int)a->pad_h + (int)(q0 * a->stride_h), -(int)a->pad_w, nq, g.Q, out, pitch, plane, a->bias,
-                      a->relu, 0, status, s);
+                      a->relu, 0, status, s, addend ? &add : nullptr);
 }
 
 // Data gradient of a strided layer.  Output row y takes the taps r with (y + pad - r * dil) divisible by the stride, a list
@@ -1426,15 +1470,17 @@ extern "C" size_t ad_conv2d_profile_read(ad_conv2d_profile_entry* out, size_t ma
   return n;
 }
 
-extern "C" int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream) {
+static int fprop_call(const ad_conv2d_args* a, const ad_tensor4* addend, void* stream) {
   return profiled(0, a, stream, [&] {
     switch (path_of(a)) {
-      case 0: g_last_conv_kernel = kConvDirectF32; return conv_direct_fprop(a, as_stream(stream));
-      case 1: return tc::conv_tc_fprop(a, as_stream(stream));
+      case 0: g_last_conv_kernel = kConvDirectF32; return addend ? (int)AD_ERR_UNSUPPORTED : conv_direct_fprop(a, as_stream(stream));
+      case 1: return tc::conv_tc_fprop(a, addend, as_stream(stream));
       default: return (int)(a ? AD_ERR_UNSUPPORTED : AD_ERR_BAD_ARG);
     }
   });
 }
+extern "C" int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream) { return fprop_call(a, nullptr, stream); }
+extern "C" int ad_conv2d_fprop_add(const ad_conv2d_args* a, const ad_tensor4* addend, void* stream) { return fprop_call(a, addend, stream); }
 static int dgrad_call(const ad_conv2d_args* a, const void* w_crsk, int32_t* status, void* stream) {
   return profiled(1, a, stream, [&] {
     switch (path_of(a)) {

@@ -323,6 +323,10 @@ public:
   void _persist(TxnId, VarIdSet&) override {}
   // The only consumer's gradient is this operator's gradient (kJoinShare): one variable, one buffer
   void share_grad(const TxnVar<Act>& grad) { y_.grad = grad; }
+  // A sum of this output (kJoinShare) and x, which is evaluated earlier, asks its last input to write the sum itself:
+  // true, and y_.val holds the sum from then on.
+  virtual bool take_sum(ActVar x) { return false; }
+  const TxnVar<Act>& value_var() const { return y_.val; }
   // Any activation can be read back, and its gradient set or read, as packed NCHW fp32 of the
   // interior: that is how a caller supplies an upstream gradient or inspects a result.
   size_t _load_grad(TxnId txn, VarIdSet& vars, size_t offset, any* reader) override;
@@ -441,6 +445,7 @@ public:
   void _forward(TxnId txn) override;
   void _backward(TxnId txn) override;
   ~CudnnConv2DOpF() override;
+  bool take_sum(ActVar x) override;
   string _debug_op_label() override { return "CudnnConv2DOp"; }
 private:
   void fill_args(ad_conv2d_args& a, Act& x);
@@ -453,6 +458,7 @@ private:
   // GPUContext::prepare_filters), fp32 KRSC gradient staging, im2col matrix (stem)
   void *w_bf16_ = nullptr, *w_crsk_ = nullptr;
   size_t filter_id_ = (size_t)-1;
+  ActVar sum_;             // take_sum: not an input of the graph (the sum is, and it orders the two)
   float* dw_krsc_ = nullptr;
   void* im2col_ = nullptr;
   size_t ck_ = 0;       // channels the tensor-core kernel reduces over per tap (padded)
@@ -526,6 +532,7 @@ public:
 private:
   vector<ActVar> xs_;
   vector<JoinGrad> grads_;
+  bool in_last_ = false;   // the last input writes the sum
 };
 
 // Re-assembly of the strips on every rank: y_r = concat_q x_q along H.  The reference builds it from

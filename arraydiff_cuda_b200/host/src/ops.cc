@@ -495,6 +495,11 @@ void CudnnConv2DOpF::fill_args(ad_conv2d_args& a, Act& x) {
   }
 }
 
+bool CudnnConv2DOpF::take_sum(ActVar x) {
+  if (gpu()->mode() != COMPUTE_BF16_NHWC || sum_) return false;
+  sum_ = x;
+  return true;
+}
 CudnnConv2DOpF::~CudnnConv2DOpF() {
   if (filter_id_ != (size_t)-1) gpu()->remove_filter(filter_id_);
 }
@@ -541,17 +546,19 @@ void CudnnConv2DOpF::_forward(TxnId txn) {
   }
   g->reserve_scratch(16);
   a.scratch = g->status_word(); a.scratch_bytes = 16;
+  ad_tensor4 add;
+  if (sum_) add = sum_->data().val.get(txn, id()).view_interior();
   if (split) {
     a.out_row_begin = (uint32_t)ph; a.out_row_count = (uint32_t)(oh - 2 * ph);
-    AD_CHECK(ad_conv2d_fprop(&a, conn.stream()));
+    AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
     g->finish_pending();
     a.out_row_begin = 0; a.out_row_count = (uint32_t)ph;
-    AD_CHECK(ad_conv2d_fprop(&a, conn.stream()));
+    AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
     a.out_row_begin = (uint32_t)(oh - ph);
-    AD_CHECK(ad_conv2d_fprop(&a, conn.stream()));
+    AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
     return;
   }
-  AD_CHECK(ad_conv2d_fprop(&a, conn.stream()));
+  AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
 }
 
 void CudnnConv2DOpF::_backward(TxnId txn) {
@@ -839,8 +846,14 @@ SumJoinOpF::SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGr
     if (op) op->share_grad(y_.grad);
     else grads_[i] = kJoinCopy;
   }
+  auto* last = dynamic_cast<ActOp*>(xs.back().get());
+  if (xs.size() == 2 && grads_[1] == kJoinShare && xs[0] != xs[1] && last->take_sum(xs[0])) {
+    in_last_ = true;
+    y_.val = last->value_var();
+  }
 }
 void SumJoinOpF::_forward(TxnId txn) {
+  if (in_last_) return;
   if (!y_.val.overwrite(txn, id())) return;
   GPUConn conn = gpu()->conn();
   ad_tensor4 yv = y_.val.get_excl(txn, id()).view_interior();

@@ -448,6 +448,9 @@ typedef struct {
 
 size_t ad_conv2d_scratch_bytes(const ad_conv2d_args* a, int32_t pass /* 0 fprop, 1 dgrad, 2 wgrad */);
 int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream);
+/* y = (the bf16 output of ad_conv2d_fprop) + addend, a whole-output view (the rows of a row range are taken from it);
+ * tensor-core path only.  addend may be NULL. */
+int ad_conv2d_fprop_add(const ad_conv2d_args* a, const ad_tensor4* addend, void* stream);
 int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream);
 int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream);
 /*

@@ -133,3 +133,38 @@ def test_forward_pairs(case, bias):
     H.sync()
     want = torch.nn.functional.conv2d(x.cpu().float().permute(0, 3, 1, 2), w.cpu().float().permute(0, 3, 1, 2), b.cpu() if bias else None)
     assert int(status[0]) == 0 and (y.cpu().float() - want.permute(0, 2, 3, 1)).abs().max() < 8e-3 * want.abs().max()
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, K, k: the epilogue's forms (pair, single CTA, one chunk per tile), ragged channels, scattered stores, row kernel
+    (2, 512, 15, 29, 256, 1), (2, 128, 9, 21, 520, 1), (1, 64, 20, 17, 264, 3), (3, 64, 7, 9, 128, 1), (2, 128, 13, 11, 64, 1),
+    (2, 128, 10, 12, 19, 1), (1, 64, 9, 140, 64, 3),
+])
+@pytest.mark.parametrize("pad", [0, 1])
+@pytest.mark.parametrize("rows", [None, (2, 3)])
+def test_forward_with_addend(case, pad, rows):
+    """To the bit: the convolution, rounded, plus the addend."""
+    import torch
+    N, Cc, Hh, W, K, k = case
+    L = abi.lib()
+    a = abi.Conv2dArgs()
+    a.dtype, a.layout = abi.AD_BF16, abi.AD_NHWC
+    a.N, a.C, a.H, a.W, a.K, a.kh, a.kw = N, Cc, Hh, W, K, k, k
+    a.stride_h = a.stride_w = a.dil_h = a.dil_w = 1
+    P, Q = Hh - k + 1, W - k + 1
+    x, w, b = (torch.randn(*n, device="cuda") for n in ((N, Hh, W, Cc), (K, k, k, Cc), (K,)))
+    x, w = x.bfloat16(), w.bfloat16()
+    add = (20 * torch.randn(N, P + 2 * pad, Q + 2 * pad, K, device="cuda")).bfloat16()
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    a.x, a.w, a.bias, a.scratch, a.scratch_bytes = x.data_ptr(), w.data_ptr(), b.data_ptr(), status.data_ptr(), 16
+    if rows:
+        a.out_row_begin, a.out_row_count = rows
+    lo, n = rows or (0, P)
+    y0, y1 = (torch.full((N, P, Q, K), 3.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    a.y = y0.data_ptr()
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    a.y = y1.data_ptr()
+    abi.check(L.ad_conv2d_fprop_add(C.byref(a), C.byref(H.view_nhwc(add, (pad, P, Q))), H.stream()))
+    H.sync()
+    y0[:, lo:lo + n] += add[:, pad + lo:pad + lo + n, pad:pad + Q]
+    assert int(status[0]) == 0 and torch.equal(y0, y1)
