@@ -155,6 +155,7 @@ int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
 int f32_gemm_dgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
 int f32_gemm_wgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
 size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q);
+size_t f32_dgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q);
 
 int conv_direct_fprop(const ad_conv2d_args* a, cudaStream_t s) {
   ConvG g;
@@ -182,10 +183,13 @@ int conv_direct_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
   return launch_status();
 }
 
-// Scratch with which a filter gradient of few outputs and many pixels is split further (optional: less or none is fine)
+// Scratch with which a filter gradient of few outputs and many pixels is split further, or a data gradient into few
+// channels takes its two-step form (optional: less or none is fine)
 size_t conv_direct_scratch_bytes(const ad_conv2d_args* a, int pass) {
   ConvG g;
-  if (pass != 2 || geometry(a, g) != AD_OK || g.kh * g.kw > 49 || !f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return 0;
+  if (geometry(a, g) != AD_OK || !f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return 0;
+  if (pass == 1) return f32_dgrad_scratch(a, g.P, g.Q);
+  if (pass != 2 || g.kh * g.kw > 49) return 0;
   return f32_wgrad_scratch(a, g.P, g.Q);
 }
 

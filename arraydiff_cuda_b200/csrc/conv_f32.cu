@@ -10,13 +10,14 @@
 // cp.async into a ring of stages, ~6 instructions per element (table entry, test, address, a predicated copy or a
 // predicated store of zero for the implicit padding).
 //
-// A shape with few output tiles splits its reduction over the CTAs of a cluster (up to 8), whose partial tiles meet
+// A shape with few output tiles splits its reduction over the CTAs of a cluster (up to 16, filter gradients 8), whose partial tiles meet
 // through distributed shared memory in rank order, and a filter gradient further over slices of the caller's scratch:
 // no atomics, reproducible.
 //
 // Measured on a B200 against one thread per output (the kernels of conv_direct.cu, which remain for geometries outside
 // f32_gemm_ok): figures at the launchers.
 #include <cooperative_groups.h>
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -45,6 +46,7 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+constexpr int kF32Most = 16;             // CTAs of a cluster, forward and data gradient
 constexpr int kF32Group = 128;           // threads that share one tile; a CTA is one or two such groups
 constexpr int kF32MaxK = 15;             // filter rows / columns: one bit each in a 32-bit word (rows 0.., columns 16..)
 constexpr uint32_t kF32Never = 1u << 31; // a bit no pixel has
@@ -58,16 +60,16 @@ template <int LM, int WM, int WN, int G> struct F32Tile {
 };
 
 // Sum of one element of the tiles of all groups of all CTAs of the cluster, in order; all loads are in flight together
-template <int G>
+template <int G, int MOST = 8>
 __device__ __forceinline__ float cluster_total(cg::cluster_group& cluster, float* sm, uint32_t cs, size_t at, size_t group_stride) {
-  float v[8 * G];
+  float v[MOST * G];
 #pragma unroll
-  for (uint32_t q = 0; q < 8; ++q)
+  for (uint32_t q = 0; q < MOST; ++q)
 #pragma unroll
     for (int g = 0; g < G; ++g) v[q * G + g] = q < cs ? (cs > 1 ? cluster.map_shared_rank(sm, q) : sm)[at + g * group_stride] : 0.f;
   float t = v[0];
 #pragma unroll
-  for (uint32_t q = 1; q < 8 * G; ++q) if (q < cs * G) t += v[q];
+  for (uint32_t q = 1; q < MOST * G; ++q) if (q < cs * G) t += v[q];
   return t;
 }
 
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(kF32Group, 3) conv_gemm_f32(const GemmF32 p) {
     const uint32_t m = rank * rows + i;
 #pragma unroll
     for (int u = 0; u < NPX; ++u) {
-      float v = cluster_total<1>(cluster, tile, cs, (size_t)m * BN + tid + u * kF32Group, 0);
+      float v = cluster_total<1, kF32Most>(cluster, tile, cs, (size_t)m * BN + tid + u * kF32Group, 0);
       if (out_px[u] && m_base + m < p.M) {
         float* o = out_px[u] + (long long)(m_base + m) * p.out_plane;
         if (!DGRAD) {
@@ -317,6 +319,7 @@ static int launch_f32(Kernel k, dim3 grid, int threads, int smem, uint32_t cs, c
       cudaGetLastError();
       return AD_ERR_CUDA;
     }
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
     attr_done |= 1u << (dev & 31);
   }
   cudaLaunchConfig_t cfg = {};
@@ -346,8 +349,9 @@ static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uin
   typedef GemmTile<LM, WM, WN> T;
   static unsigned attr_done = 0;      // one bit per device
   const uint32_t tn = (npx + T::BN - 1) / T::BN, tm = (p.M + T::BM - 1) / T::BM;
-  // three CTAs per SM are resident (BM >= 8 rows: a cluster of 8 still has a row per CTA)
-  const uint32_t cs = f32_cluster((unsigned long long)tn * tm * classes, 3ull * kNumSMs, Kd / T::KB, 8);
+  // three CTAs per SM are resident; every CTA of a cluster finishes at least one of the BM rows.  Clusters of 16 are for few
+  // tiles and long reductions: 4 x 512 x 7 x 7 -> 512, 3x3 (16 tiles) 92 -> 67 us against 8.
+  const uint32_t cs = f32_cluster((unsigned long long)tn * tm * classes, 3ull * kNumSMs, Kd / T::KB, std::min(kF32Most, (int)T::BM));
   return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, attr_done, s);
 }
 
@@ -600,7 +604,65 @@ int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
   return run_gemm_f32<false>(p, s);
 }
 
+// Data gradient into few channels (an image's three), with scratch: per pixel of dy the products of all (channel, tap) rows
+// with the filter as one GEMM -- Z[n][channel, tap][pixel], a 1x1 convolution of dy -- and then the sum over the taps of
+// each input pixel, in tap order.  As the GEMM above, 3 of 8 rows of a tile are used and every element of dy is gathered
+// once per tap: bound by the gathers.  4 x 64 x 224 x 224 -> 3, 7x7: 730 -> 393 us.
+// Images are taken as many at a time as fit kFewZ bytes; larger ones go the other way.
+constexpr size_t kFewZ = 64u << 20;
+static size_t few_z_bytes(const ad_conv2d_args* a, uint32_t P, uint32_t Q) { return (size_t)P * Q * a->C * a->kh * a->kw * 4; }   // one image
+size_t f32_dgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
+  const size_t z = few_z_bytes(a, P, Q);
+  if (a->C > 8 || a->kh * a->kw < 4 || a->K < 16 || z > kFewZ) return 0;
+  return z * std::min<size_t>(a->N, kFewZ / z);
+}
+__global__ void __launch_bounds__(256) dgrad_few_sum(const float* __restrict__ z, float* dx, uint32_t N, uint32_t C, uint32_t H, uint32_t W,
+                                                     uint32_t P, uint32_t Q, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw,
+                                                     uint32_t dh, uint32_t dw, int ph, int pw, int accumulate) {
+  grid_dependency();
+  const uint32_t total = N * C * H * W, pq = P * Q;
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    const uint32_t x = i % W, r = i / W, y = r % H, nc = r / H;
+    const float* zc = z + (size_t)nc * kh * kw * pq;
+    float v = 0.f;
+    for (uint32_t ti = 0; ti < kh; ++ti) {
+      const int ay = (int)y + ph - (int)(ti * dh);
+      if (ay < 0 || ay % (int)sh || (uint32_t)ay / sh >= P) continue;
+      const float* zr = zc + (size_t)ti * kw * pq + (size_t)((uint32_t)ay / sh) * Q;
+#pragma unroll 7
+      for (uint32_t tj = 0; tj < kw; ++tj) {
+        const int ax = (int)x + pw - (int)(tj * dw);
+        const uint32_t ox = (uint32_t)ax / sw;
+        v += ax >= 0 && ox * sw == (uint32_t)ax && ox < Q ? zr[(size_t)tj * pq + ox] : 0.f;
+      }
+    }
+    dx[i] = accumulate ? dx[i] + v : v;
+  }
+}
+static int f32_dgrad_few(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
+  const uint32_t M = a->C * a->kh * a->kw, step = (uint32_t)std::min<size_t>(a->N, kFewZ / few_z_bytes(a, P, Q));
+  for (uint32_t n0 = 0; n0 < a->N; n0 += step) {
+    const uint32_t n = std::min(step, a->N - n0);
+    GemmF32 p = {};
+    p.in_pitch = y_pitch; p.in_plane = y_plane; p.in_img = y_plane * a->K;
+    p.in = (const float*)a->y + (long long)n0 * p.in_img; p.w = (const float*)a->w; p.out = (float*)a->scratch;
+    p.M = M; p.CR = a->K; p.NI = n; p.IH = P; p.IW = Q;
+    p.OH = P; p.OW = Q; p.out_pitch = Q; p.out_plane = (long long)P * Q; p.out_img = p.out_plane * M;
+    p.w_m = 1; p.w_c = M;
+    p.kh = p.kw = p.sh = p.sw = p.dh = p.dw = 1;
+    const int rc = run_gemm_f32<false>(p, s);
+    if (rc != AD_OK) return rc;
+    launch(dgrad_few_sum, grid_for((size_t)n * a->C * a->H * a->W, 256, 16), 256, 0, s, (const float*)a->scratch,
+           (float*)a->dx + (size_t)n0 * a->C * a->H * a->W, n, a->C, a->H, a->W, P, Q, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h,
+           a->dil_w, (int)a->pad_h, (int)a->pad_w, a->accumulate);
+    count_launch();
+  }
+  return launch_status();
+}
+
 int f32_gemm_dgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
+  const size_t need = f32_dgrad_scratch(a, P, Q);
+  if (need && a->scratch && a->scratch_bytes >= need) return f32_dgrad_few(a, P, Q, y_pitch, y_plane, s);
   GemmF32 p = {};
   p.in = (const float*)a->y; p.w = (const float*)a->w; p.out = (float*)a->dx;
   p.M = a->C; p.CR = a->K; p.NI = a->N; p.IH = P; p.IW = Q;

@@ -647,6 +647,10 @@ void CudnnConv2DOpF::_backward(TxnId txn) {
     a.accumulate = mode == 1 ? 1 : 0;
     if (f32) {
       a.w = kd.val.get(txn, id()).dptr();
+      if (const size_t need = ad_conv2d_scratch_bytes(&a, 1)) {
+        g->reserve_scratch(need);
+        a.scratch = g->get_scratch(); a.scratch_bytes = g->scratch_size();
+      }
       AD_CHECK(ad_conv2d_dgrad(&a, s));
     } else {
       a.w = w_bf16_;

@@ -63,3 +63,28 @@ def test_conv_f32_tiles(case):
     assert H.max_rel(H.host(gdx) - 1, dx_w) < 1e-5
     assert H.max_rel(H.host(gdw), dw_w) < 2e-5
     assert H.max_rel(H.host(gdb), db_w) < 2e-5
+
+
+@pytest.mark.parametrize("case", [(2, 3, 40, 44, 64, 7, 2, 1, 3), (3, 1, 19, 23, 17, 3, 1, 2, 0), (1, 8, 30, 21, 33, 5, 3, 1, 1), (2, 3, 17, 18, 20, 2, 3, 1, 0)])
+@pytest.mark.parametrize("accumulate", [0, 1])
+def test_data_gradient_into_few_channels(case, accumulate):
+    """The two-step form that a caller's scratch allows."""
+    import torch
+    N, Cc, Hh, W, K, k, s, d, pd = case
+    w = H.normal(2, (K, Cc, k, k), float(np.sqrt(2.0 / (k * k * Cc))))
+    P, Q = ((n + 2 * pd - d * (k - 1) - 1) // s + 1 for n in (Hh, W))
+    dy = H.uniform(4, (N, K, P, Q))
+    want = orc.conv2d_dgrad(dy, w, (N, Cc, Hh, W), (s, s), (d, d), (pd, pd), omp=True)
+    L = abi.lib()
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, want.shape, K, k, s, d, pd)
+    need = L.ad_conv2d_scratch_bytes(C.byref(a), 1)
+    assert need == N * P * Q * Cc * k * k * 4
+    scratch, dx = torch.full((need,), 255, dtype=torch.uint8, device="cuda"), torch.ones(want.shape, device="cuda")
+    gy = torch.full((N, K, P + 1, Q + 3), float("nan"), device="cuda")
+    gy[:, :, :P, :Q] = H.dev(dy)
+    dw_ = H.dev(w)
+    a.y_pitch, a.y_plane = Q + 3, (P + 1) * (Q + 3)
+    a.y, a.w, a.dx, a.scratch, a.scratch_bytes, a.accumulate = gy.data_ptr(), dw_.data_ptr(), dx.data_ptr(), scratch.data_ptr(), need, accumulate
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    H.sync()
+    assert np.max(np.abs(H.host(dx) - accumulate - want)) < 1e-5 * np.max(np.abs(want)) + accumulate * 2e-6
