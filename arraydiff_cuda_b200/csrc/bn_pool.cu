@@ -58,11 +58,16 @@ __global__ void __launch_bounds__(256) bn_reduce_xfast(BnRed p, float* partial) 
   const uint32_t c = blockIdx.x, split = blockIdx.y, nsplit = gridDim.y;
   const size_t per = (size_t)p.N * p.H * p.W;
   float a = 0.f, b = 0.f;
-  for (size_t i = (size_t)split * 256 + threadIdx.x; i < per; i += (size_t)nsplit * 256) {
-    uint32_t x = (uint32_t)(i % p.W);
-    size_t r = i / p.W;
-    uint32_t y = (uint32_t)(r % p.H), n = (uint32_t)(r / p.H);
+  // the position moves on by the same (images, rows, columns) each time: no division per element
+  const size_t first = (size_t)split * 256 + threadIdx.x, hop = (size_t)nsplit * 256;
+  const uint32_t hx = (uint32_t)(hop % p.W), hy = (uint32_t)(hop / p.W % p.H), hn = (uint32_t)(hop / p.W / p.H);
+  uint32_t x = (uint32_t)(first % p.W), y = (uint32_t)(first / p.W % p.H), n = (uint32_t)(first / p.W / p.H);
+#pragma unroll 4
+  for (size_t i = first; i < per; i += hop) {
     bn_term<T, MODE>(p, n, c, y, x, a, b);
+    x += hx; y += hy; n += hn;
+    if (x >= p.W) { x -= p.W; ++y; }
+    if (y >= p.H) { y -= p.H; ++n; }
   }
   __shared__ float sa[8], sb[8];
   a = warp_sum(a); b = warp_sum(b);

@@ -375,59 +375,74 @@ __global__ void __launch_bounds__(256) im2col_vec_kernel(View x, uint32_t N, uin
 // shared memory as bf16 (zeros past the tensor's edge), a table maps each column to its offset inside the
 // staged rows, and every thread then assembles 16-byte pieces of the output from shared memory.  Each input
 // element is fetched from global memory once per output row instead of once per patch that holds it.
-template <typename T>
-__global__ void __launch_bounds__(256) im2col_row_kernel(View x, uint32_t C, uint32_t H, uint32_t W, uint32_t kh, uint32_t kw,
+template <typename T, bool EVEN>
+__global__ void __launch_bounds__(512) im2col_row_kernel(View x, uint32_t C, uint32_t H, uint32_t W, uint32_t kh, uint32_t kw,
                                                          uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, uint32_t P,
-                                                         uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen) {
+                                                         uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen, uint32_t qseg) {
   grid_dependency();
   extern __shared__ __align__(16) unsigned char im2col_smem[];
   __nv_bfloat16* rows = (__nv_bfloat16*)im2col_smem;                                    // [kh][rowlen]
-  uint32_t* tab = (uint32_t*)(im2col_smem + (((size_t)kh * rowlen * 2 + 15) & ~(size_t)15));  // [ldo]
-  const uint32_t p = blockIdx.x % P, n = blockIdx.x / P, cols = kh * kw * C;
-  for (uint32_t t = threadIdx.x; t < ldo; t += 256) {
-    uint32_t e = 0xffffffffu;
-    if (t < cols) { const uint32_t c = t % C, tap = t / C, s = tap % kw, r = tap / kw; e = r * rowlen + s * dw * C + c; }
-    tab[t] = e;
-  }
+  const uint32_t segs = (Q + qseg - 1) / qseg, q0 = blockIdx.x % segs * qseg, row = blockIdx.x / segs;
+  const uint32_t p = row % P, n = row / P, cols = kh * kw * C, nq = Q - q0 < qseg ? Q - q0 : qseg;
   const bool packed = x.sc == 1 && x.sx == (long long)C;
-  for (uint32_t r = 0; r < kh; ++r) {
-    const uint32_t yy = p * sh + r * dh;
-    const T* src = (const T*)x.base + n * x.sn + yy * x.sy;
-    for (uint32_t e = threadIdx.x; e < rowlen; e += 256) {
-      float v = 0.f;
-      if (yy < H) {
-        if (packed) { if (e < W * C) v = ld_f(src + e); }
-        else { const uint32_t xx = e / C, c = e - xx * C; if (xx < W) v = ld_f(src + xx * x.sx + c * x.sc); }
-      }
-      rows[r * rowlen + e] = __float2bfloat16_rn(v);
-    }
-  }
-  __syncthreads();
-  const uint32_t groups = ldo / 8;
-  __nv_bfloat16* orow = out + ((size_t)n * P + p) * Q * ldo;
-  const unsigned short* rs = (const unsigned short*)rows;
-  for (uint32_t it = threadIdx.x; it < Q * groups; it += 256) {
-    const uint32_t q = it / groups, g = it - q * groups, base = q * sw * C;
-    uint32_t w[4];
+  const T* src = (const T*)x.base + n * x.sn + (long long)p * sh * x.sy + (long long)q0 * sw * x.sx;
+  const uint32_t left = W - q0 * sw;   // input columns from the segment's first on
+  const uint32_t have = packed ? (left * C < rowlen ? left * C : rowlen) : 0u;
+  // eight rows at a time, so that a thread's loads are in flight together
+  for (uint32_t r0 = 0; r0 < kh; r0 += 8)
+    for (uint32_t e = threadIdx.x; e < rowlen; e += blockDim.x) {
+      float v[8];
+      const uint32_t xx = packed ? 0u : e / C, c = packed ? e : e - xx * C;
+      const T* at = src + (long long)(r0 * dh) * x.sy + (packed ? (long long)e : xx * x.sx + c * x.sc);
+      const bool ok = packed ? e < have : xx < left;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint32_t e0 = tab[g * 8 + 2 * j], e1 = tab[g * 8 + 2 * j + 1];
-      const uint32_t lo = e0 == 0xffffffffu ? 0u : rs[e0 + base], hi = e1 == 0xffffffffu ? 0u : rs[e1 + base];
-      w[j] = lo | (hi << 16);
+      for (uint32_t r = 0; r < 8; ++r) {
+        v[r] = ok && r0 + r < kh && p * sh + (r0 + r) * dh < H ? ld_f(at) : 0.f;
+        at += (long long)dh * x.sy;
+      }
+#pragma unroll
+      for (uint32_t r = 0; r < 8; ++r)
+        if (r0 + r < kh) rows[(r0 + r) * rowlen + e] = __float2bfloat16_rn(v[r]);
     }
-    *(uint4*)(orow + (size_t)q * ldo + g * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+  __syncthreads();
+  // A thread stays with a pair of columns and walks the pixels, so where the pair lies in the rows is in registers; a warp
+  // writes 128 contiguous bytes from 32 adjacent words of shared memory.  EVEN: the first of a pair is always at an even
+  // element, so that one 32-bit load brings both unless they are in different rows.  Bound by the stores:
+  // 7x7 x 3 stem, 1,048,576 pixels x 192: 147 us; with 8 columns per thread, a table of offsets in shared memory and a whole
+  // output row per block 183.
+  const uint32_t pairs = ldo / 2, pb = pairs < blockDim.x ? pairs : blockDim.x, lanes = blockDim.x / pb, step = sw * C;
+  uint32_t* orow = (uint32_t*)(out + (((size_t)n * P + p) * Q + q0) * ldo);
+  const unsigned short* rs = (const unsigned short*)rows;
+  if (threadIdx.x >= pb * lanes) return;
+  for (uint32_t pr = threadIdx.x % pb; pr < pairs; pr += pb) {
+    uint32_t e[2], mask = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t t = pr * 2 + h, c = t % C, tap = t / C, s = tap % kw, r = tap / kw;
+      e[h] = t < cols ? r * rowlen + s * dw * C + c : 0u;
+      if (t < cols) mask |= 0xffffu << (16 * h);
+    }
+    const bool split = !EVEN || (mask == 0xffffffffu && e[1] != e[0] + 1);
+#pragma unroll 4
+    for (uint32_t q = threadIdx.x / pb; q < nq; q += lanes) {
+      uint32_t w = EVEN ? *(const uint32_t*)(rs + e[0] + q * step) : rs[e[0] + q * step];
+      if (split) w = (w & 0xffffu) | ((uint32_t)rs[e[1] + q * step] << 16);
+      orow[(size_t)q * pairs + pr] = w & mask;
+    }
   }
 }
 template <typename T>
 static int launch_im2col_row(const View& v, const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh,
-                             uint32_t dw, uint32_t P, uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen, size_t smem,
+                             uint32_t dw, uint32_t P, uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen, uint32_t qseg, size_t smem,
                              cudaStream_t s) {
-  auto kern = im2col_row_kernel<T>;
+  const bool even = dw == 1 && ((sw * x->C) & 1u) == 0;   // and the row pitch has the parity of a row of taps
+  auto kern = even ? im2col_row_kernel<T, true> : im2col_row_kernel<T, false>;
+  const uint32_t pairs = ldo / 2, threads = pairs > 256 ? 256 : 384 / pairs * pairs > 384 ? 384 : (384 / pairs * pairs + 31) / 32 * 32;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  launch(kern, x->N * P, 256, smem, s, v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, out, ldo, rowlen);
+  launch(kern, x->N * P * ((Q + qseg - 1) / qseg), threads, smem, s, v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, out, ldo, rowlen, qseg);
   return AD_OK;
 }
 }  // namespace adk
@@ -441,12 +456,15 @@ extern "C" int ad_im2col(const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t
   adk::View v = adk::view_of(x);
   if ((ldo & 7u) == 0 && ((uintptr_t)out_bf16 & 15u) == 0) {
     // staged-row form when the rows of one output row fit shared memory
-    const uint32_t rowlen = ((Q - 1) * sw + (kw - 1) * dw + 1) * x->C;
-    const size_t smem = (((size_t)kh * rowlen * 2 + 15) & ~(size_t)15) + (size_t)ldo * 4;
-    if (smem <= 100 * 1024 && (size_t)x->N * P < (1ull << 31) && (size_t)Q * (ldo / 8) < (1ull << 31)) {
+    // of the parity of a row of taps, so that (dilation 1) a pair of columns starts at an even element in every row
+    const uint32_t qseg = Q < 128 ? Q : 128;   // output pixels per block: enough blocks per SM to keep the stores going
+    uint32_t rowlen = ((qseg - 1) * sw + (kw - 1) * dw + 1) * x->C;
+    rowlen += (rowlen ^ (kw * x->C)) & 1u;
+    const size_t smem = (((size_t)kh * rowlen * 2 + 15) & ~(size_t)15) + 16;   // a masked pair may read past the last element
+    if (smem <= 100 * 1024 && (size_t)x->N * P * Q < (1ull << 31) && (size_t)Q * (ldo / 8) < (1ull << 31)) {
       int st = AD_OK;
       AD_DISPATCH_DTYPE(x->dtype, (st = adk::launch_im2col_row<T>(v, x, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo,
-                                                                  rowlen, smem, adk::as_stream(stream))));
+                                                                  rowlen, qseg, smem, adk::as_stream(stream))));
       if (st != AD_OK) return st;
       adk::count_launch();
       return adk::launch_status();
