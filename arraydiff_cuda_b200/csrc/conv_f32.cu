@@ -310,49 +310,90 @@ __global__ void __launch_bounds__(kF32Group, 3) conv_gemm_f32(const GemmF32 p) {
   if (cs > 1) cluster.sync();         // nobody leaves while its tile is still read
 }
 
-template <typename Kernel, typename Params>
-static int launch_f32(Kernel k, dim3 grid, int threads, int smem, uint32_t cs, const Params& p, unsigned& attr_done, cudaStream_t s) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(attr_done & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
-      cudaGetLastError();
-      return AD_ERR_CUDA;
-    }
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
-    attr_done |= 1u << (dev & 31);
-  }
+// What the launches of one kernel share: on which devices (a bit each) its limits are raised, and how many clusters of
+// 1, 2, 4, 8, 16 CTAs the machine holds at a time (0: not asked yet).  That is less than CTAs per SM x 148 / size: a
+// cluster stays within one group of SMs.
+struct F32Launch { unsigned raised = 0; uint32_t held[5] = {}; };
+
+template <typename Params>
+static cudaLaunchConfig_t f32_config(void (*)(Params), dim3 grid, int threads, int smem, uint32_t cs, cudaLaunchAttribute* at, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = (size_t)smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.numAttrs = cs > 1 ? 1 : 0;
   cfg.attrs = at;
+  return cfg;
+}
+template <typename Params>
+static int raise_f32(void (*k)(Params), int smem, F32Launch& l) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (l.raised & (1u << (dev & 31))) return AD_OK;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return AD_ERR_CUDA;
+  }
+  l.raised |= 1u << (dev & 31);
+  return AD_OK;
+}
+template <typename Params>
+static int launch_f32(void (*k)(Params), dim3 grid, int threads, int smem, uint32_t cs, const Params& p, F32Launch& l, cudaStream_t s) {
+  if (int rc = raise_f32(k, smem, l)) return rc;
+  cudaLaunchAttribute at[1];
+  const cudaLaunchConfig_t cfg = f32_config(k, grid, threads, smem, cs, at, s);
   if (cudaLaunchKernelEx(&cfg, k, p) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
   count_launch();
   return launch_status();
 }
+template <typename Params>
+static uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, F32Launch& l) {
+  uint32_t i = 0;
+  while ((1u << i) < cs) ++i;
+  if (!l.held[i]) {
+    cudaLaunchAttribute at[1];
+    cudaLaunchConfig_t cfg = f32_config(k, dim3(cs), threads, smem, cs, at, nullptr);
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (raise_f32(k, smem, l) != AD_OK || cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = (int)(kNumSMs / cs); }
+    l.held[i] = (uint32_t)n;
+  }
+  return l.held[i];
+}
 
-// CTAs that share one tile: until the grid holds `want` CTAs, each with at least four stages of reduction
-static uint32_t f32_cluster(unsigned long long tiles, unsigned long long want, uint32_t steps, uint32_t most) {
-  uint32_t cs = 1;
-  while (cs < most && tiles * cs * 2 <= want && steps >= 8 * cs) cs *= 2;
-  return cs;
+// CTAs that share one tile's reduction of `steps` stages: the size with the shortest time by a count of waves.  A CTA costs
+// its stages and about six more to start and finish; one CTA on an SM takes 2.2 per stage, two 2.5, three 3 (12 warps hide
+// most of what they wait for).  Of the sizes 1 .. 16 this picks the fastest or one within a tenth of it for 18 of 20 layers
+// measured.  Before, the size went by CTAs per SM alone: 35 clusters of 8 where the machine holds 33
+// took two waves (filter gradient 64 -> 64, 4 x 112 x 112: 228 us against 168 for 30).
+template <typename Params>
+static uint32_t f32_cluster(void (*k)(Params), int threads, int smem, F32Launch& l, unsigned long long tiles, uint32_t steps, uint32_t most) {
+  static const double per_stage[4] = {0, 2.2, 2.5, 3.0};
+  uint32_t best = 1;
+  double best_cost = 0;
+  for (uint32_t cs = 1; cs <= most && (cs == 1 || steps >= 4 * cs); cs *= 2) {
+    const unsigned long long held = f32_held(k, threads, smem, cs, l);
+    auto wave = [&](unsigned long long clusters) { return per_stage[std::min<unsigned long long>((clusters * cs + kNumSMs - 1) / kNumSMs, 3)]; };
+    const double cta = (steps + cs - 1) / cs + 6, cost = cta * (tiles / held * wave(held) + (tiles % held ? wave(tiles % held) : 0));
+    if (cs == 1 || cost < best_cost) { best = cs; best_cost = cost; }
+  }
+  return best;
 }
 
 template <int LM, int WM, int WN, bool DGRAD>
 static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uint32_t Kd, cudaStream_t s) {
   typedef GemmTile<LM, WM, WN> T;
-  static unsigned attr_done = 0;      // one bit per device
+  static F32Launch l;
   const uint32_t tn = (npx + T::BN - 1) / T::BN, tm = (p.M + T::BM - 1) / T::BM;
-  // three CTAs per SM are resident; every CTA of a cluster finishes at least one of the BM rows.  Clusters of 16 are for few
-  // tiles and long reductions: 4 x 512 x 7 x 7 -> 512, 3x3 (16 tiles) 92 -> 67 us against 8.
-  const uint32_t cs = f32_cluster((unsigned long long)tn * tm * classes, 3ull * kNumSMs, Kd / T::KB, std::min(kF32Most, (int)T::BM));
-  return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, attr_done, s);
+  // every CTA of a cluster finishes at least one of the BM rows.  Clusters of 16 are for few tiles and long reductions:
+  // 4 x 512 x 7 x 7 -> 512, 3x3 (16 tiles) 92 -> 67 us against 8.
+  const uint32_t cs = f32_cluster(conv_gemm_f32<LM, WM, WN, DGRAD>, T::threads, T::smem, l, (unsigned long long)tn * tm * classes, Kd / T::KB,
+                                  std::min(kF32Most, (int)T::BM));
+  return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, l, s);
 }
 
 // Tile height by the row count: a row of the tile costs the same FMAs whether it holds a channel or not, a column is
@@ -544,13 +585,14 @@ __global__ void __launch_bounds__(256) wgrad_f32_finish(size_t n, uint32_t K, ui
 
 static uint32_t wg_rows(uint32_t K) { return K > 32 ? 64u : (K > 16 ? 32u : 16u); }
 static uint32_t wg_cols(uint32_t K) { return 8192u / wg_rows(K); }
-// Slices of the pixel range beyond a cluster of 8: until the grid holds two CTAs per SM, each with at least eight
-// stages of pixels
+// Slices of the pixel range beyond a cluster of 8, each CTA with at least eight stages of pixels: as many clusters as the
+// machine holds at a time with two CTAs per SM
+constexpr unsigned long long kWgHeld = 33;
 static uint32_t wg_slices(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
   const unsigned long long tiles = (unsigned long long)((a->K + wg_rows(a->K) - 1) / wg_rows(a->K)) *
                                    ((a->C * a->kh * a->kw + wg_cols(a->K) - 1) / wg_cols(a->K));
   const unsigned long long steps = ((unsigned long long)a->N * P * Q + kWgKB - 1) / kWgKB;
-  const unsigned long long fit = 2ull * kNumSMs / (tiles * 8), most = steps / (8 * 8);
+  const unsigned long long fit = kWgHeld / tiles, most = steps / (8 * 8);
   const unsigned long long n = fit < most ? fit : most;
   return (uint32_t)(n > 16 ? 16 : (n < 1 ? 1 : n));
 }
@@ -558,10 +600,12 @@ static uint32_t wg_slices(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
 template <int LM, int WM, int WN, int G>
 static int launch_wgrad_f32(WgradF32& p, cudaStream_t s) {
   typedef WgTile<LM, WM, WN, G> T;
-  static unsigned attr_done = 0;      // one bit per device
+  static F32Launch l;
   const uint32_t tn = (p.C * p.kh * p.kw + T::BN - 1) / T::BN, tm = (p.K + T::BM - 1) / T::BM;
-  const uint32_t cs = f32_cluster((unsigned long long)tn * tm * p.slices, (G == 1 ? 2ull : 1ull) * kNumSMs, p.N * p.P * p.Q / (kWgKB * G) / p.slices, 8);
-  int st = launch_f32(conv_wgrad_gemm_f32<LM, WM, WN, G>, dim3(tn * cs, tm, p.slices), T::threads, T::smem, cs, p, attr_done, s);
+  const uint32_t steps = p.N * p.P * p.Q / (kWgKB * G) / p.slices;
+  const uint32_t cs = p.slices > 1 ? 8u
+                                   : f32_cluster(conv_wgrad_gemm_f32<LM, WM, WN, G>, T::threads, T::smem, l, (unsigned long long)tn * tm, steps, 8);
+  int st = launch_f32(conv_wgrad_gemm_f32<LM, WM, WN, G>, dim3(tn * cs, tm, p.slices), T::threads, T::smem, cs, p, l, s);
   if (st != AD_OK || p.slices == 1) return st;
   const size_t n = (size_t)p.K * p.C * p.kh * p.kw;
   launch(wgrad_f32_finish, (unsigned)((n + p.K + 255) / 256), 256, 0, s, n, p.K, p.slices, p.part, p.dw, p.db, p.accumulate);
@@ -590,7 +634,7 @@ size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
 
 // Measured (one B200; per call, before -> now): 64 -> 64 channels, 3x3, 64 x 64 pixels, one image: forward 188 -> 19 us, data
 // gradient 158 -> 23, filter and bias gradient 286 -> 29.  4 x 64 x 112 x 112, 64 -> 64 3x3: 1440 -> 127, 1500 -> 125, 2330 ->
-// 222 us (29 / 30 / 17 TFLOP/s).  What is left above the FMA pipe: 12 warps per SM do not hide the latency of the
+// 168 us (29 / 30 / 22 TFLOP/s).  What is left above the FMA pipe: 12 warps per SM do not hide the latency of the
 // shared-memory reads (issue slots 42 % busy); 4 x 8 outputs per thread or packed pairs along the reduction were slower.
 int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
   GemmF32 p = {};
