@@ -208,10 +208,111 @@ __global__ void __launch_bounds__(256) ce_nhwc_reg(uint32_t C, size_t pixels, co
   }
 }
 
-// Few classes (C <= 32, e.g. 19): a block stages 256 consecutive pixels in shared memory as they are (16-byte vectors), a
-// thread then owns one pixel, results leave by vectors again.  One tile per block, 8 blocks per SM: the loads of one
-// block run under the exponentials of the others.  2 x 1024 x 2048 pixels, 19 classes, bf16: forward 89 us,
-// backward 155 -> 115 us (24 and 49 us of logits at the copy rate): what is left is the exponentials' arithmetic.
+// Few classes, bf16: a thread takes two neighbouring pixels, whose 2 C values are C aligned words of shared memory -- a stride
+// that is free of bank conflicts for odd C -- and keeps them in registers.  Tiles of 512 pixels in two buffers: the next
+// tile's copy is in flight while this one is worked on.  Bound by its instructions (an exponential per class).
+// 4,194,304 pixels of 19 classes: 51 us forward, 92 backward; one pixel per thread by 2-byte accesses took 63 and 104 with
+// two buffers, 87 and 117 with one.
+template <int C, bool BWD>
+__global__ void __launch_bounds__(256) ce_nhwc_pair(size_t pixels, int vec, const __nv_bfloat16* __restrict__ x,
+                                                    const uint32_t* __restrict__ label, float* loss, unsigned long long* picked,
+                                                    const float* __restrict__ dloss, __nv_bfloat16* dx, int accumulate) {
+  grid_dependency();
+  extern __shared__ __align__(16) uint32_t ce_words[];   // [2][256 pairs][C]
+  const size_t tiles = (pixels + 511) / 512;
+  auto fetch = [&](size_t tile, uint32_t buf) {
+    if (tile < tiles) {
+      const size_t p0 = tile * 512;
+      const uint32_t np = pixels - p0 < 512 ? (uint32_t)(pixels - p0) : 512u, ne = np * C, nv = vec ? ne / 8 : 0;
+      const __nv_bfloat16* xb = x + p0 * C;
+      uint32_t* sm = ce_words + buf * 256 * C;
+      for (uint32_t q = threadIdx.x; q < nv; q += 256)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared((uint4*)sm + q)), "l"((const uint4*)xb + q) : "memory");
+      for (uint32_t q = nv * 8 + threadIdx.x; q < ne; q += 256) ((__nv_bfloat16*)sm)[q] = xb[q];
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(blockIdx.x, 0);
+  uint32_t buf = 0;
+  for (size_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1u) {
+    const size_t p0 = tile * 512, i = p0 + 2 * threadIdx.x;
+    const uint32_t np = pixels - p0 < 512 ? (uint32_t)(pixels - p0) : 512u, ne = np * C, nv = vec ? ne / 8 : 0;
+    uint32_t l[2];
+    float d[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool mine = 2 * threadIdx.x + h < np;
+      l[h] = mine ? label[i + h] : 0;
+      d[h] = BWD && mine ? dloss[i + h] : 0.f;
+    }
+    fetch(tile + gridDim.x, buf ^ 1u);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    uint32_t *sm = ce_words + buf * 256 * C, *px = sm + threadIdx.x * C;
+    if (2 * threadIdx.x < np) {
+      float v[2 * C];
+#pragma unroll
+      for (int k = 0; k < C; ++k) {   // an odd last pixel leaves half of its pair's words undefined: computed, not written
+        const uint32_t w = px[k];
+        v[2 * k] = __uint_as_float(w << 16);
+        v[2 * k + 1] = __uint_as_float(w & 0xffff0000u);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float m = v[h * C], z = 0.f;
+#pragma unroll
+        for (int c = 1; c < C; ++c) m = fmaxf(m, v[h * C + c]);
+        if (!BWD) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) z += expf(v[h * C + c] - m);
+          if (2 * threadIdx.x + h < np) {
+            loss[i + h] = (logf(z) + m) - ld_f((const __nv_bfloat16*)px + h * C + l[h]);
+            if (picked) picked[i + h] = (i + h) * C + l[h];
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < C; ++c) { v[h * C + c] = expf(v[h * C + c] - m); z += v[h * C + c]; }
+          const float rz = 1.f / z;
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            float g = d[h] * (v[h * C + c] * rz - (c == (int)l[h] ? 1.f : 0.f));
+            if (accumulate && 2 * threadIdx.x + h < np) g += ld_f(dx + (i + h) * C + c);
+            v[h * C + c] = g;
+          }
+        }
+      }
+      if (BWD) {
+#pragma unroll
+        for (int k = 0; k < C; ++k) {
+          const __nv_bfloat162 g = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+          px[k] = *reinterpret_cast<const uint32_t*>(&g);
+        }
+      }
+    }
+    if (BWD) {
+      __syncthreads();
+      __nv_bfloat16* db = dx + p0 * C;
+      for (uint32_t q = threadIdx.x; q < nv; q += 256) ((uint4*)db)[q] = ((const uint4*)sm)[q];
+      for (uint32_t q = nv * 8 + threadIdx.x; q < ne; q += 256) db[q] = ((const __nv_bfloat16*)sm)[q];
+    }
+    __syncthreads();   // the buffer is free for the tile after the next
+  }
+}
+template <bool BWD, int C = 1, typename... A>
+static int launch_ce_pair(uint32_t classes, size_t pixels, cudaStream_t s, A... args) {
+  if constexpr (C <= 32) {
+    if (classes != (uint32_t)C) return launch_ce_pair<BWD, C + 1>(classes, pixels, s, args...);
+    constexpr int smem = 2 * 256 * C * 4;
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(ce_nhwc_pair<C, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      cudaGetLastError();
+      return AD_ERR_CUDA;
+    }
+    launch(ce_nhwc_pair<C, BWD>, grid_for((pixels + 511) / 512, 1, 5), 256, smem, s, pixels, args...);
+    return AD_OK;
+  } else return AD_ERR_UNSUPPORTED;
+}
+
+// Few classes (C <= 32), fp32: a thread owns one pixel of a tile in shared memory, results leave by vectors again.
 // CM: C rounded up to a multiple of 4 (the class loops are unrolled; a class past C is -inf and adds nothing).
 template <typename T, int CM, bool BWD>
 __global__ void __launch_bounds__(256) ce_nhwc_small(uint32_t C, size_t pixels, int vec, const T* __restrict__ x,
@@ -219,53 +320,74 @@ __global__ void __launch_bounds__(256) ce_nhwc_small(uint32_t C, size_t pixels, 
                                                       unsigned long long* picked, const float* __restrict__ dloss, T* dx,
                                                       int accumulate) {
   grid_dependency();
-  extern __shared__ __align__(16) uint8_t ce_raw[];   // [256][C]
-  T* sm = (T*)ce_raw;
+  // Tiles of 256 pixels, two buffers: the next tile's copy is in flight while this one is worked on (one tile per block
+  // waited for memory most of the time)
+  extern __shared__ __align__(16) uint8_t ce_raw[];   // [2][256][C]
   constexpr uint32_t V = 16 / sizeof(T);
-  const size_t p0 = (size_t)blockIdx.x * 256;
-  const uint32_t np = pixels - p0 < 256 ? (uint32_t)(pixels - p0) : 256u, ne = np * C, nv = vec ? ne / V : 0;
-  const T* xb = x + p0 * C;
-  const size_t i = p0 + threadIdx.x;
-  const bool mine = threadIdx.x < np;
-  const uint32_t l = mine ? label[i] : 0;
-  const float d = BWD && mine ? dloss[i] : 0.f;
-  for (uint32_t e = threadIdx.x; e < nv; e += 256) ((uint4*)sm)[e] = ((const uint4*)xb)[e];
-  for (uint32_t e = nv * V + threadIdx.x; e < ne; e += 256) sm[e] = xb[e];
-  __syncthreads();
-  if (mine) {
-    T* px = sm + threadIdx.x * C;
-    float m = -INFINITY, v[CM];
-#pragma unroll
-    for (uint32_t c = 0; c < CM; ++c) {
-      v[c] = c + 4 < CM || c < C ? ld_f(px + c) : -INFINITY;
-      m = fmaxf(m, v[c]);
+  const size_t tiles = (pixels + 255) / 256;
+  uint32_t l = 0, ln = 0;
+  float d = 0.f, dn = 0.f;
+  auto fetch = [&](size_t tile, uint32_t buf) {
+    if (tile < tiles) {
+      const size_t p0 = tile * 256;
+      const uint32_t np = pixels - p0 < 256 ? (uint32_t)(pixels - p0) : 256u, ne = np * C, nv = vec ? ne / V : 0;
+      const T* xb = x + p0 * C;
+      T* sm = (T*)ce_raw + buf * 256 * C;
+      for (uint32_t q = threadIdx.x; q < nv; q += 256)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared((uint4*)sm + q)), "l"((const uint4*)xb + q) : "memory");
+      for (uint32_t q = nv * V + threadIdx.x; q < ne; q += 256) sm[q] = xb[q];
+      ln = threadIdx.x < np ? label[p0 + threadIdx.x] : 0;
+      dn = BWD && threadIdx.x < np ? dloss[p0 + threadIdx.x] : 0.f;
     }
-    float z = 0.f;
-    if (!BWD) {
-      const float vl = ld_f(px + l);
-#pragma unroll
-      for (uint32_t c = 0; c < CM; ++c) z += expf(v[c] - m);
-      loss[i] = (logf(z) + m) - vl;
-      if (picked) picked[i] = i * C + l;
-    } else {
-#pragma unroll
-      for (uint32_t c = 0; c < CM; ++c) { v[c] = expf(v[c] - m); z += v[c]; }
-      const float rz = 1.f / z;
-      const T* old = dx + i * C;
-#pragma unroll
-      for (uint32_t c = 0; c < CM; ++c)
-        if (c + 4 < CM || c < C) {
-          float g = d * (v[c] * rz - (c == l ? 1.f : 0.f));
-          if (accumulate) g += ld_f(old + c);
-          st_f(px + c, g);
-        }
-    }
-  }
-  if (BWD) {
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(blockIdx.x, 0);
+  uint32_t buf = 0;
+  for (size_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, buf ^= 1u) {
+    l = ln; d = dn;
+    fetch(tile + gridDim.x, buf ^ 1u);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    T* db = dx + p0 * C;
-    for (uint32_t e = threadIdx.x; e < nv; e += 256) ((uint4*)db)[e] = ((const uint4*)sm)[e];
-    for (uint32_t e = nv * V + threadIdx.x; e < ne; e += 256) db[e] = sm[e];
+    T* sm = (T*)ce_raw + buf * 256 * C;
+    const size_t p0 = tile * 256, i = p0 + threadIdx.x;
+    const uint32_t np = pixels - p0 < 256 ? (uint32_t)(pixels - p0) : 256u, ne = np * C, nv = vec ? ne / V : 0;
+    const bool mine = threadIdx.x < np;
+    if (mine) {
+      T* px = sm + threadIdx.x * C;
+      float m = -INFINITY, v[CM];
+  #pragma unroll
+      for (uint32_t c = 0; c < CM; ++c) {
+        v[c] = c + 4 < CM || c < C ? ld_f(px + c) : -INFINITY;
+        m = fmaxf(m, v[c]);
+      }
+      float z = 0.f;
+      if (!BWD) {
+        const float vl = ld_f(px + l);
+  #pragma unroll
+        for (uint32_t c = 0; c < CM; ++c) z += expf(v[c] - m);
+        loss[i] = (logf(z) + m) - vl;
+        if (picked) picked[i] = i * C + l;
+      } else {
+  #pragma unroll
+        for (uint32_t c = 0; c < CM; ++c) { v[c] = expf(v[c] - m); z += v[c]; }
+        const float rz = 1.f / z;
+        const T* old = dx + i * C;
+  #pragma unroll
+        for (uint32_t c = 0; c < CM; ++c)
+          if (c + 4 < CM || c < C) {
+            float g = d * (v[c] * rz - (c == l ? 1.f : 0.f));
+            if (accumulate) g += ld_f(old + c);
+            st_f(px + c, g);
+          }
+      }
+    }
+    if (BWD) {
+      __syncthreads();
+      T* db = dx + p0 * C;
+      for (uint32_t q = threadIdx.x; q < nv; q += 256) ((uint4*)db)[q] = ((const uint4*)sm)[q];
+      for (uint32_t q = nv * V + threadIdx.x; q < ne; q += 256) db[q] = sm[q];
+    }
+    __syncthreads();   // the buffer is free for the tile after the next
   }
 }
 
@@ -282,18 +404,27 @@ static int launch_ce(int32_t layout, uint32_t N, uint32_t C, uint32_t HW, const 
     else launch(ce_fwd_nchw<T>, grid_for(pixels, 256), 256, 0, s, N, C, HW, x, label, loss, picked);
   } else if (C <= 32 && pixels <= (1ull << 31) * 256 - 256) {
     const int vec = ((uintptr_t)x & 15u) == 0 && (!BWD || ((uintptr_t)dx & 15u) == 0);
-    auto go = [&](auto kernel) {
-      launch(kernel, (unsigned)((pixels + 255) / 256), 256, 256 * C * sizeof(T), s, C, pixels, vec, x, label, loss, picked, dloss, dx, accumulate);
-    };
-    switch ((C + 3) / 4) {
-      case 1: go(ce_nhwc_small<T, 4, BWD>); break;
-      case 2: go(ce_nhwc_small<T, 8, BWD>); break;
-      case 3: go(ce_nhwc_small<T, 12, BWD>); break;
-      case 4: go(ce_nhwc_small<T, 16, BWD>); break;
-      case 5: go(ce_nhwc_small<T, 20, BWD>); break;
-      case 6: go(ce_nhwc_small<T, 24, BWD>); break;
-      case 7: go(ce_nhwc_small<T, 28, BWD>); break;
-      default: go(ce_nhwc_small<T, 32, BWD>); break;
+    if constexpr (sizeof(T) == 2) {
+      const int rc = launch_ce_pair<BWD>(C, pixels, s, vec, x, label, loss, picked, dloss, dx, accumulate);
+      if (rc != AD_OK) return rc;
+    } else {
+      const int smem = (int)(2 * 256 * C * sizeof(T));
+      bool ok = true;
+      auto go = [&](auto kernel) {
+        if (smem > 48 * 1024) ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+        if (ok) launch(kernel, grid_for((pixels + 255) / 256, 1, 6), 256, smem, s, C, pixels, vec, x, label, loss, picked, dloss, dx, accumulate);
+      };
+      switch ((C + 3) / 4) {
+        case 1: go(ce_nhwc_small<T, 4, BWD>); break;
+        case 2: go(ce_nhwc_small<T, 8, BWD>); break;
+        case 3: go(ce_nhwc_small<T, 12, BWD>); break;
+        case 4: go(ce_nhwc_small<T, 16, BWD>); break;
+        case 5: go(ce_nhwc_small<T, 20, BWD>); break;
+        case 6: go(ce_nhwc_small<T, 24, BWD>); break;
+        case 7: go(ce_nhwc_small<T, 28, BWD>); break;
+        default: go(ce_nhwc_small<T, 32, BWD>); break;
+      }
+      if (!ok) { cudaGetLastError(); return AD_ERR_CUDA; }
     }
   } else if (C <= 64) {
     launch(ce_nhwc_reg<T, 2, BWD>, grid_for(pixels, 32), 256, 0, s, C, pixels, x, label, loss, picked, dloss, dx, accumulate);
