@@ -245,6 +245,8 @@ __device__ __forceinline__ const void* at16(const BView& v, long long off) { ret
 
 constexpr int kBnUnroll = 4;      // pixels per thread below which a smaller grid would do (vec_grid)
 constexpr int kBnDepth = 8;       // loads in flight per thread and stream
+// of the gradient with an addend: three streams that fit beside a filter gradient's CTA
+constexpr int bn_depth(bool add) { return add ? 6 : kBnDepth; }
 
 // HBM-bound.  131,072 x 512 bf16 inside a net: 34 -> 27 us (MODE 0), 60 -> 53 us (MODE 1) against batches of 4 loads in
 // registers; 16 in flight gained nothing more.
@@ -295,7 +297,10 @@ __global__ void __launch_bounds__(256, 2) bn_reduce_vec(BnRed p, float* partial)
       }
     }
   }
-  __shared__ float sa[256][9], sb[256][9];
+  // the ring's memory is free once every thread has read its last element
+  float (*sa)[9] = (float (*)[9])ring_smem, (*sb)[9] = sa + 256;
+  static_assert(LoadRing<1, kBnDepth>::kBytes >= 2 * 256 * 9 * 4, "the sums of the lanes fit the ring");
+  __syncthreads();
 #pragma unroll
   for (int j = 0; j < 8; ++j) { sa[threadIdx.x][j] = a[j]; sb[threadIdx.x][j] = b[j]; }
   __syncthreads();
@@ -315,7 +320,7 @@ template <int MODE, bool ADD>
 __global__ void __launch_bounds__(256, 2) bn_apply_vec(BnApply p) {
   grid_dependency();
   extern __shared__ __align__(128) uint4 ring_smem[];
-  LoadRing<MODE + 1 + ADD, kBnDepth> ring(ring_smem);
+  LoadRing<MODE + 1 + ADD, bn_depth(ADD)> ring(ring_smem);
   const uint32_t G = p.C / 8, cg = threadIdx.x % G, pl = threadIdx.x / G, PL = 256 / G;
   const uint32_t per = p.N * p.H * p.W, stride = gridDim.x * PL;
   float sc[8], sh[8], mean[8], invstd[8], m1[8], m2[8];
@@ -336,7 +341,7 @@ __global__ void __launch_bounds__(256, 2) bn_apply_vec(BnApply p) {
   };
   uint32_t i = pl < PL ? blockIdx.x * PL + pl : per;
 #pragma unroll
-  for (int d = 0; d < kBnDepth - 1; ++d) issue(i + d * stride);
+  for (int d = 0; d < bn_depth(ADD) - 1; ++d) issue(i + d * stride);
   for (; i < per; i += stride) {
     ring.wait();
     float xv[8], g[8], old[8], o[8];
@@ -344,7 +349,7 @@ __global__ void __launch_bounds__(256, 2) bn_apply_vec(BnApply p) {
     if (MODE == 1) unpack8(ring.get(MODE), g);
     if (ADD) unpack8(ring.get(MODE + ADD), old);
     ring.next();
-    issue(i + (kBnDepth - 1) * stride);
+    issue(i + (bn_depth(ADD) - 1) * stride);
     if (MODE == 0) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
@@ -384,7 +389,7 @@ static unsigned vec_grid(const ad_tensor4* t) {
 static int ring_smem_failed() { cudaGetLastError(); return AD_ERR_CUDA; }
 template <int MODE, bool ADD>
 static int launch_apply_vec(const BnApply& a, cudaStream_t s) {
-  constexpr int smem = LoadRing<MODE + 1 + ADD, kBnDepth>::kSmem;
+  constexpr int smem = LoadRing<MODE + 1 + ADD, bn_depth(ADD)>::kSmem;
   if (cudaFuncSetAttribute(bn_apply_vec<MODE, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return ring_smem_failed();
   const uint32_t PL = 256 / (a.C / 8), per = a.N * a.H * a.W;
   launch(bn_apply_vec<MODE, ADD>, grid_for(per, PL * kBnUnroll, 2), 256, smem, s, a);

@@ -834,8 +834,9 @@ __global__ void __launch_bounds__(256) pad_channels_kernel(size_t pixels, uint32
 
 // db[k] (+)= sum over pixels of dy[pixel][k] (dense NHWC bf16), in two fixed-order stages: a block sums its share of the
 // pixels into part[block][k], bias_grad_finish adds the blocks in order.  HBM-bound: dy is read once.
-// K a multiple of 8: a thread owns 8 adjacent channels (16-byte loads, four pixels in flight), 256 / (K / 8) pixel lanes
-// per block (K above 2048: channel groups over blockIdx.y).  32 x 512 x 512 pixels of 64 channels: 1200 -> 205 us (5.2 TB/s).
+// K a multiple of 8: a thread owns 8 adjacent channels (16-byte loads, eight pixels in flight), 256 / (K / 8) pixel lanes
+// per block (K above 2048: channel groups over blockIdx.y).  32 x 512 x 512 pixels of 64 channels: 205 us
+// with four pixels in registers, 178 with the ring.
 __device__ __forceinline__ void bias_add8(float (&acc)[8], const uint4& v) {
   const uint32_t* w = &v.x;
 #pragma unroll
@@ -846,15 +847,31 @@ __device__ __forceinline__ void bias_add8(float (&acc)[8], const uint4& v) {
 }
 __global__ void __launch_bounds__(256) bias_grad_vec_kernel(size_t pixels, uint32_t K, uint32_t gb, const __nv_bfloat16* __restrict__ dy, float* part) {
   grid_dependency();
-  __shared__ float red[256][9];
+  typedef LoadRing<1, 8> Ring;
+  __shared__ __align__(128) uint4 ring_smem[Ring::kBytes / 16];
+  Ring ring(ring_smem);
   const uint32_t G = K / 8, gl = threadIdx.x % gb, pl = threadIdx.x / gb, PL = 256 / gb, g = blockIdx.y * gb + gl;
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  if (g < G && pl < PL) {
-    const size_t stride = (size_t)gridDim.x * PL;
-    size_t i = (size_t)blockIdx.x * PL + pl;
-    const uint4* src = (const uint4*)dy + g;
+  const size_t stride = (size_t)gridDim.x * PL;
+  size_t i = g < G && pl < PL ? (size_t)blockIdx.x * PL + pl : pixels;
+  const uint4* src = (const uint4*)dy + g;
+  if (pixels > 16 * stride) {
+    auto issue = [&](size_t at) {
+      if (at < pixels) ring.copy(0, src + at * G);
+      ring.commit();
+    };
+#pragma unroll
+    for (int u = 0; u < 7; ++u) issue(i + u * stride);
+    for (; i < pixels; i += stride) {
+      ring.wait();
+      const uint4 v = ring.get(0);
+      ring.next();
+      issue(i + 7 * stride);
+      bias_add8(acc, v);
+    }
+  } else {   // few pixels per thread: the ring's start costs more than it brings (1 us)
     for (; i + 3 * stride < pixels; i += 4 * stride) {
       uint4 v[4];
 #pragma unroll
@@ -864,6 +881,8 @@ __global__ void __launch_bounds__(256) bias_grad_vec_kernel(size_t pixels, uint3
     }
     for (; i < pixels; i += stride) bias_add8(acc, src[i * G]);
   }
+  float (*red)[9] = (float (*)[9])ring_smem;   // free once every thread has read its last element
+  __syncthreads();
 #pragma unroll
   for (int j = 0; j < 8; ++j) red[threadIdx.x][j] = acc[j];
   __syncthreads();
@@ -1121,7 +1140,9 @@ template <int BN, bool PAIR>
 static int launch_wgrad(const CUtensorMap& mdy, const CUtensorMap& mx, const WgParams& p, cudaStream_t s) {
   constexpr int kCtas = PAIR ? 2 : 1;
   constexpr int kStageBytes = 2 * kSlabBytes + (BN / 64 / kCtas) * kSlabBytes;
-  constexpr int STAGES = (200 * 1024) / kStageBytes;
+  // three stages as a pair: 146 KB leave room for a block of a batch norm pass on the main stream (LoadRing::kSmem), which
+  // waits for memory while this waits for the tensor cores (segmentation net's step 20.1 -> 19.9 ms against four)
+  constexpr int STAGES = PAIR ? 3 : (200 * 1024) / kStageBytes;
   constexpr int smem = STAGES * kStageBytes + 1024 + (int)sizeof(SmemCtl);
   static unsigned attr_done = 0;
   return launch_tc(conv_tc_wgrad_kernel<BN, STAGES, PAIR>, kCtas, p.splits * p.kh * p.kw * (p.ktiles / kCtas) * p.ctiles, kThreads, smem,
