@@ -482,8 +482,12 @@ __global__ void __launch_bounds__(kF32Group * G, G == 1 ? 2 : 1) conv_wgrad_gemm
       for (uint32_t j = 0; j < p.kw; ++j) if ((unsigned)(ix0 + col_t[j]) < p.W) bits |= 1u << (16 + j);
     }
     const float* xp = p.x + (long long)n * x_img + (long long)iy0 * p.W + ix0;
+    // columns past the last (channel, tap) are left as they are: what is summed there is not written (9 columns of 512, one
+    // input channel: most of the time went into zeros)
+    const int rows = (int)(NC - n_base < BN ? NC - n_base : BN) - (int)warp;
 #pragma unroll 16
     for (int i = 0; i < BN / 4; ++i) {
+      if (i * 4 >= rows) break;
       const int2 e = col[warp + i * 4];
       gather4(b0 + i * 4 * PITCH * 4, xp + e.x, bits, (uint32_t)e.y);
     }

@@ -111,14 +111,25 @@ __global__ void __launch_bounds__(64) avgpool_global_nhwc_seq(AvgP p) {
   float acc[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-  for (uint32_t y = 0; y < p.H; ++y)
-#pragma unroll 8
-    for (uint32_t x = 0; x < p.W; ++x) {
+  // 16 pixels in flight, added in their order
+  const uint32_t px = p.H * p.W;
+  uint32_t y = 0, x = 0;
+  for (uint32_t i = 0; i < px; i += 16) {
+    uint4 q[16];
+#pragma unroll
+    for (uint32_t u = 0; u < 16; ++u) {
+      if (i + u < px) q[u] = *(const uint4*)(X + y * p.x.sy + x * p.x.sx);
+      if (++x == p.W) { x = 0; ++y; }
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 16; ++u) {
+      if (i + u >= px) break;
       float v[8];
-      un8(*(const uint4*)(X + y * p.x.sy + x * p.x.sx), v);
+      un8(q[u], v);
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc[j] += v[j];
     }
+  }
   const float inv = 1.0f / (float)(p.H * p.W);
 #pragma unroll
   for (int j = 0; j < 8; ++j) acc[j] *= inv;

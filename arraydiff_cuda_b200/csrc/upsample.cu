@@ -363,8 +363,9 @@ static bool up_rows(const ad_tensor4* lo, const ad_tensor4* hi, bool bwd, UpRowP
     if (r.rb < 1) r.rb = 1;
     while (r.tpr > 8 && r.tpr * 2 >= r.row_len && kUpThreads / r.tpr < r.rb) r.tpr >>= 1;
   }
-  // an even, power-of-two scale whose pairs fit the block (Ci <= 64 at scale 8, <= 256 at 2)
-  r.period = !bwd && u.scale % 2 == 0 && (u.scale & (u.scale - 1)) == 0 && r.Ci * u.scale / 2 <= kUpThreads ? r.Ci * u.scale / 2 : 0;
+  // an even, power-of-two scale whose pairs fit the block (Ci <= 64 at scale 8, <= 256 at 2), rows long enough to keep the
+  // block busy one at a time (short ones share it: the general form)
+  r.period = !bwd && r.rb == 1 && u.scale % 2 == 0 && (u.scale & (u.scale - 1)) == 0 && r.Ci * u.scale / 2 <= kUpThreads ? r.Ci * u.scale / 2 : 0;
   r.wtab = (r.XC + 2) * u.scale * r.Ci + 16;
   r.smem = bwd ? ((r.XC + 2) * u.scale * r.Ci + 16 + 3 * u.scale + 2) * 4 : ((r.rb * (r.XC + 2) * r.Ci + 2) + (r.XC + 2) * 2 * u.scale) * 4;
   return r.smem <= 49152 && (unsigned long long)r.planes * (bwd ? u.XH : u.YH) * r.chunks < (1ull << 31);

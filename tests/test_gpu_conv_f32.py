@@ -29,9 +29,12 @@ CASES = [
 ]
 
 
+@pytest.mark.parametrize("tiles", [None, "1", "0"])   # by size, the tiled kernels, a thread per output
 @pytest.mark.parametrize("case", CASES)
-def test_conv_f32_tiles(case):
+def test_conv_f32_tiles(case, tiles, monkeypatch):
     import torch
+    if tiles:
+        monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", tiles)
     N, Cc, Hh, W, K, k, s, d, pd = case
     x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, k, k), float(np.sqrt(2.0 / (k * k * Cc)))), H.normal(3, (K,))
     y_w = orc.conv2d_fprop(x, w, b, (s, s), (d, d), (pd, pd), omp=True)
@@ -67,9 +70,10 @@ def test_conv_f32_tiles(case):
 
 @pytest.mark.parametrize("case", [(2, 3, 40, 44, 64, 7, 2, 1, 3), (3, 1, 19, 23, 17, 3, 1, 2, 0), (1, 8, 30, 21, 33, 5, 3, 1, 1), (2, 3, 17, 18, 20, 2, 3, 1, 0)])
 @pytest.mark.parametrize("accumulate", [0, 1])
-def test_data_gradient_into_few_channels(case, accumulate):
+def test_data_gradient_into_few_channels(case, accumulate, monkeypatch):
     """The two-step form that a caller's scratch allows."""
     import torch
+    monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", "1")
     N, Cc, Hh, W, K, k, s, d, pd = case
     w = H.normal(2, (K, Cc, k, k), float(np.sqrt(2.0 / (k * k * Cc))))
     P, Q = ((n + 2 * pd - d * (k - 1) - 1) // s + 1 for n in (Hh, W))
