@@ -170,9 +170,9 @@ static bool direct_wins(const ConvG& g, int pass) {
   const double taps = (double)g.kh * g.kw, px = (double)g.N * g.P * g.Q, mmac = px * g.K * g.C * taps * 1e-6;
   const bool one = g.kh * g.kw == 1;
   auto most = [](double x, double y) { return x > y ? x : y; };
-  if (pass == 0) return 4 + (one ? 0.36 : 0.14) * most(g.C * taps, 9 * mmac) < 21;
-  if (pass == 1) return 4 + most(0.06 * g.K * taps, 2 * mmac * g.sh * g.sw) < 20;
-  return taps <= 49 && 6 + most(px / 256 * (one ? 0.9 : 0.25 * taps), mmac * (one ? 7.8 : 2.6)) < 38;
+  if (pass == 0) return 4 + (one ? 0.36 : 0.14) * most(g.C * taps, 9 * mmac) < 25;
+  if (pass == 1) return 4 + most(0.06 * g.K * taps, 2 * mmac * g.sh * g.sw) < 25;
+  return taps <= 49 && 6 + most(px / 256 * (one ? 0.9 : 0.25 * taps), mmac * (one ? 7.8 : 2.6)) < 40;
 }
 
 int conv_direct_fprop(const ad_conv2d_args* a, cudaStream_t s) {
