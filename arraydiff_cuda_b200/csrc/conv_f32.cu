@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "conv_f32_plan.h"
 
 namespace cg = cooperative_groups;
 
@@ -311,8 +312,8 @@ __global__ void __launch_bounds__(kF32Group, 3) conv_gemm_f32(const GemmF32 p) {
 }
 
 // What the launches of one kernel share: on which devices (a bit each) its limits are raised, and how many clusters of
-// 1, 2, 4, 8, 16 CTAs the machine holds at a time (0: not asked yet).  That is less than CTAs per SM x 148 / size: a
-// cluster stays within one group of SMs.
+// 1, 2, 4, 8, 16 CTAs the machine holds at a time, plus one (0: not asked yet).  That is less than CTAs per SM x 148 / size:
+// a cluster stays within one group of SMs.
 struct F32Launch { unsigned raised = 0; uint32_t held[5] = {}; };
 
 template <typename Params>
@@ -350,6 +351,7 @@ static int launch_f32(void (*k)(Params), dim3 grid, int threads, int smem, uint3
   count_launch();
   return launch_status();
 }
+// 0: not one such cluster fits (part of a GPU, a size above what the device allows)
 template <typename Params>
 static uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, F32Launch& l) {
   uint32_t i = 0;
@@ -359,29 +361,10 @@ static uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, 
     cudaLaunchConfig_t cfg = f32_config(k, dim3(cs), threads, smem, cs, at, nullptr);
     cfg.numAttrs = 1;
     int n = 0;
-    if (raise_f32(k, smem, l) != AD_OK || cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = (int)(kNumSMs / cs); }
-    l.held[i] = (uint32_t)n;
+    if (raise_f32(k, smem, l) != AD_OK || cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 0) { cudaGetLastError(); n = 0; }
+    l.held[i] = (uint32_t)n + 1;
   }
-  return l.held[i];
-}
-
-// CTAs that share one tile's reduction of `steps` stages: the size with the shortest time by a count of waves.  A CTA costs
-// its stages and about six more to start and finish; one CTA on an SM takes 2.2 per stage, two 2.5, three 3 (12 warps hide
-// most of what they wait for).  Of the sizes 1 .. 16 this picks the fastest or one within a tenth of it for 18 of 20 layers
-// measured.  Before, the size went by CTAs per SM alone: 35 clusters of 8 where the machine holds 33
-// took two waves (filter gradient 64 -> 64, 4 x 112 x 112: 228 us against 168 for 30).
-template <typename Params>
-static uint32_t f32_cluster(void (*k)(Params), int threads, int smem, F32Launch& l, unsigned long long tiles, uint32_t steps, uint32_t most) {
-  static const double per_stage[4] = {0, 2.2, 2.5, 3.0};
-  uint32_t best = 1;
-  double best_cost = 0;
-  for (uint32_t cs = 1; cs <= most && (cs == 1 || steps >= 4 * cs); cs *= 2) {
-    const unsigned long long held = f32_held(k, threads, smem, cs, l);
-    auto wave = [&](unsigned long long clusters) { return per_stage[std::min<unsigned long long>((clusters * cs + kNumSMs - 1) / kNumSMs, 3)]; };
-    const double cta = (steps + cs - 1) / cs + 6, cost = cta * (tiles / held * wave(held) + (tiles % held ? wave(tiles % held) : 0));
-    if (cs == 1 || cost < best_cost) { best = cs; best_cost = cost; }
-  }
-  return best;
+  return l.held[i] - 1;
 }
 
 template <int LM, int WM, int WN, bool DGRAD>
@@ -391,8 +374,8 @@ static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uin
   const uint32_t tn = (npx + T::BN - 1) / T::BN, tm = (p.M + T::BM - 1) / T::BM;
   // every CTA of a cluster finishes at least one of the BM rows.  Clusters of 16 are for few tiles and long reductions:
   // 4 x 512 x 7 x 7 -> 512, 3x3 (16 tiles) 92 -> 67 us against 8.
-  const uint32_t cs = f32_cluster(conv_gemm_f32<LM, WM, WN, DGRAD>, T::threads, T::smem, l, (unsigned long long)tn * tm * classes, Kd / T::KB,
-                                  std::min(kF32Most, (int)T::BM));
+  auto held = [](uint32_t n) { return f32_held(conv_gemm_f32<LM, WM, WN, DGRAD>, T::threads, T::smem, n, l); };
+  const uint32_t cs = f32_cluster_size(held, (unsigned long long)tn * tm * classes, Kd / T::KB, std::min(kF32Most, (int)T::BM), kNumSMs);
   return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, l, s);
 }
 
@@ -607,8 +590,8 @@ static int launch_wgrad_f32(WgradF32& p, cudaStream_t s) {
   static F32Launch l;
   const uint32_t tn = (p.C * p.kh * p.kw + T::BN - 1) / T::BN, tm = (p.K + T::BM - 1) / T::BM;
   const uint32_t steps = p.N * p.P * p.Q / (kWgKB * G) / p.slices;
-  const uint32_t cs = p.slices > 1 ? 8u
-                                   : f32_cluster(conv_wgrad_gemm_f32<LM, WM, WN, G>, T::threads, T::smem, l, (unsigned long long)tn * tm, steps, 8);
+  auto held = [](uint32_t n) { return f32_held(conv_wgrad_gemm_f32<LM, WM, WN, G>, T::threads, T::smem, n, l); };
+  const uint32_t cs = p.slices > 1 ? f32_largest_cluster(held, 8) : f32_cluster_size(held, (unsigned long long)tn * tm, steps, 8, kNumSMs);
   int st = launch_f32(conv_wgrad_gemm_f32<LM, WM, WN, G>, dim3(tn * cs, tm, p.slices), T::threads, T::smem, cs, p, l, s);
   if (st != AD_OK || p.slices == 1) return st;
   const size_t n = (size_t)p.K * p.C * p.kh * p.kw;

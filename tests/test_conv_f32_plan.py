@@ -1,0 +1,61 @@
+"""Choices of the fp32 convolutions that need no GPU: conv_f32_plan.h, compiled for the host."""
+import ctypes as C
+import os
+import random
+import subprocess
+
+import pytest
+
+from tests.conftest import ROOT
+
+SOURCE = """
+#include "conv_f32_plan.h"
+extern "C" uint32_t cluster_size(const uint32_t* held, unsigned long long tiles, uint32_t steps, uint32_t most) {
+  return adk::f32_cluster_size([=](uint32_t cs) { return held[__builtin_ctz(cs)]; }, tiles, steps, most, 148);
+}
+extern "C" uint32_t largest_cluster(const uint32_t* held, uint32_t most) {
+  return adk::f32_largest_cluster([=](uint32_t cs) { return held[__builtin_ctz(cs)]; }, most);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plan(tmp_path_factory):
+    d = tmp_path_factory.mktemp("plan")
+    (d / "plan.cc").write_text(SOURCE)
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", os.path.join(ROOT, "arraydiff_cuda_b200", "csrc"),
+                           "-I", os.path.join(ROOT, "include"), str(d / "plan.cc"), "-o", str(d / "plan.so")])
+    L = C.CDLL(str(d / "plan.so"))
+    L.cluster_size.argtypes = [C.POINTER(C.c_uint32), C.c_uint64, C.c_uint32, C.c_uint32]
+    L.largest_cluster.argtypes = [C.POINTER(C.c_uint32), C.c_uint32]
+    L.cluster_size.restype = L.largest_cluster.restype = C.c_uint32
+    return L
+
+
+FULL = [296, 148, 74, 33, 14]      # clusters of 1, 2, 4, 8, 16 CTAs on a whole GPU, two CTAs per SM
+
+
+def _held(missing):
+    return [0 if i in missing else n for i, n in enumerate(FULL)]
+
+
+@pytest.mark.parametrize("missing", [(), (4,), (3, 4), (2, 3, 4), (1, 2, 3, 4), (3,), (1, 3)])
+def test_a_cluster_that_the_device_does_not_hold_is_not_chosen(plan, missing):
+    held = _held(missing)
+    h = (C.c_uint32 * 5)(*held)
+    rng = random.Random(5)
+    seen = set()
+    for _ in range(2000):
+        tiles, steps, most = int(2 ** rng.uniform(0, 12)), int(2 ** rng.uniform(0, 10)), rng.choice([1, 8, 16])
+        cs = plan.cluster_size(h, tiles, steps, most)
+        assert held[cs.bit_length() - 1] and cs <= most and (cs == 1 or steps >= 4 * cs)
+        seen.add(cs)
+    assert seen == {1 << i for i in range(5) if held[i]}
+    for most in (1, 2, 4, 8, 16):
+        cs = plan.largest_cluster(h, most)
+        assert held[cs.bit_length() - 1] and cs == max(1 << i for i in range(5) if held[i] and 1 << i <= most)
+
+
+def test_nothing_known_about_the_device(plan):
+    h = (C.c_uint32 * 5)()
+    assert plan.cluster_size(h, 16, 1024, 16) == 1 and plan.largest_cluster(h, 8) == 1
