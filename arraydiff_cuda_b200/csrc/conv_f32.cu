@@ -639,19 +639,21 @@ int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
 // with the filter as one GEMM -- Z[n][channel, tap][pixel], a 1x1 convolution of dy -- and then the sum over the taps of
 // each input pixel, in tap order.  As the GEMM above, 3 of 8 rows of a tile are used and every element of dy is gathered
 // once per tap: bound by the gathers.  4 x 64 x 224 x 224 -> 3, 7x7: 730 -> 393 us.
-// Images are taken as many at a time as fit kFewZ bytes; larger ones go the other way.
+// Images are taken as many at a time as fit kFewZ bytes (f32_few_images); larger ones go the other way.
 constexpr size_t kFewZ = 64u << 20;
 static size_t few_z_bytes(const ad_conv2d_args* a, uint32_t P, uint32_t Q) { return (size_t)P * Q * a->C * a->kh * a->kw * 4; }   // one image
+static uint32_t few_images(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
+  return f32_few_images(a->N, (unsigned long long)a->C * a->H * a->W, few_z_bytes(a, P, Q), kFewZ);
+}
 size_t f32_dgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
-  const size_t z = few_z_bytes(a, P, Q);
-  if (a->C > 8 || a->kh * a->kw < 4 || a->K < 16 || z > kFewZ) return 0;
-  return z * std::min<size_t>(a->N, kFewZ / z);
+  if (a->C > 8 || a->kh * a->kw < 4 || a->K < 16) return 0;
+  return few_z_bytes(a, P, Q) * few_images(a, P, Q);
 }
 __global__ void __launch_bounds__(256) dgrad_few_sum(const float* __restrict__ z, float* dx, uint32_t N, uint32_t C, uint32_t H, uint32_t W,
                                                      uint32_t P, uint32_t Q, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw,
                                                      uint32_t dh, uint32_t dw, int ph, int pw, int accumulate) {
   grid_dependency();
-  const uint32_t total = N * C * H * W, pq = P * Q;
+  const uint32_t total = N * C * H * W, pq = P * Q;   // below 2^31: f32_few_images
   for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
     const uint32_t x = i % W, r = i / W, y = r % H, nc = r / H;
     const float* zc = z + (size_t)nc * kh * kw * pq;
@@ -671,7 +673,7 @@ __global__ void __launch_bounds__(256) dgrad_few_sum(const float* __restrict__ z
   }
 }
 static int f32_dgrad_few(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
-  const uint32_t M = a->C * a->kh * a->kw, step = (uint32_t)std::min<size_t>(a->N, kFewZ / few_z_bytes(a, P, Q));
+  const uint32_t M = a->C * a->kh * a->kw, step = few_images(a, P, Q);
   for (uint32_t n0 = 0; n0 < a->N; n0 += step) {
     const uint32_t n = std::min(step, a->N - n0);
     GemmF32 p = {};

@@ -36,4 +36,11 @@ uint32_t f32_largest_cluster(Held held, uint32_t most) {
   return cs;
 }
 
+// Images that the two-step data gradient into few channels takes at a time: as many as fit `limit` bytes of scratch, z bytes
+// each, and whose input elements a 32-bit index counts with room for a step of the grid (an image has fewer than 2^31; with a
+// stride of 32 and more, small maps of dy belong to a gradient of more than 2^32 elements).  0: one image does not fit.
+inline uint32_t f32_few_images(uint32_t N, unsigned long long image, unsigned long long z, unsigned long long limit) {
+  return (uint32_t)std::min<unsigned long long>(N, std::min(limit / z, ((1ull << 31) - 1) / image));
+}
+
 }  // namespace adk

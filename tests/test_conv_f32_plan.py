@@ -16,6 +16,9 @@ extern "C" uint32_t cluster_size(const uint32_t* held, unsigned long long tiles,
 extern "C" uint32_t largest_cluster(const uint32_t* held, uint32_t most) {
   return adk::f32_largest_cluster([=](uint32_t cs) { return held[__builtin_ctz(cs)]; }, most);
 }
+extern "C" uint32_t few_images(uint32_t N, unsigned long long image, unsigned long long z, unsigned long long limit) {
+  return adk::f32_few_images(N, image, z, limit);
+}
 """
 
 
@@ -28,7 +31,8 @@ def plan(tmp_path_factory):
     L = C.CDLL(str(d / "plan.so"))
     L.cluster_size.argtypes = [C.POINTER(C.c_uint32), C.c_uint64, C.c_uint32, C.c_uint32]
     L.largest_cluster.argtypes = [C.POINTER(C.c_uint32), C.c_uint32]
-    L.cluster_size.restype = L.largest_cluster.restype = C.c_uint32
+    L.few_images.argtypes = [C.c_uint32, C.c_uint64, C.c_uint64, C.c_uint64]
+    L.cluster_size.restype = L.largest_cluster.restype = L.few_images.restype = C.c_uint32
     return L
 
 
@@ -59,3 +63,18 @@ def test_a_cluster_that_the_device_does_not_hold_is_not_chosen(plan, missing):
 def test_nothing_known_about_the_device(plan):
     h = (C.c_uint32 * 5)()
     assert plan.cluster_size(h, 16, 1024, 16) == 1 and plan.largest_cluster(h, 8) == 1
+
+
+@pytest.mark.parametrize("N,image,z,limit", [
+    (90, 3 * 4000 * 4000, 64 * 64 * 3 * 4 * 4, 64 << 20),   # the gradient has more than 2^32 elements, dy 65 thousand
+    (89, 3 * 4000 * 4000, 64 * 64 * 3 * 4 * 4, 64 << 20),   # just below: the step of the grid would pass 2^32
+    (5, 2 ** 31 - 1, 1 << 20, 64 << 20), (3, 2 ** 30, 1 << 20, 64 << 20),
+    (5, 8 * 134 * 134, 25690112, 64 << 20),                 # the scratch is the limit: pieces of 2, 2, 1
+    (4, 3 * 224 * 224, 3 * 49 * 218 * 218 * 4, 64 << 20), (1, 1, 4, 64 << 20),
+    (2, 100, (64 << 20) + 4, 64 << 20),                     # one image is too large: not this way
+])
+def test_pieces_of_the_gradient_into_few_channels(plan, N, image, z, limit):
+    """32-bit indices hold the elements of a piece and a step of the grid (148 x 16 blocks of 256) more."""
+    n = plan.few_images(N, image, z, limit)
+    most = max(i for i in range(N + 1) if i * z <= limit and i * image < 2 ** 31)
+    assert n == most and n * image + 148 * 16 * 256 < 2 ** 32

@@ -92,3 +92,25 @@ def test_data_gradient_into_few_channels(case, accumulate, monkeypatch):
     abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
     H.sync()
     assert np.max(np.abs(H.host(dx) - accumulate - want)) < 1e-5 * np.max(np.abs(want)) + accumulate * 2e-6
+
+
+def test_data_gradient_of_more_than_2_32_elements():
+    """A large stride: 90 images of 3 x 4000 x 4000 behind maps of 64 x 64, by pieces whose elements 32 bits count."""
+    import torch
+    N, Cc, Hh, K, k, s, P = 90, 3, 4000, 16, 2, 63, 64
+    assert N * Cc * Hh * Hh > 1 << 32 and (Hh - k) // s + 1 == P
+    L = abi.lib()
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, (N, Cc, Hh, Hh), K, k, s, 1, 0)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    dy, w = torch.rand((N, K, P, P), generator=g, device="cuda"), torch.rand((K, Cc, k, k), generator=g, device="cuda")
+    dx = torch.full((N, Cc, Hh, Hh), float("nan"), device="cuda")
+    scratch = torch.full((L.ad_conv2d_scratch_bytes(C.byref(a), 1),), 255, dtype=torch.uint8, device="cuda")
+    assert scratch.numel() == 44 * P * P * Cc * k * k * 4       # 44 images have fewer than 2^31 elements, 45 more
+    a.y, a.w, a.dx, a.scratch, a.scratch_bytes = dy.data_ptr(), w.data_ptr(), dx.data_ptr(), scratch.data_ptr(), scratch.numel()
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    for n in range(N):
+        want = torch.einsum("kpq,kcij->cpiqj", dy[n].double(), w.double())
+        full = torch.zeros((Cc, P * s, P * s), device="cuda")    # the last rows and columns are fewer than a stride
+        full[:, :Hh, :Hh] = dx[n]
+        got = full.unflatten(1, (P, s))[:, :, :k].unflatten(3, (P, s))[..., :k]
+        assert (got - want).abs().max() < 1e-5 * want.max() and torch.count_nonzero(dx[n]) == got.numel()   # zeros elsewhere
