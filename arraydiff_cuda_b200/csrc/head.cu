@@ -21,8 +21,8 @@ __global__ void __launch_bounds__(256) avgpool_fwd_kernel(AvgP p) {
   grid_dependency();
   const uint32_t total = p.N * p.C * p.P * p.Q, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)(p.kh * p.kw);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
-    uint32_t n, c, q, s, r = i;
+  for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {   // past 2^32 on the last step
+    uint32_t n, c, q, s, r = (uint32_t)i;
     if (p.c_fastest) { c = r % p.C; r /= p.C; s = r % p.Q; r /= p.Q; q = r % p.P; n = r / p.P; }
     else { s = r % p.Q; r /= p.Q; q = r % p.P; r /= p.P; c = r % p.C; n = r / p.C; }
     const T* X = (const T*)p.x.base + n * p.x.sn + c * p.x.sc;
@@ -38,8 +38,8 @@ __global__ void __launch_bounds__(256) avgpool_bwd_kernel(AvgP p) {
   grid_dependency();
   const uint32_t total = p.N * p.C * p.H * p.W, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)(p.kh * p.kw);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
-    uint32_t n, c, y, x, r = i;
+  for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {   // past 2^32 on the last step
+    uint32_t n, c, y, x, r = (uint32_t)i;
     if (p.c_fastest) { c = r % p.C; r /= p.C; x = r % p.W; r /= p.W; y = r % p.H; n = r / p.H; }
     else { x = r % p.W; r /= p.W; y = r % p.H; r /= p.H; c = r % p.C; n = r / p.C; }
     const uint32_t q_lo = y + 1 > p.kh ? (y + 1 - p.kh + p.sh - 1) / p.sh : 0;

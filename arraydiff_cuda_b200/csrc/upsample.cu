@@ -37,8 +37,8 @@ __global__ void __launch_bounds__(256) upsample_fwd_kernel(UpP p) {
   grid_dependency();
   const uint32_t total = p.N * p.C * p.YH * p.YW, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)p.scale;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
-    uint32_t n, c, oy, ox, r = i;
+  for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {   // past 2^32 on the last step
+    uint32_t n, c, oy, ox, r = (uint32_t)i;
     if (p.c_fastest) { c = r % p.C; r /= p.C; ox = r % p.YW; r /= p.YW; oy = r % p.YH; n = r / p.YH; }
     else { ox = r % p.YW; r /= p.YW; oy = r % p.YH; r /= p.YH; c = r % p.C; n = r / p.C; }
     int y0, y1, x0, x1;
@@ -62,8 +62,8 @@ __global__ void __launch_bounds__(256) upsample_bwd_kernel(UpP p) {
   const uint32_t total = p.N * p.C * p.XH * p.XW, nt = gridDim.x * blockDim.x;
   const float inv = 1.0f / (float)p.scale;
   const int s = (int)p.scale;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {
-    uint32_t n, c, yl, xl, r = i;
+  for (size_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += nt) {   // past 2^32 on the last step
+    uint32_t n, c, yl, xl, r = (uint32_t)i;
     if (p.c_fastest) { c = r % p.C; r /= p.C; xl = r % p.XW; r /= p.XW; yl = r % p.XH; n = r / p.XH; }
     else { xl = r % p.XW; r /= p.XW; yl = r % p.XH; r /= p.XH; c = r % p.C; n = r / p.C; }
     const int yg = (int)yl + p.x_row0, xg = (int)xl;
