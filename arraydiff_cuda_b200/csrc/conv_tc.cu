@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include <algorithm>
 
+#include "overlap.h"
 #include "tc_common.cuh"
 
 #include <cstdlib>
@@ -1225,6 +1226,13 @@ int conv_tc_fprop(const ad_conv2d_args* a, const ad_tensor4* addend, cudaStream_
     add = *addend;
     add.H = nq;
     add.base = (__nv_bfloat16*)addend->base + (long long)q0 * addend->sy;
+    // the forms without the sum in their epilogue write y first: an addend in its place would be the new y in those and
+    // the old one in the others
+    const long long ax = (long long)(g.Q - 1) * add.sx, ac = (long long)(a->K - 1) * add.sc;
+    const ByteRows to{(intptr_t)out, a->N, nq, plane * 2, pitch * 2, 0, (long long)g.Q * a->K * 2};
+    const ByteRows from{(intptr_t)add.base, a->N, nq, add.sn * 2, add.sy * 2, 2 * (std::min(0ll, ax) + std::min(0ll, ac)),
+                        2 * (std::max(0ll, ax) + std::max(0ll, ac) + 1)};
+    if (rows_meet(to, from)) return AD_ERR_BAD_ARG;
   }
   return run_fwd_gemm(a->x, a->N, a->H, a->W, a->C, a->w, a->K, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h,
                       a->dil_w, -(int)a->pad_h + (int)(q0 * a->stride_h), -(int)a->pad_w, nq, g.Q, out, pitch, plane, a->bias,

@@ -449,7 +449,8 @@ typedef struct {
 size_t ad_conv2d_scratch_bytes(const ad_conv2d_args* a, int32_t pass /* 0 fprop, 1 dgrad, 2 wgrad */);
 int ad_conv2d_fprop(const ad_conv2d_args* a, void* stream);
 /* y = (the bf16 output of ad_conv2d_fprop) + addend, a whole-output view (the rows of a row range are taken from it);
- * tensor-core path only.  addend may be NULL. */
+ * tensor-core path only.  addend may be NULL.  It is read while y is written: an addend that shares memory with the rows of
+ * y that the call writes is AD_ERR_BAD_ARG (a view between them, in the same buffer, is fine). */
 int ad_conv2d_fprop_add(const ad_conv2d_args* a, const ad_tensor4* addend, void* stream);
 int ad_conv2d_dgrad(const ad_conv2d_args* a, void* stream);
 int ad_conv2d_wgrad(const ad_conv2d_args* a, void* stream);

@@ -168,3 +168,42 @@ def test_forward_with_addend(case, pad, rows):
     H.sync()
     y0[:, lo:lo + n] += add[:, pad + lo:pad + lo + n, pad:pad + Q]
     assert int(status[0]) == 0 and torch.equal(y0, y1)
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, H, W, K, k: the sum in the epilogue (pair, single CTA); behind it (row kernel, scattered stores)
+    (2, 512, 15, 29, 256, 1), (3, 64, 7, 9, 128, 1), (1, 64, 9, 140, 64, 3), (2, 128, 10, 12, 24, 1),
+])
+def test_addend_in_the_output_buffer(case):
+    """Refused where it shares memory with the rows that are written, in every form alike; fine beside them."""
+    import torch
+    N, Cc, Hh, W, K, k = case
+    L = abi.lib()
+    a = abi.Conv2dArgs()
+    a.dtype, a.layout = abi.AD_BF16, abi.AD_NHWC
+    a.N, a.C, a.H, a.W, a.K, a.kh, a.kw = N, Cc, Hh, W, K, k, k
+    a.stride_h = a.stride_w = a.dil_h = a.dil_w = 1
+    P, Q = Hh - k + 1, W - k + 1
+    x, w = torch.randn(N, Hh, W, Cc, device="cuda").bfloat16(), torch.randn(K, k, k, Cc, device="cuda").bfloat16()
+    buf = torch.randn(N, P + 1, 2 * Q, K, device="cuda").bfloat16()   # y: the left half of the first P rows
+    before = buf.clone()
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    a.x, a.w, a.scratch, a.scratch_bytes, a.y = x.data_ptr(), w.data_ptr(), status.data_ptr(), 16, buf.data_ptr()
+    a.y_pitch, a.y_plane = 2 * Q * K, (P + 1) * 2 * Q * K
+
+    def add(view):
+        return L.ad_conv2d_fprop_add(C.byref(a), C.byref(H.view_nhwc(view)), H.stream())
+
+    assert add(buf[:, :P, :Q]) == -1 and add(buf[:, 1:, :Q]) == -1 and add(buf[:, :P, 1:Q + 1]) == -1
+    a.out_row_begin, a.out_row_count = 1, 2
+    assert add(buf[:, :P, :Q]) == -1
+    H.sync()
+    assert torch.equal(buf, before)
+    a.out_row_count = a.out_row_begin = 0
+    abi.check(add(buf[:, 1:, Q:]))
+    want = torch.empty((N, P, Q, K), dtype=torch.bfloat16, device="cuda")
+    a.y, a.y_pitch, a.y_plane = want.data_ptr(), 0, 0
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    H.sync()
+    assert int(status[0]) == 0 and torch.equal(buf[:, :P, :Q], want + before[:, 1:, Q:])
+    assert torch.equal(buf[:, :, Q:], before[:, :, Q:]) and torch.equal(buf[:, P], before[:, P])
