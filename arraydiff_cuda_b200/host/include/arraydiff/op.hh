@@ -324,7 +324,7 @@ public:
   // The only consumer's gradient is this operator's gradient (kJoinShare): one variable, one buffer
   void share_grad(const TxnVar<Act>& grad) { y_.grad = grad; }
   // A sum of this output (kJoinShare) and x, which is evaluated earlier, asks its last input to write the sum itself:
-  // true, and y_.val holds the sum from then on.
+  // true, and the buffer of y_.val holds the sum from then on (store_val still gives this operator's own output).
   virtual bool take_sum(ActVar x) { return false; }
   const TxnVar<Act>& value_var() const { return y_.val; }
   // Any activation can be read back, and its gradient set or read, as packed NCHW fp32 of the
@@ -446,9 +446,11 @@ public:
   void _backward(TxnId txn) override;
   ~CudnnConv2DOpF() override;
   bool take_sum(ActVar x) override;
+  size_t _store_val(TxnId txn, VarIdSet& vars, size_t offset, any* writer) override;
   string _debug_op_label() override { return "CudnnConv2DOp"; }
 private:
   void fill_args(ad_conv2d_args& a, Act& x);
+  void launch_fprop(ad_conv2d_args a, const ad_tensor4* add, cudaStream_t s);
   Conv2DShape shape_;
   ActVar x_;
   shared_ptr<Var<Kernel>> kernel_;
@@ -459,6 +461,8 @@ private:
   void *w_bf16_ = nullptr, *w_crsk_ = nullptr;
   size_t filter_id_ = (size_t)-1;
   ActVar sum_;             // take_sum: not an input of the graph (the sum is, and it orders the two)
+  ad_conv2d_args last_ = {};   // the last forward call: store_val repeats it
+  bool split_ = false;
   float* dw_krsc_ = nullptr;
   void* im2col_ = nullptr;
   size_t ck_ = 0;       // channels the tensor-core kernel reduces over per tap (padded)

@@ -495,8 +495,14 @@ void CudnnConv2DOpF::fill_args(ad_conv2d_args& a, Act& x) {
   }
 }
 
+// Only where the forward call can be repeated afterwards (_store_val): its input and x are results of this graph, not
+// variables that a caller loads, and no bias is read, which the optimizer updates in place.
 bool CudnnConv2DOpF::take_sum(ActVar x) {
-  if (gpu()->mode() != COMPUTE_BF16_NHWC || sum_) return false;
+  auto computed = [](ActVar v) {
+    while (auto* a = dynamic_cast<AliasOpF*>(v.get())) v = a->aliased();
+    return dynamic_cast<ActOp*>(v.get()) != nullptr;
+  };
+  if (gpu()->mode() != COMPUTE_BF16_NHWC || sum_ || bias_ || !computed(x_) || !computed(x)) return false;
   sum_ = x;
   return true;
 }
@@ -544,21 +550,40 @@ void CudnnConv2DOpF::_forward(TxnId txn) {
     a.x = im2col_; a.C = (uint32_t)ck_; a.H = (uint32_t)dim_.shape[1]; a.W = (uint32_t)dim_.shape[0];
     a.kh = a.kw = a.stride_h = a.stride_w = a.dil_h = a.dil_w = 1; a.pad_h = a.pad_w = 0;
   }
-  g->reserve_scratch(16);
-  a.scratch = g->status_word(); a.scratch_bytes = 16;
   ad_tensor4 add;
   if (sum_) add = sum_->data().val.get(txn, id()).view_interior();
-  if (split) {
-    a.out_row_begin = (uint32_t)ph; a.out_row_count = (uint32_t)(oh - 2 * ph);
-    AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
-    g->finish_pending();
-    a.out_row_begin = 0; a.out_row_count = (uint32_t)ph;
-    AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
-    a.out_row_begin = (uint32_t)(oh - ph);
-    AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
+  split_ = split;
+  last_ = a;
+  launch_fprop(a, sum_ ? &add : nullptr, conn.stream());
+}
+// The tensor-core convolution into y, in one piece or (split_) the interior rows before the ones that need a halo
+void CudnnConv2DOpF::launch_fprop(ad_conv2d_args a, const ad_tensor4* add, cudaStream_t s) {
+  GPUContext* g = gpu();
+  g->reserve_scratch(16);
+  a.scratch = g->status_word(); a.scratch_bytes = 16;
+  if (!split_) {
+    AD_CHECK(ad_conv2d_fprop_add(&a, add, s));
     return;
   }
-  AD_CHECK(ad_conv2d_fprop_add(&a, sum_ ? &add : nullptr, conn.stream()));
+  const uint32_t ph = (uint32_t)shape_.pad[1], oh = (uint32_t)dim_.shape[1];
+  a.out_row_begin = ph; a.out_row_count = oh - 2 * ph;
+  AD_CHECK(ad_conv2d_fprop_add(&a, add, s));
+  g->finish_pending();
+  a.out_row_begin = 0; a.out_row_count = ph;
+  AD_CHECK(ad_conv2d_fprop_add(&a, add, s));
+  a.out_row_begin = oh - ph;
+  AD_CHECK(ad_conv2d_fprop_add(&a, add, s));
+}
+// Where y holds a sum with another tensor (take_sum), what is read back is the convolution all the same: it runs again
+// without the sum, as the forward pass ran it, and then with it.  Input, filter and the other tensor are those of that pass.
+size_t CudnnConv2DOpF::_store_val(TxnId txn, VarIdSet& vars, size_t offset, any* writer) {
+  if (!sum_ || !writer || !last_.x || !vars.contains(y_.val.var())) return ActOp::_store_val(txn, vars, offset, writer);
+  GPUConn conn = gpu()->conn();
+  launch_fprop(last_, nullptr, conn.stream());
+  const size_t end = ActOp::_store_val(txn, vars, offset, writer);
+  ad_tensor4 add = sum_->data().val.raw().view_interior();
+  launch_fprop(last_, &add, conn.stream());
+  return end;
 }
 
 void CudnnConv2DOpF::_backward(TxnId txn) {
@@ -852,13 +877,12 @@ SumJoinOpF::SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGr
   }
   auto* last = dynamic_cast<ActOp*>(xs.back().get());
   if (xs.size() == 2 && grads_[1] == kJoinShare && xs[0] != xs[1] && last->take_sum(xs[0])) {
-    in_last_ = true;
-    y_.val = last->value_var();
+    in_last_ = true;   // a variable of its own in the same buffer
+    y_.val = TxnVar<Act>(VAR_KIND_VAL, [val = last->value_var()]() mutable { return val.raw(); });
   }
 }
 void SumJoinOpF::_forward(TxnId txn) {
-  if (in_last_) return;
-  if (!y_.val.overwrite(txn, id())) return;
+  if (!y_.val.overwrite(txn, id()) || in_last_) return;
   GPUConn conn = gpu()->conn();
   ad_tensor4 yv = y_.val.get_excl(txn, id()).view_interior();
   ad_tensor4 a = xs_[0]->data().val.get(txn, id()).view_interior(), b = xs_[1]->data().val.get(txn, id()).view_interior();
