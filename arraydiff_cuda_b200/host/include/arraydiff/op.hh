@@ -321,8 +321,10 @@ public:
   VarData<Act> data() override { return y_; }
   size_t rank() const override { return rank_; }
   void _persist(TxnId, VarIdSet&) override {}
-  // The only consumer's gradient is this operator's gradient (kJoinShare): one variable, one buffer
-  void share_grad(const TxnVar<Act>& grad) { y_.grad = grad; }
+  // The only consumer's gradient is this operator's gradient (kJoinShare): a variable of its own over one buffer
+  virtual void share_grad(const TxnVar<Act>& grad) {
+    y_.grad = TxnVar<Act>(VAR_KIND_GRAD, [g = grad]() mutable { return g.raw(); });
+  }
   // A sum of this output (kJoinShare) and x, which is evaluated earlier, asks its last input to write the sum itself:
   // true, and the buffer of y_.val holds the sum from then on (store_val still gives this operator's own output).
   virtual bool take_sum(ActVar x) { return false; }
@@ -531,6 +533,7 @@ class SumJoinOpF : public ActOp {
 public:
   static ActVar Make(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGrad> grads = {});
   SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGrad> grads);
+  void share_grad(const TxnVar<Act>& grad) override;   // passed on to the inputs that share this one's
   void _forward(TxnId txn) override;
   void _backward(TxnId txn) override;
 private:

@@ -881,6 +881,11 @@ SumJoinOpF::SumJoinOpF(vector<ActVar> xs, shared_ptr<Context> ctx, vector<JoinGr
     y_.val = TxnVar<Act>(VAR_KIND_VAL, [val = last->value_var()]() mutable { return val.raw(); });
   }
 }
+void SumJoinOpF::share_grad(const TxnVar<Act>& grad) {
+  ActOp::share_grad(grad);
+  for (size_t i = 0; i < xs_.size(); ++i)
+    if (grads_[i] == kJoinShare) dynamic_cast<ActOp*>(xs_[i].get())->share_grad(y_.grad);
+}
 void SumJoinOpF::_forward(TxnId txn) {
   if (!y_.val.overwrite(txn, id()) || in_last_) return;
   GPUConn conn = gpu()->conn();
@@ -896,8 +901,8 @@ void SumJoinOpF::_backward(TxnId txn) {
   GPUConn conn = gpu()->conn();
   ad_tensor4 dyv = y_.grad.get(txn, id()).view_interior();
   for (size_t i = 0; i < xs_.size(); ++i) {
-    if (grads_[i] == kJoinShare) continue;
     auto xd = xs_[i]->data();
+    if (grads_[i] == kJoinShare) { xd.grad.accumulate_full(txn, id(), always, nullptr); continue; }   // written: the buffer is this gradient's
     if (grads_[i] == kJoinDefer) { xd.grad.defer(txn, &y_.grad.get(txn, id())); continue; }
     const int mode = xd.grad.accumulate_full(txn, id(), unpadded, zero_init(gpu()));
     if (!mode) continue;

@@ -1,4 +1,4 @@
-// A residual sum written by its branch's last convolution: every value of the graph can still be read back.
+// A residual sum written by its branch's last convolution: every value and gradient of the graph can still be read back.
 // Two graphs over the same variables, with gradients shared at the join (the convolution may write the sum) and copied (it
 // may not), have to agree to the bit.  Prints "ok" or what differs.
 #include <cstdio>
@@ -13,7 +13,7 @@ typedef GPUArray1D<float> Bias;
 
 struct Graph {
   shared_ptr<CudnnConv2DOpF> trunk, branch;
-  ActVar sum;
+  ActVar sum, top;   // top: a sum over the sum
 };
 
 static size_t failures = 0;
@@ -43,6 +43,7 @@ int main() {
     g.trunk = CudnnConv2DOpF::Make(s, in, k[0], nullptr, ctx);
     g.branch = CudnnConv2DOpF::Make(s, loaded_input ? ActVar(in) : ActVar(g.trunk), k[1], with_bias ? bias : nullptr, ctx);
     g.sum = SumJoinOpF::Make({loaded_addend ? ActVar(in) : ActVar(g.trunk), g.branch}, ctx, {kJoinCopy, last});
+    g.top = SumJoinOpF::Make({ActVar(g.trunk), g.sum}, ctx, {kJoinCopy, last});
     return g;
   };
   auto load = [&](shared_ptr<Op> sink, TxnId txn, VarId v, vector<float>& from) {
@@ -53,7 +54,7 @@ int main() {
   for (int form = 0; form < 8; ++form) {
     const bool loaded_input = form & 1, loaded_addend = form & 2, with_bias = form & 4;
     Graph g[2] = {make(loaded_input, loaded_addend, with_bias, kJoinShare), make(loaded_input, loaded_addend, with_bias, kJoinCopy)};
-    auto sink = std::make_shared<GroupSinkOp>(vector<shared_ptr<Op>>{g[0].sum, g[1].sum});
+    auto sink = std::make_shared<GroupSinkOp>(vector<shared_ptr<Op>>{g[0].top, g[1].top});
     auto read = [&](TxnId txn, ActVar v) {
       VarIdSet set = VarIdSet::Singleton(v->data().val.var());
       vector<float> out(n);
@@ -71,6 +72,7 @@ int main() {
       sink->eval(txn);
       const vector<float> sum = read(txn, g[0].sum), conv = read(txn, g[0].branch);
       same("sum", sum, read(txn, g[1].sum));
+      same("top", read(txn, g[0].top), read(txn, g[1].top));
       same("convolution", conv, read(txn, g[1].branch));
       same("convolution and sum", conv, sum, false);
       same("sum after the convolution was read", sum, read(txn, g[0].sum));
@@ -83,6 +85,27 @@ int main() {
         if (sink->store_val(txn, set, 0, &w) != 2 * n) { std::printf("form %d: size of two\n", form); ++failures; }
         same("first of two", vector<float>(out.begin(), out.begin() + n), conv);
         same("second of two", vector<float>(out.begin() + n, out.end()), sum);
+      }
+      {
+        // gradients: of the top (loaded), the sum and the branch's output (the same)
+        vector<float> dy = draw(n, 1.f);
+        VarIdSet sums = VarIdSet::Singleton(g[0].top->data().grad.var());
+        sums.insert(g[1].top->data().grad.var());
+        vector<float> both(dy);
+        both.insert(both.end(), dy.begin(), dy.end());
+        any rd = both.data();
+        sink->load_grad(txn, sums, 0, &rd);
+        sink->backward(txn);
+        vector<float> of[2];
+        for (int i = 0; i < 2; ++i) {
+          VarIdSet set = VarIdSet::Singleton(g[i].branch->data().grad.var());
+          set.insert(g[i].sum->data().grad.var());
+          set.insert(g[i].trunk->data().grad.var());
+          of[i].resize(3 * n);
+          any w = of[i].data();
+          if (sink->store_grad(txn, set, 0, &w) != 3 * n) { std::printf("form %d: size of three gradients\n", form); ++failures; }
+        }
+        same("gradients of trunk, branch and sum", of[0], of[1]);
       }
       // the next batch and other parameters are loaded, nothing is evaluated: results are those of the last pass
       vector<float> x2 = draw(n, 1.f), b2 = draw(C, 1.f), v0 = draw(C * C, 0.125f), v1 = draw(C * C, 0.125f);
