@@ -60,6 +60,14 @@ def test_a_cluster_that_the_device_does_not_hold_is_not_chosen(plan, missing):
         assert held[cs.bit_length() - 1] and cs == max(1 << i for i in range(5) if held[i] and 1 << i <= most)
 
 
+def test_clusters_of_16(plan):
+    """The layers of tests/test_gpu_conv_f32.py that are there for them: tiles and stages of each pass."""
+    for held in (FULL, [444, 222, 111, 50, 21]):       # two or three CTAs per SM
+        h = (C.c_uint32 * 5)(*held)
+        for tiles, steps in ((3, 128 * 9 // 16), (2, 130 * 9 // 16), (1, 120 * 9 // 16)):
+            assert plan.cluster_size(h, tiles, steps, 16) == 16
+
+
 def test_nothing_known_about_the_device(plan):
     h = (C.c_uint32 * 5)()
     assert plan.cluster_size(h, 16, 1024, 16) == 1 and plan.largest_cluster(h, 8) == 1

@@ -74,6 +74,12 @@ def test_filter_gradient_order(K, Cc, k, accumulate):
     (2, 64, 17, 16, 64, 2, 3, 1, 0, (2, 9)),     # a kernel smaller than the stride
     (1, 64, 23, 26, 64, 5, 4, 3, 4, None), (1, 19, 12, 12, 64, 3, 2, 1, 1, None), (2, 32, 14, 14, 19, 4, 2, 1, 1, None),
     (1, 64, 31, 33, 64, 7, 2, 1, 3, None),
+    # more than 128 channels and 8 slabs of 64: CTA pairs
+    (2, 256, 17, 19, 512, 1, 2, 1, 0, None),     # three of four classes have no taps
+    (1, 200, 15, 22, 128, 3, 2, 1, 1, (2, 17)),  # ragged channels, a range of columns
+    (3, 264, 13, 9, 64, 3, 2, 1, 1, None),       # two channel tiles, the second one of 8
+    (1, 256, 20, 47, 64, 3, 3, 1, 1, None),      # nine classes
+    (1, 130, 11, 12, 64, 3, 2, 1, 1, None),      # scattered stores
 ])
 @pytest.mark.parametrize("accumulate", [0, 1])
 def test_strided_data_gradient(case, accumulate):
