@@ -575,15 +575,27 @@ void CudnnConv2DOpF::launch_fprop(ad_conv2d_args a, const ad_tensor4* add, cudaS
   AD_CHECK(ad_conv2d_fprop_add(&a, add, s));
 }
 // Where y holds a sum with another tensor (take_sum), what is read back is the convolution all the same: it runs again
-// without the sum, as the forward pass ran it, and then with it.  Input, filter and the other tensor are those of that pass.
+// without the sum, as the forward pass ran it, into scratch (another rank may be reading y).
 size_t CudnnConv2DOpF::_store_val(TxnId txn, VarIdSet& vars, size_t offset, any* writer) {
-  if (!sum_ || !writer || !last_.x || !vars.contains(y_.val.var())) return ActOp::_store_val(txn, vars, offset, writer);
-  GPUConn conn = gpu()->conn();
-  launch_fprop(last_, nullptr, conn.stream());
-  const size_t end = ActOp::_store_val(txn, vars, offset, writer);
-  ad_tensor4 add = sum_->data().val.raw().view_interior();
-  launch_fprop(last_, &add, conn.stream());
-  return end;
+  if (!sum_ || !writer || !last_.x) return ActOp::_store_val(txn, vars, offset, writer);
+  if (!vars.mask(y_.val.var())) return offset;
+  float* host = host_floats(writer);
+  assert(host);
+  GPUContext* g = gpu();
+  GPUConn conn = g->conn();
+  const size_t n = dim_.flat_size() * batch_, as_f32 = (n * 4 + 255) / 256 * 256;
+  g->reserve_scratch(as_f32 + n * 2);
+  ad_conv2d_args a = last_;
+  a.y = (char*)g->get_scratch() + as_f32;
+  launch_fprop(a, nullptr, conn.stream());
+  ad_tensor4 from = y_.val.raw().view_interior(), to = from;
+  from.base = a.y;
+  to.base = g->get_scratch(); to.dtype = AD_F32;
+  to.sx = 1; to.sy = to.W; to.sc = (int64_t)to.H * to.W; to.sn = to.C * to.sc;
+  AD_CHECK(ad_convert(&from, &to, 0, conn.stream()));
+  CUDA_CHECK(cudaMemcpyAsync(host + offset, to.base, n * 4, cudaMemcpyDeviceToHost, conn.stream()));
+  conn.sync();
+  return offset + n;
 }
 
 void CudnnConv2DOpF::_backward(TxnId txn) {
