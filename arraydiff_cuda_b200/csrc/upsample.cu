@@ -159,11 +159,10 @@ __global__ void __launch_bounds__(kUpThreads) upsample_fwd_rows(UpRowP p) {
     bilin_src(u.y_row0 + oy, inv, u.in_rows_total, y0, y1, fy);
     const T* X = (const T*)u.x.base + plane_off(u.x, plane, per_n) + (long long)lo * p.Ci;
     const T *X0 = X + (y0 - u.x_row0) * u.x.sy, *X1 = X + (y1 - u.x_row0) * u.x.sy;
-    // one column past the last is a copy of it: the right edge blends it with weight 0
-    for (uint32_t i = threadIdx.x; i < cols + (hi == u.XW ? p.Ci : 0); i += kUpThreads) {
-      const uint32_t k = i < cols ? i : i - p.Ci;
-      L[r * pitch + i] = (1.f - fy) * ld_f(X0 + k) + fy * ld_f(X1 + k);
-    }
+    // one column of zeros past the last: the right edge blends it with weight 0 (an infinity there, times 0, would be NaN)
+    for (uint32_t i = threadIdx.x; i < cols; i += kUpThreads) L[r * pitch + i] = (1.f - fy) * ld_f(X0 + i) + fy * ld_f(X1 + i);
+    if (hi == u.XW)
+      for (uint32_t i = threadIdx.x; i < p.Ci; i += kUpThreads) L[r * pitch + cols + i] = 0.f;
   }
   if (p.period) {
     // Scale a power of two: the pairs of one source column's outputs, scale * Ci / 2 of them, recur from column to column with
@@ -252,15 +251,16 @@ __global__ void __launch_bounds__(kUpThreads) upsample_bwd_rows(UpRowP p) {
   const int yg = (int)yl + u.x_row0;
   int oy_lo = 0, oy_hi = -1;
   if (yg >= 0 && yg < (int)u.in_rows_total) {
-    // outputs whose source coordinate lies in (g - 1, g + 1); edge cells also take the clamped ones
-    oy_lo = yg == 0 ? 0 : (yg - 1) * s + s / 2;
-    oy_hi = yg == (int)u.in_rows_total - 1 ? (int)u.in_rows_total * s - 1 : (yg + 1) * s + (s - 1) / 2;
+    // outputs whose source coordinate lies in (g - 1, g + 1); edge cells also take the clamped ones.  At an odd scale the
+    // outputs at g - 1 and g + 1 have no part in g: an infinite gradient there must not meet a weight of 0.
+    oy_lo = yg == 0 ? 0 : (yg - 1) * s + (s + 1) / 2;
+    oy_hi = yg == (int)u.in_rows_total - 1 ? (int)u.in_rows_total * s - 1 : (yg + 1) * s + s / 2 - 1;
     if (oy_lo < (int)u.y_row0) oy_lo = (int)u.y_row0;
     if (oy_hi > (int)(u.y_row0 + u.YH) - 1) oy_hi = (int)(u.y_row0 + u.YH) - 1;
   }
   const T* G = (const T*)u.y.base + plane_off(u.y, plane, per_n);
   const uint32_t e0 = oxa * p.Ci, e1 = oxb * p.Ci, v0 = e0 / V, nv = (e1 + V - 1) / V - v0;
-  // weights of the output rows, and of the output columns (xg - 1) * s + s / 2 + t around a column xg away from the edges
+  // weights of the output rows, and of the output columns (xg - 1) * s + (s + 1) / 2 + t around a column xg away from the edges
   float* const wyt = S + p.wtab;
   for (int oy = oy_lo + (int)threadIdx.x; oy <= oy_hi; oy += kUpThreads) {
     int y0, y1;
@@ -297,11 +297,11 @@ __global__ void __launch_bounds__(kUpThreads) upsample_bwd_rows(UpRowP p) {
   }
   __syncthreads();
   // the column weights take the place of the row weights
-  const int nt = s + (s - 1) / 2 - s / 2 + s + 1;      // outputs whose source pair can contain an inner column
+  const int nt = 2 * s + s / 2 - (s + 1) / 2;          // outputs that an inner column has a part in
   for (int t = (int)threadIdx.x; t < nt; t += kUpThreads) {
     int x0, x1;
     float fx;
-    bilin_src((uint32_t)(s / 2 + t), inv, 1u << 20, x0, x1, fx);      // around column 1 of a wide row
+    bilin_src((uint32_t)((s + 1) / 2 + t), inv, 1u << 20, x0, x1, fx);      // around column 1 of a wide row
     wyt[t] = (x0 == 1 ? 1.f - fx : 0.f) + (x1 == 1 ? fx : 0.f);
   }
   __syncthreads();
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kUpThreads) upsample_bwd_rows(UpRowP p) {
   for (uint32_t i = threadIdx.x; i < (xb - xa) * p.Ci; i += kUpThreads) {
     const uint32_t xl = xa + i / p.Ci, c = i % p.Ci;
     const int xg = (int)xl;
-    const int ox_lo = xg == 0 ? 0 : (xg - 1) * s + s / 2, ox_hi = xg == (int)u.XW - 1 ? (int)u.XW * s - 1 : (xg + 1) * s + (s - 1) / 2;
+    const int ox_lo = xg == 0 ? 0 : (xg - 1) * s + (s + 1) / 2, ox_hi = xg == (int)u.XW - 1 ? (int)u.XW * s - 1 : (xg + 1) * s + s / 2 - 1;
     float acc = 0.f;
     const float* sp = Sr + ((uint32_t)ox_lo - oxa) * p.Ci + c;
     if (xg > 0 && xg < (int)u.XW - 1) {

@@ -52,6 +52,59 @@ def test_upsample_rows(dtype, shape, scale):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape,scale", [((1, 3, 6, 40), 8), ((2, 3, 5, 90), 3), ((1, 19, 5, 33), 2), ((1, 1, 4, 700), 5), ((1, 2, 5, 9), 2)])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_upsample_rows_of_infinities(dtype, shape, scale, bad):
+    """Logits masked with an infinity, at the right and lower edge and inside, and gradients that overflowed: each reaches the
+    elements that it has a weight in and no other (weights of 0 multiply nothing but the next source row and column)."""
+    import torch
+    N, Cc, Hh, W = shape
+
+    def weights(n):                                  # [output][source], of the half-pixel rule
+        o = np.arange(n * scale)
+        src = np.maximum((o + 0.5) / scale - 0.5, 0.0)
+        i0 = np.minimum(np.floor(src + 1e-9).astype(int), n - 1)
+        f = np.where(src - i0 < 1e-9, 0.0, src - i0)
+        w = np.zeros((n * scale, n))
+        np.add.at(w, (o, i0), 1 - f)
+        np.add.at(w, (o, np.minimum(i0 + 1, n - 1)), f)
+        touch, zero = w > 0, np.zeros_like(w, bool)  # multiplied at all: with a weight of 0, or one that rounds to it
+        touch[o, np.minimum(i0 + 1, n - 1)] = True
+        touch[o, np.where(f == 0, np.maximum(i0 - 1, 0), i0)] = True
+        zero[o, np.minimum(i0 + 1, n - 1)] = f == 0
+        return w, touch, zero
+
+    (wy, ty, zy), (wx, tx, zx) = weights(Hh), weights(W)
+    _, _, view = FMT[dtype]
+    L = abi.lib()
+
+    def reach(a, b, at):                             # which results an element set at `at` reaches through a and b
+        m = np.zeros((a.shape[1], b.shape[1]))
+        m[at] = 1
+        return a @ m @ b.T > 0
+
+    for at in [(Hh - 1, W - 1), (Hh - 1, 2), (2, W - 1), (2, 3)]:
+        x = _q(H.normal(1, shape), dtype)
+        x[:, :, at[0], at[1]] = bad
+        dx_ = _dev(x, dtype)
+        y = _dev(np.zeros((N, Cc, Hh * scale, W * scale), np.float32), dtype)
+        abi.check(L.ad_upsample_bilinear_fwd(C.byref(view(dx_)), C.byref(view(y)), scale, 0, Hh, 0, H.stream()))
+        H.sync()
+        got = ~np.isfinite(_host(y, dtype))
+        assert np.all(got >= reach(wy, wx, at)) and np.all(got <= reach(ty, tx, at))
+        if not np.isnan(bad):                        # the value itself wherever it is not multiplied with 0 as well
+            itself = reach(wy, wx, at) & ~zy[:, at[0], None] & ~zx[None, :, at[1]]
+            assert np.all(_host(y, dtype)[:, :, itself] == bad)
+        oy, ox = at[0] * scale + scale // 2, at[1] * scale + scale // 2
+        dy = _q(H.normal(2, (N, Cc, Hh * scale, W * scale)), dtype)
+        dy[:, :, oy, ox] = bad
+        ddy = _dev(dy, dtype)
+        abi.check(L.ad_upsample_bilinear_bwd(C.byref(view(ddy)), C.byref(view(dx_)), scale, 0, Hh, 0, 0, H.stream()))
+        H.sync()
+        assert np.array_equal(~np.isfinite(_host(dx_, dtype)), np.broadcast_to(reach(wy.T, wx.T, (oy, ox)), shape))
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
 @pytest.mark.parametrize("Cc,HW", [(1, 300), (8, 257), (9, 255), (32, 256), (33, 130), (64, 31), (65, 77), (128, 3), (129, 9), (256, 5), (257, 4), (1000, 1)])
 def test_ce_class_counts(dtype, layout, Cc, HW):
