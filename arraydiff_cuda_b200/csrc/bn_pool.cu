@@ -620,8 +620,9 @@ __global__ void __launch_bounds__(256) maxpool_bwd_vec(PoolP p) {
 // Phase 1, once per window that touches the patch: the position of the window's first maximum (a small bf16 number per
 // channel, so that packed comparisons serve it) and its gradient go to shared memory; phase 2 lets every input pixel pick
 // its gradients there.  Same first-maximum rule and the same summation order (q, then s, ascending) as the kernels above.
-// The bound is HBM (x, dy and dx once); packed 16-bit comparisons keep the arithmetic below it.
-// 2 x 64 x 514 x 1026, 3x3 / 2: forward 57 -> 32 us, gradient 208 -> 90 us (46 us at the copy rate).
+// The bound is HBM (x, dy and dx once) for windows that do not overlap much; packed 16-bit comparisons keep the arithmetic
+// near it.  Gradient of 2 x 64 x 514 x 1026 (46 us at the copy rate for 2 x 2 / 2): 2 x 2 / 2 132 -> 56 us, 3 x 3 / 3 142 -> 99,
+// 3 x 3 / 1 560 -> 296, 5 x 5 / 2 6650 -> 278; 3 x 3 / 2 goes to maxpool_bwd_quads.
 constexpr uint32_t kPoolTile = 16, kPoolMaxWin = 400;
 // K x K windows of stride S, or any extents (K = 0)
 template <int K, int S>

@@ -1,6 +1,6 @@
 // fp32 NCHW convolution with fp32 FMA accumulate: the exact-precision path (max-relative 1e-5 against a
 // double-accumulating CPU result).  The tiled kernels of conv_f32.cu serve every geometry within their limits
-// (f32_gemm_ok: 32-bit offsets, at most 63 taps) but the smallest calls (direct_wins); the one-thread-per-output kernels
+// (f32_gemm_ok: 32-bit offsets, at most 64 taps) but the smallest calls (direct_wins); the one-thread-per-output kernels
 // here take those and what is left.
 #include <cstdlib>
 

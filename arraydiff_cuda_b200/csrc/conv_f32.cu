@@ -1,6 +1,6 @@
 // fp32 NCHW convolution with fp32 FMA accumulate, as tiled implicit GEMMs: forward, data gradient, filter and bias
 // gradient.  Every product and every sum is an fp32 FMA (packed two to an instruction: fma.rn.f32x2 rounds each half as
-// fmaf does), and long sums are kept short in two levels: a running sum of at most a few hundred terms is added to the
+// fmaf does), and long sums are kept short in two levels: a running sum of 64 terms (filter gradient: 128) is added to the
 // main accumulator and restarted.
 //
 // The bound is the fp32 FMA pipe (148 SMs x 128 FMA per clock: 74 TFLOP/s on paper, 60-68 in a loop of nothing else)
@@ -15,7 +15,7 @@
 // no atomics, reproducible.
 //
 // Measured on a B200 against one thread per output (the kernels of conv_direct.cu, which remain for geometries outside
-// f32_gemm_ok): figures at the launchers.
+// f32_gemm_ok and for the smallest calls, direct_wins): figures at the launchers.
 #include <cooperative_groups.h>
 #include <algorithm>
 
@@ -573,7 +573,9 @@ __global__ void __launch_bounds__(256) wgrad_f32_finish(size_t n, uint32_t K, ui
 static uint32_t wg_rows(uint32_t K) { return K > 32 ? 64u : (K > 16 ? 32u : 16u); }
 static uint32_t wg_cols(uint32_t K) { return 8192u / wg_rows(K); }
 // Slices of the pixel range beyond a cluster of 8, each CTA with at least eight stages of pixels: as many clusters as the
-// machine holds at a time with two CTAs per SM
+// machine holds at a time with two CTAs per SM.  That is the number of the form with 64 rows and one group (88 KB); the forms
+// of 32 and 16 rows and the one of two groups (116 to 185 KB) have one CTA per SM and hold about half as many, so that
+// their last slices are a second wave.
 constexpr unsigned long long kWgHeld = 33;
 static uint32_t wg_slices(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
   const unsigned long long tiles = (unsigned long long)((a->K + wg_rows(a->K) - 1) / wg_rows(a->K)) *

@@ -10,12 +10,12 @@
 //       The data gradient of a stride-1 convolution is the same kernel run over dy with the
 //       taps mirrored and the filter transposed to C,R,S,K.
 //       Persistent CTAs (one per SM) loop over tiles; warp 0 = TMA producer, warp 1 = MMA
-//       issuer (one elected thread), warps 2-5 = epilogue.  Two accumulators in tensor memory
-//       let the epilogue of tile i overlap the MMAs of tile i+1.
+//       issuer (one elected thread), warps 2-9 = two epilogue groups of four.  Two accumulators in
+//       tensor memory let the epilogue of tile i overlap the MMAs of tile i+1.
 //   filter gradient           conv_tc_wgrad_kernel
 //       GEMM  M = 128 output channels of dy, N = BN input channels of x, K = pixels.  Both
 //       operands are the NHWC tiles as TMA delivers them ([pixel][64 ch] rows), consumed as
-//       MN-major operands.  The pixel range is split across CTAs; each split writes an fp32
+//       MN-major operands; warps 2-5 are the epilogue.  The pixel range is split across CTAs; each split writes an fp32
 //       partial to caller scratch and a second kernel sums the partials in a fixed order
 //       (reproducible, no atomics).
 //
@@ -702,7 +702,8 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(size_t n, size_t part
   dw[o] = accumulate ? dw[o] + t : t;
 }
 // KCRS filters of several taps: a block owns 32 channels x all taps of one filter, a contiguous run of dw, and turns them
-// round in shared memory; element by element, each 4-byte store met its own 32-byte sector (3x3 512 x 512: the segmentation net's 50 filter gradients: 1.77 -> 1.06 ms).
+// round in shared memory; element by element, each 4-byte store met its own 32-byte sector (the reductions of the
+// segmentation net's 50 filter gradients: 1.77 -> 1.06 ms).
 constexpr uint32_t kWgRedPitch = 36;
 __global__ void wgrad_reduce_kcrs_kernel(size_t part_stride, uint32_t splits, const float* __restrict__ partial, float* dw,
                                          int accumulate, uint32_t taps, uint32_t C) {

@@ -240,7 +240,8 @@ int adh_net_backward(void* h) {
   n->ctx->end_phase();
   return AD_OK;
 }
-// flat gradient of rank's parameters (this rank's strip only, before the allreduce)
+// flat gradient of rank's parameters, between the backward pass and the update: of this rank's strip only.  (The update sums
+// the ranks' gradients and adds the weight decay in the same buffer: after it, that is what is there.)
 int adh_net_get_param_grads(void* h, int rank, float* host) {
   auto* n = (Net*)h;
   GPUContext* g = n->ctx->device_context((size_t)rank).get();

@@ -407,6 +407,8 @@ int ad_im2col(const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t sh, uint32
  *   AD_F32 / AD_NCHW : fp32 operands, fp32 accumulate (SIMT FMA).  Filter KCRS fp32.
  *   AD_BF16 / AD_NHWC: bf16 operands, fp32 accumulate in tensor memory (tcgen05.mma), operands
  *                      staged by TMA.  Filter KRSC bf16 (K, kh, kw, C), C and K multiples of 8 ...
+ * Implicit padding (pad_h, pad_w) takes part as zeros: in a filter gradient an infinite or NaN element of dy gives NaN at the
+ * taps that reach from it into the padding.
  * y / dy / dx may be views into larger (e.g. halo-padded) buffers: *_pitch give the row pitch
  * (elements between consecutive y) and *_plane the pitch between images (NHWC) or planes (NCHW);
  * 0 means packed.
