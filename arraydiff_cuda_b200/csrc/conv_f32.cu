@@ -16,41 +16,14 @@
 //
 // Measured on a B200 against one thread per output (the kernels of conv_direct.cu, which remain for geometries outside
 // f32_gemm_ok and for the smallest calls, direct_wins): figures at the launchers.
-#include <cooperative_groups.h>
 #include <algorithm>
 
-#include "common.cuh"
-#include "conv_f32_plan.h"
-
-namespace cg = cooperative_groups;
+#include "conv_f32.cuh"
 
 namespace adk {
 
-typedef unsigned long long u64;
-
-__device__ __forceinline__ void ffma2(u64& d, u64 a, u64 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b)); }
-__device__ __forceinline__ u64 dup2(float v) {
-  u64 r;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(u64 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-// 4 bytes global -> shared asynchronously where all bits of `need` are in `have`, else a zero (source size 0: not read)
-__device__ __forceinline__ void gather4(uint32_t dst, const float* src, uint32_t have, uint32_t need) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"((have & need) == need ? 4u : 0u) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-constexpr int kF32Most = 16;             // CTAs of a cluster, forward and data gradient
 constexpr int kF32Group = 128;           // threads that share one tile; a CTA is one or two such groups
 constexpr int kF32MaxK = 15;             // filter rows / columns: one bit each in a 32-bit word (rows 0.., columns 16..)
-constexpr uint32_t kF32Never = 1u << 31; // a bit no pixel has
 
 // A group is 4 warps, WM x WN of them over rows and columns; a warp's lanes are LM x (32 / LM) over rows and columns, a
 // thread owns 8 rows x 8 columns.  A CTA of G = 2 groups (filter gradients) halves every stage's pixels between them: 8
@@ -79,19 +52,6 @@ __device__ __forceinline__ float cluster_total(cg::cluster_group& cluster, float
 // A data gradient of a strided layer is one such GEMM per residue class of its pixels (blockIdx.z): the pixels
 // (y mod sh, x mod sw) = (ry, rx) meet only the taps whose distance is a multiple of the stride, so no tap is multiplied
 // that does not contribute.
-struct GemmF32 {
-  const float *in, *w, *bias;
-  float* out;
-  uint32_t M, CR, NI;
-  uint32_t IH, IW;                    // extent of `in`
-  long long in_pitch, in_plane, in_img;
-  uint32_t OH, OW;                    // full output extent
-  long long out_pitch, out_plane, out_img;
-  long long w_m, w_c;                 // filter strides of m and of the reduction channel (taps are contiguous)
-  uint32_t kh, kw, sh, sw, dh, dw;
-  int ph, pw;
-  int relu, accumulate;
-};
 // Shared memory: a ring of stages ([kd][m], pitch BM + 4, and [kd][pixel]; KB reduction indices each) beside the BM x BN
 // tile of main accumulators, to which the running sums of 64 terms go
 template <int LM, int WM, int WN> struct GemmTile : F32Tile<LM, WM, WN, 1> {
@@ -311,62 +271,6 @@ __global__ void __launch_bounds__(kF32Group, 3) conv_gemm_f32(const GemmF32 p) {
   if (cs > 1) cluster.sync();         // nobody leaves while its tile is still read
 }
 
-// What the launches of one kernel share: on which devices (a bit each) its limits are raised, and how many clusters of
-// 1, 2, 4, 8, 16 CTAs the machine holds at a time, plus one (0: not asked yet).  That is less than CTAs per SM x 148 / size:
-// a cluster stays within one group of SMs.
-struct F32Launch { unsigned raised = 0; uint32_t held[5] = {}; };
-
-template <typename Params>
-static cudaLaunchConfig_t f32_config(void (*)(Params), dim3 grid, int threads, int smem, uint32_t cs, cudaLaunchAttribute* at, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = (size_t)smem;
-  cfg.stream = s;
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.numAttrs = cs > 1 ? 1 : 0;
-  cfg.attrs = at;
-  return cfg;
-}
-template <typename Params>
-static int raise_f32(void (*k)(Params), int smem, F32Launch& l) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (l.raised & (1u << (dev & 31))) return AD_OK;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-    cudaGetLastError();
-    return AD_ERR_CUDA;
-  }
-  l.raised |= 1u << (dev & 31);
-  return AD_OK;
-}
-template <typename Params>
-static int launch_f32(void (*k)(Params), dim3 grid, int threads, int smem, uint32_t cs, const Params& p, F32Launch& l, cudaStream_t s) {
-  if (int rc = raise_f32(k, smem, l)) return rc;
-  cudaLaunchAttribute at[1];
-  const cudaLaunchConfig_t cfg = f32_config(k, grid, threads, smem, cs, at, s);
-  if (cudaLaunchKernelEx(&cfg, k, p) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
-  count_launch();
-  return launch_status();
-}
-// 0: not one such cluster fits (part of a GPU, a size above what the device allows)
-template <typename Params>
-static uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, F32Launch& l) {
-  uint32_t i = 0;
-  while ((1u << i) < cs) ++i;
-  if (!l.held[i]) {
-    cudaLaunchAttribute at[1];
-    cudaLaunchConfig_t cfg = f32_config(k, dim3(cs), threads, smem, cs, at, nullptr);
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (raise_f32(k, smem, l) != AD_OK || cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 0) { cudaGetLastError(); n = 0; }
-    l.held[i] = (uint32_t)n + 1;
-  }
-  return l.held[i] - 1;
-}
-
 template <int LM, int WM, int WN, bool DGRAD>
 static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uint32_t Kd, cudaStream_t s) {
   typedef GemmTile<LM, WM, WN> T;
@@ -379,6 +283,17 @@ static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uin
   return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, l, s);
 }
 
+// The 3x3 kernels own blocks of 4 x 2 pixels.  Where more than a fifth of them lies past the edges of the map (a third, if the
+// reduction is long), for 16 rows and fewer, and for long reductions into few tiles of 32 rows, which go to 8 CTAs at
+// most, the general tiles are as fast or faster: 17 x 42 x 13 x 5 -> 346 channels, two thirds used, 25 against 31 us;
+// 9 x 440 x 18 x 22 -> 27, 16 tiles, 48 against 65.  The other way: 4 x 512 x 7 x 7 -> 512 data gradient, two thirds used, 94 -> 66.
+static bool f32_k3_gemm_wins(const GemmF32& p) {
+  if (p.kh != 3 || p.kw != 3 || p.sh != 1 || p.sw != 1 || p.dh != 1 || p.dw != 1 || p.M <= 16) return false;
+  const unsigned long long used = (unsigned long long)p.OH * p.OW, blocks = (unsigned long long)((p.OH + 3) / 4) * ((p.OW + 1) / 2);
+  if (p.M <= 32 && p.CR > 128 && p.NI * blocks < 24 * 32) return false;
+  return used * 20 >= blocks * 8 * (p.CR >= 192 ? 13 : 16);
+}
+
 // Tile height by the row count: a row of the tile costs the same FMAs whether it holds a channel or not, a column is
 // gathered once per tile row: 64 x 128 for more than 32 channels, 32 x 256, 16 x 512 and 8 x 1024 below.
 template <bool DGRAD>
@@ -386,6 +301,7 @@ static int run_gemm_f32(const GemmF32& p, cudaStream_t s) {
   const uint32_t classes = DGRAD ? p.sh * p.sw : 1;
   const uint32_t OHc = DGRAD ? (p.OH + p.sh - 1) / p.sh : p.OH, OWc = DGRAD ? (p.OW + p.sw - 1) / p.sw : p.OW;
   const uint32_t npx = p.NI * OHc * OWc, Kd = p.CR * ((p.kh * p.kw + classes - 1) / classes);
+  if (f32_k3_gemm_wins(p)) return f32_k3_gemm<DGRAD>(p, s);
   if (p.M <= 8) return launch_gemm_f32<1, 1, 4, DGRAD>(p, npx, classes, Kd, s);
   if (p.M <= 16) return launch_gemm_f32<2, 1, 4, DGRAD>(p, npx, classes, Kd, s);
   if (p.M <= 32) return launch_gemm_f32<4, 1, 4, DGRAD>(p, npx, classes, Kd, s);
@@ -396,15 +312,6 @@ static int run_gemm_f32(const GemmF32& p, cudaStream_t s) {
 // GEMM: rows m = output channels, columns n = (input channel, tap), reduction = output pixels, which is the order both
 // operands have in memory.  The reduction is split over the CTAs of a cluster and over `slices` of the grid; with more
 // than one slice the clusters write partial gradients to scratch and wgrad_f32_finish adds them in order.
-struct WgradF32 {
-  const float *x, *dy;
-  float *dw, *db, *part;
-  uint32_t K, C, N, P, Q, H, W, kh, kw, sh, sw, dh, dw_;
-  int ph, pw;
-  long long dy_pitch, dy_plane;
-  int accumulate;
-  uint32_t slices;
-};
 // Shared memory: a ring of stages ([row][32 pixels], pitch 36: reads and writes free of bank conflicts) beside the BM x BN
 // tile of main accumulators.  One packed FMA multiplies two neighbouring pixels; the halves are added at the end.
 constexpr int kWgKB = 32, kWgPitch = 36, kWgStages = 2, kWgFlush = 8;
@@ -586,6 +493,13 @@ static uint32_t wg_slices(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
   return (uint32_t)(n > 16 ? 16 : (n < 1 ? 1 : n));
 }
 
+static int finish_wgrad_f32(const WgradF32& p, cudaStream_t s) {
+  const size_t n = (size_t)p.K * p.C * p.kh * p.kw;
+  launch(wgrad_f32_finish, (unsigned)((n + p.K + 255) / 256), 256, 0, s, n, p.K, p.slices, p.part, p.dw, p.db, p.accumulate);
+  count_launch();
+  return launch_status();
+}
+
 template <int LM, int WM, int WN, int G>
 static int launch_wgrad_f32(WgradF32& p, cudaStream_t s) {
   typedef WgTile<LM, WM, WN, G> T;
@@ -595,11 +509,7 @@ static int launch_wgrad_f32(WgradF32& p, cudaStream_t s) {
   auto held = [](uint32_t n) { return f32_held(conv_wgrad_gemm_f32<LM, WM, WN, G>, T::threads, T::smem, n, l); };
   const uint32_t cs = p.slices > 1 ? f32_largest_cluster(held, 8) : f32_cluster_size(held, (unsigned long long)tn * tm, steps, 8, kNumSMs);
   int st = launch_f32(conv_wgrad_gemm_f32<LM, WM, WN, G>, dim3(tn * cs, tm, p.slices), T::threads, T::smem, cs, p, l, s);
-  if (st != AD_OK || p.slices == 1) return st;
-  const size_t n = (size_t)p.K * p.C * p.kh * p.kw;
-  launch(wgrad_f32_finish, (unsigned)((n + p.K + 255) / 256), 256, 0, s, n, p.K, p.slices, p.part, p.dw, p.db, p.accumulate);
-  count_launch();
-  return launch_status();
+  return st != AD_OK || p.slices == 1 ? st : finish_wgrad_f32(p, s);
 }
 
 // ---------------------------------------------------------------- entry points (called by conv_direct.cu)
@@ -616,15 +526,34 @@ bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pi
          a->K <= 65535u * 8 && a->C <= 65535u * 8 && y_pitch >= 0 && y_plane >= 0;
 }
 
+// The 3x3 kernel's tiles are 64 x 16 channels (32 x 32 for up to 32 output channels), the general one's 64 x 128 (channel, tap)
+// columns: it wins from 16 channels on where more than half of its tiles is used (11 channels: 35 against 47 us, 14: 36
+// against 63, 17: 109 against 137, 33 output channels: 79 against 103; the other way 25: 430 -> 367, 32: 54 -> 52).
+static bool f32_k3_wgrad_wins(const ad_conv2d_args* a) {
+  if (a->kh != 3 || a->kw != 3 || a->stride_h != 1 || a->stride_w != 1 || a->dil_h != 1 || a->dil_w != 1 || a->K <= 16 || a->C < 16) return false;
+  if (a->K <= 32) return true;
+  const unsigned long long k = (a->K + 63) / 64 * 64, c = (a->C + 15) / 16 * 16;
+  return 25ull * a->K * a->C >= 14ull * k * c;
+}
+// Whether the 3x3 kernels serve the pass: their smallest calls take 10 - 13 us (filter gradient 17 - 19)
+bool f32_k3_takes(const ad_conv2d_args* a, int pass, uint32_t P, uint32_t Q) {
+  if (pass == 2) return f32_k3_wgrad_wins(a);
+  GemmF32 p = {};
+  p.M = pass ? a->C : a->K; p.OH = pass ? a->H : P; p.OW = pass ? a->W : Q;
+  p.kh = a->kh; p.kw = a->kw; p.sh = a->stride_h; p.sw = a->stride_w; p.dh = a->dil_h; p.dw = a->dil_w;
+  return f32_k3_gemm_wins(p);
+}
+
 size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
-  const uint32_t s = wg_slices(a, P, Q);
+  const uint32_t s = f32_k3_wgrad_wins(a) ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q).slices : wg_slices(a, P, Q);
   return s > 1 ? (size_t)s * ((size_t)a->K * a->C * a->kh * a->kw + a->K) * 4 : 0;
 }
 
-// Measured (one B200; per call, before -> now): 64 -> 64 channels, 3x3, 64 x 64 pixels, one image: forward 188 -> 19 us, data
-// gradient 158 -> 23, filter and bias gradient 286 -> 29.  4 x 64 x 112 x 112, 64 -> 64 3x3: 1440 -> 127, 1500 -> 125, 2330 ->
-// 168 us (29 / 30 / 22 TFLOP/s).  What is left above the FMA pipe: 12 warps per SM do not hide the latency of the
-// shared-memory reads (issue slots 42 % busy); 4 x 8 outputs per thread or packed pairs along the reduction were slower.
+// Measured (one B200; per call, thread per output -> these tiles): 64 -> 64 channels, 3x3, 64 x 64 pixels, one image: forward
+// 188 -> 21 us, data gradient 158 -> 25, filter and bias gradient 286 -> 31.  4 x 64 x 112 x 112, 64 -> 64 3x3: 1440 -> 135, 1500 ->
+// 134, 2330 -> 172 us (27 / 28 / 21 TFLOP/s); conv_f32_k3.cu, which serves these two now, takes 19, 25, 25 and 94, 92, 127.
+// What is left above the FMA pipe: 12 warps per SM do not hide the latency of the shared-memory reads (issue slots 42 % busy);
+// 4 x 8 outputs per thread or packed pairs along the reduction were slower.
 int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
   GemmF32 p = {};
   p.in = (const float*)a->x; p.w = (const float*)a->w; p.bias = a->bias; p.out = (float*)a->y;
@@ -718,7 +647,13 @@ int f32_gemm_wgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
   p.dy_pitch = y_pitch; p.dy_plane = y_plane; p.accumulate = a->accumulate;
   p.slices = 1;
   const size_t need = f32_wgrad_scratch(a, P, Q);
-  if (need && a->scratch && a->scratch_bytes >= need) { p.slices = wg_slices(a, P, Q); p.part = (float*)a->scratch; }
+  const bool k3 = f32_k3_wgrad_wins(a), parts = need && a->scratch && a->scratch_bytes >= need;
+  const F32Split split = k3 ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q) : F32Split{8, wg_slices(a, P, Q)};
+  if (parts) { p.slices = split.slices; p.part = (float*)a->scratch; }
+  if (k3) {
+    const int rc = f32_k3_wgrad(p, parts || split.slices == 1 ? split.cs : 8, s);
+    return rc != AD_OK || p.slices == 1 ? rc : finish_wgrad_f32(p, s);
+  }
   // clusters of 8 fill at most one CTA per SM: two groups per CTA (9 tiles of 4096 pixels: 31 -> 27 us)
   const unsigned long long tiles = (unsigned long long)((a->K + 63) / 64) * ((a->C * a->kh * a->kw + 127) / 128) * p.slices;
   switch (wg_rows(a->K)) {

@@ -28,6 +28,48 @@ uint32_t f32_cluster_size(Held held, unsigned long long tiles, uint32_t steps, u
   return best ? best : 1;
 }
 
+// The 3x3 kernels (conv_f32_k3.cu) keep the FMA pipe busy with one CTA per SM, so that CTAs on one SM take turns (a stage
+// measured 1.1 us alone, 1.9 beside one other, 2.7 beside two), and the SM with the most of them counts.  A cluster stays
+// within one group of SMs, so that larger ones are spread less evenly: 36 clusters of 4 leave some SMs two CTAs (filter gradient
+// 64 -> 64, 4 x 112 x 112: 184 us, 32 clusters of 4 133), and so do 16 of 8 already (half of the SMs were idle).
+inline double f32_k3_share(unsigned long long ctas, uint32_t cs, uint32_t sms) {
+  static const double per_stage[4] = {0, 1.2, 2.1, 3.0};
+  const double even = (double)ctas * (cs >= 8 ? 1.15 : cs >= 4 ? 1.1 : cs == 2 ? 1.02 : 1.0) / sms;
+  return per_stage[even > 2 ? 3 : even > 1 || (cs >= 8 && even > 0.5) ? 2 : ctas ? 1 : 0];
+}
+template <typename Held>
+uint32_t f32_k3_cluster(Held held, unsigned long long tiles, uint32_t steps, uint32_t most, uint32_t sms) {
+  uint32_t best = 0;
+  double best_cost = 0;
+  for (uint32_t cs = 1; cs <= most && (cs == 1 || steps >= 2 * cs); cs *= 2) {
+    const unsigned long long h = held(cs);
+    if (!h) continue;
+    const double cta = (steps + cs - 1) / cs + 3 + 0.5 * cs, cost = cta * (tiles / h * f32_k3_share(h * cs, cs, sms) + f32_k3_share(tiles % h * cs, cs, sms));
+    // a CTA sums over 128 stages (256 channels) at most where that can be: the sum of its running sums loses precision with
+    // their number (371 channels in one CTA: 2.0e-7 against 1.7e-7 in two)
+    if (!best || cost < best_cost || (steps > 128 * best)) { best = cs; best_cost = cost; }
+  }
+  return best ? best : 1;
+}
+
+// Filter gradient of the 3x3 kernels: CTAs of a cluster x slices of the grid that share a tile's `all` stages of pixels
+struct F32Split { uint32_t cs, slices; };
+inline F32Split f32_k3_split(unsigned long long tiles, unsigned long long all, uint32_t sms) {
+  static const unsigned held[4] = {444, 222, 104, 48};      // clusters of 1, 2, 4, 8 CTAs, three CTAs per SM
+  F32Split best = {1, 1};
+  double best_cost = 0;
+  for (uint32_t i = 0; i < 4; ++i)
+    for (uint32_t sl = 1; sl <= 16; ++sl) {
+      const uint32_t cs = 1u << i, parts = cs * sl;
+      if (parts > 1 && all < 2ull * parts) break;
+      const unsigned long long h = held[i], n = tiles * sl;
+      const double cta = (double)((all + parts - 1) / parts) + 2 + 0.25 * cs;
+      const double cost = cta * (n / h * f32_k3_share(h * cs, cs, sms) + f32_k3_share(n % h * cs, cs, sms)) + (sl > 1 ? 3 + 0.3 * sl : 0);
+      if (best_cost == 0 || cost < best_cost) { best = {cs, sl}; best_cost = cost; }
+    }
+  return best;
+}
+
 // `most` CTAs, or the largest smaller power of two of which the machine holds a cluster
 template <typename Held>
 uint32_t f32_largest_cluster(Held held, uint32_t most) {

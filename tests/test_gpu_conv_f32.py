@@ -118,3 +118,71 @@ def test_data_gradient_of_more_than_2_32_elements():
         full[:, :Hh, :Hh] = dx[n]
         got = full.unflatten(1, (P, s))[:, :, :k].unflatten(3, (P, s))[..., :k]
         assert (got - want).abs().max() < 1e-5 * want.max() and torch.count_nonzero(dx[n]) == got.numel()   # zeros elsewhere
+
+
+K3_CASES = [
+    # N, C, H, W (of x), K, pad: 3x3, stride and dilation 1
+    (1, 16, 3, 3, 17, 0),          # one output pixel; the smallest channel counts of the 3x3 kernels
+    (1, 17, 6, 4, 33, 0),          # one block of 4 x 2 pixels; a channel past a pair of stages, a row past the 32-row tile
+    (3, 20, 11, 13, 64, 1),        # blocks past both edges, implicit padding, images that share a tile
+    (2, 33, 10, 17, 65, 2),        # padding of 2: the gradient's map is smaller than y; a row past the 64-row tile
+    (1, 130, 9, 12, 24, 1),        # 32-row tiles, reduction split over a cluster; rows of 12 = 8 + 4 pixels
+    (5, 48, 18, 19, 80, 1),        # running sums that restart, 19 = 8 + 8 + 3 pixels
+    (1, 300, 23, 25, 40, 0),       # more than 256 channels per CTA of a cluster of one
+    (4, 64, 58, 61, 32, 0),        # filter gradient in clusters and slices of the scratch
+]
+
+
+@pytest.mark.parametrize("scratch", [True, False])
+@pytest.mark.parametrize("case", K3_CASES)
+def test_conv_f32_3x3(case, scratch, monkeypatch):
+    """The 3x3 kernels at the edges of their tiles, blocks, segments and splits; infinities stay where they have a weight."""
+    import torch
+    monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", "1")
+    N, Cc, Hh, W, K, pd = case
+    x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, 3, 3), float(np.sqrt(2.0 / (9 * Cc)))), H.normal(3, (K,))
+    y_w = orc.conv2d_fprop(x, w, b, (1, 1), (1, 1), (pd, pd), omp=True)
+    dy = H.uniform(4, y_w.shape)
+    dx_w = orc.conv2d_dgrad(dy, w, x.shape, (1, 1), (1, 1), (pd, pd), omp=True)
+    db_w = np.zeros(K, np.float32)
+    dw_w = orc.conv2d_wgrad(x, dy, w.shape, (1, 1), (1, 1), (pd, pd), db=db_w, omp=True)
+    L = abi.lib()
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, 3, 1, 1, pd)
+    P, Q = y_w.shape[2:]
+    y, gy = torch.full((N, K, P + 1, Q + 3), 7.0, device="cuda"), torch.full((N, K, P + 1, Q + 3), float("nan"), device="cuda")
+    gy[:, :, :P, :Q] = H.dev(dy)
+    xd, wd, bd = H.dev(x), H.dev(w), H.dev(b)
+    dx, dw, db = torch.ones(x.shape, device="cuda"), torch.ones(w.shape, device="cuda"), torch.ones(K, device="cuda")
+    a.x, a.w, a.bias, a.y, a.y_pitch, a.y_plane = xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), y.data_ptr(), Q + 3, (P + 1) * (Q + 3)
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    a.y, a.dx, a.dw, a.db, a.accumulate = gy.data_ptr(), dx.data_ptr(), dw.data_ptr(), db.data_ptr(), 1
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    if scratch:
+        part = torch.full((max(16, L.ad_conv2d_scratch_bytes(C.byref(a), 2)),), 255, dtype=torch.uint8, device="cuda")
+        a.scratch, a.scratch_bytes = part.data_ptr(), part.numel()
+    abi.check(L.ad_conv2d_wgrad(C.byref(a), H.stream()))
+    H.sync()
+    got = H.host(y)
+    assert H.max_rel(got[:, :, :P, :Q], y_w) < 1e-5
+    assert np.all(got[:, :, P:, :] == 7.0) and np.all(got[:, :, :, Q:] == 7.0)
+    # 1 + v rounds to 2^-24 of its size
+    assert np.max(np.abs(H.host(dx) - 1 - dx_w)) < 1e-5 * np.max(np.abs(dx_w)) + 1e-6
+    assert np.max(np.abs(H.host(dw) - 1 - dw_w)) < 2e-5 * np.max(np.abs(dw_w)) + 1e-6
+    assert np.max(np.abs(H.host(db) - 1 - db_w)) < 2e-5 * np.max(np.abs(db_w)) + 1e-6
+    # an infinite pixel of x reaches the outputs and filter entries that it has a product in, and no others
+    n, c, iy, ix = N - 1, Cc - 1, Hh - 1, W - 1
+    xd[n, c, iy, ix] = float("inf")
+    a.y, a.accumulate = y.data_ptr(), 0
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    a.y = gy.data_ptr()
+    abi.check(L.ad_conv2d_wgrad(C.byref(a), H.stream()))
+    H.sync()
+    hit = np.zeros((N, P, Q), bool)
+    taps = np.zeros((Cc, 3, 3), bool)
+    for i in range(3):
+        for j in range(3):
+            oy, ox = iy + pd - i, ix + pd - j
+            if 0 <= oy < P and 0 <= ox < Q:
+                hit[n, oy, ox] = taps[c, i, j] = True
+    assert np.array_equal(~np.isfinite(H.host(y)[:, :, :P, :Q]).all(1), hit)
+    assert np.array_equal(~np.isfinite(H.host(dw)).all(0), taps)
