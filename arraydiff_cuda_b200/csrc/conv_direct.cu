@@ -153,7 +153,6 @@ static int geometry(const ad_conv2d_args* a, ConvG& g) {
   return AD_OK;
 }
 
-bool f32_k3_takes(const ad_conv2d_args* a, int pass, uint32_t P, uint32_t Q);
 bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane);
 int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
 int f32_gemm_dgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s);
@@ -165,17 +164,17 @@ size_t f32_dgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q);
 // the sums over the cluster.  A thread per output is bound by its chain of loads (0.36 us per term of a 1x1 filter, whose
 // terms are planes apart, 0.14 of a larger one, 0.06 per term of a data gradient), by the number of terms in all, and as a
 // filter gradient by the rounds of 256 pixels of a block.  These times come within a quarter of 60 measured layers of up to
-// 25 M multiplications; of those the smallest ran three times faster this way.  A 3x3 layer that conv_f32_k3.cu serves takes
-// 10 - 13 us there (a filter gradient 17 - 19), so that only smaller calls stay here.
-static bool direct_wins(const ad_conv2d_args* a, const ConvG& g, int pass) {
+// 25 M multiplications; of those the smallest ran three times faster this way.  (The 3x3 kernels of conv_f32_k3.cu would take
+// 10 - 19 us for the smallest calls too; but these sums of 9 terms and of channels are the more precise ones, 0.75e-7 against
+// 0.85 - 1.2e-7, and the calls stay here.)
+static bool direct_wins(const ConvG& g, int pass) {
   if (const char* t = getenv("ARRAYDIFF_B200_F32_TILES")) return t[0] == '0';   // the parity tests: "1" tiled, "0" direct
   const double taps = (double)g.kh * g.kw, px = (double)g.N * g.P * g.Q, mmac = px * g.K * g.C * taps * 1e-6;
   const bool one = g.kh * g.kw == 1;
-  const bool k3 = f32_k3_takes(a, pass, g.P, g.Q);
   auto most = [](double x, double y) { return x > y ? x : y; };
-  if (pass == 0) return 4 + (one ? 0.36 : 0.14) * most(g.C * taps, 9 * mmac) < (k3 ? 12 : 25);
-  if (pass == 1) return 4 + most(0.06 * g.K * taps, 2 * mmac * g.sh * g.sw) < (k3 ? 12 : 25);
-  return taps <= 49 && 6 + most(px / 256 * (one ? 0.9 : 0.25 * taps), mmac * (one ? 7.8 : 2.6)) < (k3 ? 18 : 40);
+  if (pass == 0) return 4 + (one ? 0.36 : 0.14) * most(g.C * taps, 9 * mmac) < 25;
+  if (pass == 1) return 4 + most(0.06 * g.K * taps, 2 * mmac * g.sh * g.sw) < 25;
+  return taps <= 49 && 6 + most(px / 256 * (one ? 0.9 : 0.25 * taps), mmac * (one ? 7.8 : 2.6)) < 40;
 }
 
 int conv_direct_fprop(const ad_conv2d_args* a, cudaStream_t s) {
@@ -184,7 +183,7 @@ int conv_direct_fprop(const ad_conv2d_args* a, cudaStream_t s) {
   if (st != AD_OK) return st;
   if (!a->x || !a->w || !a->y) return AD_ERR_BAD_ARG;
   if (a->out_row_count) return AD_ERR_UNSUPPORTED;   // row ranges: tensor-core path only
-  if (!direct_wins(a, g, 0) && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_fprop(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
+  if (!direct_wins(g, 0) && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_fprop(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
   const size_t total = (size_t)g.N * g.K * g.P * g.Q;
   conv_fprop_f32<<<grid_for(total, 256, 16), 256, 0, s>>>(g, (const float*)a->x, (const float*)a->w, a->bias, (float*)a->y);
   count_launch();
@@ -197,7 +196,7 @@ int conv_direct_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
   if (st != AD_OK) return st;
   if (!a->y || !a->w || !a->dx) return AD_ERR_BAD_ARG;
   if (a->dx_col_count) return AD_ERR_UNSUPPORTED;   // column ranges: tensor-core path only
-  if (!direct_wins(a, g, 1) && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_dgrad(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
+  if (!direct_wins(g, 1) && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_dgrad(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
   const size_t total = (size_t)g.N * g.C * g.H * g.W;
   conv_dgrad_f32<<<grid_for(total, 256, 16), 256, 0, s>>>(g, (const float*)a->y, (const float*)a->w, (float*)a->dx);
   count_launch();
@@ -208,7 +207,7 @@ int conv_direct_dgrad(const ad_conv2d_args* a, cudaStream_t s) {
 // channels takes its two-step form (optional: less or none is fine)
 size_t conv_direct_scratch_bytes(const ad_conv2d_args* a, int pass) {
   ConvG g;
-  if (geometry(a, g) != AD_OK || direct_wins(a, g, pass) || !f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return 0;
+  if (geometry(a, g) != AD_OK || direct_wins(g, pass) || !f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return 0;
   if (pass == 1) return f32_dgrad_scratch(a, g.P, g.Q);
   if (pass != 2 || g.kh * g.kw > 49) return 0;
   return f32_wgrad_scratch(a, g.P, g.Q);
@@ -220,7 +219,7 @@ int conv_direct_wgrad(const ad_conv2d_args* a, cudaStream_t s) {
   if (st != AD_OK) return st;
   if (!a->x || !a->y || !a->dw) return AD_ERR_BAD_ARG;
   const uint32_t taps = g.kh * g.kw;
-  if (taps <= 49 && !direct_wins(a, g, 2) && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_wgrad(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
+  if (taps <= 49 && !direct_wins(g, 2) && f32_gemm_ok(a, g.P, g.Q, g.y_pitch, g.y_plane)) return f32_gemm_wgrad(a, g.P, g.Q, g.y_pitch, g.y_plane, s);
   if (taps <= 9) conv_wgrad_f32<9><<<g.K * g.C, 256, 0, s>>>(g, (const float*)a->x, (const float*)a->y, (float*)a->dw);
   else if (taps <= 49) conv_wgrad_f32<49><<<g.K * g.C, 256, 0, s>>>(g, (const float*)a->x, (const float*)a->y, (float*)a->dw);
   else return AD_ERR_UNSUPPORTED;

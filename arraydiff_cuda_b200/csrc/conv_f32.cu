@@ -535,15 +535,6 @@ static bool f32_k3_wgrad_wins(const ad_conv2d_args* a) {
   const unsigned long long k = (a->K + 63) / 64 * 64, c = (a->C + 15) / 16 * 16;
   return 25ull * a->K * a->C >= 14ull * k * c;
 }
-// Whether the 3x3 kernels serve the pass: their smallest calls take 10 - 13 us (filter gradient 17 - 19)
-bool f32_k3_takes(const ad_conv2d_args* a, int pass, uint32_t P, uint32_t Q) {
-  if (pass == 2) return f32_k3_wgrad_wins(a);
-  GemmF32 p = {};
-  p.M = pass ? a->C : a->K; p.OH = pass ? a->H : P; p.OW = pass ? a->W : Q;
-  p.kh = a->kh; p.kw = a->kw; p.sh = a->stride_h; p.sw = a->stride_w; p.dh = a->dil_h; p.dw = a->dil_w;
-  return f32_k3_gemm_wins(p);
-}
-
 size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
   const uint32_t s = f32_k3_wgrad_wins(a) ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q).slices : wg_slices(a, P, Q);
   return s > 1 ? (size_t)s * ((size_t)a->K * a->C * a->kh * a->kw + a->K) * 4 : 0;
