@@ -5,6 +5,7 @@
 // to caller scratch, stage 2 combines them in double.  No atomics, so results are
 // reproducible run to run.  Threads walk the tensor along its fastest axis (x for
 // NCHW-like views, channel for NHWC-like views) so that warps read whole sectors.
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -33,51 +34,95 @@ struct BnRed {
   const float *gamma, *beta, *mean, *invstd;
 };
 
-template <typename T, int MODE>
-__device__ __forceinline__ void bn_term(const BnRed& p, uint32_t n, uint32_t c, uint32_t y, uint32_t x, float& a,
-                                        float& b) {
+// what an x-fastest reduction sums in
+template <int MODE> struct BnSum { using type = float; };
+template <> struct BnSum<0> { using type = double; };
+
+template <typename T, int MODE, typename A>
+__device__ __forceinline__ void bn_term(const BnRed& p, uint32_t n, uint32_t c, uint32_t y, uint32_t x, A& a, A& b) {
   const long long ox = n * p.x.sn + c * p.x.sc + y * p.x.sy + x * p.x.sx;
   const float xv = ld_f((const T*)p.x.base + ox);
   if (MODE == 0) {
-    a += xv;
-    b = fmaf(xv, xv, b);
+    a += (A)xv;
+    b = fma((A)xv, (A)xv, b);
   } else {
     const long long od = n * p.dy.sn + c * p.dy.sc + y * p.dy.sy + x * p.dy.sx;
     float g = ld_f((const T*)p.dy.base + od);
     const float xhat = (xv - p.mean[c]) * p.invstd[c];
     if (p.relu && fmaf(p.gamma[c], xhat, p.beta[c]) <= 0.f) g = 0.f;
     a += g;
-    b = fmaf(g, xhat, b);
+    b = fma(g, xhat, b);
   }
 }
 
-// NCHW-like: block (256) per (channel, split); threads stride over (n, y, x).
-template <typename T, int MODE>
+// Views whose planes are runs of floats that 16-byte loads reach
+static bool planes_vec_ok(const ad_tensor4* t) {
+  return t->dtype == AD_F32 && t->sx == 1 && t->sy == (int64_t)t->W && !((uintptr_t)t->base & 15u) && !(t->sn & 3) && !(t->sc & 3) &&
+         ((unsigned long long)t->H * t->W) % 4 == 0 && (unsigned long long)t->H * t->W < (1ull << 31);
+}
+
+// NCHW-like: block (256) per (channel, split); threads stride over (n, y, x), 4 pixels at a time where the planes allow it (VEC).
+// The forward statistics are summed in double, and a split writes its sums as two rows of floats, high and low parts: the
+// variance is the small difference of E[x^2] and E[x]^2, and with sums in fp32 its error was what the gradients of a small fp32
+// net differed by from a double-precision one (18 layers, 16 pixels per channel at the end: 8e-4 -> 4e-5 of a filter
+// gradient).  The conversions and double additions are a tenth of what the SM can do in the time of the loads.
+template <typename T, int MODE, bool VEC>
 __global__ void __launch_bounds__(256) bn_reduce_xfast(BnRed p, float* partial) {
   grid_dependency();
   const uint32_t c = blockIdx.x, split = blockIdx.y, nsplit = gridDim.y;
-  const size_t per = (size_t)p.N * p.H * p.W;
-  float a = 0.f, b = 0.f;
+  using A = typename BnSum<MODE>::type;
+  A a = 0, b = 0;
   // the position moves on by the same (images, rows, columns) each time: no division per element
   const size_t first = (size_t)split * 256 + threadIdx.x, hop = (size_t)nsplit * 256;
-  const uint32_t hx = (uint32_t)(hop % p.W), hy = (uint32_t)(hop / p.W % p.H), hn = (uint32_t)(hop / p.W / p.H);
-  uint32_t x = (uint32_t)(first % p.W), y = (uint32_t)(first / p.W % p.H), n = (uint32_t)(first / p.W / p.H);
+  if constexpr (VEC) {
+    const uint32_t hw = p.H * p.W / 4, hi = (uint32_t)(hop % hw), hn = (uint32_t)(hop / hw);
+    uint32_t i = (uint32_t)(first % hw), n = (uint32_t)(first / hw);
+    const float *xb = (const float*)p.x.base + c * p.x.sc, *db = (const float*)p.dy.base + c * p.dy.sc;
+    const float mean = MODE ? p.mean[c] : 0.f, invstd = MODE ? p.invstd[c] : 0.f, gam = MODE ? p.gamma[c] : 0.f, bet = MODE ? p.beta[c] : 0.f;
 #pragma unroll 4
-  for (size_t i = first; i < per; i += hop) {
-    bn_term<T, MODE>(p, n, c, y, x, a, b);
-    x += hx; y += hy; n += hn;
-    if (x >= p.W) { x -= p.W; ++y; }
-    if (y >= p.H) { y -= p.H; ++n; }
+    for (; n < p.N;) {
+      const float4 v = *(const float4*)(xb + n * p.x.sn + (size_t)i * 4);
+      const float xv[4] = {v.x, v.y, v.z, v.w};
+      if constexpr (MODE == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { const double d = (double)xv[j]; a += d; b = fma(d, d, b); }
+      } else {
+        const float4 w = *(const float4*)(db + n * p.dy.sn + (size_t)i * 4);
+        const float gv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float xhat = (xv[j] - mean) * invstd;
+          const float g = p.relu && fmaf(gam, xhat, bet) <= 0.f ? 0.f : gv[j];
+          a += g;
+          b = fmaf(g, xhat, b);
+        }
+      }
+      i += hi; n += hn;
+      if (i >= hw) { i -= hw; ++n; }
+    }
+  } else {
+    const size_t per = (size_t)p.N * p.H * p.W;
+    const uint32_t hx = (uint32_t)(hop % p.W), hy = (uint32_t)(hop / p.W % p.H), hn = (uint32_t)(hop / p.W / p.H);
+    uint32_t x = (uint32_t)(first % p.W), y = (uint32_t)(first / p.W % p.H), n = (uint32_t)(first / p.W / p.H);
+#pragma unroll 4
+    for (size_t i = first; i < per; i += hop) {
+      bn_term<T, MODE>(p, n, c, y, x, a, b);
+      x += hx; y += hy; n += hn;
+      if (x >= p.W) { x -= p.W; ++y; }
+      if (y >= p.H) { y -= p.H; ++n; }
+    }
   }
-  __shared__ float sa[8], sb[8];
-  a = warp_sum(a); b = warp_sum(b);
+  __shared__ A sa[8], sb[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); }
   if ((threadIdx.x & 31) == 0) { sa[threadIdx.x >> 5] = a; sb[threadIdx.x >> 5] = b; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float ta = 0.f, tb = 0.f;
-    for (int w = 0; w < 8; ++w) { ta += sa[w]; tb += sb[w]; }
-    partial[(size_t)split * 2 * p.C + c] = ta;
-    partial[(size_t)split * 2 * p.C + p.C + c] = tb;
+  if (threadIdx.x < 2) {
+    A t = 0;
+    for (int w = 0; w < 8; ++w) t += threadIdx.x ? sb[w] : sa[w];
+    float* out = partial + (size_t)split * (MODE == 0 ? 4 : 2) * p.C + threadIdx.x * p.C + c;
+    *out = (float)t;
+    if (MODE == 0) out[2 * p.C] = isfinite((float)t) ? (float)(t - (A)(float)t) : 0.f;
   }
 }
 
@@ -213,6 +258,72 @@ __global__ void __launch_bounds__(256) bn_apply(BnApply p) {
       if (p.accumulate) v += ld_f((const T*)p.add.base + (n * p.add.sn + c * p.add.sc + y * p.add.sy + x * p.add.sx));
       st_f(op, v);
     }
+  }
+}
+// The same for views that are not channel-fastest: a block serves part of one (image, channel) plane, so that the channel's
+// constants are read once and a pixel's place costs one 32-bit division (VEC: none, 4 pixels per load).  Element by
+// element over the whole tensor (bn_apply, with 64-bit divisions and the sums divided by the count for each) the 34
+// normalisations of an 18-layer net on 4 x 224 x 224 took 527 us, so 205; with the sums 867 -> 372.
+constexpr uint32_t kPlaneApply = 1024, kPlaneApplyVec = 2048;   // pixels per block
+template <typename T, int MODE, bool VEC>
+__global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunks) {
+  grid_dependency();
+  const uint32_t plane = blockIdx.x / chunks, chunk = blockIdx.x - plane * chunks, n = plane / p.C, c = plane - n * p.C, hw = p.H * p.W;
+  const float mean = p.mean[c], invstd = p.invstd[c], gam = p.gamma[c], bet = p.beta[c];
+  const float m1 = MODE ? p.partial[2 * p.C + c] : 0.f, m2 = MODE ? p.partial[3 * p.C + c] : 0.f, scale = gam * invstd;
+  const T *xb = (const T*)p.x.base + n * p.x.sn + c * p.x.sc, *db = (const T*)p.dy.base + n * p.dy.sn + c * p.dy.sc;
+  const T* ab = (const T*)p.add.base + n * p.add.sn + c * p.add.sc;
+  T* ob = (T*)p.out.base + n * p.out.sn + c * p.out.sc;
+  auto value = [&](float xv, float g, float old) {
+    const float xhat = (xv - mean) * invstd;
+    if (MODE == 0) {
+      const float v = fmaf(gam, xhat, bet);
+      return p.relu ? fmaxf(v, 0.f) : v;
+    }
+    if (p.relu && fmaf(gam, xhat, bet) <= 0.f) g = 0.f;
+    const float v = scale * (g - m1 - xhat * m2);
+    return p.accumulate ? v + old : v;
+  };
+  if constexpr (VEC) {
+    constexpr int U = kPlaneApplyVec / 1024;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 xv[U], g[U], old[U];
+    const uint32_t i0 = chunk * kPlaneApplyVec + threadIdx.x * 4;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = i0 + u * 1024;
+      xv[u] = g[u] = old[u] = zero;
+      if (i < hw) {
+        xv[u] = *(const float4*)(xb + i);
+        if (MODE == 1) g[u] = *(const float4*)(db + i);
+        if (MODE == 1 && p.accumulate) old[u] = *(const float4*)(ab + i);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = i0 + u * 1024;
+      if (i < hw)
+        *(float4*)(ob + i) = make_float4(value(xv[u].x, g[u].x, old[u].x), value(xv[u].y, g[u].y, old[u].y), value(xv[u].z, g[u].z, old[u].z),
+                                         value(xv[u].w, g[u].w, old[u].w));
+    }
+  } else {
+    constexpr int U = kPlaneApply / 256;
+    float xv[U], g[U], old[U];
+    long long at[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t i = chunk * kPlaneApply + u * 256 + threadIdx.x, y = i / p.W, x = i - y * p.W;
+      xv[u] = g[u] = old[u] = 0.f;
+      at[u] = y * p.out.sy + x * p.out.sx;
+      if (i < hw) {
+        xv[u] = ld_f(xb + (y * p.x.sy + x * p.x.sx));
+        if (MODE == 1) g[u] = ld_f(db + (y * p.dy.sy + x * p.dy.sx));
+        if (MODE == 1 && p.accumulate) old[u] = ld_f(ab + (y * p.add.sy + x * p.add.sx));
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (chunk * kPlaneApply + u * 256 + threadIdx.x < hw) st_f(ob + at[u], value(xv[u], g[u], old[u]));
   }
 }
 
@@ -414,7 +525,7 @@ static void launch_finish(const BnFin& f, int nsplit, const float* partial, cuda
 }
 // Both stages of the statistics of x (MODE 0) or of the backward sums (MODE 1) into what `f` names
 template <int MODE>
-static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, float* partial, cudaStream_t s) {
+static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, float* partial, cudaStream_t s, bool vec) {
   const bool cfast = x->sc == 1 && x->C > 1;
   int nsplit;
   if (vec_view_ok(x) && (MODE == 0 || (p.dy.sc == 1 && !((uintptr_t)p.dy.base & 15u) && !(p.dy.sn & 7) && !(p.dy.sy & 7) && !(p.dy.sx & 7)))) {
@@ -429,8 +540,11 @@ static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, fl
       dim3 grid((x->C + 31) / 32, nsplit), block(32, 8);
       AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_cfast<T, MODE>, grid, block, 0, s, p, partial)));
     } else {
+      if (MODE == 0) nsplit = std::max(1, std::min(nsplit, bn_max_splits(x->C) / 2));   // two rows per split
       dim3 grid(x->C, nsplit);
-      AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_xfast<T, MODE>, grid, 256, 0, s, p, partial)));
+      if (vec) launch(bn_reduce_xfast<float, MODE, true>, grid, 256, 0, s, p, partial);
+      else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_xfast<T, MODE, false>, grid, 256, 0, s, p, partial)));
+      if (MODE == 0) nsplit *= 2;
     }
   }
   count_launch();
@@ -919,13 +1033,18 @@ extern "C" size_t ad_bn_scratch_bytes(uint32_t C) { return (size_t)(bn_max_split
 
 // y = the normalised x with the statistics a.mean / a.invstd, or the backward pass over them
 template <int MODE>
-static int launch_apply(const BnApply& a, const ad_tensor4* x, bool vec, cudaStream_t s) {
+static int launch_apply(const BnApply& a, const ad_tensor4* x, bool vec, bool planes_vec, cudaStream_t s) {
   if (vec) {
     const int rc = MODE == 1 && a.accumulate ? launch_apply_vec<MODE, MODE == 1>(a, s) : launch_apply_vec<MODE, false>(a, s);
     if (rc != AD_OK) return rc;
   } else {
     const size_t total = (size_t)x->N * x->C * x->H * x->W;
-    AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply<T, MODE>, grid_for(total, 256, 16), 256, 0, s, a)));
+    const unsigned long long hw = (unsigned long long)x->H * x->W, chunks = planes_vec ? (hw + kPlaneApplyVec - 1) / kPlaneApplyVec : (hw + kPlaneApply - 1) / kPlaneApply;
+    if (!a.c_fastest && hw < (1ull << 31) && (unsigned long long)x->N * x->C * chunks < (1ull << 31)) {
+      const unsigned grid = (unsigned)(x->N * x->C * chunks);
+      if (planes_vec) launch(bn_apply_planes<float, MODE, true>, grid, 256, 0, s, a, (uint32_t)chunks);
+      else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply_planes<T, MODE, false>, grid, 256, 0, s, a, (uint32_t)chunks)));
+    } else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply<T, MODE>, grid_for(total, 256, 16), 256, 0, s, a)));
   }
   count_launch();
   return launch_status();
@@ -935,7 +1054,7 @@ extern "C" int ad_bn_partial_stats(const ad_tensor4* x, float* sums, void* scrat
   if (!x || !x->base || !sums || !scratch) return AD_ERR_BAD_ARG;
   if (scratch_bytes < ad_bn_scratch_bytes(x->C)) return AD_ERR_SCRATCH;
   BnRed p{bview(x), bview(x), x->N, x->C, x->H, x->W, 0, nullptr, nullptr, nullptr, nullptr};
-  return launch_reduce<0>(p, x, BnFin{2, x->C, 1.0, 0.f, nullptr, nullptr, nullptr, sums, nullptr, nullptr, 0}, (float*)scratch, as_stream(stream));
+  return launch_reduce<0>(p, x, BnFin{2, x->C, 1.0, 0.f, nullptr, nullptr, nullptr, sums, nullptr, nullptr, 0}, (float*)scratch, as_stream(stream), planes_vec_ok(x));
 }
 
 extern "C" int ad_bn_finalize_apply(const ad_tensor4* x, const ad_tensor4* y, const float* sums, double count,
@@ -947,7 +1066,7 @@ extern "C" int ad_bn_finalize_apply(const ad_tensor4* x, const ad_tensor4* y, co
   launch_finish(BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, 1, sums, s);
   BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, save_mean, save_invstd, nullptr, 1, count};
-  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), s);
+  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), planes_vec_ok(x) && planes_vec_ok(y), s);
 }
 
 extern "C" int ad_bn_fwd_train(const ad_tensor4* x, const ad_tensor4* y, const float* gamma, const float* beta,
@@ -961,11 +1080,11 @@ extern "C" int ad_bn_fwd_train(const ad_tensor4* x, const ad_tensor4* y, const f
   cudaStream_t s = as_stream(stream);
   BnRed p{bview(x), bview(x), x->N, x->C, x->H, x->W, 0, nullptr, nullptr, nullptr, nullptr};
   const double count = (double)x->N * x->H * x->W;
-  int st = launch_reduce<0>(p, x, BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, (float*)scratch, s);
+  int st = launch_reduce<0>(p, x, BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, (float*)scratch, s, planes_vec_ok(x));
   if (st != AD_OK) return st;
   BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, save_mean, save_invstd, nullptr, 1, count};
-  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), s);
+  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), planes_vec_ok(x) && planes_vec_ok(y), s);
 }
 
 // invstd[c] = 1 / sqrt(var[c] + eps), in double as the training path does
@@ -987,7 +1106,7 @@ extern "C" int ad_bn_fwd_inference(const ad_tensor4* x, const ad_tensor4* y, con
   count_launch();
   BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, mean, invstd_out, nullptr, 1, (double)x->N * x->H * x->W};
-  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), s);
+  return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), planes_vec_ok(x) && planes_vec_ok(y), s);
 }
 
 extern "C" int ad_bn_bwd_add(const ad_tensor4* x, const ad_tensor4* dy, const ad_tensor4* addend, const ad_tensor4* dx, const float* gamma,
@@ -1006,11 +1125,12 @@ extern "C" int ad_bn_bwd_add(const ad_tensor4* x, const ad_tensor4* dy, const ad
   float* partial = (float*)scratch;
   float* sums = partial + (size_t)bn_max_splits(x->C) * 2 * x->C;
   const double count = (double)x->N * x->H * x->W;
-  int st = launch_reduce<1>(p, x, BnFin{1, x->C, count, 0.f, nullptr, nullptr, nullptr, sums, dgamma, dbeta, accumulate_params}, partial, s);
+  int st = launch_reduce<1>(p, x, BnFin{1, x->C, count, 0.f, nullptr, nullptr, nullptr, sums, dgamma, dbeta, accumulate_params}, partial, s, planes_vec_ok(x) && planes_vec_ok(dy));
   if (st != AD_OK) return st;
   BnApply a{bview(x), bview(dy), bview(dx), bview(addend ? addend : dx), x->N, x->C, x->H, x->W, dx->sc == 1 && dx->C > 1, relu, addend != nullptr,
             gamma, beta, save_mean, save_invstd, sums, 1, count};
-  return launch_apply<1>(a, x, vec_view_ok(x) && vec_view_ok(dy) && vec_view_ok(dx) && (!addend || vec_view_ok(addend)), s);
+  return launch_apply<1>(a, x, vec_view_ok(x) && vec_view_ok(dy) && vec_view_ok(dx) && (!addend || vec_view_ok(addend)),
+                         planes_vec_ok(x) && planes_vec_ok(dy) && planes_vec_ok(dx) && (!addend || planes_vec_ok(addend)), s);
 }
 
 extern "C" int ad_bn_bwd(const ad_tensor4* x, const ad_tensor4* dy, const ad_tensor4* dx, const float* gamma,
