@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include <algorithm>
 
+#include "bias_grad.cuh"
 #include "overlap.h"
 #include "tc_common.cuh"
 
@@ -680,15 +681,16 @@ __device__ __forceinline__ float4 wgrad_lane_sum(const float* src, size_t part_s
 // KRSC filters, and 1x1 ones in either order (kcrs): 64 x 4 outputs x 4 lanes per block.  C is a multiple of 64.
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(size_t n, size_t part_stride, uint32_t splits,
                                                            const float* __restrict__ partial, float* dw, int accumulate,
-                                                           uint32_t taps, uint32_t C, int kcrs) {
+                                                           uint32_t taps, uint32_t C, int kcrs, BiasParts bias) {
   grid_dependency();
-  const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6;
-  const size_t i = ((size_t)blockIdx.x * 64 + tx) * 4;
+  if (bias_finish_blocks(bias, accumulate)) return;
+  const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6, block = blockIdx.x - bias.blocks;
+  const size_t i = ((size_t)block * 64 + tx) * 4;
   __shared__ float4 sh[4][64];
   if (i < n) sh[pl][tx] = wgrad_lane_sum(partial + i, part_stride, splits, pl);
   __syncthreads();
   // thread t finishes output t of the block's 256
-  const size_t j = (size_t)blockIdx.x * 256 + threadIdx.x;
+  const size_t j = (size_t)block * 256 + threadIdx.x;
   if (j >= n) return;
   const float* f = (const float*)sh + threadIdx.x;
   const float t = ((f[0] + f[256]) + f[512]) + f[768];
@@ -706,10 +708,11 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(size_t n, size_t part
 // segmentation net's 50 filter gradients: 1.77 -> 1.06 ms).
 constexpr uint32_t kWgRedPitch = 36;
 __global__ void wgrad_reduce_kcrs_kernel(size_t part_stride, uint32_t splits, const float* __restrict__ partial, float* dw,
-                                         int accumulate, uint32_t taps, uint32_t C) {
+                                         int accumulate, uint32_t taps, uint32_t C, BiasParts bias) {
   grid_dependency();
+  if (bias_finish_blocks(bias, accumulate)) return;
   extern __shared__ float wr[];   // [4][taps][kWgRedPitch]
-  const uint32_t ctiles = C / 32, k = blockIdx.x / ctiles, c0 = blockIdx.x % ctiles * 32, items = taps * 8;
+  const uint32_t block = blockIdx.x - bias.blocks, ctiles = C / 32, k = block / ctiles, c0 = block % ctiles * 32, items = taps * 8;
   for (uint32_t w = threadIdx.x; w < items * 4; w += blockDim.x) {
     const uint32_t pl = w / items, e = w - pl * items, tap = e >> 3, c4 = e & 7;
     *(float4*)(wr + (pl * taps + tap) * kWgRedPitch + c4 * 4) =
@@ -725,18 +728,6 @@ __global__ void wgrad_reduce_kcrs_kernel(size_t part_stride, uint32_t splits, co
     out[i] = accumulate ? out[i] + t : t;
   }
 }
-static void launch_wgrad_reduce(uint32_t K, uint32_t taps, uint32_t C, size_t part_stride, uint32_t splits, const float* partial,
-                                float* dw, int accumulate, int kcrs, cudaStream_t s) {
-  const size_t n = (size_t)K * taps * C, smem = (size_t)4 * taps * kWgRedPitch * 4;
-  if (kcrs && taps > 1 && smem <= 48 * 1024) {   // more taps than shared memory holds (over 85) take the form below
-    const uint32_t threads = std::min((taps * 32 + 31) / 32 * 32, 512u);
-    launch(wgrad_reduce_kcrs_kernel, K * (C / 32), threads, smem, s, part_stride, splits, partial, dw, accumulate, taps, C);
-  } else {
-    launch(wgrad_reduce_kernel, (unsigned)((n + 255) / 256), 256, 0, s, n, part_stride, splits, partial, dw, accumulate, taps, C, kcrs && taps > 1);
-  }
-  count_launch();
-}
-
 // Filter for the data gradient: wt[c][kh-1-r][kw-1-s][k] = w[k][r][s][c]  (bf16); rows of Kp >= K
 // entries, zero past K.
 __global__ void __launch_bounds__(256) filter_transpose_flip_kernel(uint32_t K, uint32_t Kp, uint32_t kh, uint32_t kw,
@@ -835,7 +826,7 @@ __global__ void __launch_bounds__(256) pad_channels_kernel(size_t pixels, uint32
 }
 
 // db[k] (+)= sum over pixels of dy[pixel][k] (dense NHWC bf16), in two fixed-order stages: a block sums its share of the
-// pixels into part[block][k], bias_grad_finish adds the blocks in order.  HBM-bound: dy is read once.
+// pixels into part[block][k], bias_finish_blocks adds the blocks in order.  HBM-bound: dy is read once.
 // K a multiple of 8: a thread owns 8 adjacent channels (16-byte loads, eight pixels in flight), 256 / (K / 8) pixel lanes
 // per block (K above 2048: channel groups over blockIdx.y).  32 x 512 x 512 pixels of 64 channels: 205 us
 // with four pixels in registers, 178 with the ring.
@@ -916,42 +907,42 @@ __global__ void __launch_bounds__(256) bias_grad_nhwc_kernel(size_t pixels, uint
     part[(size_t)split * K + k] = t;
   }
 }
-// a block per 32 channels: 8 lanes of blocks' rows, combined in order
-__global__ void __launch_bounds__(256) bias_grad_finish(uint32_t K, uint32_t nsplit, const float* __restrict__ part, float* db, int accumulate) {
-  grid_dependency();
-  __shared__ float red[8][33];
-  const uint32_t tx = threadIdx.x & 31, ty = threadIdx.x >> 5, k = blockIdx.x * 32 + tx;
-  float t = 0.f;
-  if (k < K) {
-#pragma unroll 8
-    for (uint32_t s = ty; s < nsplit; s += 8) t += part[(size_t)s * K + k];
-  }
-  red[ty][tx] = t;
-  __syncthreads();
-  if (ty == 0 && k < K) {
-#pragma unroll
-    for (int w = 1; w < 8; ++w) t += red[w][tx];
-    db[k] = accumulate ? db[k] + t : t;
-  }
-}
 // Blocks (= partial rows of K floats) of the first stage: four per SM, each thread with at least two batches of pixels.
-// conv_tc_scratch_bytes sets that much aside; the filter partials, already reduced, lie in the same memory.
+// Their sum is part of the reduction of the filter gradient's partials (BiasParts), which lie in front of them in scratch.
 static uint32_t bias_grad_blocks(size_t pixels, uint32_t K) {
   const bool vec = K % 8 == 0;
   const uint32_t gb = vec ? std::min(K / 8, 256u) : 32u, lanes = vec ? 256 / gb : 8, groups = vec ? (K / 8 + gb - 1) / gb : (K + 31) / 32;
   const size_t most = pixels / ((size_t)lanes * 8), want = std::max(1u, 4u * kNumSMs / groups);
   return (uint32_t)std::max<size_t>(1, std::min(most, want));
 }
-static void launch_bias_grad(size_t pixels, uint32_t K, const void* dy, float* db, int accumulate, float* part, cudaStream_t s) {
-  const uint32_t nsplit = bias_grad_blocks(pixels, K);
+size_t bias_grad_bytes(size_t pixels, uint32_t K) { return (size_t)bias_grad_blocks(pixels, K) * K * 4; }
+// The first stage, if there is a db; part: at least bias_grad_bytes (less: one block does with what there is)
+BiasParts bias_grad_parts(size_t pixels, uint32_t K, const void* dy, float* db, float* part, size_t part_bytes, cudaStream_t s) {
+  if (!db) return BiasParts{};
+  const uint32_t nsplit = (uint32_t)std::min<size_t>(bias_grad_blocks(pixels, K), part_bytes / ((size_t)K * 4));
   if (K % 8 == 0 && ((uintptr_t)dy & 15u) == 0) {
     const uint32_t gb = K / 8 < 256 ? K / 8 : 256;
     launch(bias_grad_vec_kernel, dim3(nsplit, (K / 8 + gb - 1) / gb), 256, 0, s, pixels, K, gb, (const __nv_bfloat16*)dy, part);
   } else {
     launch(bias_grad_nhwc_kernel, dim3(nsplit, (K + 31) / 32), dim3(32, 8), 0, s, pixels, K, (const __nv_bfloat16*)dy, part);
   }
-  launch(bias_grad_finish, (K + 31) / 32, 256, 0, s, K, nsplit, part, db, accumulate);
-  count_launch(2);
+  count_launch();
+  return BiasParts{part, nsplit, K, K, db, (K + 31) / 32};
+}
+
+struct BiasGrad { size_t pixels; const void* dy; float *db, *part; size_t part_bytes; };
+// The reduction over the splits, with that of the bias gradient's partials in blocks of its own
+static void launch_wgrad_reduce(uint32_t K, uint32_t taps, uint32_t C, size_t part_stride, uint32_t splits, const float* partial,
+                                float* dw, int accumulate, int kcrs, const BiasGrad& b, cudaStream_t s) {
+  const size_t n = (size_t)K * taps * C, smem = (size_t)4 * taps * kWgRedPitch * 4;
+  const BiasParts bias = bias_grad_parts(b.pixels, K, b.dy, b.db, b.part, b.part_bytes, s);
+  if (kcrs && taps > 1 && smem <= 48 * 1024) {   // more taps than shared memory holds (over 85) take the form below
+    const uint32_t threads = std::min((taps * 32 + 31) / 32 * 32, 512u);
+    launch(wgrad_reduce_kcrs_kernel, bias.blocks + K * (C / 32), threads, smem, s, part_stride, splits, partial, dw, accumulate, taps, C, bias);
+  } else {
+    launch(wgrad_reduce_kernel, bias.blocks + (uint32_t)((n + 255) / 256), 256, 0, s, n, part_stride, splits, partial, dw, accumulate, taps, C, kcrs && taps > 1, bias);
+  }
+  count_launch();
 }
 
 // ---------------------------------------------------------------- host side
@@ -1038,7 +1029,7 @@ size_t conv_tc_row_wgrad_scratch(uint32_t NI, uint32_t CI, uint32_t KO, uint32_t
                                  uint32_t dh, uint32_t dw, uint32_t OP, uint32_t OQ);
 int conv_tc_row_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CI, const void* dy, uint32_t KO,
                       uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, int offy, int offx,
-                      uint32_t OP, uint32_t OQ, float* dwt, int accumulate, int kcrs, void* partial, size_t partial_bytes,
+                      uint32_t OP, uint32_t OQ, float* dwt, float* db, int accumulate, int kcrs, void* partial, size_t partial_bytes,
                       int32_t* status, cudaStream_t s);
 
 // The launch of the general kernel: everything but the tensor maps and the channel tiles is in p (and cl, NC > 1).
@@ -1155,12 +1146,23 @@ static int launch_wgrad(const CUtensorMap& mdy, const CUtensorMap& mx, const WgP
 // tile but leaves room for two pipeline stages only: measured 15 % slower on the 512 -> 512 layers.)
 static int wgrad_bn(uint32_t C) { return C > 64 ? 128 : 64; }
 
-static uint32_t wgrad_splits(uint32_t sp_tiles, uint32_t outer) {
-  uint32_t want = (2 * kNumSMs + outer - 1) / outer;
-  if (want > sp_tiles) want = sp_tiles;
-  if (want > 64) want = 64;
-  if (want < 1) want = 1;
-  return want;
+// Splits of the pixel range: the count with the shortest time by rounds of the machine's CTAs (pairs) and by what the partial
+// gradients cost on their way out and back (a pixel tile of an item takes about 0.5 us, 2.5 MB).  Most often that is as
+// many as fill one round; a count that leaves the last round nearly empty costs most: 1024 -> 256 channels 1x1, 65,536 pixels, 19
+// splits (152 items, 74 pairs) 62 us, 9 splits 45; 512 -> 512 3x3 on 64 x 4 x 7 pixels 3 splits 44, one 34.
+static uint32_t wgrad_splits(uint32_t sp_tiles, uint32_t KO, uint32_t C, uint32_t taps) {
+  const uint32_t BN = (uint32_t)wgrad_bn(C), ktiles = (KO + 127) / 128;
+  const bool pair = BN == 128 && ktiles % 2 == 0;
+  const unsigned long long outer = (unsigned long long)taps * (pair ? ktiles / 2 : ktiles) * ((C + BN - 1) / BN), units = pair ? kNumSMs / 2 : kNumSMs;
+  const double part = (double)KO * taps * C * 8 / 2.5e6;
+  uint32_t best = 1;
+  double best_cost = 0;
+  for (uint32_t n = 1; n <= sp_tiles && n <= 64; ++n) {   // above 64 the reduction takes a third trip to the L2 (64 -> 256: 36 us, 74 splits 39)
+    const double cost = (double)((outer * n + units - 1) / units) * ((sp_tiles + n - 1) / n) + n * part;
+    if (n == 1 || cost < best_cost) { best = n; best_cost = cost; }
+    if (outer * n > 8 * units) break;
+  }
+  return best;
 }
 
 static size_t round_1k(size_t b) { return (b + 1023) / 1024 * 1024; }
@@ -1189,12 +1191,9 @@ size_t conv_tc_scratch_bytes(const ad_conv2d_args* a, int pass) {
     uint32_t TN, TH, TW;
     pick_tile3(a->N, g.P, g.Q, a->stride_h, a->stride_w, TN, TH, TW);
     const uint32_t sp = ((a->N + TN - 1) / TN) * ((g.P + TH - 1) / TH) * ((g.Q + TW - 1) / TW);
-    const uint32_t BN = (uint32_t)wgrad_bn(a->C);
-    const uint32_t outer = a->kh * a->kw * ((Kp + 127) / 128) * ((a->C + BN - 1) / BN);
-    size_t general = (size_t)wgrad_splits(sp, outer) * wcount * 4;
+    size_t general = (size_t)wgrad_splits(sp, Kp, a->C, a->kh * a->kw) * wcount * 4;
     size_t row = conv_tc_row_wgrad_scratch(a->N, a->C, a->K, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h, a->dil_w, g.P, g.Q);
-    size_t part = general > row ? general : row;
-    part = std::max(part, (size_t)bias_grad_blocks(pixels, a->K) * a->K * 4);
+    const size_t part = std::max(general + bias_grad_bytes(pixels, a->K), row);
     size_t b = 1024 + part;
     if (Kp != a->K) b += round_1k(pixels * Kp * 2);
     return b;
@@ -1366,9 +1365,8 @@ int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
   if (Kp == a->K && !getenv("ARRAYDIFF_B200_NO_ROW_KERNEL")) {
     // 64-channel layers: one CTA serves all taps from one fetch of x and dy (conv_tc_row.cu)
     st = conv_tc_row_wgrad(a->x, a->N, a->H, a->W, a->C, a->y, a->K, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h,
-                           a->dil_w, -(int)a->pad_h, -(int)a->pad_w, g.P, g.Q, (float*)a->dw, a->accumulate, a->dw_kcrs,
+                           a->dil_w, -(int)a->pad_h, -(int)a->pad_w, g.P, g.Q, (float*)a->dw, a->db, a->accumulate, a->dw_kcrs,
                            part_base, part_bytes, status, s);
-    if (st == AD_OK && a->db) launch_bias_grad((size_t)a->N * g.P * g.Q, a->K, a->y, a->db, a->accumulate, (float*)part_base, s);
     if (st != AD_ERR_UNSUPPORTED) {
       g_last_conv_kernel = kConvTcRow;
       return st;
@@ -1388,7 +1386,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
   p.ktiles = (Kp + 127) / 128;
   p.ctiles = (a->C + BN - 1) / BN;
   const uint32_t sp_tiles = p.tiles_b * p.tiles_y * p.tiles_x;
-  p.splits = wgrad_splits(sp_tiles, p.kh * p.kw * p.ktiles * p.ctiles);
+  p.splits = wgrad_splits(sp_tiles, Kp, a->C, p.kh * p.kw);
   p.status = status;
   p.partial = (float*)part_base;
   const size_t wcount_p = (size_t)Kp * a->kh * a->kw * a->C;
@@ -1415,8 +1413,9 @@ int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
   st = BN == 128 ? (p.ktiles % 2 == 0 ? launch_wgrad<128, true>(mdy, mx, p, s) : launch_wgrad<128, false>(mdy, mx, p, s))
                  : launch_wgrad<64, false>(mdy, mx, p, s);
   if (st != AD_OK) return st;
-  launch_wgrad_reduce(a->K, a->kh * a->kw, a->C, wcount_p, p.splits, p.partial, (float*)a->dw, a->accumulate, a->dw_kcrs, s);
-  if (a->db) launch_bias_grad((size_t)a->N * g.P * g.Q, a->K, a->y, a->db, a->accumulate, p.partial, s);
+  const size_t filter_bytes = (size_t)p.splits * wcount_p * 4;
+  launch_wgrad_reduce(a->K, a->kh * a->kw, a->C, wcount_p, p.splits, p.partial, (float*)a->dw, a->accumulate, a->dw_kcrs,
+                      BiasGrad{(size_t)a->N * g.P * g.Q, a->y, a->db, (float*)(part_base + filter_bytes), part_bytes - filter_bytes}, s);
   return launch_status();
 }
 

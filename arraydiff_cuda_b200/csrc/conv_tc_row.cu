@@ -14,6 +14,7 @@
 //
 // Same bounded-wait, abort-flag and tensor-memory discipline as conv_tc.cu; no multicast loads.
 #include "common.cuh"
+#include "bias_grad.cuh"
 #include "tc_common.cuh"
 
 #include <cstdlib>
@@ -28,6 +29,7 @@ struct RowCtl {
   unsigned long long full[4], empty[4], tfull[2], tempty[2], wbar, stg_full[2], stg_free[2];
   uint32_t tmem_base;
   volatile int abort_flag;
+  float db[4][64];     // rows filter gradient: the epilogue warps' sums of dy
 };
 
 struct RowFwdParams {
@@ -1053,12 +1055,16 @@ conv_tc_row_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gri
 //   D[(s, c)][(r, k)]: ceil(kw / 2) accumulators of 64 * kh columns.
 // A 3x3 needs 2 MMAs of N = 192 (math-bound, 96 cycles) per 16 pixels instead of 5 of N = 64, fetches one input row
 // instead of three, and walks oy over OP + (kh - 1)*dil rows (output-gradient rows outside [0, OP) are zero-filled by TMA).
+// The bias gradient comes along: the epilogue warps, idle until the end, add up the pixels of dy[oy], which every output row
+// is exactly once, from the stages (16 KB of the 80 that the MMAs read per tile).  As a kernel of its own it read all
+// of dy once more: 32 x 512 x 512 pixels 178 us of 2195 for the three passes of the layer.
 struct RowsWgParams {
   uint32_t NI, OP, OQ, KO;
   uint32_t kh, kw, dh, dw;
   int32_t offy, offx;
   uint32_t tiles_x, rows_ext, pw, stage_bytes, stages, naccs;
   float* partial;   // [grid][naccs][128][64 * kh]
+  float* db_part;   // [grid][64] or NULL: no bias gradient
   int32_t* status;
 };
 
@@ -1076,7 +1082,7 @@ conv_tc_rows_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gr
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < p.stages; ++s) {
       mbar_init(smem_u32(&ctl->full[s]), 1);
-      mbar_init(smem_u32(&ctl->empty[s]), 1);
+      mbar_init(smem_u32(&ctl->empty[s]), p.db_part ? 5 : 1);   // the MMAs and the four warps that read dy
     }
     mbar_init(smem_u32(&ctl->tfull[0]), 1);
     ctl->abort_flag = 0;
@@ -1154,6 +1160,49 @@ conv_tc_rows_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gr
     const uint32_t row = q * 32 + lane;
     float* out = p.partial + ((size_t)blockIdx.x * kAccs * 128 + row) * kN;
     const bool have = blockIdx.x < total_tiles;
+    if (p.db_part) {
+      // thread: 8 channels (16 bytes of a pixel's 128, swizzled by the pixel) of every 16th pixel; sums over 32 tiles restart
+      const uint32_t j = threadIdx.x & 7u, px0 = (threadIdx.x - 64u) >> 3;
+      float sum[8], run[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum[i] = run[i] = 0.f;
+      uint32_t stage = 0, phase = 0, it = 0;
+      for (uint32_t tile = blockIdx.x; tile < total_tiles && !*abortf; tile += gridDim.x) {
+        if (!__all_sync(0xffffffffu, mbar_wait_relaxed(smem_u32(&ctl->full[stage]), phase, abortf))) break;
+        const uint8_t* dy = smem + (size_t)stage * p.stage_bytes;
+        uint4 v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; ++i) {
+          const uint32_t px = px0 + 16u * i;
+          v[i] = *(const uint4*)(dy + px * 128u + ((j ^ (px & 7u)) << 4));
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&ctl->empty[stage]));
+#pragma unroll
+        for (uint32_t w = 0; w < 4; ++w) {
+          auto word = [&](uint32_t i) { return (&v[i].x)[w]; };
+          auto lo = [&](uint32_t i) { return __uint_as_float(word(i) << 16); };
+          auto hi = [&](uint32_t i) { return __uint_as_float(word(i) & 0xffff0000u); };
+          run[2 * w] += ((lo(0) + lo(1)) + (lo(2) + lo(3))) + ((lo(4) + lo(5)) + (lo(6) + lo(7)));
+          run[2 * w + 1] += ((hi(0) + hi(1)) + (hi(2) + hi(3))) + ((hi(4) + hi(5)) + (hi(6) + hi(7)));
+        }
+        if ((++it & 31u) == 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { sum[i] += run[i]; run[i] = 0.f; }
+        }
+        if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        sum[i] += run[i];
+        sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 8);
+        sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 16);
+        if (lane < 8) ctl->db[warp - 2][lane * 8 + i] = sum[i];
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");   // the four epilogue warps
+      const uint32_t k = threadIdx.x - 64u;
+      if (k < 64u) p.db_part[(size_t)blockIdx.x * 64 + k] = (ctl->db[0][k] + ctl->db[1][k]) + (ctl->db[2][k] + ctl->db[3][k]);
+    }
     if (!have) {
       for (uint32_t a = 0; a < kAccs; ++a)
         for (uint32_t c = 0; c < kN; c += 4) *(float4*)(out + (size_t)a * 128 * kN + c) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1192,10 +1241,11 @@ conv_tc_rows_wgrad_kernel(const __grid_constant__ CUtensorMap map_dy, const __gr
 // dw[k][r*kw + s][c] (+)= sum over CTAs of partial[cta][s / 2][(s % 2)*64 + c][r*64 + k], fixed order (as below).
 __global__ void __launch_bounds__(256) wgrad_rows_reduce_kernel(uint32_t nparts, uint32_t naccs, uint32_t KO, uint32_t kh,
                                                                 uint32_t kw, const float* __restrict__ partial, float* dw,
-                                                                int accumulate, int kcrs) {
+                                                                int accumulate, int kcrs, BiasParts bias) {
   grid_dependency();
+  if (bias_finish_blocks(bias, accumulate)) return;
   const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6;
-  const uint32_t cols4 = 16 * kh, item = blockIdx.x * 64 + tx, nitems = naccs * 128 * cols4;
+  const uint32_t cols4 = 16 * kh, item = (blockIdx.x - bias.blocks) * 64 + tx, nitems = naccs * 128 * cols4;
   float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
   if (item < nitems) {
     const size_t part_stride = (size_t)naccs * 128 * 64 * kh;
@@ -1235,10 +1285,11 @@ __global__ void __launch_bounds__(256) wgrad_rows_reduce_kernel(uint32_t nparts,
 // lane sums parts lane, lane+4, ... with 8 loads in flight, the lanes are combined in order.
 __global__ void __launch_bounds__(256) wgrad_row_reduce_kernel(uint32_t nparts, uint32_t naccs, uint32_t KO, uint32_t kh,
                                                                uint32_t kw, const float* __restrict__ partial, float* dw,
-                                                               int accumulate, int kcrs) {
+                                                               int accumulate, int kcrs, BiasParts bias) {
   grid_dependency();
+  if (bias_finish_blocks(bias, accumulate)) return;
   const uint32_t tx = threadIdx.x & 63, pl = threadIdx.x >> 6;
-  const uint32_t item = blockIdx.x * 64 + tx, nitems = naccs * 128 * 16;
+  const uint32_t item = (blockIdx.x - bias.blocks) * 64 + tx, nitems = naccs * 128 * 16;
   float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
   if (item < nitems) {
     const size_t part_stride = (size_t)naccs * 128 * 64;
@@ -1295,14 +1346,14 @@ static uint32_t rows_wgrad_grid(uint32_t NI, uint32_t OP, uint32_t OQ, uint32_t 
 size_t conv_tc_row_wgrad_scratch(uint32_t NI, uint32_t CI, uint32_t KO, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw,
                                  uint32_t dh, uint32_t dw, uint32_t OP, uint32_t OQ) {
   if (!row_wgrad_ok(CI, KO, kh, kw, sh, sw, dh, dw, OQ)) return 0;
-  const size_t pairs = (size_t)row_wgrad_grid(NI, OP, OQ) * ((kh * kw + 1) / 2) * 128 * 64 * 4;
-  const size_t rows = kh == 3 && kw == 3 ? (size_t)rows_wgrad_grid(NI, OP, OQ, kh, dh) * ((kw + 1) / 2) * 128 * 64 * kh * 4 : 0;
+  const size_t pairs = (size_t)row_wgrad_grid(NI, OP, OQ) * ((kh * kw + 1) / 2) * 128 * 64 * 4 + bias_grad_bytes((size_t)NI * OP * OQ, KO);
+  const size_t rows = kh == 3 && kw == 3 ? (size_t)rows_wgrad_grid(NI, OP, OQ, kh, dh) * (((kw + 1) / 2) * 128 * 64 * kh + 64) * 4 : 0;   // + bias
   return pairs > rows ? pairs : rows;
 }
 
 static int conv_tc_rows_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CI, const void* dy, uint32_t KO,
                               uint32_t kh, uint32_t kw, uint32_t dh, uint32_t dw, int offy, int offx, uint32_t OP, uint32_t OQ,
-                              float* dwt, int accumulate, int kcrs, void* partial, size_t partial_bytes, int32_t* status,
+                              float* dwt, float* db, int accumulate, int kcrs, void* partial, size_t partial_bytes, int32_t* status,
                               cudaStream_t s) {
   RowsWgParams p{};
   p.NI = NI; p.OP = OP; p.OQ = OQ; p.KO = KO;
@@ -1318,8 +1369,9 @@ static int conv_tc_rows_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t 
   if (stages > 4) stages = 4;
   p.stages = (uint32_t)stages;
   const uint32_t grid = rows_wgrad_grid(NI, OP, OQ, kh, dh);
-  if (partial_bytes < (size_t)grid * p.naccs * 128 * 64 * kh * 4) return AD_ERR_SCRATCH;
+  if (partial_bytes < (size_t)grid * (p.naccs * 128 * 64 * kh + 64) * 4) return AD_ERR_SCRATCH;
   p.partial = (float*)partial;
+  if (db) p.db_part = p.partial + (size_t)grid * p.naccs * 128 * 64 * kh;
   p.status = status;
   CUtensorMap mdy, mx;
   {
@@ -1345,18 +1397,19 @@ static int conv_tc_rows_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t 
   }
   launch(conv_tc_rows_wgrad_kernel<3, 3>, grid, kRowThreads, smem, s, mdy, mx, p);
   count_launch();
-  launch(wgrad_rows_reduce_kernel, (p.naccs * 128 * 16 * kh + 63) / 64, 256, 0, s, grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs);
+  const BiasParts bias{p.db_part, grid, 64, KO, db, db ? (KO + 31) / 32 : 0};
+  launch(wgrad_rows_reduce_kernel, bias.blocks + (p.naccs * 128 * 16 * kh + 63) / 64, 256, 0, s, grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs, bias);
   count_launch();
   return launch_status();
 }
 
 int conv_tc_row_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CI, const void* dy, uint32_t KO,
                       uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, int offy, int offx,
-                      uint32_t OP, uint32_t OQ, float* dwt, int accumulate, int kcrs, void* partial, size_t partial_bytes,
+                      uint32_t OP, uint32_t OQ, float* dwt, float* db, int accumulate, int kcrs, void* partial, size_t partial_bytes,
                       int32_t* status, cudaStream_t s) {
   if (!row_wgrad_ok(CI, KO, kh, kw, sh, sw, dh, dw, OQ)) return AD_ERR_UNSUPPORTED;
   if (rows_wgrad_ok(kh, kw)) {
-    const int st = conv_tc_rows_wgrad(x, NI, IH, IW, CI, dy, KO, kh, kw, dh, dw, offy, offx, OP, OQ, dwt, accumulate, kcrs, partial,
+    const int st = conv_tc_rows_wgrad(x, NI, IH, IW, CI, dy, KO, kh, kw, dh, dw, offy, offx, OP, OQ, dwt, db, accumulate, kcrs, partial,
                                       partial_bytes, status, s);
     if (st != AD_ERR_UNSUPPORTED) return st;
   }
@@ -1373,7 +1426,8 @@ int conv_tc_row_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t IW, uint
   if (stages > 4) stages = 4;
   p.stages = (uint32_t)stages;
   const uint32_t grid = row_wgrad_grid(NI, OP, OQ);
-  if (partial_bytes < (size_t)grid * p.naccs * 128 * 64 * 4) return AD_ERR_SCRATCH;
+  const size_t filter = (size_t)grid * p.naccs * 128 * 64;
+  if (partial_bytes < filter * 4) return AD_ERR_SCRATCH;
   p.partial = (float*)partial;
   p.status = status;
   CUtensorMap mdy, mx;
@@ -1404,7 +1458,8 @@ int conv_tc_row_wgrad(const void* x, uint32_t NI, uint32_t IH, uint32_t IW, uint
   launch(kern, grid, kRowThreads, smem, s, mdy, mx, p);
   count_launch();
   const size_t wcount = (size_t)KO * kh * kw * 64;
-  launch(wgrad_row_reduce_kernel, (p.naccs * 128 * 16 + 63) / 64, 256, 0, s, grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs);
+  const BiasParts bias = bias_grad_parts((size_t)NI * OP * OQ, KO, dy, db, p.partial + filter, partial_bytes - filter * 4, s);
+  launch(wgrad_row_reduce_kernel, bias.blocks + (p.naccs * 128 * 16 + 63) / 64, 256, 0, s, grid, p.naccs, KO, kh, kw, p.partial, dwt, accumulate, kcrs, bias);
   count_launch();
   return launch_status();
 }

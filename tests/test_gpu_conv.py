@@ -419,3 +419,34 @@ def test_conv_tc_filter_gradient_forms_agree(case, kcrs, accumulate, monkeypatch
     monkeypatch.delenv("ARRAYDIFF_B200_WGRAD_PAIRS", raising=False)
     assert H.max_rel(got["rows"], dw_w) < 1e-4 and H.max_rel(got["pairs"], dw_w) < 1e-4
     assert H.max_rel(got["rows"], got["pairs"]) < 1e-5
+
+
+@pytest.mark.parametrize("case", [(1, 512, 9, 10, 512, 3, 1), (1, 1024, 6, 7, 2048, 1, 1), (2, 64, 40, 90, 256, 1, 1), (3, 128, 20, 17, 384, 3, 2), (2, 64, 12, 400, 64, 3, 1)])
+@pytest.mark.parametrize("kcrs", [0, 1])
+def test_filter_and_bias_gradient_splits(case, kcrs):
+    """One split with nearly as many items as CTA pairs, more items than pairs, the largest split count, a few; the bias gradient from
+    the stages of the 64-channel kernel and from its own kernel; its blocks behind those of every reduction."""
+    import torch
+    N, Cc, Hh, W, K, k, s = case
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.rand((N, Cc, Hh, W), generator=g, device="cuda").sub_(0.5).bfloat16()
+    P, Q = (Hh - k) // s + 1, (W - k) // s + 1
+    dy = torch.rand((N, K, P, Q), generator=g, device="cuda").bfloat16()
+    want = torch.nn.grad.conv2d_weight(x.double(), (K, Cc, k, k), dy.double(), stride=s)
+    db_w = dy.double().sum((0, 2, 3))
+    L = abi.lib()
+    a = conv_args(abi.AD_BF16, abi.AD_NHWC, (N, Cc, Hh, W), K, k, s, 1, 0)
+    xd, dyd = x.permute(0, 2, 3, 1).contiguous(), dy.permute(0, 2, 3, 1).contiguous()
+    dw = torch.ones((K, Cc, k, k) if kcrs else (K, k, k, Cc), device="cuda")
+    db = torch.ones(K, device="cuda")
+    scratch = torch.full((L.ad_conv2d_scratch_bytes(C.byref(a), 2),), 255, dtype=torch.uint8, device="cuda")
+    scratch[:16] = 0
+    a.x, a.y, a.dw, a.db, a.dw_kcrs, a.accumulate = xd.data_ptr(), dyd.data_ptr(), dw.data_ptr(), db.data_ptr(), kcrs, 1
+    a.scratch, a.scratch_bytes = scratch.data_ptr(), scratch.numel()
+    abi.check(L.ad_conv2d_wgrad(C.byref(a), H.stream()))
+    H.sync()
+    assert scratch[:4].view(torch.int32).item() == 0
+    got = dw.double() - 1 if kcrs else dw.double().permute(0, 3, 1, 2) - 1
+    # exact products, fp32 sums; 1 + v rounds to 2^-24 of its size
+    assert (got - want).abs().max() < 1e-5 * want.abs().max() + 1e-6
+    assert (db.double() - 1 - db_w).abs().max() < 1e-6 * db_w.abs().max() + 1e-6
