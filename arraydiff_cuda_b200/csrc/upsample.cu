@@ -6,6 +6,8 @@
 // and rows [y_row0, y_row0 + y.H) of the upsampled output; source rows are computed in global
 // coordinates, so a strip with one halo row on each inner edge gives exactly the rows of the
 // unpartitioned result.  HBM-bound: the output is scale^2 times the input.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace adk {
@@ -119,6 +121,7 @@ struct UpRowP {
   uint32_t row_len;       // elements of a high-resolution row
   int vec;                // high-resolution rows start on the boundaries of the vectors
   uint32_t period;        // forward: pairs of outputs per low-resolution column (0: the general form)
+  uint32_t cell0, cells;  // forward by cells: the first row of cells (between two source rows) that the strip meets, their number
 };
 constexpr uint32_t kUpThreads = 256, kUpFloats = 5120;    // 20 KB of rows per block where that holds three columns: 8 blocks per SM
 constexpr uint32_t kUpFloatsMax = 12000;
@@ -164,44 +167,6 @@ __global__ void __launch_bounds__(kUpThreads) upsample_fwd_rows(UpRowP p) {
     if (hi == u.XW)
       for (uint32_t i = threadIdx.x; i < p.Ci; i += kUpThreads) L[r * pitch + cols + i] = 0.f;
   }
-  if (p.period) {
-    // Scale a power of two: the pairs of one source column's outputs, scale * Ci / 2 of them, recur from column to column with
-    // the same channels and exactly the same weights.  A thread stays with its pair of them and steps over columns, so an
-    // output costs two reads and two FMAs and little else; with a table of columns and weights (below) the kernel was
-    // bound by its instructions: 2 x 19 x 128 x 256 x 8 bf16 99 -> 58 us.
-    __syncthreads();
-    const uint32_t m = kUpThreads / p.period, k0 = threadIdx.x / p.period, e = threadIdx.x % p.period * 2;
-    if (k0 >= m) return;
-    const uint32_t ph0 = e / p.Ci, c0 = e - ph0 * p.Ci, ph1 = (e + 1) / p.Ci, c1 = e + 1 - ph1 * p.Ci;
-    const int d0 = 2 * ph0 < u.scale ? -1 : 0, d1 = 2 * ph1 < u.scale ? -1 : 0;
-    const float f0 = ((float)ph0 + 0.5f) * inv - 0.5f - (float)d0, f1 = ((float)ph1 + 0.5f) * inv - 0.5f - (float)d1;
-    const float g0 = 1.f - f0, g1 = 1.f - f1;
-    const uint32_t Ci = p.Ci, hop = m * Ci, ohop = hop * u.scale;
-    for (uint32_t r = 0; r < nr; ++r) {
-      const uint32_t oy = (row0 + r) % u.YH, plane = (row0 + r) / u.YH;
-      T* o = (T*)u.y.base + plane_off(u.y, plane, per_n) + (long long)oy * u.y.sy + (size_t)(xa + k0) * u.scale * Ci + e;
-      const float *a0 = L + r * pitch + (int)(xa + k0 - lo + d0) * (int)Ci + (int)c0, *a1 = L + r * pitch + (int)(xa + k0 - lo + d1) * (int)Ci + (int)c1;
-      uint32_t x = xa + k0;
-      auto edge = [&] {   // left of the first or right of the last column: that column's value, weight 0 on its neighbour
-        const int x0 = (int)x + d0, x1 = (int)x + d1, last = (int)u.XW - 1;
-        const float h0 = x0 < 0 || x0 >= last ? 0.f : f0, h1 = x1 < 0 || x1 >= last ? 0.f : f1;
-        const float *b0 = x0 < 0 ? a0 + Ci : a0, *b1 = x1 < 0 ? a1 + Ci : a1;
-        st_f(o, (1.f - h0) * b0[0] + h0 * b0[Ci]);
-        st_f(o + 1, (1.f - h1) * b1[0] + h1 * b1[Ci]);
-      };
-      auto next = [&] { x += m; a0 += hop; a1 += hop; o += ohop; };
-      if (x == 0 && x < xb) { edge(); next(); }
-      const uint32_t xe = xb == u.XW ? xb - 1 : xb;
-      if (p.vec) {
-#pragma unroll 4
-        for (; x < xe; next()) st_pair<T>(o, g0 * a0[0] + f0 * a0[Ci], g1 * a1[0] + f1 * a1[Ci]);
-      } else {
-        for (; x < xe; next()) { st_f(o, g0 * a0[0] + f0 * a0[Ci]); st_f(o + 1, g1 * a1[0] + f1 * a1[Ci]); }
-      }
-      if (x < xb) edge();
-    }
-    return;
-  }
   int2* tab = (int2*)(L + (((size_t)p.rb * pitch + 1) & ~(size_t)1));   // per output column: where its left source column lies, weight of the right one
   const uint32_t oxa = xa * u.scale, oxb = xb * u.scale;
   for (uint32_t i = threadIdx.x; i < oxb - oxa; i += kUpThreads) {
@@ -235,6 +200,98 @@ __global__ void __launch_bounds__(kUpThreads) upsample_fwd_rows(UpRowP p) {
       if (c >= p.Ci) { c -= p.Ci; ++ox; }
     }
   }
+}
+
+// Forward, scale a power of two (S, 0: at run time): the output rows between two neighbouring source rows, scale of them, are
+// blends of the same two blended rows, and the pairs of one source column's outputs, scale * Ci / 2 of them, recur from column
+// to column with the same channels and exactly the same weights.  A block takes such a cell of rows and some columns, a thread
+// stays with its pair and steps over columns: 8 reads of shared memory and 8 FMAs for the two blends, then two FMAs, a
+// conversion and a store per pair and row.  Bound by instructions before (a table of columns and weights, a row per block: 99
+// us and 92 M; pairs with a row per block 55 us and 49 M), by the stores now: 2 x 19 x 128 x 256 x 8 bf16
+// 32 us (25 at the copy rate), 2 x 19 x 64 x 128 x 8 fp32, whose planes took the table, 60 -> 16.
+template <typename T, int S>
+__global__ void __launch_bounds__(kUpThreads) upsample_fwd_cells(UpRowP p) {
+  grid_dependency();
+  extern __shared__ __align__(16) float L[];   // [2 source rows][XC + 2 columns, clamped to the image][Ci], weights of the cell's rows
+  const UpP& u = p.u;
+  const int s = S ? S : (int)u.scale;
+  const float inv = 1.0f / (float)s;
+  const uint32_t chunk = blockIdx.x % p.chunks, at = blockIdx.x / p.chunks, plane = at / p.cells, cell = p.cell0 + at % p.cells;
+  const uint32_t xa = chunk * p.XC, xb = xa + p.XC < u.XW ? xa + p.XC : u.XW;
+  const uint32_t lo = xa > 0 ? xa - 1 : 0, hi = xb < u.XW ? xb + 1 : u.XW, cols = (hi - lo) * p.Ci, pitch = (p.XC + 2) * p.Ci, Ci = p.Ci;
+  // rows ra .. rb - 1 of the cell's s lie in this strip
+  const int oy0 = (int)cell * s - s / 2, first = (int)u.y_row0, last_y = (int)(u.y_row0 + u.YH);
+  const int ra = oy0 < first ? first - oy0 : 0, rb = oy0 + s > last_y ? last_y - oy0 : s;
+  int y0, y1;
+  float fy;
+  bilin_src((uint32_t)(oy0 + ra), inv, u.in_rows_total, y0, y1, fy);   // the same two rows for the whole cell
+  const uint32_t per_n = u.C / Ci;
+  const T* X = (const T*)u.x.base + plane_off(u.x, plane, per_n) + (long long)lo * Ci;
+  const T *X0 = X + (y0 - u.x_row0) * u.x.sy, *X1 = X + (y1 - u.x_row0) * u.x.sy;
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < cols; i += kUpThreads) { L[i] = ld_f(X0 + i); L[pitch + i] = ld_f(X1 + i); }
+  if (hi == u.XW)   // a column of zeros past the last: the right edge blends it with weight 0 (an infinity there, times 0, would be NaN)
+    for (uint32_t i = threadIdx.x; i < Ci; i += kUpThreads) L[cols + i] = L[pitch + cols + i] = 0.f;
+  float* const W = L + 2 * pitch;
+  if ((int)threadIdx.x >= ra && (int)threadIdx.x < rb) {
+    bilin_src((uint32_t)(oy0 + (int)threadIdx.x), inv, u.in_rows_total, y0, y1, fy);
+    W[threadIdx.x] = fy;
+  }
+  __syncthreads();
+  const uint32_t m = kUpThreads / p.period, k0 = threadIdx.x / p.period, e = threadIdx.x % p.period * 2;
+  if (k0 >= m) return;
+  const uint32_t ph0 = e / Ci, c0 = e - ph0 * Ci, ph1 = (e + 1) / Ci, c1 = e + 1 - ph1 * Ci;
+  const int d0 = 2 * (int)ph0 < s ? -1 : 0, d1 = 2 * (int)ph1 < s ? -1 : 0;
+  const float f0 = ((float)ph0 + 0.5f) * inv - 0.5f - (float)d0, f1 = ((float)ph1 + 0.5f) * inv - 0.5f - (float)d1;
+  const float g0 = 1.f - f0, g1 = 1.f - f1;
+  const uint32_t hop = m * Ci, ohop = hop * (uint32_t)s;
+  const long long sy = u.y.sy;
+  T* o = (T*)u.y.base + plane_off(u.y, plane, per_n) + (long long)(oy0 - first) * sy + (long long)(xa + k0) * s * Ci + e;
+  const float *a0 = L + (int)(xa + k0 - lo + d0) * (int)Ci + (int)c0, *a1 = L + (int)(xa + k0 - lo + d1) * (int)Ci + (int)c1;
+  uint32_t x = xa + k0;
+  auto edge = [&] {   // left of the first or right of the last column: that column's value, weight 0 on its neighbour
+    const int x0 = (int)x + d0, x1 = (int)x + d1, last = (int)u.XW - 1;
+    const float h0 = x0 < 0 || x0 >= last ? 0.f : f0, h1 = x1 < 0 || x1 >= last ? 0.f : f1;
+    const float *b0 = x0 < 0 ? a0 + Ci : a0, *b1 = x1 < 0 ? a1 + Ci : a1;
+    const float t0 = (1.f - h0) * b0[0] + h0 * b0[Ci], t1 = (1.f - h1) * b1[0] + h1 * b1[Ci];
+    const float v0 = (1.f - h0) * b0[pitch] + h0 * b0[pitch + Ci], v1 = (1.f - h1) * b1[pitch] + h1 * b1[pitch + Ci];
+    for (int r = ra; r < rb; ++r) {
+      const float w = W[r];
+      st_f(o + r * sy, (1.f - w) * t0 + w * v0);
+      st_f(o + r * sy + 1, (1.f - w) * t1 + w * v1);
+    }
+  };
+  auto next = [&] { x += m; a0 += hop; a1 += hop; o += ohop; };
+  if (x == 0 && x < xb) { edge(); next(); }
+  const uint32_t xe = xb == u.XW ? xb - 1 : xb;
+  auto blends = [&](float& t0, float& t1, float& v0, float& v1) {
+    t0 = g0 * a0[0] + f0 * a0[Ci]; t1 = g1 * a1[0] + f1 * a1[Ci];
+    v0 = g0 * a0[pitch] + f0 * a0[pitch + Ci]; v1 = g1 * a1[pitch] + f1 * a1[pitch + Ci];
+  };
+  if (S && p.vec && ra == 0 && rb == s) {
+    float w[S ? S : 1], q[S ? S : 1];
+#pragma unroll
+    for (int r = 0; r < S; ++r) { w[r] = W[r]; q[r] = 1.f - w[r]; }
+#pragma unroll 2
+    for (; x < xe; next()) {
+      float t0, t1, v0, v1;
+      blends(t0, t1, v0, v1);
+      T* or_ = o;
+#pragma unroll
+      for (int r = 0; r < S; ++r, or_ += sy) st_pair<T>(or_, q[r] * t0 + w[r] * v0, q[r] * t1 + w[r] * v1);
+    }
+  } else {
+    for (; x < xe; next()) {
+      float t0, t1, v0, v1;
+      blends(t0, t1, v0, v1);
+      for (int r = ra; r < rb; ++r) {
+        const float w = W[r], a = (1.f - w) * t0 + w * v0, b = (1.f - w) * t1 + w * v1;
+        if (p.vec) st_pair<T>(o + r * sy, a, b);
+        else { st_f(o + r * sy, a); st_f(o + r * sy + 1, b); }
+      }
+    }
+  }
+  if (x < xb) edge();
 }
 
 template <typename T>
@@ -365,9 +422,24 @@ static bool up_rows(const ad_tensor4* lo, const ad_tensor4* hi, bool bwd, UpRowP
     if (r.rb < 1) r.rb = 1;
     while (r.tpr > 8 && r.tpr * 2 >= r.row_len && kUpThreads / r.tpr < r.rb) r.tpr >>= 1;
   }
-  // an even, power-of-two scale whose pairs fit the block (Ci <= 64 at scale 8, <= 256 at 2), rows long enough to keep the
-  // block busy one at a time (short ones share it: the general form)
-  r.period = !bwd && r.rb == 1 && u.scale % 2 == 0 && (u.scale & (u.scale - 1)) == 0 && r.Ci * u.scale / 2 <= kUpThreads ? r.Ci * u.scale / 2 : 0;
+  // an even, power-of-two scale whose pairs fit the block (Ci <= 64 at scale 8, <= 256 at 2), 16 outputs per thread in a cell of
+  // one row (shorter rows share a block in the general form)
+  r.period = !bwd && u.scale % 2 == 0 && (u.scale & (u.scale - 1)) == 0 && r.Ci * u.scale / 2 <= kUpThreads &&
+                     (unsigned long long)r.row_len * u.scale >= 16 * kUpThreads ? r.Ci * u.scale / 2 : 0;
+  if (r.period) {
+    // two source rows in shared memory; blocks of so few columns that the machine has six per SM
+    r.cell0 = (u.y_row0 + u.scale / 2) / u.scale;
+    r.cells = (u.y_row0 + u.YH - 1 + u.scale / 2) / u.scale - r.cell0 + 1;
+    const uint32_t most = std::max(1u, (kUpFloats / (2 * r.Ci)) - 2), lanes = kUpThreads / r.period;
+    const unsigned long long rows = (unsigned long long)r.planes * r.cells;
+    const uint32_t want = (uint32_t)std::max<unsigned long long>(1, (unsigned long long)u.XW * rows / (6 * kNumSMs));
+    r.XC = std::min(std::min(most, u.XW), std::max(want, std::min(4 * lanes, u.XW)));
+    r.chunks = (u.XW + r.XC - 1) / r.XC;
+    r.XC = (u.XW + r.chunks - 1) / r.chunks;
+    r.chunks = (u.XW + r.XC - 1) / r.XC;
+    r.smem = (2 * (r.XC + 2) * r.Ci + u.scale) * 4;
+    return u.scale <= kUpThreads && r.smem <= 49152 && rows * r.chunks < (1ull << 31);
+  }
   r.wtab = (r.XC + 2) * u.scale * r.Ci + 16;
   r.smem = bwd ? ((r.XC + 2) * u.scale * r.Ci + 16 + 3 * u.scale + 2) * 4 : ((r.rb * (r.XC + 2) * r.Ci + 2) + (r.XC + 2) * 2 * u.scale) * 4;
   return r.smem <= 49152 && (unsigned long long)r.planes * (bwd ? u.XH : u.YH) * r.chunks < (1ull << 31);
@@ -415,8 +487,10 @@ extern "C" int ad_upsample_bilinear_fwd(const ad_tensor4* x, const ad_tensor4* y
   UpRowP r{};
   r.u = p;
   if (up_rows(x, y, false, r)) {
-    const unsigned grid = (unsigned)((((size_t)r.planes * p.YH + r.rb - 1) / r.rb) * r.chunks);
-    AD_DISPATCH_DTYPE(x->dtype, (launch(upsample_fwd_rows<T>, grid, kUpThreads, r.smem, as_stream(stream), r)));
+    const unsigned grid = r.period ? (unsigned)((size_t)r.planes * r.cells * r.chunks) : (unsigned)((((size_t)r.planes * p.YH + r.rb - 1) / r.rb) * r.chunks);
+    const auto go = [&](auto kernel) { launch(kernel, grid, kUpThreads, r.smem, as_stream(stream), r); };
+    AD_DISPATCH_DTYPE(x->dtype, (!r.period ? go(upsample_fwd_rows<T>) : scale == 2 ? go(upsample_fwd_cells<T, 2>) : scale == 4 ? go(upsample_fwd_cells<T, 4>)
+                                                                      : scale == 8 ? go(upsample_fwd_cells<T, 8>) : go(upsample_fwd_cells<T, 0>)));
   } else
     AD_DISPATCH_DTYPE(x->dtype, (launch(upsample_fwd_kernel<T>, grid_for(total, 256, 16), 256, 0, as_stream(stream), p)));
   count_launch();

@@ -52,6 +52,40 @@ def test_upsample_rows(dtype, shape, scale):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
+@pytest.mark.parametrize("Cc,W,scale", [(19, 40, 8), (3, 300, 4), (1, 1100, 2), (31, 70, 4), (2, 33, 16), (64, 18, 8), (5, 300, 2)])
+def test_upsample_cells_of_strips(dtype, layout, Cc, W, scale):
+    """Rows between two source rows as one block: cells cut by the strips, rows that start on odd elements, odd channel counts, one
+    thread group per block (64 channels at scale 8); every element of the strip and none beside it."""
+    import torch
+    N, Hh = 2, 5
+    x = _q(H.normal(1, (N, Cc, Hh, W)), dtype)
+    want = orc.upsample_bilinear_fwd(x, scale)
+    YW = W * scale
+    nchw = layout == abi.AD_NCHW
+    tx = H.dev(x).to(torch.float32 if dtype == "f32" else torch.bfloat16)
+    tx = tx if nchw else tx.permute(0, 2, 3, 1).contiguous()
+    es = abi.AD_F32 if dtype == "f32" else abi.AD_BF16
+    for y0, rows, odd in [(0, Hh * scale, 0), (0, scale + 1, 1), (scale // 2 + 1, 2 * scale, 0), ((Hh - 1) * scale + 1, scale - 1, 1)]:
+        pitch = YW * (1 if nchw else Cc) + odd
+        buf = torch.full((N, Cc if nchw else 1, rows, pitch), 7.0, dtype=tx.dtype, device="cuda")
+        if nchw:
+            vx = abi.Tensor4(tx.data_ptr(), es, N, Cc, Hh, W, Cc * Hh * W, Hh * W, W, 1)
+            vy = abi.Tensor4(buf.data_ptr(), es, N, Cc, rows, YW, Cc * rows * pitch, rows * pitch, pitch, 1)
+        else:
+            vx = abi.Tensor4(tx.data_ptr(), es, N, Cc, Hh, W, Hh * W * Cc, 1, W * Cc, Cc)
+            vy = abi.Tensor4(buf.data_ptr(), es, N, Cc, rows, YW, rows * pitch, 1, pitch, Cc)
+        abi.check(abi.lib().ad_upsample_bilinear_fwd(C.byref(vx), C.byref(vy), scale, 0, Hh, y0, H.stream()))
+        H.sync()
+        got = H.host(buf)
+        assert np.all(got[..., pitch - odd:] == 7.0)
+        got = got[..., :pitch - odd]
+        got = got if nchw else np.transpose(got.reshape(N, rows, YW, Cc), (0, 3, 1, 2))
+        # two blends of two values: a rounding of each, and bf16's own
+        assert H.max_rel(got, want[:, :, y0:y0 + rows]) < (1e-6 if dtype == "f32" else 8e-3)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("shape,scale", [((1, 3, 6, 40), 8), ((2, 3, 5, 90), 3), ((1, 19, 5, 33), 2), ((1, 1, 4, 700), 5), ((1, 2, 5, 9), 2)])
 @pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
 def test_upsample_rows_of_infinities(dtype, shape, scale, bad):
