@@ -1,6 +1,8 @@
 // Packed fp32 array arithmetic, the fused SGD update, and strided ReLU / add / convert.
 // All HBM-bound: one read of each input and one write of each output, 16-byte vectors
 // where the pointers allow, grid-stride loops sized from the SM count.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace adk {
@@ -197,6 +199,49 @@ static bool ew_vec_ok(const ad_tensor4* t) {
          !(t->sy & 7) && !(t->sx & 7);
 }
 
+// fp32 planes -> bf16 pixels of C <= 4 channels (a host image on its way into a tensor-core net): four pixels per thread, 16-byte
+// loads from each plane and C 8-byte stores where rows are aligned (VEC).  Element by element, each 2-byte store and 4-byte
+// load on its own with three divisions, 2 x 3 x 1024 x 2048 took 67 us (12 us of memory).
+template <int C, bool VEC>
+__global__ void __launch_bounds__(256) planes_to_pixels_kernel(Dims d, View a, View yv) {
+  grid_dependency();
+  const uint32_t quads = (d.W + 3) / 4, total = d.N * d.H * quads;
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    const uint32_t q = i % quads, r = i / quads, y = r % d.H, n = r / d.H, x = q * 4;
+    const float* src = (const float*)a.base + n * a.sn + y * a.sy + x;
+    __nv_bfloat16* dst = (__nv_bfloat16*)yv.base + n * yv.sn + y * yv.sy + (long long)x * C;
+    float v[C][4];
+    if (VEC) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) *(float4*)v[c] = *(const float4*)(src + c * a.sc);
+      uint2 w[C];
+      __nv_bfloat162* h = (__nv_bfloat162*)w;
+#pragma unroll
+      for (int k = 0; k < 2 * C; ++k) h[k] = __floats2bfloat162_rn(v[2 * k % C][2 * k / C], v[(2 * k + 1) % C][(2 * k + 1) / C]);
+#pragma unroll
+      for (int k = 0; k < C; ++k) ((uint2*)dst)[k] = w[k];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (x + j < d.W)
+#pragma unroll
+          for (int c = 0; c < C; ++c) v[c][j] = src[c * a.sc + j];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (x + j < d.W)
+#pragma unroll
+          for (int c = 0; c < C; ++c) dst[j * C + c] = __float2bfloat16_rn(v[c][j]);
+    }
+  }
+}
+template <int C = 1>
+static void launch_planes_to_pixels(const Dims& d, const View& a, const View& y, bool vec, cudaStream_t s) {
+  if constexpr (C <= 4) {
+    if (d.C != C) return launch_planes_to_pixels<C + 1>(d, a, y, vec, s);
+    launch(vec ? planes_to_pixels_kernel<C, true> : planes_to_pixels_kernel<C, false>, grid_for((size_t)d.N * d.H * ((d.W + 3) / 4), 256, 8), 256, 0, s, d, a, y);
+  }
+}
+
 static int same_dims(const ad_tensor4* a, const ad_tensor4* b) {
   return a->N == b->N && a->C == b->C && a->H == b->H && a->W == b->W;
 }
@@ -218,6 +263,14 @@ static int ew_launch(const ad_tensor4* a, const ad_tensor4* b, const ad_tensor4*
       return AD_ERR_CUDA;
     }
     launch(ew_vec_kernel<OP>, grid_for(total / 8, 256, 2), 256, smem, s, d, va, vb, vy, accumulate);
+    count_launch();
+    return launch_status();
+  }
+  if (OP == kConvert && !accumulate && a->dtype == AD_F32 && y->dtype == AD_BF16 && y->C <= 4 && a->sx == 1 && y->sc == 1 && y->sx == (int64_t)y->C &&
+      (size_t)y->N * y->H * ((y->W + 3) / 4) < (1ull << 31)) {
+    auto in4 = [](int64_t v) { return v % 4 == 0; };
+    const bool vec = in4(y->W) && in4(a->sn) && in4(a->sc) && in4(a->sy) && in4(y->sn) && in4(y->sy) && !((uintptr_t)a->base & 15u) && !((uintptr_t)y->base & 7u);
+    launch_planes_to_pixels(d, va, vy, vec, s);
     count_launch();
     return launch_status();
   }
@@ -431,6 +484,94 @@ __global__ void __launch_bounds__(512) im2col_row_kernel(View x, uint32_t C, uin
     }
   }
 }
+// Rows of packed bf16 pixels behind a 16-byte aligned base (the input of a tensor-core net), as a pipeline: a block works through
+// segments of one output row; while it assembles one (two words and a permutation of bytes for a pair of columns), the input rows of the next come by 16-byte asynchronous copies
+// (from the aligned element in front of the segment on, so that each row has a phase of its own), and the part of the matrix
+// that it assembled before, one run of memory, leaves by a bulk copy.  Bound by instructions: a block per segment with a branch
+// for the pairs that lie in two rows (im2col_row_kernel) spent 47 per word and warp on a 7x7 x 3 stem of 1,048,576 pixels x
+// 192, 141 us; 90 now (57 at the rate of a fill).  Segments of 64 pixels with two tiles took 104: what is worked out once per
+// segment counts.
+__global__ void __launch_bounds__(384) im2col_pipe_kernel(View x, uint32_t C, uint32_t H, uint32_t W, uint32_t kh, uint32_t kw, uint32_t sh,
+                                                          uint32_t sw, uint32_t dh, uint32_t dw, uint32_t P, uint32_t Q, __nv_bfloat16* out,
+                                                          uint32_t ldo, uint32_t rowlen, uint32_t qseg, uint32_t total) {
+  grid_dependency();
+  extern __shared__ __align__(16) unsigned char im2col_smem[];
+  const uint32_t pairs = ldo / 2, rows_bytes = kh * rowlen * 2 + 16, segs = (Q + qseg - 1) / qseg, cols = kh * kw * C, step = sw * C;
+  unsigned char* const tiles = im2col_smem + 2 * rows_bytes;
+  // a segment's place, moved on by the grid's size without divisions
+  struct Place { uint32_t q, p, n; };              // segment of the row, row, image
+  const uint32_t hop_q = gridDim.x % segs, hop_p = gridDim.x / segs % P, hop_n = gridDim.x / segs / P;
+  auto advance = [&](Place t) {
+    t.q += hop_q; t.p += hop_p; t.n += hop_n;
+    if (t.q >= segs) { t.q -= segs; ++t.p; }
+    if (t.p >= P) { t.p -= P; ++t.n; }
+    return t;
+  };
+  auto first_of = [&](const Place& t) { return t.n * x.sn + (long long)(t.p * sh) * x.sy + (long long)(t.q * qseg * sw) * x.sx; };   // element
+  const uint32_t per_row = rowlen / 8, r0 = threadIdx.x / per_row, k0 = threadIdx.x - r0 * per_row;
+  auto fetch = [&](const Place& t, bool any, uint32_t buf) {
+    if (any) {
+      const uint32_t left = (W - t.q * qseg * sw) * C, have = left < rowlen ? left : rowlen;
+      const long long base = first_of(t);
+      __nv_bfloat16* rows = (__nv_bfloat16*)(im2col_smem + buf * rows_bytes);
+      for (uint32_t i = threadIdx.x, r = r0, k = k0; i < kh * per_row; i += blockDim.x, r = i / per_row, k = i - r * per_row) {
+        const long long first = base + (long long)(r * dh) * x.sy;
+        const uint32_t phase = (uint32_t)first & 7u, end = t.p * sh + r * dh < H ? phase + have : 0u;   // elements of the copy that exist
+        const __nv_bfloat16* from = (const __nv_bfloat16*)x.base + (first - phase) + k * 8;
+        __nv_bfloat16* to = rows + r * rowlen + k * 8;
+        if (k * 8 + 8 <= end)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+        else
+#pragma unroll
+          for (uint32_t j = 0; j < 8; ++j) to[j] = k * 8 + j >= phase && k * 8 + j < end ? from[j] : __float2bfloat16_rn(0.f);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // a thread's pair of columns: which rows and elements of a row of taps it lies in
+  const uint32_t lanes = blockDim.x / pairs, pr = threadIdx.x % pairs;
+  uint32_t row[2], off[2], mask = 0;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint32_t t = pr * 2 + h, c = t % C, tap = t / C, s = tap % kw, r = tap / kw;
+    row[h] = t < cols ? r : 0u;
+    off[h] = t < cols ? s * dw * C + c : 0u;
+    if (t < cols) mask |= 0xffffu << (16 * h);
+  }
+  Place now{blockIdx.x % segs, blockIdx.x / segs % P, blockIdx.x / segs / P}, next;
+  fetch(now, blockIdx.x < total, 0);
+  uint32_t buf = 0;
+  for (uint32_t seg = blockIdx.x; seg < total; seg += gridDim.x, buf ^= 1u, now = next) {
+    next = advance(now);
+    fetch(next, seg + gridDim.x < total, buf ^ 1u);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the tile before has left
+    __syncthreads();
+    const uint32_t q0 = now.q * qseg, nq = Q - q0 < qseg ? Q - q0 : qseg;
+    const long long base = first_of(now);
+    uint32_t* const tile = (uint32_t*)tiles;
+    const unsigned char* rows = im2col_smem + buf * rows_bytes;
+    if (threadIdx.x < pairs * lanes) {
+      uint32_t e[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) e[h] = row[h] * rowlen + off[h] + ((uint32_t)(base + (long long)(row[h] * dh) * x.sy) & 7u);
+      // the halves of two words (of one, or neighbours, or in two rows); the step from pixel to pixel is even, so which halves stays
+      const uint32_t sel = (e[0] & 1u ? 0x32u : 0x10u) | (e[1] & 1u ? 0x7600u : 0x5400u), q1 = threadIdx.x / pairs, hop = lanes * (step / 2);
+      const uint32_t *a = (const uint32_t*)rows + e[0] / 2 + q1 * (step / 2), *b = (const uint32_t*)rows + e[1] / 2 + q1 * (step / 2);
+      uint32_t* o = tile + q1 * pairs + pr;
+#pragma unroll 4
+      for (uint32_t q = q1; q < nq; q += lanes, a += hop, b += hop, o += lanes * pairs) *o = __byte_perm(*a, *b, sel) & mask;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out + (((size_t)now.n * P + now.p) * Q + q0) * ldo),
+                   "r"((uint32_t)__cvta_generic_to_shared(tile)), "r"(nq * pairs * 4) : "memory");
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+  }
+  if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
 template <typename T>
 static int launch_im2col_row(const View& v, const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh,
                              uint32_t dw, uint32_t P, uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen, uint32_t qseg, size_t smem,
@@ -457,6 +598,24 @@ extern "C" int ad_im2col(const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t
   if ((ldo & 7u) == 0 && ((uintptr_t)out_bf16 & 15u) == 0) {
     // staged-row form when the rows of one output row fit shared memory
     // of the parity of a row of taps, so that (dilation 1) a pair of columns starts at an even element in every row
+    const uint32_t pairs = ldo / 2, reach = (kw - 1) * dw + 1;
+    if (x->dtype == AD_BF16 && x->sc == 1 && x->sx == (int64_t)x->C && !((uintptr_t)x->base & 15u) && x->sn >= 0 && x->sy >= 0 && pairs <= 384 &&
+        (sw * x->C) % 2 == 0) {
+      // two stages of input rows and a tile of 48 KB at most, three or four blocks per SM
+      const uint32_t qs = std::max(1u, std::min(Q, 24576u / ldo)), len = (((qs - 1) * sw + reach) * x->C + 14) / 8 * 8;
+      const size_t need = 2 * ((size_t)kh * len * 2 + 16) + (size_t)qs * ldo * 2, segs = (size_t)x->N * P * ((Q + qs - 1) / qs);
+      if (need <= 96 * 1024 && segs < (1ull << 31)) {
+        if (need > 48 * 1024 && cudaFuncSetAttribute(adk::im2col_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) != cudaSuccess) {
+          cudaGetLastError();
+          return AD_ERR_CUDA;
+        }
+        const uint32_t per_sm = std::min(4u, (uint32_t)(220 * 1024 / (need + 1024)));
+        launch(adk::im2col_pipe_kernel, (unsigned)std::min<size_t>(segs, adk::kNumSMs * per_sm), 384 / pairs * pairs > 32 ? (384 / pairs * pairs + 31) / 32 * 32 : 32,
+               need, adk::as_stream(stream), v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo, len, qs, (uint32_t)segs);
+        adk::count_launch();
+        return adk::launch_status();
+      }
+    }
     const uint32_t qseg = Q < 128 ? Q : 128;   // output pixels per block: enough blocks per SM to keep the stores going
     uint32_t rowlen = ((qseg - 1) * sw + (kw - 1) * dw + 1) * x->C;
     rowlen += (rowlen ^ (kw * x->C)) & 1u;

@@ -443,3 +443,51 @@ def test_sgd_step_guard_skips_the_update_after_a_timed_out_wait():
             assert torch.equal(ref, theta)
         else:
             assert np.array_equal(H.host(m), np.zeros(n, np.float32))
+
+
+@pytest.mark.parametrize("Cc,Hh,W,k,stride,dil,ldo", [
+    (3, 30, 40, 7, 2, 1, 192), (3, 21, 301, 7, 2, 1, 152), (3, 9, 270, 3, 2, 3, 32),     # several segments per row; rows of odd length: a phase each
+    (2, 12, 19, 5, 1, 1, 64), (4, 8, 11, 2, 3, 1, 16), (1, 10, 33, 3, 2, 1, 16),         # other channel counts
+    (3, 14, 17, 3, 1, 1, 32), (5, 9, 20, 3, 1, 1, 48),                                    # an odd step between pixels: the general form
+    (6, 40, 15, 11, 2, 1, 728),                                                           # a wide matrix, one row of pixels per tile
+])
+@pytest.mark.parametrize("lift", [0, 8, 3])
+def test_patch_matrix(Cc, Hh, W, k, stride, dil, ldo, lift):
+    """Patches of bf16 pixels from bases of every alignment; output rows that reach past the input's lower and right edge get zeros."""
+    import torch
+    N = 3
+    g = torch.Generator(device="cuda").manual_seed(11)
+    buf = torch.rand(N * Hh * W * Cc + 64, generator=g, device="cuda").bfloat16()
+    x = buf[lift:lift + N * Hh * W * Cc].view(N, Hh, W, Cc)
+    reach = dil * (k - 1) + 1
+    P, Q = (Hh - reach) // stride + 2, (W - reach) // stride + 2          # one more than fits, each way
+    out = torch.full((N * P * Q + 1, ldo), 7.0, dtype=torch.bfloat16, device="cuda")
+    vx = H.view_nhwc(x)
+    abi.check(abi.lib().ad_im2col(C.byref(vx), k, k, stride, stride, dil, dil, P, Q, out.data_ptr(), ldo, H.stream()))
+    H.sync()
+    pad = torch.zeros((N, (P - 1) * stride + reach, (Q - 1) * stride + reach, Cc), device="cuda", dtype=torch.bfloat16)
+    hh, ww = min(Hh, pad.shape[1]), min(W, pad.shape[2])
+    pad[:, :hh, :ww] = x[:, :hh, :ww]
+    want = torch.stack([pad[:, r * dil:r * dil + (P - 1) * stride + 1:stride, s * dil:s * dil + (Q - 1) * stride + 1:stride] for r in range(k) for s in range(k)], 3)
+    assert torch.equal(out[:-1, :k * k * Cc], want.reshape(N * P * Q, k * k * Cc))
+    assert torch.count_nonzero(out[:-1, k * k * Cc:]) == 0 and (out[-1] == 7).all()
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 5, 8), (1, 3, 4, 13), (3, 1, 7, 4), (2, 4, 3, 40), (1, 2, 6, 257)])
+@pytest.mark.parametrize("lift,gap", [(0, 0), (1, 0), (4, 4), (0, 5)])
+def test_planes_to_pixels(shape, lift, gap):
+    """fp32 planes into bf16 pixels: rows and bases of every alignment, wider rows on both sides; nothing beside them is written."""
+    import torch
+    N, Cc, Hh, W = shape
+    g = torch.Generator(device="cuda").manual_seed(3)
+    src = torch.rand(lift + N * Cc * Hh * (W + gap) + 8, generator=g, device="cuda")
+    x = src[lift:lift + N * Cc * Hh * (W + gap)].view(N, Cc, Hh, W + gap)
+    dst = torch.full((lift + N * Hh * (W + gap) * Cc + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    y = dst[lift:lift + N * Hh * (W + gap) * Cc].view(N, Hh, W + gap, Cc)
+    vx = abi.Tensor4(x.data_ptr(), abi.AD_F32, N, Cc, Hh, W, Cc * Hh * (W + gap), Hh * (W + gap), W + gap, 1)
+    vy = abi.Tensor4(y.data_ptr(), abi.AD_BF16, N, Cc, Hh, W, Hh * (W + gap) * Cc, 1, (W + gap) * Cc, Cc)
+    abi.check(abi.lib().ad_convert(C.byref(vx), C.byref(vy), 0, H.stream()))
+    H.sync()
+    assert torch.equal(y[:, :, :W], x[..., :W].permute(0, 2, 3, 1).bfloat16())
+    y[:, :, :W] = 7.0
+    assert (dst == 7.0).all()
