@@ -528,21 +528,24 @@ bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pi
 
 // The 3x3 kernel's tiles are 64 x 16 channels (32 x 32 for up to 32 output channels), the general one's 64 x 128 (channel, tap)
 // columns: it wins from 16 channels on where more than half of its tiles is used (11 channels: 35 against 47 us, 14: 36
-// against 63, 17: 109 against 137, 33 output channels: 79 against 103; the other way 25: 430 -> 367, 32: 54 -> 52).
-static bool f32_k3_wgrad_wins(const ad_conv2d_args* a) {
+// against 63, 17: 109 against 137, 33 output channels: 79 against 103; the other way 25: 430 -> 367, 32: 54 -> 52).  One tile
+// alone is split into 128 CTAs at most: with more than four stages for each, the general kernel, which has more of them, is
+// faster (8 x 24 x 60 x 60 -> 32: 47 against 56 us).
+static bool f32_k3_wgrad_wins(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
   if (a->kh != 3 || a->kw != 3 || a->stride_h != 1 || a->stride_w != 1 || a->dil_h != 1 || a->dil_w != 1 || a->K <= 16 || a->C < 16) return false;
+  if (a->K <= 64 && a->C <= (a->K <= 32 ? 32u : 16u) && (unsigned long long)a->N * P * ((Q + 7) / 8) > 4 * 4 * 128) return false;
   if (a->K <= 32) return true;
   const unsigned long long k = (a->K + 63) / 64 * 64, c = (a->C + 15) / 16 * 16;
   return 25ull * a->K * a->C >= 14ull * k * c;
 }
 size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
-  const uint32_t s = f32_k3_wgrad_wins(a) ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q).slices : wg_slices(a, P, Q);
+  const uint32_t s = f32_k3_wgrad_wins(a, P, Q) ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q).slices : wg_slices(a, P, Q);
   return s > 1 ? (size_t)s * ((size_t)a->K * a->C * a->kh * a->kw + a->K) * 4 : 0;
 }
 
 // Measured (one B200; per call, thread per output -> these tiles): 64 -> 64 channels, 3x3, 64 x 64 pixels, one image: forward
 // 188 -> 21 us, data gradient 158 -> 25, filter and bias gradient 286 -> 31.  4 x 64 x 112 x 112, 64 -> 64 3x3: 1440 -> 135, 1500 ->
-// 134, 2330 -> 172 us (27 / 28 / 21 TFLOP/s); conv_f32_k3.cu, which serves these two now, takes 19, 25, 25 and 94, 92, 127.
+// 134, 2330 -> 172 us (27 / 28 / 21 TFLOP/s); conv_f32_k3.cu, which serves these two now, takes 17, 21, 23 and 94, 92, 127.
 // What is left above the FMA pipe: 12 warps per SM do not hide the latency of the shared-memory reads (issue slots 42 % busy);
 // 4 x 8 outputs per thread or packed pairs along the reduction were slower.
 int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pitch, long long y_plane, cudaStream_t s) {
@@ -638,7 +641,7 @@ int f32_gemm_wgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
   p.dy_pitch = y_pitch; p.dy_plane = y_plane; p.accumulate = a->accumulate;
   p.slices = 1;
   const size_t need = f32_wgrad_scratch(a, P, Q);
-  const bool k3 = f32_k3_wgrad_wins(a), parts = need && a->scratch && a->scratch_bytes >= need;
+  const bool k3 = f32_k3_wgrad_wins(a, P, Q), parts = need && a->scratch && a->scratch_bytes >= need;
   const F32Split split = k3 ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q) : F32Split{8, wg_slices(a, P, Q)};
   if (parts) { p.slices = split.slices; p.part = (float*)a->scratch; }
   if (k3) {

@@ -9,7 +9,7 @@
 // Measured (one B200, 3.7 GFLOP each; before -> now): 4 x 64 x 112 x 112 -> 64: forward 135 -> 94 us, data gradient 134 -> 92, filter
 // and bias gradient 172 -> 127; 4 x 128 x 56 x 56 -> 128: 131 -> 94, 131 -> 90, 261 -> 115; 4 x 512 x 14 x 14 -> 512: 181 -> 127,
 // 180 -> 123, 135 -> 125.  Over 630 drawn layers: forward 1.33, data gradient 1.33, filter gradient 1.2 times as fast.
-// Sums, splits over clusters and slices, and their order of addition are as in conv_f32.cu: fp32 FMAs, running sums of 18 or
+// Sums, splits over clusters and slices, and their order of addition are as in conv_f32.cu: fp32 FMAs, running sums of 18 to
 // 54 (filter gradient: 32 to 128) terms, partial tiles in rank order; no atomics.
 #include <algorithm>
 
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kK3Threads, 3) conv3_f32(const GemmF32 p) {
     cp_async_commit();
   }
   bool first = true;
-  const uint32_t period = steps <= 8 ? 1 : 3;     // running sums of 18 or 54 terms
+  const uint32_t period = steps <= 2 ? 1 : steps <= 8 ? 2 : 3;     // running sums of 18, 36, 54 terms
   uint32_t slot = 0, to_flush = period;
 #pragma unroll 1
   for (uint32_t st = 0; st < steps; ++st) {
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kK3Threads, 3) conv3_wgrad_f32(const WgradF32 
   };
   if (steps) load(0);
   cp_async_commit();
-  const uint32_t period = steps <= 8 ? 1 : steps <= 24 ? 2 : 4;     // running sums of 32, 64, 128 pixels: a flush costs as much as 8
+  const uint32_t period = steps <= 2 ? 1 : steps <= 24 ? 2 : 4;     // running sums of 32, 64, 128 pixels: a flush costs as much as 8
   uint32_t to_flush = period;
   bool first = true;
   for (uint32_t st = 0; st < steps; ++st) {

@@ -44,7 +44,7 @@ uint32_t f32_k3_cluster(Held held, unsigned long long tiles, uint32_t steps, uin
   for (uint32_t cs = 1; cs <= most && (cs == 1 || steps >= 2 * cs); cs *= 2) {
     const unsigned long long h = held(cs);
     if (!h) continue;
-    const double cta = (steps + cs - 1) / cs + 3 + 0.5 * cs, cost = cta * (tiles / h * f32_k3_share(h * cs, cs, sms) + f32_k3_share(tiles % h * cs, cs, sms));
+    const double cost = (steps + cs - 1) / cs * (tiles / h * f32_k3_share(h * cs, cs, sms) + f32_k3_share(tiles % h * cs, cs, sms)) + 0.75 * cs;
     // a CTA sums over 128 stages (256 channels) at most where that can be: the sum of its running sums loses precision with
     // their number (371 channels in one CTA: 2.0e-7 against 1.7e-7 in two)
     if (!best || cost < best_cost || (steps > 128 * best)) { best = cs; best_cost = cost; }
