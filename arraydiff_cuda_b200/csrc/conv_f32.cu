@@ -294,6 +294,12 @@ static bool f32_k3_gemm_wins(const GemmF32& p) {
   return used * 20 >= blocks * 8 * (p.CR >= 192 ? 13 : 16);
 }
 
+// Tiles of 32 rows and more: for 16 and fewer most of one would be zeros.  Faster or equal at every size measured above that
+// (150 layers of 17 to 600 channels, maps from 7 x 7).
+static bool f32_k1_gemm_wins(const GemmF32& p) {
+  return p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && !p.ph && !p.pw && p.IH == p.OH && p.IW == p.OW && p.M > 16;
+}
+
 // Tile height by the row count: a row of the tile costs the same FMAs whether it holds a channel or not, a column is
 // gathered once per tile row: 64 x 128 for more than 32 channels, 32 x 256, 16 x 512 and 8 x 1024 below.
 template <bool DGRAD>
@@ -302,6 +308,7 @@ static int run_gemm_f32(const GemmF32& p, cudaStream_t s) {
   const uint32_t OHc = DGRAD ? (p.OH + p.sh - 1) / p.sh : p.OH, OWc = DGRAD ? (p.OW + p.sw - 1) / p.sw : p.OW;
   const uint32_t npx = p.NI * OHc * OWc, Kd = p.CR * ((p.kh * p.kw + classes - 1) / classes);
   if (f32_k3_gemm_wins(p)) return f32_k3_gemm<DGRAD>(p, s);
+  if (f32_k1_gemm_wins(p)) return f32_k1_gemm(p, s);
   if (p.M <= 8) return launch_gemm_f32<1, 1, 4, DGRAD>(p, npx, classes, Kd, s);
   if (p.M <= 16) return launch_gemm_f32<2, 1, 4, DGRAD>(p, npx, classes, Kd, s);
   if (p.M <= 32) return launch_gemm_f32<4, 1, 4, DGRAD>(p, npx, classes, Kd, s);
@@ -563,7 +570,7 @@ int f32_gemm_fprop(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
 // Data gradient into few channels (an image's three), with scratch: per pixel of dy the products of all (channel, tap) rows
 // with the filter as one GEMM -- Z[n][channel, tap][pixel], a 1x1 convolution of dy -- and then the sum over the taps of
 // each input pixel, in tap order.  As the GEMM above, 3 of 8 rows of a tile are used and every element of dy is gathered
-// once per tap: bound by the gathers.  4 x 64 x 224 x 224 -> 3, 7x7: 730 -> 393 us.
+// once per tap: bound by the gathers.  4 x 64 x 224 x 224 -> 3, 7x7: 730 -> 250 us.
 // Images are taken as many at a time as fit kFewZ bytes (f32_few_images); larger ones go the other way.
 constexpr size_t kFewZ = 64u << 20;
 static size_t few_z_bytes(const ad_conv2d_args* a, uint32_t P, uint32_t Q) { return (size_t)P * Q * a->C * a->kh * a->kw * 4; }   // one image

@@ -36,6 +36,22 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+__device__ __forceinline__ void fadd2(u64& d, u64 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
+
+// Sum of four neighbouring floats of the tiles of all CTAs of the cluster, in rank order; all loads are in flight together
+template <int MOST>
+__device__ __forceinline__ float4 cluster_total4(cg::cluster_group& cluster, float* sm, uint32_t cs, size_t at) {
+  float4 v[MOST];
+#pragma unroll
+  for (uint32_t q = 0; q < MOST; ++q)
+    v[q] = q < cs ? *(const float4*)((cs > 1 ? cluster.map_shared_rank(sm, q) : sm) + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 t = v[0];
+#pragma unroll
+  for (uint32_t q = 1; q < MOST; ++q)
+    if (q < cs) { t.x += v[q].x; t.y += v[q].y; t.z += v[q].z; t.w += v[q].w; }
+  return t;
+}
+
 constexpr int kF32Most = 16;             // CTAs of a cluster, forward and data gradient
 constexpr uint32_t kF32Never = 1u << 31; // a bit no pixel has
 
@@ -122,6 +138,8 @@ inline uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, 
 
 // 3x3, stride and dilation 1 (conv_f32_k3.cu)
 template <bool DGRAD> int f32_k3_gemm(const GemmF32& p, cudaStream_t s);
+// 1x1, stride 1, no padding (conv_f32_k1.cu)
+int f32_k1_gemm(const GemmF32& p, cudaStream_t s);
 F32Split f32_k3_wgrad_split(uint32_t K, uint32_t C, uint32_t N, uint32_t P, uint32_t Q);
 int f32_k3_wgrad(const WgradF32& p, uint32_t cs, cudaStream_t s);
 

@@ -17,22 +17,6 @@
 
 namespace adk {
 
-__device__ __forceinline__ void fadd2(u64& d, u64 a) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
-
-// Sum of four neighbouring floats of the tiles of all CTAs of the cluster, in rank order; all loads are in flight together
-template <int MOST>
-__device__ __forceinline__ float4 cluster_total4(cg::cluster_group& cluster, float* sm, uint32_t cs, size_t at) {
-  float4 v[MOST];
-#pragma unroll
-  for (uint32_t q = 0; q < MOST; ++q)
-    v[q] = q < cs ? *(const float4*)((cs > 1 ? cluster.map_shared_rank(sm, q) : sm) + at) : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 t = v[0];
-#pragma unroll
-  for (uint32_t q = 1; q < MOST; ++q)
-    if (q < cs) { t.x += v[q].x; t.y += v[q].y; t.z += v[q].z; t.w += v[q].w; }
-  return t;
-}
-
 constexpr int kK3Threads = 128;
 
 // ---------------------------------------------------------------- forward / data gradient

@@ -28,7 +28,7 @@ uint32_t f32_cluster_size(Held held, unsigned long long tiles, uint32_t steps, u
   return best ? best : 1;
 }
 
-// The 3x3 kernels (conv_f32_k3.cu) keep the FMA pipe busy with one CTA per SM, so that CTAs on one SM take turns (a stage
+// The 3x3 and 1x1 kernels (conv_f32_k3.cu, conv_f32_k1.cu: stages of 18 and 16 terms) keep the FMA pipe busy with one CTA per SM, so that CTAs on one SM take turns (a stage
 // measured 1.1 us alone, 1.9 beside one other, 2.7 beside two), and the SM with the most of them counts.  A cluster stays
 // within one group of SMs, so that larger ones are spread less evenly: 36 clusters of 4 leave some SMs two CTAs (filter gradient
 // 64 -> 64, 4 x 112 x 112: 184 us, 32 clusters of 4 133), and so do 16 of 8 already (half of the SMs were idle).

@@ -120,6 +120,53 @@ def test_data_gradient_of_more_than_2_32_elements():
         assert (got - want).abs().max() < 1e-5 * want.max() and torch.count_nonzero(dx[n]) == got.numel()   # zeros elsewhere
 
 
+K1_CASES = [
+    # N, C, H, W, K of 1x1 layers: both directions
+    (1, 17, 1, 1, 17),             # one pixel, the smallest channel counts of the 1x1 kernels
+    (1, 32, 2, 2, 33),             # one vector of pixels; a row past the 32-row tile, filters of the gradient one by one
+    (3, 31, 5, 13, 64),            # planes of 65 pixels: gathers one by one; a channel short of two stages
+    (2, 65, 6, 22, 36),            # vectors that cross rows, images that share a tile; a row past the 64-row tile
+    (1, 130, 9, 12, 24),           # 32-row tiles, reduction split over a cluster
+    (5, 48, 16, 20, 148),          # running sums that restart, three tiles of rows
+    (1, 2100, 8, 8, 20),           # the largest clusters, shares of unequal length
+]
+
+
+@pytest.mark.parametrize("pitched", [0, 1])
+@pytest.mark.parametrize("case", K1_CASES)
+def test_conv_f32_1x1(case, pitched, monkeypatch):
+    """The 1x1 kernels at the edges of their tiles, vectors and splits; dense planes and padded ones; operands off by four bytes."""
+    import torch
+    monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", "1")
+    N, Cc, Hh, W, K = case
+    x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, 1, 1), float(np.sqrt(2.0 / Cc))), H.normal(3, (K,))
+    dy = H.uniform(4, (N, K, Hh, W))
+    y_w = np.einsum("nchw,kc->nkhw", x.astype(np.float64), w[:, :, 0, 0].astype(np.float64)) + b[None, :, None, None]
+    dx_w = np.einsum("nkhw,kc->nchw", dy.astype(np.float64), w[:, :, 0, 0].astype(np.float64)) + 1.0
+    # a sum of n products, |terms| t: running sums of 64 and n / 64 partial sums round at 2^-24 of what they hold
+    eps = lambda n: (min(n, 64) + n // 64 + 4) * 2.0 ** -24  # noqa: E731
+    L = abi.lib()
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, 1, 1, 1, 0)
+    flat = torch.empty(x.size + 1, device="cuda")
+    xd = flat[pitched:pitched + x.size].view(x.shape).copy_(H.dev(x))          # one off: no longer 16-byte aligned
+    wflat = torch.empty(w.size + 1, device="cuda")
+    wd = wflat[pitched:pitched + w.size].view(w.shape).copy_(H.dev(w))
+    bd = H.dev(b)
+    ph, pw = Hh + pitched, W + 3 * pitched
+    y, gy = torch.full((N, K, ph, pw), 7.0, device="cuda"), torch.full((N, K, ph, pw), float("nan"), device="cuda")
+    gy[:, :, :Hh, :W] = H.dev(dy)
+    dx = torch.ones(x.shape, device="cuda")
+    a.x, a.w, a.bias, a.y, a.y_pitch, a.y_plane = xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), y.data_ptr(), pw, ph * pw
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    a.y, a.dx, a.accumulate = gy.data_ptr(), dx.data_ptr(), 1
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    mag_y = np.einsum("nchw,kc->nkhw", np.abs(x), np.abs(w[:, :, 0, 0])) + np.abs(b)[None, :, None, None]
+    mag_x = np.einsum("nkhw,kc->nchw", np.abs(dy), np.abs(w[:, :, 0, 0])) + 1.0
+    assert (np.abs(y[:, :, :Hh, :W].cpu().numpy() - y_w) <= eps(Cc) * mag_y).all()
+    assert (np.abs(dx.cpu().numpy() - dx_w) <= eps(K) * mag_x).all()
+    assert (y[:, :, Hh:] == 7).all() and (y[:, :, :, W:] == 7).all()
+
+
 K3_CASES = [
     # N, C, H, W (of x), K, pad: 3x3, stride and dilation 1
     (1, 16, 3, 3, 17, 0),          # one output pixel; the smallest channel counts of the 3x3 kernels
