@@ -287,17 +287,23 @@ static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uin
 // reduction is long), for 16 rows and fewer, and for long reductions into few tiles of 32 rows, which go to 8 CTAs at
 // most, the general tiles are as fast or faster: 17 x 42 x 13 x 5 -> 346 channels, two thirds used, 25 against 31 us;
 // 9 x 440 x 18 x 22 -> 27, 16 tiles, 48 against 65.  The other way: 4 x 512 x 7 x 7 -> 512 data gradient, two thirds used, 94 -> 66.
-static bool f32_k3_gemm_wins(const GemmF32& p) {
-  if (p.kh != 3 || p.kw != 3 || p.sh != 1 || p.sw != 1 || p.dh != 1 || p.dw != 1 || p.M <= 16) return false;
-  const unsigned long long used = (unsigned long long)p.OH * p.OW, blocks = (unsigned long long)((p.OH + 3) / 4) * ((p.OW + 1) / 2);
-  if (p.M <= 32 && p.CR > 128 && p.NI * blocks < 24 * 32) return false;
+// A map under dilation is counted as the maps that it falls into.  With a stride of 2 (forward only) a patch is 45 elements
+// instead of 24 and three quarters of a tile's rows and pixels have to be used: 137 -> 209, 2 x 14 x 34, 0.71, 33 against 39 us;
+// 156 -> 276, 4 x 12 x 21, 0.82, the other way, 47 -> 43.
+static bool f32_k3_gemm_wins(const GemmF32& p, bool dgrad) {
+  if (p.kh != 3 || p.kw != 3 || p.sh != p.sw || p.sh > (dgrad ? 1u : 2u) || (p.sh == 2 && (p.dh != 1 || p.dw != 1)) || p.M <= 16) return false;
+  const unsigned long long used = (unsigned long long)p.OH * p.OW, blocks = f32_k3_blocks(p.OH, p.OW, p.dh, p.dw);
+  if (p.M <= 32 && p.CR > 128 && p.NI * blocks < (p.sh == 2 ? 48 : 24) * 32) return false;
+  if (p.sh == 2 && p.M > 32 && 4 * used * p.M < 3 * 8 * blocks * ((p.M + 63) / 64 * 64)) return false;
   return used * 20 >= blocks * 8 * (p.CR >= 192 ? 13 : 16);
 }
 
 // Tiles of 32 rows and more: for 16 and fewer most of one would be zeros.  Faster or equal at every size measured above that
-// (150 layers of 17 to 600 channels, maps from 7 x 7).
-static bool f32_k1_gemm_wins(const GemmF32& p) {
-  return p.kh == 1 && p.kw == 1 && p.sh == 1 && p.sw == 1 && !p.ph && !p.pw && p.IH == p.OH && p.IW == p.OW && p.M > 16;
+// (300 layers of 17 to 600 channels, strides 1 to 3, maps from 7 x 7) but where single pixels are gathered from far apart for
+// few rows (8 x 192 x 235 x 280 -> 21, stride 3: 68 against 60 us).
+static bool f32_k1_gemm_wins(const GemmF32& p, bool dgrad) {
+  if (!dgrad && p.M <= 32 && p.sh * p.sw > 4) return false;
+  return p.kh == 1 && p.kw == 1 && !p.ph && !p.pw && p.M > 16;
 }
 
 // Tile height by the row count: a row of the tile costs the same FMAs whether it holds a channel or not, a column is
@@ -307,8 +313,8 @@ static int run_gemm_f32(const GemmF32& p, cudaStream_t s) {
   const uint32_t classes = DGRAD ? p.sh * p.sw : 1;
   const uint32_t OHc = DGRAD ? (p.OH + p.sh - 1) / p.sh : p.OH, OWc = DGRAD ? (p.OW + p.sw - 1) / p.sw : p.OW;
   const uint32_t npx = p.NI * OHc * OWc, Kd = p.CR * ((p.kh * p.kw + classes - 1) / classes);
-  if (f32_k3_gemm_wins(p)) return f32_k3_gemm<DGRAD>(p, s);
-  if (f32_k1_gemm_wins(p)) return f32_k1_gemm(p, s);
+  if (f32_k3_gemm_wins(p, DGRAD)) return f32_k3_gemm<DGRAD>(p, s);
+  if (f32_k1_gemm_wins(p, DGRAD)) return f32_k1_gemm<DGRAD>(p, s);
   if (p.M <= 8) return launch_gemm_f32<1, 1, 4, DGRAD>(p, npx, classes, Kd, s);
   if (p.M <= 16) return launch_gemm_f32<2, 1, 4, DGRAD>(p, npx, classes, Kd, s);
   if (p.M <= 32) return launch_gemm_f32<4, 1, 4, DGRAD>(p, npx, classes, Kd, s);
@@ -539,14 +545,19 @@ bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pi
 // alone is split into 128 CTAs at most: with more than four stages for each, the general kernel, which has more of them, is
 // faster (8 x 24 x 60 x 60 -> 32: 47 against 56 us).
 static bool f32_k3_wgrad_wins(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
-  if (a->kh != 3 || a->kw != 3 || a->stride_h != 1 || a->stride_w != 1 || a->dil_h != 1 || a->dil_w != 1 || a->K <= 16 || a->C < 16) return false;
-  if (a->K <= 64 && a->C <= (a->K <= 32 ? 32u : 16u) && (unsigned long long)a->N * P * ((Q + 7) / 8) > 4 * 4 * 128) return false;
+  if (a->kh != 3 || a->kw != 3 || a->stride_h != a->stride_w || a->stride_h > 2 || a->K <= 16 || a->C < 16) return false;
+  if (a->stride_h == 2 && (a->dil_h != 1 || a->dil_w != 1)) return false;
+  if (a->K <= 64 && a->C <= (a->K <= 32 ? 32u : 16u) && (unsigned long long)a->N * P * f32_k3_segments(Q, a->dil_w) > 4 * 4 * 128) return false;
+  // under dilation a segment's pixels are dil apart: seven tenths of segments and tiles together (27 x 41 x 14 x 33 -> 57, dilation 4,
+  // 0.37: 39 against 54 us; 29 x 26 x 16 x 58 -> 177, 0.68: 118 against 131)
+  const unsigned bk = a->K <= 32 ? 32 : 64, bc = a->K <= 32 ? 32 : 16;
+  const unsigned long long k = (a->K + bk - 1) / bk * bk, c = (a->C + bc - 1) / bc * bc;
+  if (a->dil_w > 1 && (a->dil_w > Q || 10ull * a->K * a->C * Q < 7ull * k * c * f32_k3_segments(Q, a->dil_w) * 8)) return false;
   if (a->K <= 32) return true;
-  const unsigned long long k = (a->K + 63) / 64 * 64, c = (a->C + 15) / 16 * 16;
   return 25ull * a->K * a->C >= 14ull * k * c;
 }
 size_t f32_wgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
-  const uint32_t s = f32_k3_wgrad_wins(a, P, Q) ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q).slices : wg_slices(a, P, Q);
+  const uint32_t s = f32_k3_wgrad_wins(a, P, Q) ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q, a->stride_w, a->dil_w).slices : wg_slices(a, P, Q);
   return s > 1 ? (size_t)s * ((size_t)a->K * a->C * a->kh * a->kw + a->K) * 4 : 0;
 }
 
@@ -649,7 +660,7 @@ int f32_gemm_wgrad(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_
   p.slices = 1;
   const size_t need = f32_wgrad_scratch(a, P, Q);
   const bool k3 = f32_k3_wgrad_wins(a, P, Q), parts = need && a->scratch && a->scratch_bytes >= need;
-  const F32Split split = k3 ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q) : F32Split{8, wg_slices(a, P, Q)};
+  const F32Split split = k3 ? f32_k3_wgrad_split(a->K, a->C, a->N, P, Q, a->stride_w, a->dil_w) : F32Split{8, wg_slices(a, P, Q)};
   if (parts) { p.slices = split.slices; p.part = (float*)a->scratch; }
   if (k3) {
     const int rc = f32_k3_wgrad(p, parts || split.slices == 1 ? split.cs : 8, s);

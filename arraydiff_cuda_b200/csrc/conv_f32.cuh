@@ -41,6 +41,7 @@ __device__ __forceinline__ void fadd2(u64& d, u64 a) { asm("add.rn.f32x2 %0, %0,
 // Sum of four neighbouring floats of the tiles of all CTAs of the cluster, in rank order; all loads are in flight together
 template <int MOST>
 __device__ __forceinline__ float4 cluster_total4(cg::cluster_group& cluster, float* sm, uint32_t cs, size_t at) {
+  if (cs == 1) return *(const float4*)(sm + at);
   float4 v[MOST];
 #pragma unroll
   for (uint32_t q = 0; q < MOST; ++q)
@@ -138,9 +139,9 @@ inline uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, 
 
 // 3x3, stride and dilation 1 (conv_f32_k3.cu)
 template <bool DGRAD> int f32_k3_gemm(const GemmF32& p, cudaStream_t s);
-// 1x1, stride 1, no padding (conv_f32_k1.cu)
-int f32_k1_gemm(const GemmF32& p, cudaStream_t s);
-F32Split f32_k3_wgrad_split(uint32_t K, uint32_t C, uint32_t N, uint32_t P, uint32_t Q);
+// 1x1 without padding (conv_f32_k1.cu)
+template <bool DGRAD> int f32_k1_gemm(const GemmF32& p, cudaStream_t s);
+F32Split f32_k3_wgrad_split(uint32_t K, uint32_t C, uint32_t N, uint32_t P, uint32_t Q, uint32_t stride, uint32_t dil);
 int f32_k3_wgrad(const WgradF32& p, uint32_t cs, cudaStream_t s);
 
 }  // namespace adk

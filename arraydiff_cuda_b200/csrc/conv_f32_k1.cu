@@ -1,13 +1,15 @@
-// fp32 NCHW convolution, 1x1 filters of stride 1 without padding: forward and data gradient, and the products of the two-step
+// fp32 NCHW convolution, 1x1 filters without padding: forward and data gradient, and the products of the two-step
 // data gradient into few channels.  A plain GEMM over channels whose right operand, planes of pixels, is contiguous as it
 // lies: 16-byte asynchronous copies where planes and images are multiples of four floats apart, per-pixel gathers otherwise.
 // The general tiles of conv_f32.cu work an address and a test out for every element.  Packed FMAs, splits over clusters
 // and the order of sums are those of conv_f32_k3.cu; running sums of 64 terms.  Long reductions are bound by the issue of
 // packed FMAs, short ones by the start of a CTA and its way out through the tile.
+// A strided layer gathers every stride-th pixel forward; its data gradient writes them between zeros set in front.
 // Measured (one B200; before -> now, the other direction has the sizes exchanged): 2 x 64 x 224 x 224 -> 147: forward 154 -> 82 us,
 // data gradient 99 -> 62; 4 x 512 x 14 x 14 -> 2048: 92 -> 59 and 86 -> 62; 4 x 64 x 56 x 56 -> 256: 35 -> 21 and 25 -> 19.  Over 150
 // drawn layers: forward 1.63, data gradient 1.45 times as fast in sum, none slower; error against 64 bits as before
-// (means 1.17 -> 1.15e-7, 1.34 -> 1.31e-7).
+// (means 1.17 -> 1.15e-7, 1.34 -> 1.31e-7).  Strides 2 and 3, 150 layers: 1.36 and 2.3 times (4 x 64 x 112 x 112 -> 128, stride 2: 27 -> 17,
+// 31 -> 21 us).
 #include <algorithm>
 
 #include "conv_f32.cuh"
@@ -25,8 +27,9 @@ template <int WM> struct K1Tile {
   static constexpr int smem = (STAGES * stage_floats + BN * PT) * 4;
 };
 
-// VX: 16-byte copies of pixels.  VW: output channels are contiguous in the filter (data gradient) and come by 16 bytes
-template <int WM, bool VX, bool VW>
+// VX: 16-byte copies of pixels.  VW: output channels are contiguous in the filter (data gradient) and come by 16 bytes.
+// SPREAD: the data gradient of a strided layer: a pixel of dy adds to or writes every stride-th pixel of every stride-th row
+template <int WM, bool VX, bool VW, bool SPREAD>
 __global__ void __launch_bounds__(kK1Threads, 3) conv1_f32(const GemmF32 p) {
   grid_dependency();
   typedef K1Tile<WM> T;
@@ -36,14 +39,14 @@ __global__ void __launch_bounds__(kK1Threads, 3) conv1_f32(const GemmF32 p) {
   cg::cluster_group cluster = cg::this_cluster();
   const uint32_t cs = cluster.num_blocks(), rank = cluster.block_rank();
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t m_base = blockIdx.y * BM, n_base = blockIdx.x / cs * BN, hw = p.OH * p.OW, npx = p.NI * hw;
+  const uint32_t m_base = blockIdx.y * BM, n_base = blockIdx.x / cs * BN, PW = SPREAD ? p.IW : p.OW, hw = (SPREAD ? p.IH : p.OH) * PW, npx = p.NI * hw;
   const uint32_t per = ((p.CR + cs - 1) / cs + CH - 1) / CH * CH;   // this CTA's share of the input channels
   const uint32_t c_lo = rank * per < p.CR ? rank * per : p.CR, c_hi = c_lo + per < p.CR ? c_lo + per : p.CR;
   const uint32_t steps = (c_hi - c_lo + CH - 1) / CH;
 
   auto in_at = [&](uint32_t px) {
-    const uint32_t n = px / hw, r = px - n * hw, y = r / p.OW;
-    return p.in + (long long)n * p.in_img + (long long)y * p.in_pitch + (r - y * p.OW);
+    const uint32_t n = px / hw, r = px - n * hw, y = r / PW, x = r - y * PW;
+    return p.in + (long long)n * p.in_img + (long long)(SPREAD ? y : y * p.sh) * p.in_pitch + (SPREAD ? x : x * p.sw);
   };
   // what this thread copies of the input: 4 pixels of every XS-th channel, or XN pixels of every channel
   constexpr uint32_t XT = BN / 4, XS = kK1Threads / XT, XN = BN / kK1Threads;
@@ -161,8 +164,8 @@ __global__ void __launch_bounds__(kK1Threads, 3) conv1_f32(const GemmF32 p) {
   for (uint32_t e = tid; e < (uint32_t)BN; e += kK1Threads) {
     const uint32_t px = n_base + e;
     if (px >= npx) continue;
-    const uint32_t n = px / hw, r = px - n * hw, y = r / p.OW;
-    float* out = p.out + (long long)n * p.out_img + (long long)y * p.out_pitch + (r - y * p.OW);
+    const uint32_t n = px / hw, r = px - n * hw, y = r / PW, x = r - y * PW;
+    float* out = p.out + (long long)n * p.out_img + (long long)(SPREAD ? y * p.sh : y) * p.out_pitch + (SPREAD ? x * p.sw : x);
     const uint32_t row = tile_row((e >> 5 & 1u) * 4 + (e & 3u), (e >> 6) * 8 + (e >> 2 & 7u));
 #pragma unroll 1
     for (uint32_t m = rank * rows; m < (rank + 1) * rows; m += 4) {
@@ -183,23 +186,35 @@ __global__ void __launch_bounds__(kK1Threads, 3) conv1_f32(const GemmF32 p) {
   if (cs > 1) cluster.sync();           // nobody leaves while its tile is still read
 }
 
-template <int WM, bool VX, bool VW>
+template <int WM, bool VX, bool VW, bool SPREAD>
 static int launch_conv1_f32(const GemmF32& p, cudaStream_t s) {
   typedef K1Tile<WM> T;
   static F32Launch l;
-  const uint32_t npx = p.NI * p.OH * p.OW, tn = (npx + T::BN - 1) / T::BN, tm = (p.M + T::BM - 1) / T::BM;
-  auto held = [](uint32_t n) { return f32_held(conv1_f32<WM, VX, VW>, kK1Threads, T::smem, n, l); };
+  const uint32_t npx = SPREAD ? p.NI * p.IH * p.IW : p.NI * p.OH * p.OW, tn = (npx + T::BN - 1) / T::BN, tm = (p.M + T::BM - 1) / T::BM;
+  auto held = [](uint32_t n) { return f32_held(conv1_f32<WM, VX, VW, SPREAD>, kK1Threads, T::smem, n, l); };
   const uint32_t cs = f32_k3_cluster(held, (unsigned long long)tn * tm, (p.CR + T::CH - 1) / T::CH, std::min(kF32Most, T::BM / 4), kNumSMs);
-  return launch_f32(conv1_f32<WM, VX, VW>, dim3(tn * cs, tm), kK1Threads, T::smem, cs, p, l, s);
+  return launch_f32(conv1_f32<WM, VX, VW, SPREAD>, dim3(tn * cs, tm), kK1Threads, T::smem, cs, p, l, s);
 }
-int f32_k1_gemm(const GemmF32& p, cudaStream_t s) {
+template <bool SPREAD>
+static int run_conv1_f32(const GemmF32& p, cudaStream_t s) {
   auto in4 = [](long long v) { return v % 4 == 0; };
-  const bool vx = p.in_pitch == p.OW && in4(p.in_plane) && in4(p.in_img) && in4((long long)p.OH * p.OW) && !((uintptr_t)p.in & 15u);
+  const long long px = SPREAD ? (long long)p.IH * p.IW : (long long)p.OH * p.OW;
+  const bool vx = p.in_pitch * p.IH == px && in4(p.in_plane) && in4(p.in_img) && in4(px) && !((uintptr_t)p.in & 15u);
   const bool vw = p.w_m == 1 && in4(p.w_c) && in4(p.M) && !((uintptr_t)p.w & 15u);
-  if (p.M <= 32) return vx ? (vw ? launch_conv1_f32<1, true, true>(p, s) : launch_conv1_f32<1, true, false>(p, s))
-                           : (vw ? launch_conv1_f32<1, false, true>(p, s) : launch_conv1_f32<1, false, false>(p, s));
-  return vx ? (vw ? launch_conv1_f32<2, true, true>(p, s) : launch_conv1_f32<2, true, false>(p, s))
-            : (vw ? launch_conv1_f32<2, false, true>(p, s) : launch_conv1_f32<2, false, false>(p, s));
+  if (p.M <= 32) return vx ? (vw ? launch_conv1_f32<1, true, true, SPREAD>(p, s) : launch_conv1_f32<1, true, false, SPREAD>(p, s))
+                           : (vw ? launch_conv1_f32<1, false, true, SPREAD>(p, s) : launch_conv1_f32<1, false, false, SPREAD>(p, s));
+  return vx ? (vw ? launch_conv1_f32<2, true, true, SPREAD>(p, s) : launch_conv1_f32<2, true, false, SPREAD>(p, s))
+            : (vw ? launch_conv1_f32<2, false, true, SPREAD>(p, s) : launch_conv1_f32<2, false, false, SPREAD>(p, s));
 }
+template <bool DGRAD>
+int f32_k1_gemm(const GemmF32& p, cudaStream_t s) {
+  if (!DGRAD || (p.sh == 1 && p.sw == 1)) return run_conv1_f32<false>(p, s);
+  // the pixels between: zeroed in front.  Written along by the kernel, one by one, they took most of its time for few tiles
+  // (168 -> 33 channels, 27 x 22, stride 3: 39 us)
+  if (!p.accumulate && cudaMemsetAsync(p.out, 0, (size_t)p.NI * p.out_img * 4, s) != cudaSuccess) { cudaGetLastError(); return AD_ERR_CUDA; }
+  return run_conv1_f32<true>(p, s);
+}
+template int f32_k1_gemm<false>(const GemmF32&, cudaStream_t);
+template int f32_k1_gemm<true>(const GemmF32&, cudaStream_t);
 
 }  // namespace adk

@@ -32,8 +32,8 @@ uint32_t f32_cluster_size(Held held, unsigned long long tiles, uint32_t steps, u
 // measured 1.1 us alone, 1.9 beside one other, 2.7 beside two), and the SM with the most of them counts.  A cluster stays
 // within one group of SMs, so that larger ones are spread less evenly: 36 clusters of 4 leave some SMs two CTAs (filter gradient
 // 64 -> 64, 4 x 112 x 112: 184 us, 32 clusters of 4 133), and so do 16 of 8 already (half of the SMs were idle).
-inline double f32_k3_share(unsigned long long ctas, uint32_t cs, uint32_t sms) {
-  static const double per_stage[4] = {0, 1.2, 2.1, 3.0};
+inline double f32_k3_share(unsigned long long ctas, uint32_t cs, uint32_t sms, double one, double two) {
+  const double per_stage[4] = {0, one, two, 3.0};
   const double even = (double)ctas * (cs >= 8 ? 1.15 : cs >= 4 ? 1.1 : cs == 2 ? 1.02 : 1.0) / sms;
   return per_stage[even > 2 ? 3 : even > 1 || (cs >= 8 && even > 0.5) ? 2 : ctas ? 1 : 0];
 }
@@ -44,7 +44,7 @@ uint32_t f32_k3_cluster(Held held, unsigned long long tiles, uint32_t steps, uin
   for (uint32_t cs = 1; cs <= most && (cs == 1 || steps >= 2 * cs); cs *= 2) {
     const unsigned long long h = held(cs);
     if (!h) continue;
-    const double cost = (steps + cs - 1) / cs * (tiles / h * f32_k3_share(h * cs, cs, sms) + f32_k3_share(tiles % h * cs, cs, sms)) + 0.75 * cs;
+    const double cost = (steps + cs - 1) / cs * (tiles / h * f32_k3_share(h * cs, cs, sms, 1.2, 2.1) + f32_k3_share(tiles % h * cs, cs, sms, 1.2, 2.1)) + 0.75 * cs;
     // a CTA sums over 128 stages (256 channels) at most where that can be: the sum of its running sums loses precision with
     // their number (371 channels in one CTA: 2.0e-7 against 1.7e-7 in two)
     if (!best || cost < best_cost || (steps > 128 * best)) { best = cs; best_cost = cost; }
@@ -52,19 +52,32 @@ uint32_t f32_k3_cluster(Held held, unsigned long long tiles, uint32_t steps, uin
   return best ? best : 1;
 }
 
+// Blocks of 4 x 2 pixels of the 3x3 kernels in an image: a map under dilation falls into dh x dw maps without
+inline unsigned long long f32_k3_blocks(uint32_t OH, uint32_t OW, uint32_t dh, uint32_t dw) {
+  return (unsigned long long)(((OH + dh - 1) / dh + 3) / 4) * (((OW + dw - 1) / dw + 1) / 2) * dh * dw;
+}
+// Segments of up to 8 pixels of a row
+inline uint32_t f32_k3_segments(uint32_t Q, uint32_t dw) { return ((Q + dw - 1) / dw + 7) / 8 * dw; }
+
 // Filter gradient of the 3x3 kernels: CTAs of a cluster x slices of the grid that share a tile's `all` stages of pixels
 struct F32Split { uint32_t cs, slices; };
-inline F32Split f32_k3_split(unsigned long long tiles, unsigned long long all, uint32_t sms) {
-  static const unsigned held[4] = {444, 222, 104, 48};      // clusters of 1, 2, 4, 8 CTAs, three CTAs per SM
+// A stage takes 3.0 us alone, 4.8 beside one other, 7.0 beside two: the most CTAs that are resident together win, up to what
+// their start, and writing and adding the slices' `words` (the gradient's size), cost.  The constants are a fit to 1000 times of
+// 40 layers: the choice is on average 1.6 % above the fastest (7.6 % with the forward kernels' ones: 256 -> 256, 4 x 14 x 14
+// 52 -> 44 us, 191 -> 75, 3 x 71 x 10 68 -> 54).  The slices' scratch stays within 32 MB.
+inline F32Split f32_k3_split(unsigned long long tiles, unsigned long long all, unsigned long long words, uint32_t sms, uint32_t per_sm) {
+  // clusters of 1, 2, 4, 8 CTAs at a time, two or three CTAs per SM
+  static const unsigned held2[4] = {296, 148, 70, 33}, held3[4] = {444, 222, 104, 48}, *const held = per_sm == 2 ? held2 : held3;
   F32Split best = {1, 1};
   double best_cost = 0;
   for (uint32_t i = 0; i < 4; ++i)
     for (uint32_t sl = 1; sl <= 16; ++sl) {
       const uint32_t cs = 1u << i, parts = cs * sl;
-      if (parts > 1 && all < 2ull * parts) break;
+      if ((parts > 1 && all < 2ull * parts) || (sl > 1 && sl * words > (8ull << 20))) break;
       const unsigned long long h = held[i], n = tiles * sl;
-      const double cta = (double)((all + parts - 1) / parts) + 2 + 0.25 * cs;
-      const double cost = cta * (n / h * f32_k3_share(h * cs, cs, sms) + f32_k3_share(n % h * cs, cs, sms)) + (sl > 1 ? 3 + 0.3 * sl : 0);
+      const double cta = (double)((all + parts - 1) / parts) + 1.75 + 0.5 * cs;
+      const double cost = cta * (n / h * f32_k3_share(h * cs, cs, sms, 1.8, 2.35) + f32_k3_share(n % h * cs, cs, sms, 1.8, 2.35)) +
+                          (sl > 1 ? 2.1 + (0.1 + 0.63e-6 * words) * sl : 0);
       if (best_cost == 0 || cost < best_cost) { best = {cs, sl}; best_cost = cost; }
     }
   return best;

@@ -121,14 +121,16 @@ def test_data_gradient_of_more_than_2_32_elements():
 
 
 K1_CASES = [
-    # N, C, H, W, K of 1x1 layers: both directions
-    (1, 17, 1, 1, 17),             # one pixel, the smallest channel counts of the 1x1 kernels
-    (1, 32, 2, 2, 33),             # one vector of pixels; a row past the 32-row tile, filters of the gradient one by one
-    (3, 31, 5, 13, 64),            # planes of 65 pixels: gathers one by one; a channel short of two stages
-    (2, 65, 6, 22, 36),            # vectors that cross rows, images that share a tile; a row past the 64-row tile
-    (1, 130, 9, 12, 24),           # 32-row tiles, reduction split over a cluster
-    (5, 48, 16, 20, 148),          # running sums that restart, three tiles of rows
-    (1, 2100, 8, 8, 20),           # the largest clusters, shares of unequal length
+    # N, C, H, W (of x), K, stride of 1x1 layers: both directions
+    (1, 17, 1, 1, 17, 1),          # one pixel, the smallest channel counts of the 1x1 kernels
+    (1, 32, 2, 2, 33, 1),          # one vector of pixels; a row past the 32-row tile, filters of the gradient one by one
+    (3, 31, 5, 13, 64, 1),         # planes of 65 pixels: gathers one by one; a channel short of two stages
+    (2, 65, 6, 22, 36, 1),         # vectors that cross rows, images that share a tile; a row past the 64-row tile
+    (1, 130, 9, 12, 24, 1),        # 32-row tiles, reduction split over a cluster
+    (5, 48, 16, 20, 148, 1),       # running sums that restart, three tiles of rows
+    (1, 2100, 8, 8, 20, 1),        # the largest clusters, shares of unequal length
+    (2, 33, 15, 16, 40, 2),        # 8 x 8 planes of dy: vectors; rows and columns between and past the last that belong to no pixel
+    (3, 20, 16, 20, 65, 3),        # 6 x 7
 ]
 
 
@@ -138,63 +140,73 @@ def test_conv_f32_1x1(case, pitched, monkeypatch):
     """The 1x1 kernels at the edges of their tiles, vectors and splits; dense planes and padded ones; operands off by four bytes."""
     import torch
     monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", "1")
-    N, Cc, Hh, W, K = case
+    N, Cc, Hh, W, K, s = case
+    P, Q = (Hh - 1) // s + 1, (W - 1) // s + 1
     x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, 1, 1), float(np.sqrt(2.0 / Cc))), H.normal(3, (K,))
-    dy = H.uniform(4, (N, K, Hh, W))
-    y_w = np.einsum("nchw,kc->nkhw", x.astype(np.float64), w[:, :, 0, 0].astype(np.float64)) + b[None, :, None, None]
-    dx_w = np.einsum("nkhw,kc->nchw", dy.astype(np.float64), w[:, :, 0, 0].astype(np.float64)) + 1.0
+    dy = H.uniform(4, (N, K, P, Q))
+    y_w = np.einsum("nchw,kc->nkhw", x[:, :, ::s, ::s].astype(np.float64), w[:, :, 0, 0].astype(np.float64)) + b[None, :, None, None]
+    add = float(pitched)             # the padded form accumulates, into ones
+    dx_w, mag_x = np.full(x.shape, add), np.full(x.shape, add)
+    dx_w[:, :, ::s, ::s] += np.einsum("nkhw,kc->nchw", dy.astype(np.float64), w[:, :, 0, 0].astype(np.float64))
+    mag_x[:, :, ::s, ::s] += np.einsum("nkhw,kc->nchw", np.abs(dy), np.abs(w[:, :, 0, 0]))
     # a sum of n products, |terms| t: running sums of 64 and n / 64 partial sums round at 2^-24 of what they hold
     eps = lambda n: (min(n, 64) + n // 64 + 4) * 2.0 ** -24  # noqa: E731
     L = abi.lib()
-    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, 1, 1, 1, 0)
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, 1, s, 1, 0)
     flat = torch.empty(x.size + 1, device="cuda")
     xd = flat[pitched:pitched + x.size].view(x.shape).copy_(H.dev(x))          # one off: no longer 16-byte aligned
     wflat = torch.empty(w.size + 1, device="cuda")
     wd = wflat[pitched:pitched + w.size].view(w.shape).copy_(H.dev(w))
     bd = H.dev(b)
-    ph, pw = Hh + pitched, W + 3 * pitched
+    ph, pw = P + pitched, Q + 3 * pitched
     y, gy = torch.full((N, K, ph, pw), 7.0, device="cuda"), torch.full((N, K, ph, pw), float("nan"), device="cuda")
-    gy[:, :, :Hh, :W] = H.dev(dy)
+    gy[:, :, :P, :Q] = H.dev(dy)
     dx = torch.ones(x.shape, device="cuda")
     a.x, a.w, a.bias, a.y, a.y_pitch, a.y_plane = xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), y.data_ptr(), pw, ph * pw
     abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
-    a.y, a.dx, a.accumulate = gy.data_ptr(), dx.data_ptr(), 1
+    a.y, a.dx, a.accumulate = gy.data_ptr(), dx.data_ptr(), pitched
     abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
-    mag_y = np.einsum("nchw,kc->nkhw", np.abs(x), np.abs(w[:, :, 0, 0])) + np.abs(b)[None, :, None, None]
-    mag_x = np.einsum("nkhw,kc->nchw", np.abs(dy), np.abs(w[:, :, 0, 0])) + 1.0
-    assert (np.abs(y[:, :, :Hh, :W].cpu().numpy() - y_w) <= eps(Cc) * mag_y).all()
+    mag_y = np.einsum("nchw,kc->nkhw", np.abs(x[:, :, ::s, ::s]), np.abs(w[:, :, 0, 0])) + np.abs(b)[None, :, None, None]
+    assert (np.abs(y[:, :, :P, :Q].cpu().numpy() - y_w) <= eps(Cc) * mag_y).all()
     assert (np.abs(dx.cpu().numpy() - dx_w) <= eps(K) * mag_x).all()
-    assert (y[:, :, Hh:] == 7).all() and (y[:, :, :, W:] == 7).all()
+    assert (y[:, :, P:] == 7).all() and (y[:, :, :, Q:] == 7).all()
 
 
 K3_CASES = [
-    # N, C, H, W (of x), K, pad: 3x3, stride and dilation 1
-    (1, 16, 3, 3, 17, 0),          # one output pixel; the smallest channel counts of the 3x3 kernels
-    (1, 17, 6, 4, 33, 0),          # one block of 4 x 2 pixels; a channel past a pair of stages, a row past the 32-row tile
-    (3, 20, 11, 13, 64, 1),        # blocks past both edges, implicit padding, images that share a tile
-    (2, 33, 10, 17, 65, 2),        # padding of 2: the gradient's map is smaller than y; a row past the 64-row tile
-    (1, 130, 9, 12, 24, 1),        # 32-row tiles, reduction split over a cluster; rows of 12 = 8 + 4 pixels
-    (5, 48, 18, 19, 80, 1),        # running sums that restart, 19 = 8 + 8 + 3 pixels
-    (1, 300, 23, 25, 40, 0),       # more than 256 channels per CTA of a cluster of one
-    (4, 64, 58, 61, 32, 0),        # filter gradient in clusters and slices of the scratch
+    # N, C, H, W (of x), K, pad, stride, dilation of 3x3 layers
+    (1, 16, 3, 3, 17, 0, 1, 1),          # one output pixel; the smallest channel counts of the 3x3 kernels
+    (1, 17, 6, 4, 33, 0, 1, 1),          # one block of 4 x 2 pixels; a channel past a pair of stages, a row past the 32-row tile
+    (3, 20, 11, 13, 64, 1, 1, 1),        # blocks past both edges, implicit padding, images that share a tile
+    (2, 33, 10, 17, 65, 2, 1, 1),        # padding of 2: the gradient's map is smaller than y; a row past the 64-row tile
+    (1, 130, 9, 12, 24, 1, 1, 1),        # 32-row tiles, reduction split over a cluster; rows of 12 = 8 + 4 pixels
+    (5, 48, 18, 19, 80, 1, 1, 1),        # running sums that restart, 19 = 8 + 8 + 3 pixels
+    (1, 300, 23, 25, 40, 0, 1, 1),       # more than 256 channels per CTA of a cluster of one
+    (4, 64, 58, 61, 32, 0, 1, 1),  # filter gradient in clusters and slices of the scratch
+    (1, 16, 3, 3, 17, 0, 2, 1),    # one output pixel of stride 2
+    (2, 33, 18, 18, 96, 0, 2, 1),  # 8 x 8 pixels; a row and a column of x that no tap meets
+    (3, 21, 17, 33, 64, 1, 2, 1),  # 9 x 17: blocks past both edges, rows of 8 + 8 + 1 pixels, implicit padding
+    (4, 40, 39, 49, 30, 2, 2, 1),  # 32-row tiles of stride 2; padding of 2
+    (2, 20, 20, 21, 64, 2, 1, 2),  # 20 x 21 under dilation 2: maps of 10 x 11 and 10 x 10
+    (1, 30, 16, 27, 24, 0, 1, 3),  # 10 x 21: 4, 3 and 3 rows
+    (2, 18, 24, 32, 70, 4, 1, 4),  # 24 x 32
 ]
 
 
 @pytest.mark.parametrize("scratch", [True, False])
 @pytest.mark.parametrize("case", K3_CASES)
 def test_conv_f32_3x3(case, scratch, monkeypatch):
-    """The 3x3 kernels at the edges of their tiles, blocks, segments and splits; infinities stay where they have a weight."""
+    """The 3x3 kernels at the edges of their tiles, blocks, segments and splits, with strides and dilations; infinities stay where they have a weight."""
     import torch
     monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", "1")
-    N, Cc, Hh, W, K, pd = case
+    N, Cc, Hh, W, K, pd, s, d = case
     x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, 3, 3), float(np.sqrt(2.0 / (9 * Cc)))), H.normal(3, (K,))
-    y_w = orc.conv2d_fprop(x, w, b, (1, 1), (1, 1), (pd, pd), omp=True)
+    y_w = orc.conv2d_fprop(x, w, b, (s, s), (d, d), (pd, pd), omp=True)
     dy = H.uniform(4, y_w.shape)
-    dx_w = orc.conv2d_dgrad(dy, w, x.shape, (1, 1), (1, 1), (pd, pd), omp=True)
+    dx_w = orc.conv2d_dgrad(dy, w, x.shape, (s, s), (d, d), (pd, pd), omp=True)
     db_w = np.zeros(K, np.float32)
-    dw_w = orc.conv2d_wgrad(x, dy, w.shape, (1, 1), (1, 1), (pd, pd), db=db_w, omp=True)
+    dw_w = orc.conv2d_wgrad(x, dy, w.shape, (s, s), (d, d), (pd, pd), db=db_w, omp=True)
     L = abi.lib()
-    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, 3, 1, 1, pd)
+    a = conv_args(abi.AD_F32, abi.AD_NCHW, x.shape, K, 3, s, d, pd)
     P, Q = y_w.shape[2:]
     y, gy = torch.full((N, K, P + 1, Q + 3), 7.0, device="cuda"), torch.full((N, K, P + 1, Q + 3), float("nan"), device="cuda")
     gy[:, :, :P, :Q] = H.dev(dy)
@@ -228,8 +240,8 @@ def test_conv_f32_3x3(case, scratch, monkeypatch):
     taps = np.zeros((Cc, 3, 3), bool)
     for i in range(3):
         for j in range(3):
-            oy, ox = iy + pd - i, ix + pd - j
-            if 0 <= oy < P and 0 <= ox < Q:
-                hit[n, oy, ox] = taps[c, i, j] = True
+            oy, ox = iy + pd - i * d, ix + pd - j * d
+            if 0 <= oy < P * s and 0 <= ox < Q * s and oy % s == 0 and ox % s == 0:
+                hit[n, oy // s, ox // s] = taps[c, i, j] = True
     assert np.array_equal(~np.isfinite(H.host(y)[:, :, :P, :Q]).all(1), hit)
     assert np.array_equal(~np.isfinite(H.host(dw)).all(0), taps)
