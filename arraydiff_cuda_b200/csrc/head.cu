@@ -234,166 +234,201 @@ static int avg_params(const ad_tensor4* x, const ad_tensor4* y, uint32_t kh, uin
 }
 
 // ------------------------------------------------------------------ fully connected
-// The weights (fp32) are the traffic: every kernel reads them for 8 images at a time.  64 x 2048 -> 1000: forward 73 -> 49,
-// data gradient 75 -> 53, weight gradient 116 -> 25 us (beside the other strip's, which reads the same memory system).
+// Each kernel reads the fp32 weights for 8 images (the weight gradient x for 8 rows) at a time, four features per thread and
+// load: a warp meets 128 products with every 12 loads forward, 32 with 3 in the gradients, so that neither loads nor
+// shared memory bound them but the latency of a chain of loads, which more warps and loads in flight cut.  With a product per
+// read of shared memory (forward), one chain over all rows per column (data gradient) and one load at a time (weight
+// gradient), 64 x 2048 -> 1000 took 37, 40 and 19 us, 4 x 512 -> 1000 6, 39 and 6; now 15, 15 and 12, 5, 13 and 5 (5 of them the
+// launch).  Sums over 62 rows and 16 warps are also closer than a chain over 1000: 5.7e-7 -> 1.6e-7 against 64 bits.
+// VEC: rows are multiples of four elements and aligned: 16-byte loads of weights; else a thread's four features are 32 apart.
 constexpr uint32_t kLinB = 8;
 static unsigned lin_groups(uint32_t n, uint32_t per) { const uint32_t g = n / per + (n % per != 0); return g > 65535 ? 65535 : g; }
-// y[b][o] = bias[o] + sum_i x[b][i] * w[o][i]: one warp per output and 8 images, lanes stride over i, shuffle sums; the 8
-// images lie in shared memory as fp32 (1024 features at a time), read by the 8 warps of the block
-constexpr uint32_t kFwdI = 1024;
-template <typename T>
+// a thread's four features of the 128 from c0 on
+template <bool VEC> __device__ __forceinline__ uint32_t lin_col(uint32_t c0, uint32_t lane, uint32_t e) { return c0 + (VEC ? lane * 4 + e : lane + e * 32); }
+template <typename T, bool VEC>
+__device__ __forceinline__ void lin_ld4(const T* row, uint32_t c0, uint32_t lane, uint32_t I, bool have, float (&v)[4]) {
+  if (VEC) {
+    const uint32_t c = c0 + lane * 4;
+    if (sizeof(T) == 4) {
+      const float4 q = have && c < I ? *(const float4*)(row + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+      const uint2 q = have && c < I ? *(const uint2*)(row + c) : make_uint2(0u, 0u);
+      v[0] = __uint_as_float(q.x << 16); v[1] = __uint_as_float(q.x & 0xffff0000u);
+      v[2] = __uint_as_float(q.y << 16); v[3] = __uint_as_float(q.y & 0xffff0000u);
+    }
+  } else {
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) { const uint32_t c = lin_col<false>(c0, lane, e); v[e] = have && c < I ? ld_f(row + c) : 0.f; }
+  }
+}
+// y[b][o] = bias[o] + sum_i x[b][i] * w[o][i]: a warp for four outputs and 8 images, its lanes along i; the 32 sums over the
+// lanes in 31 exchanges, after which a lane holds one
+template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) linear_fwd_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
                                                          const float* __restrict__ w, const float* __restrict__ bias, T* y) {
   grid_dependency();
-  __shared__ float xs[kLinB][kFwdI];
-  const uint32_t o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const uint32_t o0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 4, lane = threadIdx.x & 31;
+  if (o0 >= O) return;
   for (uint32_t b0 = blockIdx.y * kLinB; b0 < B; b0 += gridDim.y * kLinB) {
     const uint32_t nb = B - b0 < kLinB ? B - b0 : kLinB;
-    float acc[kLinB];
+    float acc[32];                      // [output][image]
 #pragma unroll
-    for (uint32_t j = 0; j < kLinB; ++j) acc[j] = 0.f;
-    for (uint32_t i0 = 0; i0 < I; i0 += kFwdI) {
-      const uint32_t ni = I - i0 < kFwdI ? I - i0 : kFwdI;
-      __syncthreads();
-      for (uint32_t j = 0; j < kLinB; ++j)
-        for (uint32_t i = threadIdx.x; i < ni; i += 256) xs[j][i] = j < nb ? ld_f(x + (size_t)(b0 + j) * I + i0 + i) : 0.f;
-      __syncthreads();
-      if (o < O) {
-        const float* wr = w + (size_t)o * I + i0;
-        uint32_t i = lane;
-        for (; i + 7 * 32 < ni; i += 8 * 32) {
-          float wv[8];
+    for (int k = 0; k < 32; ++k) acc[k] = 0.f;
+#pragma unroll 2
+    for (uint32_t c0 = 0; c0 < I; c0 += 128) {
+      float wv[4][4], xv[kLinB][4];
 #pragma unroll
-          for (int u = 0; u < 8; ++u) wv[u] = wr[i + u * 32];
+      for (uint32_t o = 0; o < 4; ++o) lin_ld4<float, VEC>(w + (size_t)(o0 + o) * I, c0, lane, I, o0 + o < O, wv[o]);
 #pragma unroll
-          for (int u = 0; u < 8; ++u)
+      for (uint32_t j = 0; j < kLinB; ++j) lin_ld4<T, VEC>(x + (size_t)(b0 + j) * I, c0, lane, I, j < nb, xv[j]);
 #pragma unroll
-            for (uint32_t j = 0; j < kLinB; ++j) acc[j] = fmaf(xs[j][i + u * 32], wv[u], acc[j]);
-        }
-        for (; i < ni; i += 32) {
-          const float wv = wr[i];
+      for (int e = 0; e < 4; ++e)
 #pragma unroll
-          for (uint32_t j = 0; j < kLinB; ++j) acc[j] = fmaf(xs[j][i], wv, acc[j]);
-        }
+        for (int o = 0; o < 4; ++o)
+#pragma unroll
+          for (uint32_t j = 0; j < kLinB; ++j) acc[o * 8 + j] = fmaf(xv[j][e], wv[o][e], acc[o * 8 + j]);
+    }
+#pragma unroll
+    for (int n = 16; n >= 1; n >>= 1) {
+      const bool up = lane & n;
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        const float other = __shfl_xor_sync(0xffffffffu, up ? acc[k] : acc[k + n], n);
+        acc[k] = (up ? acc[k + n] : acc[k]) + other;
       }
     }
-    if (o < O) {
-#pragma unroll
-      for (uint32_t j = 0; j < kLinB; ++j) {
-        const float v = warp_sum(acc[j]);
-        if (lane == 0 && j < nb) st_f(y + (size_t)(b0 + j) * O + o, v + (bias ? bias[o] : 0.f));
-      }
-    }
+    const uint32_t o = o0 + lane / 8, j = lane % 8;
+    if (o < O && j < nb) st_f(y + (size_t)(b0 + j) * O + o, acc[0] + (bias ? bias[o] : 0.f));
   }
 }
-// dx[b][i] (+)= sum_o dy[b][o] * w[o][i]: a thread owns a column i and 8 images and adds the rows o in order; weights come
-// through a ring of asynchronous copies (96 rows ahead), the gradients of the 8 images from shared memory
-constexpr uint32_t kDxCols = 128, kDxRows = 32, kDxStages = 4, kDxMaxO = 1024;
-template <typename T>
-__global__ void __launch_bounds__(kDxCols) linear_dx_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ dy,
-                                                            const float* __restrict__ w, T* dx, int accumulate) {
+// dx[b][i] (+)= sum_o dy[b][o] * w[o][i]: 16 warps share the rows o of 128 columns and 8 images, every 16th each; their sums are
+// added in order.  The gradients of the 8 images lie in shared memory, 1024 rows at a time.
+constexpr uint32_t kDxWarps = 16, kDxMaxO = 1024;
+constexpr int kDxSmem = (kDxMaxO * kLinB + kDxWarps * 32 * 32) * 4;
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(kDxWarps * 32) linear_dx_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ dy,
+                                                                  const float* __restrict__ w, T* dx, int accumulate) {
   grid_dependency();
   extern __shared__ __align__(16) float lin_sm[];
-  float* const ring = lin_sm;                                      // [stage][row][column]
-  float* const g = lin_sm + kDxStages * kDxRows * kDxCols;         // [row][image]
-  const uint32_t tx = threadIdx.x, i = blockIdx.x * kDxCols + tx;
-  const uint32_t bytes = i < I ? 4u : 0u;
+  float* const g = lin_sm;                                         // [row][image]
+  float* const part = lin_sm + kDxMaxO * kLinB;                    // [warp][image, column of four][lane]
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = blockIdx.x * 128;
   for (uint32_t b0 = blockIdx.y * kLinB; b0 < B; b0 += gridDim.y * kLinB) {
     const uint32_t nb = B - b0 < kLinB ? B - b0 : kLinB;
-    float acc[kLinB];
+    float acc[kLinB][4];
 #pragma unroll
-    for (uint32_t j = 0; j < kLinB; ++j) acc[j] = 0.f;
+    for (uint32_t j = 0; j < kLinB; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
     for (uint32_t oc = 0; oc < O; oc += kDxMaxO) {
-      const uint32_t no = O - oc < kDxMaxO ? O - oc : kDxMaxO, steps = (no + kDxRows - 1) / kDxRows;
+      const uint32_t no = O - oc < kDxMaxO ? O - oc : kDxMaxO;
       __syncthreads();
-      auto load = [&](uint32_t st) {
-        float* d = ring + (st % kDxStages) * kDxRows * kDxCols + tx;
-#pragma unroll 8
-        for (uint32_t r = 0; r < kDxRows; ++r) {
-          const uint32_t o = st * kDxRows + r;
-          const float* src = w + (size_t)(oc + (o < no ? o : 0)) * I + (i < I ? i : 0);
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(d + r * kDxCols)), "l"(src),
-                       "r"(o < no ? bytes : 0u) : "memory");
-        }
-      };
-      for (uint32_t st = 0; st < kDxStages - 1; ++st) {
-        if (st < steps) load(st);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-      }
-      for (uint32_t j = 0; j < kLinB; ++j)
-        for (uint32_t o = tx; o < steps * kDxRows; o += kDxCols)
-          g[o * kLinB + j] = j < nb && o < no ? ld_f(dy + (size_t)(b0 + j) * O + oc + o) : 0.f;
-      for (uint32_t st = 0; st < steps; ++st) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kDxStages - 2) : "memory");
-        __syncthreads();
-        if (st + kDxStages - 1 < steps) load(st + kDxStages - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        const float* wr = ring + (st % kDxStages) * kDxRows * kDxCols + tx;
-        const float* gr = g + st * kDxRows * kLinB;
-        const uint32_t rows = no - st * kDxRows < kDxRows ? no - st * kDxRows : kDxRows;
-#pragma unroll 8
-        for (uint32_t r = 0; r < rows; ++r) {
-          const float wv = wr[r * kDxCols];
-          const float4 g0 = *(const float4*)(gr + r * kLinB), g1 = *(const float4*)(gr + r * kLinB + 4);
-          const float gv[kLinB] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
-          for (uint32_t j = 0; j < kLinB; ++j) acc[j] = fmaf(gv[j], wv, acc[j]);
-        }
+      for (uint32_t j = 0; j < kLinB; ++j)
+        for (uint32_t o = threadIdx.x; o < no; o += kDxWarps * 32) g[o * kLinB + j] = j < nb ? ld_f(dy + (size_t)(b0 + j) * O + oc + o) : 0.f;
+      __syncthreads();
+#pragma unroll 8
+      for (uint32_t o = warp; o < no; o += kDxWarps) {
+        float wv[4];
+        lin_ld4<float, VEC>(w + (size_t)(oc + o) * I, c0, lane, I, true, wv);
+        const float4 g0 = *(const float4*)(g + o * kLinB), g1 = *(const float4*)(g + o * kLinB + 4);
+        const float gv[kLinB] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+        for (uint32_t j = 0; j < kLinB; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[j][e] = fmaf(gv[j], wv[e], acc[j][e]);
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
-    if (i < I) {
 #pragma unroll
-      for (uint32_t j = 0; j < kLinB; ++j)
-        if (j < nb) {
-          T* d = dx + (size_t)(b0 + j) * I + i;
-          st_f(d, accumulate ? ld_f(d) + acc[j] : acc[j]);
-        }
+    for (uint32_t j = 0; j < kLinB; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) part[(warp * 32 + j * 4 + e) * 32 + lane] = acc[j][e];
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < 32 * 32; t += kDxWarps * 32) {
+      const uint32_t j = t >> 7, e = (t >> 5) & 3, i = lin_col<VEC>(c0, t & 31, e);
+      if (j >= nb || i >= I) continue;
+      float v = 0.f;
+#pragma unroll
+      for (uint32_t q = 0; q < kDxWarps; ++q) v += part[q * 32 * 32 + t];
+      T* d = dx + (size_t)(b0 + j) * I + i;
+      st_f(d, accumulate ? ld_f(d) + v : v);
     }
   }
 }
-constexpr int kDxSmem = (kDxStages * kDxRows * kDxCols + kDxMaxO * kLinB) * 4;
-// dw[o][i] (+)= sum_b dy[b][o] * x[b][i]; db[o] (+)= sum_b dy[b][o]: one thread per (8 rows o, i), batch in order; the 8
+// dw[o][i] (+)= sum_b dy[b][o] * x[b][i]; db[o] (+)= sum_b dy[b][o]: a thread for 8 rows o and four columns i, batch in order; the 8
 // rows' gradients of 64 images at a time in shared memory
-template <typename T>
-__global__ void __launch_bounds__(256) linear_dw_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(128) linear_dw_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
                                                         const T* __restrict__ dy, float* dw, float* db, int accumulate) {
   grid_dependency();
   __shared__ __align__(16) float g[64][8];
-  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+  const uint32_t lane = threadIdx.x & 31, c0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 128;
   for (uint32_t o0 = blockIdx.y * 8; o0 < O; o0 += gridDim.y * 8) {
     const uint32_t no = O - o0 < 8 ? O - o0 : 8;
-    float acc[8], accb[8], old[8];
+    float acc[8][4], accb = 0.f;
 #pragma unroll
-    for (uint32_t j = 0; j < 8; ++j) {
-      acc[j] = accb[j] = 0.f;
-      old[j] = accumulate && j < no && i < I ? dw[(size_t)(o0 + j) * I + i] : 0.f;
-    }
+    for (uint32_t k = 0; k < 8; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[k][e] = 0.f;
     for (uint32_t b0 = 0; b0 < B; b0 += 64) {
       const uint32_t nb = B - b0 < 64 ? B - b0 : 64;
       __syncthreads();
-      for (uint32_t t = threadIdx.x; t < nb * 8; t += 256) g[t >> 3][t & 7] = (t & 7) < no ? ld_f(dy + (size_t)(b0 + (t >> 3)) * O + o0 + (t & 7)) : 0.f;
+      for (uint32_t t = threadIdx.x; t < nb * 8; t += 128) g[t >> 3][t & 7] = (t & 7) < no ? ld_f(dy + (size_t)(b0 + (t >> 3)) * O + o0 + (t & 7)) : 0.f;
       __syncthreads();
-      if (i < I) {
+      if (db && blockIdx.x == 0 && threadIdx.x < 8) {
 #pragma unroll 8
-        for (uint32_t b = 0; b < nb; ++b) {
-          const float xv = ld_f(x + (size_t)(b0 + b) * I + i);
-          const float4 g0 = *(const float4*)&g[b][0], g1 = *(const float4*)&g[b][4];
+        for (uint32_t b = 0; b < nb; ++b) accb += g[b][threadIdx.x];
+      }
+      for (uint32_t b = 0; b < nb; b += 8) {
+        float xv[8][4];
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) {
+          const T* row = x + (size_t)(b0 + (b + r < nb ? b + r : b)) * I;      // past the last image and feature: others, not used
+          if (VEC) {
+            lin_ld4<T, VEC>(row, c0, lane, I, true, xv[r]);
+          } else {
+#pragma unroll
+            for (uint32_t e = 0; e < 4; ++e) xv[r][e] = ld_f(row + min(lin_col<false>(c0, lane, e), I - 1));
+          }
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < 8; ++r) {
+          if (b + r >= nb) break;
+          const float4 g0 = *(const float4*)&g[b + r][0], g1 = *(const float4*)&g[b + r][4];
           const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
 #pragma unroll
-          for (uint32_t j = 0; j < 8; ++j) { acc[j] = fmaf(gv[j], xv, acc[j]); accb[j] += gv[j]; }
+          for (uint32_t k = 0; k < 8; ++k)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[k][e] = fmaf(gv[k], xv[r][e], acc[k][e]);
         }
       }
     }
-    if (i < I) {
 #pragma unroll
-      for (uint32_t j = 0; j < 8; ++j)
-        if (j < no) {
-          dw[(size_t)(o0 + j) * I + i] = accumulate ? old[j] + acc[j] : acc[j];
-          if (db && i == 0) db[o0 + j] = accumulate ? db[o0 + j] + accb[j] : accb[j];
+    for (uint32_t k = 0; k < 8; ++k) {
+      if (k >= no) break;
+      float* d = dw + (size_t)(o0 + k) * I;
+      if (VEC) {
+        const uint32_t c = lin_col<true>(c0, lane, 0);
+        if (c < I) {
+          float4 v = make_float4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
+          if (accumulate) { const float4 old = *(const float4*)(d + c); v = make_float4(old.x + v.x, old.y + v.y, old.z + v.z, old.w + v.w); }
+          *(float4*)(d + c) = v;
         }
+      } else {
+#pragma unroll
+        for (uint32_t e = 0; e < 4; ++e) {
+          const uint32_t c = lin_col<false>(c0, lane, e);
+          if (c < I) d[c] = accumulate ? d[c] + acc[k][e] : acc[k][e];
+        }
+      }
     }
+    if (db && blockIdx.x == 0 && threadIdx.x < no) db[o0 + threadIdx.x] = accumulate ? db[o0 + threadIdx.x] + accb : accb;
   }
+}
+// rows of four elements per load: x and dx of `es` bytes each
+static bool lin_vec(uint32_t I, const void* w, const void* x, size_t es) {
+  return I % 4 == 0 && ((uintptr_t)w & 15u) == 0 && ((uintptr_t)x & (4 * es - 1)) == 0;
 }
 
 }  // namespace adk
@@ -438,25 +473,26 @@ extern "C" int ad_linear_fwd(int32_t dtype, uint32_t batch, uint32_t in_features
   if (!x || !w || !y) return AD_ERR_BAD_ARG;
   if ((size_t)batch * out_features >= (1ull << 31) || (size_t)batch * in_features >= (1ull << 31)) return AD_ERR_LIMIT;
   if (batch == 0 || out_features == 0) return AD_OK;
-  const dim3 grid((unsigned)(((size_t)out_features + 7) / 8), lin_groups(batch, kLinB));
-  AD_DISPATCH_DTYPE(dtype, (launch(linear_fwd_kernel<T>, grid, 256, 0, as_stream(stream), batch, in_features, out_features, (const T*)x, w, bias, (T*)y)));
+  const dim3 grid((unsigned)(((size_t)out_features + 31) / 32), lin_groups(batch, kLinB));
+  AD_DISPATCH_DTYPE(dtype, (launch(lin_vec(in_features, w, x, sizeof(T)) ? linear_fwd_kernel<T, true> : linear_fwd_kernel<T, false>, grid, 256, 0,
+                                   as_stream(stream), batch, in_features, out_features, (const T*)x, w, bias, (T*)y)));
   count_launch();
   return launch_status();
 }
 
-template <typename T>
+template <typename T, bool VEC>
 static int launch_linear_dx(uint32_t B, uint32_t I, uint32_t O, const T* dy, const float* w, T* dx, int accumulate, cudaStream_t s) {
   static unsigned attr_done = 0;       // one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(linear_dx_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDxSmem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(linear_dx_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDxSmem) != cudaSuccess) {
       cudaGetLastError();
       return AD_ERR_CUDA;
     }
     attr_done |= 1u << (dev & 31);
   }
-  launch(linear_dx_kernel<T>, dim3((I + kDxCols - 1) / kDxCols, lin_groups(B, kLinB)), kDxCols, kDxSmem, s, B, I, O, dy, w, dx, accumulate);
+  launch(linear_dx_kernel<T, VEC>, dim3((I + 127) / 128, lin_groups(B, kLinB)), kDxWarps * 32, kDxSmem, s, B, I, O, dy, w, dx, accumulate);
   return AD_OK;
 }
 
@@ -470,12 +506,16 @@ extern "C" int ad_linear_bwd(int32_t dtype, uint32_t batch, uint32_t in_features
   if (batch == 0) return AD_OK;
   cudaStream_t s = as_stream(stream);
   if (dx && in_features) {
-    AD_DISPATCH_DTYPE(dtype, { const int st = launch_linear_dx<T>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s); if (st != AD_OK) return st; });
+    AD_DISPATCH_DTYPE(dtype, {
+      const int st = lin_vec(in_features, w, w, sizeof(T)) ? launch_linear_dx<T, true>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s)
+                                                           : launch_linear_dx<T, false>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s);
+      if (st != AD_OK) return st;
+    });
     count_launch();
   }
   if (dw && in_features && out_features) {
-    const dim3 grid((in_features + 255) / 256, lin_groups(out_features, 8));
-    AD_DISPATCH_DTYPE(dtype, (launch(linear_dw_kernel<T>, grid, 256, 0, s, batch, in_features, out_features, (const T*)x, (const T*)dy, dw, db, accumulate_dw)));
+    const dim3 grid((in_features + 511) / 512, lin_groups(out_features, 8));
+    AD_DISPATCH_DTYPE(dtype, (launch(lin_vec(in_features, dw, x, sizeof(T)) ? linear_dw_kernel<T, true> : linear_dw_kernel<T, false>, grid, 128, 0, s, batch, in_features, out_features, (const T*)x, (const T*)dy, dw, db, accumulate_dw)));
     count_launch();
   }
   return launch_status();

@@ -398,7 +398,7 @@ def test_average_pool(layout, dtype, k, s):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
-@pytest.mark.parametrize("B,I,O", [(4, 512, 1000), (3, 70, 19)])
+@pytest.mark.parametrize("B,I,O", [(4, 512, 1000), (3, 70, 19), (9, 132, 33), (70, 516, 1030), (1, 1, 1)])
 def test_linear_layer(dtype, B, I, O):
     """y = x w^T + b and its three gradients against the numpy restatement."""
     x, w, b = H.normal(70, (B, I)), H.normal(71, (O, I), 0.05), H.normal(72, (O,))
