@@ -1100,8 +1100,9 @@ static int run_fwd_gemm(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, 
                         long long out_plane, const float* bias, int relu, int accumulate, int32_t* status,
                         cudaStream_t s, const ad_tensor4* add = nullptr) {
   if (CK % 64 != 0) return AD_ERR_UNSUPPORTED;
-  if (!getenv("ARRAYDIFF_B200_NO_ROW_KERNEL")) {
-    // 64-channel layers: the row-tile kernel fetches each activation patch once (conv_tc_row.cu)
+  if (!getenv("ARRAYDIFF_B200_NO_ROW_KERNEL") && !(add && OQ < 96)) {
+    // 64-channel layers: the row kernels fetch each activation patch once (conv_tc_row.cu); narrow maps with an addend stay with the
+    // general kernel, whose epilogue adds it
     int st = conv_tc_row_fwd(act, NI, IH, IW, CK, filt, OC, kh, kw, sh, sw, dh, dw, offy, offx, OP, OQ, out, out_pitch,
                              out_plane, bias, relu, accumulate, status, s);
     if (st != AD_ERR_UNSUPPORTED) {

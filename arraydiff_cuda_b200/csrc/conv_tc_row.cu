@@ -23,6 +23,7 @@ namespace adk {
 namespace tc {
 
 constexpr int kRowThreads = 192;
+constexpr int kStreamThreads = 320;      // the streaming kernel: two sets of epilogue warps
 constexpr uint32_t kTapBytes = 8192;  // one [64 out ch][64 in ch] filter tap, K-major SW128
 
 struct RowCtl {
@@ -309,19 +310,32 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
                        uint32_t OP, uint32_t OQ, void* out, long long out_pitch, long long out_plane, const float* bias,
                        int relu, int accumulate, int32_t* status, cudaStream_t s);
 
+// Images whose rows the streaming kernel lays side by side in a 128-pixel tile of a narrow map: the rows of 2, 4 or 8 with their
+// filter's reach fit it (a wider map leaves more of the tile unused than the general kernel's tiles do).  0: not that way, nor for
+// an output that the general kernel makes in one round of 128-pixel tiles: 6.6 us, the streaming kernel takes 7.3 to 8.4 for
+// those.  From two rounds on (3x3): 13.4 -> 8.9 us at 16 x 56 x 56, 10.2 -> 8.5 at 32 x 28 x 28; 1x1: 8.6 -> 7.6 at 64 x 28 x 56.
+static uint32_t stream_images(uint32_t NI, uint32_t OP, uint32_t OQ, uint32_t kw, uint32_t dw) {
+  if ((unsigned long long)NI * OP * OQ <= 128ull * kNumSMs) return 0;
+  uint32_t g = 0;
+  for (uint32_t t = 2; t <= 8 && OQ + (kw - 1) * dw <= 128 / t; t *= 2) g = t;
+  return g;
+}
+
 // Returns AD_ERR_UNSUPPORTED when the shape is outside what this variant serves, so that the
 // caller falls back to the general kernel.
 int conv_tc_row_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CK, const void* filt, uint32_t OC,
                     uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, int offy, int offx,
                     uint32_t OP, uint32_t OQ, void* out, long long out_pitch, long long out_plane, const float* bias,
                     int relu, int accumulate, int32_t* status, cudaStream_t s) {
-  if (sh != 1 || sw != 1 || CK != 64 || OC > 64 || OQ < 96) return AD_ERR_UNSUPPORTED;
+  if (sh != 1 || sw != 1 || CK != 64 || OC > 64) return AD_ERR_UNSUPPORTED;
+  if (OQ < 96 && !stream_images(NI, OP, OQ, kw, dw)) return AD_ERR_UNSUPPORTED;
   if (!getenv("ARRAYDIFF_B200_ROW_TILES")) {
     // the row-streaming kernel (below) serves every shape it can; the one-row tile kernel takes the rest
     int st = conv_tc_stream_fwd(act, NI, IH, IW, CK, filt, OC, kh, kw, sh, sw, dh, dw, offy, offx, OP, OQ, out, out_pitch,
                                 out_plane, bias, relu, accumulate, status, s);
     if (st != AD_ERR_UNSUPPORTED) return st;
   }
+  if (OQ < 96) return AD_ERR_UNSUPPORTED;
   const uint32_t taps = kh * kw;
   const uint32_t pw = (128 + (kw - 1) * dw + 7) / 8 * 8;
   if (pw > 256 || (kh - 1) * dh + 1 > 256 || taps > 16) return AD_ERR_UNSUPPORTED;
@@ -400,6 +414,12 @@ int conv_tc_row_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint
 // warps (bias / ReLU / bf16 / swizzled staging / one TMA tile store, as above) while later rows accumulate.  The
 // new row's slot must be overwritten, the older rows' slots accumulated: the first MMA of an input row is split
 // in two for that reason; an MMA whose slots would wrap around the ring is split at the wrap.
+// The bound, where it is not HBM, is an output row's way out: tensor memory, bias and ReLU, staging, store.  One set of four
+// warps took 1.46 us for it (waits that sleep, 64 loads of the bias, the slot and the staging buffer held to the end); two sets
+// with a buffer each take 0.42: 148 columns of 16 rows 29.8 -> 20.4 us, of 32 rows 53 -> 38 (24 at the copy rate).
+// Narrow maps: the rows of several images lie side by side in the tile (stream_images), each followed by its own filter
+// reach; what the MMAs make of the pixels in between is clipped by the store.  64 x 28 x 56, 3x3: 22.2 -> 11.5 us, 64 x 56 x 56
+// 36.7 -> 18.5 against the general kernel.
 // What the MMA thread needs to know about an input row, worked out by the producer thread when it fetches the row (one
 // record per stage, visible to the MMA thread through the stage's `full` barrier).  All descriptor entries are the low
 // 32-bit words (start address in 16-byte units); A and B share the high word.
@@ -420,6 +440,7 @@ struct StreamCtl {
   alignas(16) StreamRow row[8];
   uint32_t swait_bar[8], swait_par[8], ecount[8];   // producer thread only: what frees each stage, uses of empty[]
   unsigned long long full[8], empty[8], afull[8], aempty[8], wbar, stg_full[2], stg_free[2];
+  alignas(16) float bias[64];
   uint32_t tmem_base;
   volatile int abort_flag;
 };
@@ -429,6 +450,7 @@ struct StreamParams {
   uint32_t kh, kw, dh, dw;
   int32_t offy, offx;
   uint32_t tiles_x, pw, row_bytes, stages;
+  uint32_t images, load_bytes;         // images side by side in a tile, bytes of the row box
   uint32_t L, nchunks, items;
   long long out_pitch, out_plane;
   __nv_bfloat16* out;
@@ -457,7 +479,7 @@ __device__ __forceinline__ StreamItem stream_item(const StreamParams& p, uint32_
 }
 
 template <int KH, int KW>
-__global__ void __launch_bounds__(kRowThreads, 1)
+__global__ void __launch_bounds__(kStreamThreads, 1)
 conv_tc_stream_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           const __grid_constant__ CUtensorMap map_o, const StreamParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -500,6 +522,10 @@ conv_tc_stream_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   __syncthreads();
   tc_fence_after();
   grid_dependency();
+  if (warp >= 2 && p.bias) {      // both sets write the same values; a warp reads behind its own writes and the other's equal ones
+    for (uint32_t j = (uint32_t)lane; j < 64; j += 32) ctl->bias[j] = j < p.OC ? p.bias[j] : 0.f;
+    __syncwarp();
+  }
   const uint32_t tmem_base = ctl->tmem_base;
   volatile int* abortf = &ctl->abort_flag;
 
@@ -574,9 +600,9 @@ conv_tc_stream_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
             const uint4* src = (const uint4*)&r;
             dst[0] = src[0]; dst[1] = src[1]; dst[2] = src[2]; dst[3] = src[3];
             // the arrive below releases these stores to the thread that waits on the barrier
-            mbar_expect_tx(full, p.row_bytes);
+            mbar_expect_tx(full, p.load_bytes);
             tma_load_4d(smem_u32(psm + (size_t)stage * p.row_bytes), &map_a, full, 0, (int)(it.tx * 128) + p.offx,
-                        (int)(it.rho + (it.i0 + (uint32_t)j) * p.dh) + p.offy, (int)it.n);
+                        (int)(it.rho + (it.i0 + (uint32_t)j) * p.dh) + p.offy, (int)(it.n * p.images));
           }
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
@@ -671,39 +697,57 @@ conv_tc_stream_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       if (pend_s) umma_commit(pend_s);
     }
   } else {
-    const uint32_t q = (uint32_t)warp & 3u;
+    // two sets of four warps, every other output row each, with a staging buffer of its own
+    const uint32_t q = (uint32_t)warp & 3u, set = ((uint32_t)warp - 2u) >> 2;
     uint32_t tt = 0;
     bool go = true;
     for (uint32_t item = blockIdx.x; go && item < p.items && !*abortf; item += gridDim.x) {
       const StreamItem it = stream_item(p, item);
       if (it.Lc <= 0) continue;
       for (int32_t i = 0; i < it.Lc; ++i, ++tt) {
+        if ((tt & 1u) != set) continue;
         const uint32_t slot = tt & 7u;
         const uint32_t oy = it.rho + (it.i0 + (uint32_t)i) * p.dh, n = it.n, tx = it.tx;
         bool ok = mbar_wait_relaxed(smem_u32(&ctl->afull[slot]), (tt >> 3) & 1u, abortf);
         if (!__all_sync(0xffffffffu, ok)) { go = false; break; }
         tc_fence_after();
         if (p.tma_store) {
-          const uint32_t b = tt & 1u;
+          const uint32_t b = set;
           const uint32_t m = q * 32 + lane;
           uint8_t* stg = osm + (size_t)b * 16384;
-          if (tt >= 2) ok = mbar_wait_relaxed(smem_u32(&ctl->stg_free[b]), ((tt >> 1) - 1u) & 1u, abortf);
-          if (!__all_sync(0xffffffffu, ok)) { go = false; break; }   // leave together: the tensor-memory loads below are warp-wide
           {
             uint32_t v[64];
             const uint32_t taddr = tmem_base + ((q * 32u) << 16) + slot * 64u;
             tmem_ld32(taddr, *(uint32_t(*)[32])&v[0]);
             tmem_ld32(taddr + 32, *(uint32_t(*)[32])&v[32]);
             tmem_ld_wait();
+            // accumulator slot drained: hand it back to the MMA warp
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl->aempty[slot]));
             if (p.bias) {
 #pragma unroll
-              for (int j = 0; j < 64; ++j)
-                if ((uint32_t)j < p.OC) v[j] = __float_as_uint(__uint_as_float(v[j]) + p.bias[j]);
+              for (int j = 0; j < 64; j += 4) {
+                const float4 b4 = *(const float4*)&ctl->bias[j];
+                v[j] = __float_as_uint(__uint_as_float(v[j]) + b4.x);
+                v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + b4.y);
+                v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + b4.z);
+                v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + b4.w);
+              }
             }
             if (p.relu) {
 #pragma unroll
               for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.f));
             }
+            // the set's previous store has finished reading the staging buffer
+            if (tt >= 2) {
+              if (q == 0 && lane == 0) {
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                mbar_arrive(smem_u32(&ctl->stg_free[b]));
+              }
+              ok = mbar_wait(smem_u32(&ctl->stg_free[b]), ((tt >> 1) - 1u) & 1u, abortf);
+            }
+            if (!__all_sync(0xffffffffu, ok)) { go = false; break; }   // leave together: the next tensor-memory load is warp-wide
             uint8_t* srow = stg + m * 128u;
             const uint32_t m7 = m & 7u;
 #pragma unroll
@@ -716,24 +760,16 @@ conv_tc_stream_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
               *(uint4*)(srow + ((g8 ^ m7) * 16u)) = pk;
             }
           }
-          // accumulator slot drained: hand it back to the MMA warp
-          tc_fence_before();
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-          if (lane == 0) {
-            mbar_arrive(smem_u32(&ctl->aempty[slot]));
-            mbar_arrive(smem_u32(&ctl->stg_full[b]));
-          }
+          if (lane == 0) mbar_arrive(smem_u32(&ctl->stg_full[b]));
           if (q == 0 && lane == 0) {
             // on a failed wait the abort flag is up and every warp leaves at its next wait
-            if (mbar_wait_relaxed(smem_u32(&ctl->stg_full[b]), (tt >> 1) & 1u, abortf)) {
+            if (mbar_wait(smem_u32(&ctl->stg_full[b]), (tt >> 1) & 1u, abortf)) {
               asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(&map_o),
-                           "r"(smem_u32(stg)), "r"(0), "r"((int)(tx * 128)), "r"((int)oy), "r"((int)n)
+                           "r"(smem_u32(stg)), "r"(0), "r"((int)(tx * 128)), "r"((int)oy), "r"((int)(n * p.images))
                            : "memory");
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-              // every store but the newest has finished reading its staging buffer: free the other one
-              asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-              if (tt >= 1) mbar_arrive(smem_u32(&ctl->stg_free[b ^ 1u]));
             }
           }
           __syncwarp();
@@ -833,13 +869,15 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
                        uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, int offy, int offx,
                        uint32_t OP, uint32_t OQ, void* out, long long out_pitch, long long out_plane, const float* bias,
                        int relu, int accumulate, int32_t* status, cudaStream_t s) {
-  if (sh != 1 || sw != 1 || CK != 64 || OC > 64 || OQ < 96) return AD_ERR_UNSUPPORTED;
-  const uint32_t taps = kh * kw;
+  if (sh != 1 || sw != 1 || CK != 64 || OC > 64) return AD_ERR_UNSUPPORTED;
+  const uint32_t taps = kh * kw, images = OQ < 96 ? stream_images(NI, OP, OQ, kw, dw) : 1;
   const uint32_t pw = (128 + (kw - 1) * dw + 7) / 8 * 8;
-  if (pw > 256 || kh > 4 || taps > 16) return AD_ERR_UNSUPPORTED;
+  if (!images || pw > 256 || kh > 4 || taps > 16) return AD_ERR_UNSUPPORTED;
   const uint32_t row_bytes = pw * 128;
   const long long op_ = out_pitch ? out_pitch : (long long)OQ * OC, opl_ = out_plane ? out_plane : (long long)OP * OQ * OC;
   const bool tma_store = !accumulate && (OC & 7u) == 0 && !((uintptr_t)out & 15u) && (op_ % 8) == 0 && (opl_ % 8) == 0;
+  if (images > 1 && !tma_store) return AD_ERR_UNSUPPORTED;
+  const uint32_t groups = (NI + images - 1) / images;
   const long long avail = (long long)kMaxDynSmem - 1024 - (long long)sizeof(StreamCtl) - (long long)taps * kTapBytes -
                           (tma_store ? 2 * 16384 : 0);
   long long stages = avail / row_bytes;
@@ -849,8 +887,9 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
   p.NI = NI; p.OP = OP; p.OQ = OQ; p.OC = OC;
   p.kh = kh; p.kw = kw; p.dh = dh; p.dw = dw; p.offy = offy; p.offx = offx;
   p.tiles_x = (OQ + 127) / 128; p.pw = pw; p.row_bytes = row_bytes; p.stages = (uint32_t)stages;
-  stream_chunks(NI, p.tiles_x, dh, OP, kh, p.L, p.nchunks);
-  const unsigned long long items = (unsigned long long)NI * p.tiles_x * dh * p.nchunks;
+  p.images = images; p.load_bytes = images > 1 ? 16384u : row_bytes;
+  stream_chunks(groups, p.tiles_x, dh, OP, kh, p.L, p.nchunks);
+  const unsigned long long items = (unsigned long long)groups * p.tiles_x * dh * p.nchunks;
   if (items > 0xffffffffull) return AD_ERR_UNSUPPORTED;
   p.items = (uint32_t)items;
   p.out_pitch = op_; p.out_plane = opl_;
@@ -861,7 +900,7 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
   {
     uint64_t dims[4] = {CK, IW, IH, NI};
     uint64_t str[4] = {0, (uint64_t)CK * 2, (uint64_t)IW * CK * 2, (uint64_t)IH * IW * CK * 2};
-    uint32_t box[4] = {64, pw, 1, 1};
+    uint32_t box[4] = {64, images > 1 ? 128 / images : pw, 1, images};
     uint32_t es[4] = {1, 1, 1, 1};
     int st = make_tmap_bf16(&ma, act, 4, dims, str, box, es);
     if (st != AD_OK) return st;
@@ -878,7 +917,7 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
   if (tma_store) {
     uint64_t dims[4] = {OC, OQ, OP, NI};
     uint64_t str[4] = {0, (uint64_t)OC * 2, (uint64_t)p.out_pitch * 2, (uint64_t)p.out_plane * 2};
-    uint32_t box[4] = {64, 128, 1, 1};
+    uint32_t box[4] = {64, 128 / images, 1, images};
     uint32_t es[4] = {1, 1, 1, 1};
     int st = make_tmap_bf16(&mo, out, 4, dims, str, box, es);
     if (st != AD_OK) return st;
@@ -892,7 +931,7 @@ int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, u
     cudaGetLastError();
     return AD_ERR_CUDA;
   }
-  launch(kern, grid, kRowThreads, smem, s, ma, mb, mo, p);
+  launch(kern, grid, kStreamThreads, smem, s, ma, mb, mo, p);
   count_launch();
   return launch_status();
 }

@@ -379,6 +379,55 @@ def test_conv_tc_row_kernels_agree_with_general_kernels(case, monkeypatch):
         assert H.max_rel(got, ref) < tol
 
 
+@pytest.mark.parametrize("case", [
+    # N, K, H, W (of x), filter, dilation, padding; more than 148 x 128 output pixels, 64 input channels
+    (39, 64, 11, 58, 3, 1, 0),     # pairs of images, the last alone; the gradient is 58 wide
+    (339, 64, 3, 58, 3, 1, 0),     # one output row per image
+    (150, 32, 11, 32, 3, 3, 0),    # four side by side, 26 + 6 pixels: no room left; the gradient in pairs
+    (103, 64, 14, 14, 3, 1, 1),    # eight side by side, implicit padding, the last seven
+    (41, 8, 14, 64, 3, 3, 0),      # 58 + 6: no room left; the gradient is too wide
+    (75, 64, 8, 32, 1, 1, 0),      # 1x1
+])
+def test_conv_tc_rows_of_several_images_in_a_tile(case, monkeypatch):
+    """Narrow maps in the streaming kernel, several images side by side, against the general kernel: both accumulate in fp32 and
+    round once.  Bias, ReLU and a padded output whose margins stay as they are; nothing leaks between neighbours: one
+    image is NaN."""
+    import torch
+    N, K, Hh, W, k, d, pd = case
+    x, w, b = H.uniform(1, (N, Hh, W, 64)), H.normal(2, (K, k, k, 64), (2.0 / (64 * k * k)) ** 0.5), H.normal(3, (K,))
+    L = abi.lib()
+    a = conv_args(abi.AD_BF16, abi.AD_NHWC, (N, 64, Hh, W), K, k, 1, d, pd)
+    P, Q = Hh + 2 * pd - d * (k - 1), W + 2 * pd - d * (k - 1)
+    xd, wd, bd = H.dev_bf16(x), H.dev_bf16(w), H.dev(b)
+    dy = H.dev_bf16(H.uniform(4, (N, P, Q, K)))
+    xd[N // 2] = float("nan")
+    dy[N // 2] = float("nan")
+    nscr = L.ad_conv2d_scratch_bytes(C.byref(a), 1)
+    scratch = torch.zeros(max(nscr, 16), dtype=torch.uint8, device="cuda")
+    a.scratch, a.scratch_bytes = scratch.data_ptr(), nscr
+    out, kinds = {}, {}
+    for mode in ("row", "general"):
+        monkeypatch.setenv("ARRAYDIFF_B200_NO_ROW_KERNEL", "1") if mode == "general" else monkeypatch.delenv("ARRAYDIFF_B200_NO_ROW_KERNEL", raising=False)
+        y = torch.full((N, P + 1, Q + 2, K), 7.0, dtype=torch.bfloat16, device="cuda")
+        gx = torch.full((N, Hh, W, 64), 7.0, dtype=torch.bfloat16, device="cuda")
+        a.x, a.w, a.bias, a.y, a.relu = xd.data_ptr(), wd.data_ptr(), bd.data_ptr(), y.data_ptr(), 1
+        a.y_pitch, a.y_plane = (Q + 2) * K, (P + 1) * (Q + 2) * K
+        abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+        kinds[mode] = L.ad_conv2d_last_kernel()
+        a.y, a.dx, a.y_pitch, a.y_plane = dy.data_ptr(), gx.data_ptr(), 0, 0
+        abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+        H.sync()
+        assert scratch[:4].view(torch.int32).item() == 0
+        out[mode] = y, gx
+    assert kinds == {"row": ROW, "general": GEN}
+    others = [n for n in range(N) if n != N // 2]
+    for got, ref in zip(out["row"], out["general"]):
+        assert torch.isfinite(got[others]).all()
+        assert H.max_rel(got[others].float().cpu().numpy(), ref[others].float().cpu().numpy()) < TOL_BF16
+    y = out["row"][0]
+    assert (y[:, P:] == 7).all() and (y[:, :, Q:] == 7).all()
+
+
 @pytest.mark.parametrize("case", [(2, 64, 22, 140, 64, 3, 1, 3, 0), (1, 64, 18, 262, 64, 3, 1, 1, 0), (3, 64, 12, 104, 32, 3, 1, 2, 0),
                                   (1, 64, 9, 132, 8, 3, 1, 3, 1)])
 @pytest.mark.parametrize("kcrs,accumulate", [(0, 0), (1, 1)])
