@@ -308,17 +308,25 @@ conv_tc_row_fwd_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CK, const void* filt, uint32_t OC,
                        uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, int offy, int offx,
                        uint32_t OP, uint32_t OQ, void* out, long long out_pitch, long long out_plane, const float* bias,
-                       int relu, int accumulate, int32_t* status, cudaStream_t s);
+                       int relu, int accumulate, int32_t* status, uint32_t images, cudaStream_t s);
 
 // Images whose rows the streaming kernel lays side by side in a 128-pixel tile of a narrow map: the rows of 2, 4 or 8 with their
 // filter's reach fit it (a wider map leaves more of the tile unused than the general kernel's tiles do).  0: not that way, nor for
 // an output that the general kernel makes in one round of 128-pixel tiles: 6.6 us, the streaming kernel takes 7.3 to 8.4 for
 // those.  From two rounds on (3x3): 13.4 -> 8.9 us at 16 x 56 x 56, 10.2 -> 8.5 at 32 x 28 x 28; 1x1: 8.6 -> 7.6 at 64 x 28 x 56.
-static uint32_t stream_images(uint32_t NI, uint32_t OP, uint32_t OQ, uint32_t kw, uint32_t dw) {
-  if ((unsigned long long)NI * OP * OQ <= 128ull * kNumSMs) return 0;
+static uint32_t stream_fit(uint32_t OQ, uint32_t kw, uint32_t dw) {
   uint32_t g = 0;
-  for (uint32_t t = 2; t <= 8 && OQ + (kw - 1) * dw <= 128 / t; t *= 2) g = t;
+  for (uint32_t t = 2; t <= 8 && (unsigned long long)OQ + (unsigned long long)(kw - 1) * dw <= 128 / t; t *= 2) g = t;
   return g;
+}
+static uint32_t stream_images(uint32_t NI, uint32_t OP, uint32_t OQ, uint32_t kw, uint32_t dw) {
+  return (unsigned long long)NI * OP * OQ <= 128ull * kNumSMs ? 0 : stream_fit(OQ, kw, dw);
+}
+// A few columns past the last whole tile (the data gradient of a 512-wide layer under dilation 3 is 518 wide) are a narrow map
+// of their own where that saves each SM 16 rows of a nearly empty tile, against some 8 us for the second launch.
+static uint32_t stream_tail(uint32_t NI, uint32_t OP, uint32_t OQ, uint32_t kw, uint32_t dw) {
+  const uint32_t g = OQ > 128 && OQ % 128 ? stream_fit(OQ % 128, kw, dw) : 0;
+  return g && (unsigned long long)(NI - (NI + g - 1) / g) * OP >= 16ull * kNumSMs ? g : 0;
 }
 
 // Returns AD_ERR_UNSUPPORTED when the shape is outside what this variant serves, so that the
@@ -328,11 +336,22 @@ int conv_tc_row_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint
                     uint32_t OP, uint32_t OQ, void* out, long long out_pitch, long long out_plane, const float* bias,
                     int relu, int accumulate, int32_t* status, cudaStream_t s) {
   if (sh != 1 || sw != 1 || CK != 64 || OC > 64) return AD_ERR_UNSUPPORTED;
-  if (OQ < 96 && !stream_images(NI, OP, OQ, kw, dw)) return AD_ERR_UNSUPPORTED;
+  const uint32_t images = OQ < 96 ? stream_images(NI, OP, OQ, kw, dw) : 1;
+  if (!images) return AD_ERR_UNSUPPORTED;
   if (!getenv("ARRAYDIFF_B200_ROW_TILES")) {
     // the row-streaming kernel (below) serves every shape it can; the one-row tile kernel takes the rest
+    if (const uint32_t g = accumulate ? 0 : stream_tail(NI, OP, OQ, kw, dw)) {
+      const uint32_t whole = OQ / 128 * 128;
+      const long long pitch = out_pitch ? out_pitch : (long long)OQ * OC, plane = out_plane ? out_plane : (long long)OP * OQ * OC;
+      int st = conv_tc_stream_fwd(act, NI, IH, IW, CK, filt, OC, kh, kw, sh, sw, dh, dw, offy, offx + (int)whole, OP, OQ - whole,
+                                  (__nv_bfloat16*)out + (size_t)whole * OC, pitch, plane, bias, relu, 0, status, g, s);
+      if (st == AD_OK)
+        return conv_tc_stream_fwd(act, NI, IH, IW, CK, filt, OC, kh, kw, sh, sw, dh, dw, offy, offx, OP, whole, out, pitch, plane, bias, relu, 0,
+                                  status, 1, s);
+      if (st != AD_ERR_UNSUPPORTED) return st;
+    }
     int st = conv_tc_stream_fwd(act, NI, IH, IW, CK, filt, OC, kh, kw, sh, sw, dh, dw, offy, offx, OP, OQ, out, out_pitch,
-                                out_plane, bias, relu, accumulate, status, s);
+                                out_plane, bias, relu, accumulate, status, images, s);
     if (st != AD_ERR_UNSUPPORTED) return st;
   }
   if (OQ < 96) return AD_ERR_UNSUPPORTED;
@@ -868,11 +887,11 @@ static void stream_chunks(uint32_t NI, uint32_t tiles_x, uint32_t dh, uint32_t O
 int conv_tc_stream_fwd(const void* act, uint32_t NI, uint32_t IH, uint32_t IW, uint32_t CK, const void* filt, uint32_t OC,
                        uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh, uint32_t dw, int offy, int offx,
                        uint32_t OP, uint32_t OQ, void* out, long long out_pitch, long long out_plane, const float* bias,
-                       int relu, int accumulate, int32_t* status, cudaStream_t s) {
+                       int relu, int accumulate, int32_t* status, uint32_t images, cudaStream_t s) {
   if (sh != 1 || sw != 1 || CK != 64 || OC > 64) return AD_ERR_UNSUPPORTED;
-  const uint32_t taps = kh * kw, images = OQ < 96 ? stream_images(NI, OP, OQ, kw, dw) : 1;
+  const uint32_t taps = kh * kw;
   const uint32_t pw = (128 + (kw - 1) * dw + 7) / 8 * 8;
-  if (!images || pw > 256 || kh > 4 || taps > 16) return AD_ERR_UNSUPPORTED;
+  if (pw > 256 || kh > 4 || taps > 16) return AD_ERR_UNSUPPORTED;
   const uint32_t row_bytes = pw * 128;
   const long long op_ = out_pitch ? out_pitch : (long long)OQ * OC, opl_ = out_plane ? out_plane : (long long)OP * OQ * OC;
   const bool tma_store = !accumulate && (OC & 7u) == 0 && !((uintptr_t)out & 15u) && (op_ % 8) == 0 && (opl_ % 8) == 0;

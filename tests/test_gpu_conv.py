@@ -387,6 +387,8 @@ def test_conv_tc_row_kernels_agree_with_general_kernels(case, monkeypatch):
     (103, 64, 14, 14, 3, 1, 1),    # eight side by side, implicit padding, the last seven
     (41, 8, 14, 64, 3, 3, 0),      # 58 + 6: no room left; the gradient is too wide
     (75, 64, 8, 32, 1, 1, 0),      # 1x1
+    (16, 64, 172, 134, 3, 3, 0),   # the gradient's last 6 columns of 134 in eights
+    (28, 32, 120, 146, 3, 1, 1),   # 18 columns past a whole tile in fours, both directions
 ])
 def test_conv_tc_rows_of_several_images_in_a_tile(case, monkeypatch):
     """Narrow maps in the streaming kernel, several images side by side, against the general kernel: both accumulate in fp32 and
