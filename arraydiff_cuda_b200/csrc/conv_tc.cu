@@ -1039,7 +1039,13 @@ static int run_fwd_tiles(const void* act, uint32_t IH, uint32_t IW, const void* 
                          cudaStream_t s) {
   g_last_conv_kernel = kConvTcGeneral;
   const uint32_t tiles_m = NC > 1 ? p.tiles_x : p.tiles_b * p.tiles_y * p.tiles_x;
-  const int BN = p.OC > 128 ? 256 : (p.OC > 64 ? 128 : (p.OC > 32 ? 64 : 32));
+  int BN = p.OC > 128 ? 256 : (p.OC > 64 ? 128 : (p.OC > 32 ? 64 : 32));
+  // Short contractions: narrower channel tiles where they still make one round, which takes as long at any width (0.3 us per 64
+  // terms) while more SMs share the stores.  2 x 64 x 79 x 21 -> 512, 3x3 9.3 -> 6.5 us, 5 x 256 x 29 x 16 -> 256, 1x1 5.8 -> 4.5; in two rounds
+  // 9.7 -> 10.0.  A long contraction occupies twice the SMs for almost as long: 8 - 23 % faster alone, but kernels of other
+  // streams wait (two strips of a 50-layer net side by side: 10.93 -> 11.21 ms).
+  if (all_taps * (p.CK / 64) <= 9)
+    while (BN > 64 && tiles_m * ((p.OC + BN / 2 - 1) / (BN / 2)) <= (uint32_t)kNumSMs) BN /= 2;
   p.tiles_n = (p.OC + BN - 1) / BN;
   const bool aligned = !((uintptr_t)p.out & 15u) && p.out_pitch % 8 == 0 && p.out_plane % 8 == 0;
   if (!aligned && (p.OC & 7u) == 0) return AD_ERR_ALIGN;

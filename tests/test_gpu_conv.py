@@ -380,6 +380,46 @@ def test_conv_tc_row_kernels_agree_with_general_kernels(case, monkeypatch):
 
 
 @pytest.mark.parametrize("case", [
+    # N, C, H, W (of x), K, filter, stride: few pixels, a contraction of up to 9 steps of 64, channel tiles of 64 or 128
+    (1, 64, 5, 5, 200, 1, 1),      # four tiles of 64, the last with 8 channels
+    (2, 64, 9, 7, 136, 3, 1),      # 9 steps
+    (1, 128, 7, 9, 96, 1, 2),      # 64 + 32 channels
+    (3, 128, 37, 90, 200, 1, 1),   # 79 pixel tiles: 158 channel tiles of 128 would be two rounds
+    (2, 64, 61, 80, 256, 1, 1),    # 77 pixel tiles: 154
+    (2, 64, 59, 79, 256, 1, 1),    # 74: 148 of 128
+    (1, 64, 37, 127, 256, 1, 1),   # 37 or 38: 148 of 64, or 76 of 128
+])
+def test_conv_tc_channel_tiles_of_short_contractions(case):
+    """Channel tiles narrowed to fill one round of the machine: forward (bias, ReLU) and data gradient against fp64."""
+    import torch
+    import torch.nn.functional as F
+    N, Cc, Hh, W, K, k, s = case
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    rnd = lambda *d: torch.randn(d, generator=g, device="cuda")  # noqa: E731
+    x, w, b = rnd(N, Hh, W, Cc).bfloat16(), (rnd(K, k, k, Cc) * (2.0 / (Cc * k * k)) ** 0.5).bfloat16(), rnd(K)
+    xn, wn = x.double().permute(0, 3, 1, 2).requires_grad_(), w.double().permute(0, 3, 1, 2)
+    lin = F.conv2d(xn, wn, stride=s)
+    P, Q = lin.shape[2:]
+    dy = rnd(N, P, Q, K).bfloat16()
+    lin.backward(dy.double().permute(0, 3, 1, 2))
+    want = (lin.detach() + b.double()[None, :, None, None]).clamp_min(0).permute(0, 2, 3, 1)
+    L = abi.lib()
+    a = conv_args(abi.AD_BF16, abi.AD_NHWC, (N, Cc, Hh, W), K, k, s, 1, 0)
+    y, dx = torch.full((N, P, Q, K), 7.0, device="cuda").bfloat16(), torch.full_like(x, 7.0)
+    nscr = max(16, L.ad_conv2d_scratch_bytes(C.byref(a), 1))
+    scratch = torch.zeros(nscr, dtype=torch.uint8, device="cuda")
+    a.x, a.w, a.bias, a.y, a.relu, a.scratch, a.scratch_bytes = x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), 1, scratch.data_ptr(), nscr
+    abi.check(L.ad_conv2d_fprop(C.byref(a), H.stream()))
+    a.y, a.dx = dy.data_ptr(), dx.data_ptr()
+    abi.check(L.ad_conv2d_dgrad(C.byref(a), H.stream()))
+    H.sync()
+    assert scratch[:4].view(torch.int32).item() == 0
+    assert H.max_rel(y.float().cpu().numpy(), want.float().cpu().numpy()) < TOL_BF16
+    assert H.max_rel(dx.float().cpu().numpy(), xn.grad.permute(0, 2, 3, 1).float().cpu().numpy()) < TOL_BF16
+
+
+@pytest.mark.parametrize("case", [
     # N, K, H, W (of x), filter, dilation, padding; more than 148 x 128 output pixels, 64 input channels
     (39, 64, 11, 58, 3, 1, 0),     # pairs of images, the last alone; the gradient is 58 wide
     (339, 64, 3, 58, 3, 1, 0),     # one output row per image
