@@ -67,7 +67,8 @@ struct F32Split { uint32_t cs, slices; };
 // 52 -> 44 us, 191 -> 75, 3 x 71 x 10 68 -> 54).  The slices' scratch stays within 32 MB.
 inline F32Split f32_k3_split(unsigned long long tiles, unsigned long long all, unsigned long long words, uint32_t sms, uint32_t per_sm) {
   // clusters of 1, 2, 4, 8 CTAs at a time, two or three CTAs per SM
-  static const unsigned held2[4] = {296, 148, 70, 33}, held3[4] = {444, 222, 104, 48}, *const held = per_sm == 2 ? held2 : held3;
+  static const unsigned held2[4] = {296, 148, 70, 33}, held3[4] = {444, 222, 104, 48};
+  const unsigned* const held = per_sm == 2 ? held2 : held3;
   F32Split best = {1, 1};
   double best_cost = 0;
   for (uint32_t i = 0; i < 4; ++i)

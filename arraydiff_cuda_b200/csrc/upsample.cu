@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(kUpThreads) upsample_fwd_cells(UpRowP p) {
   const T *X0 = X + (y0 - u.x_row0) * u.x.sy, *X1 = X + (y1 - u.x_row0) * u.x.sy;
 #pragma unroll 4
   for (uint32_t i = threadIdx.x; i < cols; i += kUpThreads) { L[i] = ld_f(X0 + i); L[pitch + i] = ld_f(X1 + i); }
-  if (hi == u.XW)   // a column of zeros past the last: the right edge blends it with weight 0 (an infinity there, times 0, would be NaN)
+  if (xb == u.XW)   // a column of zeros past the last: the right edge blends it with weight 0 (an infinity there, times 0, would be NaN)
     for (uint32_t i = threadIdx.x; i < Ci; i += kUpThreads) L[cols + i] = L[pitch + cols + i] = 0.f;
   float* const W = L + 2 * pitch;
   if ((int)threadIdx.x >= ra && (int)threadIdx.x < rb) {

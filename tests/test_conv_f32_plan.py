@@ -16,6 +16,10 @@ extern "C" uint32_t cluster_size(const uint32_t* held, unsigned long long tiles,
 extern "C" uint32_t largest_cluster(const uint32_t* held, uint32_t most) {
   return adk::f32_largest_cluster([=](uint32_t cs) { return held[__builtin_ctz(cs)]; }, most);
 }
+extern "C" uint32_t k3_split(unsigned long long tiles, unsigned long long all, unsigned long long words, uint32_t per_sm) {
+  const adk::F32Split s = adk::f32_k3_split(tiles, all, words, 148, per_sm);
+  return s.cs << 16 | s.slices;
+}
 extern "C" uint32_t few_images(uint32_t N, unsigned long long image, unsigned long long z, unsigned long long limit) {
   return adk::f32_few_images(N, image, z, limit);
 }
@@ -31,8 +35,9 @@ def plan(tmp_path_factory):
     L = C.CDLL(str(d / "plan.so"))
     L.cluster_size.argtypes = [C.POINTER(C.c_uint32), C.c_uint64, C.c_uint32, C.c_uint32]
     L.largest_cluster.argtypes = [C.POINTER(C.c_uint32), C.c_uint32]
+    L.k3_split.argtypes = [C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint32]
     L.few_images.argtypes = [C.c_uint32, C.c_uint64, C.c_uint64, C.c_uint64]
-    L.cluster_size.restype = L.largest_cluster.restype = L.few_images.restype = C.c_uint32
+    L.k3_split.restype = L.cluster_size.restype = L.largest_cluster.restype = L.few_images.restype = C.c_uint32
     return L
 
 
@@ -86,3 +91,20 @@ def test_pieces_of_the_gradient_into_few_channels(plan, N, image, z, limit):
     n = plan.few_images(N, image, z, limit)
     most = max(i for i in range(N + 1) if i * z <= limit and i * image < 2 ** 31)
     assert n == most and n * image + 148 * 16 * 256 < 2 ** 32
+
+
+def test_filter_gradient_split_depends_on_its_arguments_alone(plan):
+    """The same split whatever was asked for before; at least two stages per CTA, at most 16 slices and 32 MB of them."""
+    rng = random.Random(6)
+    calls = []
+    for _ in range(500):
+        tiles, stages, words = int(2 ** rng.uniform(0, 9)), int(2 ** rng.uniform(0, 12)), int(2 ** rng.uniform(10, 23))
+        calls.append((tiles, stages, words, rng.choice([2, 3])))
+    first = [plan.k3_split(*c) for c in calls]
+    assert [plan.k3_split(*c) for c in reversed(calls)] == first[::-1]
+    assert any(plan.k3_split(t, s, w, 2) != plan.k3_split(t, s, w, 3) for t, s, w, _ in calls)
+    for (tiles, stages, words, _), split in zip(calls, first):
+        cs, slices = split >> 16, split & 0xffff
+        assert cs in (1, 2, 4, 8) and 1 <= slices <= 16
+        assert cs * slices == 1 or stages >= 2 * cs * slices
+        assert slices == 1 or slices * words * 4 <= 32 << 20

@@ -53,7 +53,8 @@ def test_upsample_rows(dtype, shape, scale):
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
-@pytest.mark.parametrize("Cc,W,scale", [(19, 40, 8), (3, 300, 4), (1, 1100, 2), (31, 70, 4), (2, 33, 16), (64, 18, 8), (5, 300, 2)])
+@pytest.mark.parametrize("Cc,W,scale", [(19, 40, 8), (3, 300, 4), (1, 1100, 2), (31, 70, 4), (2, 33, 16), (64, 18, 8), (5, 300, 2),
+                                        (36, 25, 8), (107, 21, 4)])   # 6 blocks of 4 columns and one of the last, 5 and one
 def test_upsample_cells_of_strips(dtype, layout, Cc, W, scale):
     """Rows between two source rows as one block: cells cut by the strips, rows that start on odd elements, odd channel counts, one
     thread group per block (64 channels at scale 8); every element of the strip and none beside it."""
