@@ -32,29 +32,26 @@ struct BnRed {
   uint32_t N, C, H, W;
   int relu;
   const float *gamma, *beta, *mean, *invstd;
+  int dual;               // forward sums of an x-fastest view: in double too
 };
 
-// what an x-fastest reduction sums in
-template <int MODE> struct BnSum { using type = float; };
-template <> struct BnSum<0> { using type = double; };
-
-template <typename T, int MODE, typename A>
-__device__ __forceinline__ void bn_term(const BnRed& p, uint32_t n, uint32_t c, uint32_t y, uint32_t x, A& a, A& b) {
+template <typename T, int MODE>
+__device__ __forceinline__ float bn_term(const BnRed& p, uint32_t n, uint32_t c, uint32_t y, uint32_t x, float& a, float& b) {
   const long long ox = n * p.x.sn + c * p.x.sc + y * p.x.sy + x * p.x.sx;
   const float xv = ld_f((const T*)p.x.base + ox);
   if (MODE == 0) {
-    a += (A)xv;
-    b = fma((A)xv, (A)xv, b);
+    a += xv;
+    b = fmaf(xv, xv, b);
   } else {
     const long long od = n * p.dy.sn + c * p.dy.sc + y * p.dy.sy + x * p.dy.sx;
     float g = ld_f((const T*)p.dy.base + od);
     const float xhat = (xv - p.mean[c]) * p.invstd[c];
     if (p.relu && fmaf(p.gamma[c], xhat, p.beta[c]) <= 0.f) g = 0.f;
     a += g;
-    b = fma(g, xhat, b);
+    b = fmaf(g, xhat, b);
   }
+  return xv;
 }
-
 // Views whose planes are runs of floats that 16-byte loads reach
 static bool planes_vec_ok(const ad_tensor4* t) {
   return t->dtype == AD_F32 && t->sx == 1 && t->sy == (int64_t)t->W && !((uintptr_t)t->base & 15u) && !(t->sn & 3) && !(t->sc & 3) &&
@@ -62,40 +59,34 @@ static bool planes_vec_ok(const ad_tensor4* t) {
 }
 
 // NCHW-like: block (256) per (channel, split); threads stride over (n, y, x), 4 pixels at a time where the planes allow it (VEC).
-// The forward statistics are summed in double, and a split writes its sums as two rows of floats, high and low parts: the
-// variance is the small difference of E[x^2] and E[x]^2, and with sums in fp32 its error was what the gradients of a small fp32
-// net differed by from a double-precision one (18 layers, 16 pixels per channel at the end: 8e-4 -> 4e-5 of a filter
-// gradient).  The conversions and double additions are a tenth of what the SM can do in the time of the loads.
+// The forward statistics are summed in fp32, one pixel after the other, and beside that in double, which a split writes as two
+// more rows of floats, high and low parts; bn_finish takes the double ones where the two differ (bn_statistics).  The
+// conversions and double additions are a tenth of what the SM can do in the time of the loads.
 template <typename T, int MODE, bool VEC>
 __global__ void __launch_bounds__(256) bn_reduce_xfast(BnRed p, float* partial) {
   grid_dependency();
   const uint32_t c = blockIdx.x, split = blockIdx.y, nsplit = gridDim.y;
-  using A = typename BnSum<MODE>::type;
-  A a = 0, b = 0;
+  float a = 0.f, b = 0.f;
+  double da = 0.0, db = 0.0;
   // the position moves on by the same (images, rows, columns) each time: no division per element
   const size_t first = (size_t)split * 256 + threadIdx.x, hop = (size_t)nsplit * 256;
-  if constexpr (VEC) {
+  if constexpr (VEC) {       // MODE 1
     const uint32_t hw = p.H * p.W / 4, hi = (uint32_t)(hop % hw), hn = (uint32_t)(hop / hw);
     uint32_t i = (uint32_t)(first % hw), n = (uint32_t)(first / hw);
-    const float *xb = (const float*)p.x.base + c * p.x.sc, *db = (const float*)p.dy.base + c * p.dy.sc;
-    const float mean = MODE ? p.mean[c] : 0.f, invstd = MODE ? p.invstd[c] : 0.f, gam = MODE ? p.gamma[c] : 0.f, bet = MODE ? p.beta[c] : 0.f;
+    const float *xb = (const float*)p.x.base + c * p.x.sc, *gb = (const float*)p.dy.base + c * p.dy.sc;
+    const float mean = p.mean[c], invstd = p.invstd[c], gam = p.gamma[c], bet = p.beta[c];
 #pragma unroll 4
     for (; n < p.N;) {
       const float4 v = *(const float4*)(xb + n * p.x.sn + (size_t)i * 4);
       const float xv[4] = {v.x, v.y, v.z, v.w};
-      if constexpr (MODE == 0) {
+      const float4 w = *(const float4*)(gb + n * p.dy.sn + (size_t)i * 4);
+      const float gv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) { const double d = (double)xv[j]; a += d; b = fma(d, d, b); }
-      } else {
-        const float4 w = *(const float4*)(db + n * p.dy.sn + (size_t)i * 4);
-        const float gv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float xhat = (xv[j] - mean) * invstd;
-          const float g = p.relu && fmaf(gam, xhat, bet) <= 0.f ? 0.f : gv[j];
-          a += g;
-          b = fmaf(g, xhat, b);
-        }
+      for (int j = 0; j < 4; ++j) {
+        const float xhat = (xv[j] - mean) * invstd;
+        const float g = p.relu && fmaf(gam, xhat, bet) <= 0.f ? 0.f : gv[j];
+        a += g;
+        b = fmaf(g, xhat, b);
       }
       i += hi; n += hn;
       if (i >= hw) { i -= hw; ++n; }
@@ -106,23 +97,34 @@ __global__ void __launch_bounds__(256) bn_reduce_xfast(BnRed p, float* partial) 
     uint32_t x = (uint32_t)(first % p.W), y = (uint32_t)(first / p.W % p.H), n = (uint32_t)(first / p.W / p.H);
 #pragma unroll 4
     for (size_t i = first; i < per; i += hop) {
-      bn_term<T, MODE>(p, n, c, y, x, a, b);
+      const float v = bn_term<T, MODE>(p, n, c, y, x, a, b);
+      if (MODE == 0) { da += (double)v; db = fma((double)v, (double)v, db); }
       x += hx; y += hy; n += hn;
       if (x >= p.W) { x -= p.W; ++y; }
       if (y >= p.H) { y -= p.H; ++n; }
     }
   }
-  __shared__ A sa[8], sb[8];
+  __shared__ float sa[8], sb[8];
+  __shared__ double sd[2][8];
+  a = warp_sum(a); b = warp_sum(b);
+  if (MODE == 0) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); }
-  if ((threadIdx.x & 31) == 0) { sa[threadIdx.x >> 5] = a; sb[threadIdx.x >> 5] = b; }
+    for (int o = 16; o > 0; o >>= 1) { da += __shfl_xor_sync(0xffffffffu, da, o); db += __shfl_xor_sync(0xffffffffu, db, o); }
+  }
+  if ((threadIdx.x & 31) == 0) { sa[threadIdx.x >> 5] = a; sb[threadIdx.x >> 5] = b; sd[0][threadIdx.x >> 5] = da; sd[1][threadIdx.x >> 5] = db; }
   __syncthreads();
   if (threadIdx.x < 2) {
-    A t = 0;
+    float t = 0.f;
     for (int w = 0; w < 8; ++w) t += threadIdx.x ? sb[w] : sa[w];
-    float* out = partial + (size_t)split * (MODE == 0 ? 4 : 2) * p.C + threadIdx.x * p.C + c;
-    *out = (float)t;
-    if (MODE == 0) out[2 * p.C] = isfinite((float)t) ? (float)(t - (A)(float)t) : 0.f;
+    float* out = partial + (size_t)split * 2 * p.C + threadIdx.x * p.C + c;
+    *out = t;
+    if (MODE == 0 && p.dual) {
+      double d = 0.0;
+      for (int w = 0; w < 8; ++w) d += sd[threadIdx.x][w];
+      out = partial + (size_t)(nsplit + 2 * split) * 2 * p.C + threadIdx.x * p.C + c;
+      *out = (float)d;
+      out[2 * p.C] = isfinite((float)d) ? (float)(d - (double)(float)d) : 0.f;
+    }
   }
 }
 
@@ -163,7 +165,17 @@ struct BnFin {
   float eps;
   float *mean, *invstd, *var, *sums, *dgamma, *dbeta;
   int accumulate;     // kind 1: add to dgamma / dbeta (else overwrite)
+  double rows;        // pixels behind the sums
 };
+// The sums that statistics are made of: those in fp32 (s, ss), or where the mean or the variance made of them is more than 1e-6 of
+// the spread or the variance off, those in double.  The variance is the small difference of E[x^2] and E[x]^2: with fp32
+// sums throughout, the gradients of a small net in strips differed from a double-precision one by 8e-4 (18 layers, 16
+// pixels per channel at the end), now by 4e-5.  Statistics that agree keep their last digit from call to call of either form: one
+// rounding moves pixels across the edge of the ReLU behind (2e-4 of the gradient of 10 M pixels).
+__device__ __forceinline__ void bn_statistics(double count, double& s, double& ss, double ds, double dss) {
+  const double m = s / count, v = ss / count - m * m, dm = ds / count, dv = dss / count - dm * dm;
+  if (!(fabs(v - dv) <= 1e-6 * dv && (m - dm) * (m - dm) <= 1e-12 * dv)) { s = ds; ss = dss; }
+}
 __device__ __forceinline__ void bn_finish_channel(const BnFin& f, uint32_t c, double s, double ss) {
   if (f.kind == 0) {
     double m = s / f.count, v = ss / f.count - m * m;
@@ -187,18 +199,18 @@ __device__ __forceinline__ void bn_finish_channel(const BnFin& f, uint32_t c, do
 // flight at once, so the kernel is one trip to L2 and a short tree.  As 32 channels per block with 8 rows in flight and a
 // serial sum of 32 lanes it took 5.6 us, this form 3.3 us at 256 channels.
 constexpr uint32_t kFinishThreads = 512, kFinishRows = 10;
-__global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit, const float* __restrict__ partial) {
-  grid_dependency();
+// dual: behind the rows of fp32 sums lie twice as many of double ones
+__device__ __forceinline__ double bn_finish_rows(const BnFin& f, uint32_t nsplit, const float* __restrict__ partial) {
   const uint32_t v = threadIdx.x & 15, rl = threadIdx.x >> 4, which = v >> 3, c = blockIdx.x * 8 + (v & 7);
   double t = 0.0;
   if (c < f.C) {
     const float* src = partial + which * f.C + c;
-    for (uint32_t k0 = rl; k0 < (uint32_t)nsplit; k0 += 32 * kFinishRows) {
+    for (uint32_t k0 = rl; k0 < nsplit; k0 += 32 * kFinishRows) {
       float r[kFinishRows];
 #pragma unroll
       for (uint32_t u = 0; u < kFinishRows; ++u) {
         const uint32_t k = k0 + u * 32;
-        r[u] = k < (uint32_t)nsplit ? src[(size_t)k * 2 * f.C] : 0.f;
+        r[u] = k < nsplit ? src[(size_t)k * 2 * f.C] : 0.f;
       }
 #pragma unroll
       for (uint32_t u = 0; u < kFinishRows; ++u) t += (double)r[u];
@@ -208,15 +220,30 @@ __global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit,
   __shared__ double sh[16][17];
   if ((threadIdx.x & 31) < 16) sh[threadIdx.x >> 5][v] = t;
   __syncthreads();
-  if (threadIdx.x >= 32) return;
-  // lane: value v, half of the 16 warps' sums
-  const uint32_t h = threadIdx.x >> 4;
-  t = 0.0;
+  if (threadIdx.x < 32) {
+    // lane: value v, half of the 16 warps' sums
+    const uint32_t h = threadIdx.x >> 4;
+    t = 0.0;
 #pragma unroll
-  for (uint32_t w = 0; w < 8; ++w) t += sh[h * 8 + w][v];
-  t += __shfl_xor_sync(0xffffffffu, t, 16);
-  const double ss = __shfl_down_sync(0xffffffffu, t, 8);
-  if (threadIdx.x < 8 && c < f.C) bn_finish_channel(f, c, t, ss);
+    for (uint32_t w = 0; w < 8; ++w) t += sh[h * 8 + w][v];
+    t += __shfl_xor_sync(0xffffffffu, t, 16);
+  }
+  return t;                   // of the first warp: lanes 0 .. 7 the first sum of channel c, 8 .. 15 the second
+}
+__global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit, int dual, const float* __restrict__ partial) {
+  grid_dependency();
+  double t = bn_finish_rows(f, (uint32_t)nsplit, partial), d = 0.0;
+  if (dual) {
+    __syncthreads();
+    d = bn_finish_rows(f, 2u * nsplit, partial + (size_t)nsplit * 2 * f.C);
+  }
+  if (threadIdx.x >= 32) return;
+  double ss = __shfl_down_sync(0xffffffffu, t, 8);
+  const double dss = __shfl_down_sync(0xffffffffu, d, 8);
+  const uint32_t c = blockIdx.x * 8 + threadIdx.x;
+  if (threadIdx.x >= 8 || c >= f.C) return;
+  if (dual) bn_statistics(f.kind == 0 ? f.count : f.rows, t, ss, d, dss);
+  bn_finish_channel(f, c, t, ss);
 }
 
 struct BnApply {
@@ -519,15 +546,17 @@ static int pick_splits(const ad_tensor4* x, bool cfast) {
   return (int)want;
 }
 
-static void launch_finish(const BnFin& f, int nsplit, const float* partial, cudaStream_t s) {
-  launch(bn_finish, (f.C + 7) / 8, kFinishThreads, 0, s, f, nsplit, partial);
+static void launch_finish(const BnFin& f, int nsplit, int dual, const float* partial, cudaStream_t s) {
+  launch(bn_finish, (f.C + 7) / 8, kFinishThreads, 0, s, f, nsplit, dual, partial);
   count_launch();
 }
 // Both stages of the statistics of x (MODE 0) or of the backward sums (MODE 1) into what `f` names
 template <int MODE>
 static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, float* partial, cudaStream_t s, bool vec) {
   const bool cfast = x->sc == 1 && x->C > 1;
-  int nsplit;
+  int nsplit, dual = 0;
+  BnFin fin = f;
+  fin.rows = (double)x->N * x->H * x->W;
   if (vec_view_ok(x) && (MODE == 0 || (p.dy.sc == 1 && !((uintptr_t)p.dy.base & 15u) && !(p.dy.sn & 7) && !(p.dy.sy & 7) && !(p.dy.sx & 7)))) {
     nsplit = (int)vec_grid(x);
     constexpr int smem = LoadRing<MODE + 1, kBnDepth>::kSmem;
@@ -540,15 +569,15 @@ static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, fl
       dim3 grid((x->C + 31) / 32, nsplit), block(32, 8);
       AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_cfast<T, MODE>, grid, block, 0, s, p, partial)));
     } else {
-      if (MODE == 0) nsplit = std::max(1, std::min(nsplit, bn_max_splits(x->C) / 2));   // two rows per split
-      dim3 grid(x->C, nsplit);
-      if (vec) launch(bn_reduce_xfast<float, MODE, true>, grid, 256, 0, s, p, partial);
-      else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_xfast<T, MODE, false>, grid, 256, 0, s, p, partial)));
-      if (MODE == 0) nsplit *= 2;
+      BnRed r = p;
+      r.dual = dual = MODE == 0 && 3 * nsplit <= bn_max_splits(x->C);
+      const dim3 grid(x->C, nsplit);
+      if (MODE == 1 && vec) launch(bn_reduce_xfast<float, 1, true>, grid, 256, 0, s, r, partial);
+      else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_reduce_xfast<T, MODE, false>, grid, 256, 0, s, r, partial)));
     }
   }
   count_launch();
-  launch_finish(f, nsplit, partial, s);
+  launch_finish(fin, nsplit, dual, partial, s);
   return launch_status();
 }
 
@@ -1063,7 +1092,7 @@ extern "C" int ad_bn_finalize_apply(const ad_tensor4* x, const ad_tensor4* y, co
   if (!x || !y || !x->base || !y->base || !sums || !gamma || !beta || !save_mean || !save_invstd) return AD_ERR_BAD_ARG;
   if (!dims_eq(x, y) || count <= 0.0) return AD_ERR_BAD_ARG;
   cudaStream_t s = as_stream(stream);
-  launch_finish(BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, 1, sums, s);
+  launch_finish(BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, 1, 0, sums, s);
   BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, save_mean, save_invstd, nullptr, 1, count};
   return launch_apply<0>(a, x, vec_view_ok(x) && vec_view_ok(y), planes_vec_ok(x) && planes_vec_ok(y), s);
