@@ -199,7 +199,6 @@ __device__ __forceinline__ void bn_finish_channel(const BnFin& f, uint32_t c, do
 // flight at once, so the kernel is one trip to L2 and a short tree.  As 32 channels per block with 8 rows in flight and a
 // serial sum of 32 lanes it took 5.6 us, this form 3.3 us at 256 channels.
 constexpr uint32_t kFinishThreads = 512, kFinishRows = 10;
-// dual: behind the rows of fp32 sums lie twice as many of double ones
 __device__ __forceinline__ double bn_finish_rows(const BnFin& f, uint32_t nsplit, const float* __restrict__ partial) {
   const uint32_t v = threadIdx.x & 15, rl = threadIdx.x >> 4, which = v >> 3, c = blockIdx.x * 8 + (v & 7);
   double t = 0.0;
@@ -230,19 +229,21 @@ __device__ __forceinline__ double bn_finish_rows(const BnFin& f, uint32_t nsplit
   }
   return t;                   // of the first warp: lanes 0 .. 7 the first sum of channel c, 8 .. 15 the second
 }
-__global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit, int dual, const float* __restrict__ partial) {
+// DUAL: behind the rows of fp32 sums lie twice as many of double ones
+template <bool DUAL>
+__global__ void __launch_bounds__(kFinishThreads) bn_finish(BnFin f, int nsplit, const float* __restrict__ partial) {
   grid_dependency();
   double t = bn_finish_rows(f, (uint32_t)nsplit, partial), d = 0.0;
-  if (dual) {
+  if constexpr (DUAL) {
     __syncthreads();
     d = bn_finish_rows(f, 2u * nsplit, partial + (size_t)nsplit * 2 * f.C);
   }
   if (threadIdx.x >= 32) return;
-  double ss = __shfl_down_sync(0xffffffffu, t, 8);
-  const double dss = __shfl_down_sync(0xffffffffu, d, 8);
+  double ss = __shfl_down_sync(0xffffffffu, t, 8), dss = 0.0;
+  if constexpr (DUAL) dss = __shfl_down_sync(0xffffffffu, d, 8);
   const uint32_t c = blockIdx.x * 8 + threadIdx.x;
   if (threadIdx.x >= 8 || c >= f.C) return;
-  if (dual) bn_statistics(f.kind == 0 ? f.count : f.rows, t, ss, d, dss);
+  if constexpr (DUAL) bn_statistics(f.kind == 0 ? f.count : f.rows, t, ss, d, dss);
   bn_finish_channel(f, c, t, ss);
 }
 
@@ -547,7 +548,7 @@ static int pick_splits(const ad_tensor4* x, bool cfast) {
 }
 
 static void launch_finish(const BnFin& f, int nsplit, int dual, const float* partial, cudaStream_t s) {
-  launch(bn_finish, (f.C + 7) / 8, kFinishThreads, 0, s, f, nsplit, dual, partial);
+  launch(dual ? bn_finish<true> : bn_finish<false>, (f.C + 7) / 8, kFinishThreads, 0, s, f, nsplit, partial);
   count_launch();
 }
 // Both stages of the statistics of x (MODE 0) or of the backward sums (MODE 1) into what `f` names
