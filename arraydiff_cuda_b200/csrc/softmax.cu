@@ -4,6 +4,8 @@
 //   NHWC: up to 32 classes a block stages 256 pixels in shared memory by 16-byte vectors, a thread per pixel; up to 256
 //   classes a warp holds several pixels in registers; more: a warp per pixel.
 // A map of one position is the same memory in both layouts (a classifier's [batch][classes]) and takes the NHWC kernels.
+// A label that is no class (255 for "void", -1) is compared, never used as an index: its pixel's loss is logsumexp(logits), whose
+// gradient is dloss * softmax, zero under a weight of zero.
 #include "common.cuh"
 
 namespace adk {
@@ -84,7 +86,7 @@ __global__ void __launch_bounds__(256) ce_fwd_nchw(uint32_t N, uint32_t C, uint3
     for (uint32_t c = 0; c < C; ++c) z += expf(ld_f(px + (size_t)c * HW) - m);
     const uint32_t l = label[i];
     const size_t li = (n * C + l) * HW + t;
-    loss[i] = (logf(z) + m) - ld_f(x + li);
+    loss[i] = (logf(z) + m) - (l < C ? ld_f(x + li) : 0.f);
     if (picked) picked[i] = li;
   }
 }
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(256) ce_nhwc(uint32_t C, size_t pixels, const 
     const uint32_t l = label[i];
     if (!BWD) {
       if (lane == 0) {
-        loss[i] = (logf(z) + m) - ld_f(px + l);
+        loss[i] = (logf(z) + m) - (l < C ? ld_f(px + l) : 0.f);
         if (picked) picked[i] = i * C + l;
       }
     } else {
@@ -181,7 +183,7 @@ __global__ void __launch_bounds__(256) ce_nhwc_reg(uint32_t C, size_t pixels, co
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const uint32_t c = lane + k * 32;
-        if (c == l) vl = v[q][k];
+        if (c == l && c < C) vl = v[q][k];
         v[q][k] = c < C ? expf(v[q][k] - m[q]) : 0.f;
         z[q] += v[q][k];
       }
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(256) ce_nhwc_pair(size_t pixels, int vec, cons
       uint32_t top[2] = {0xff80ff80u, 0xff80ff80u};   // packed maxima of the words that lie in one pixel (from -infinity)
       __nv_bfloat16* pe = (__nv_bfloat16*)px;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) xl[h] = ld_f(pe + h * C + l[h]);
+      for (int h = 0; h < 2; ++h) xl[h] = l[h] < C ? ld_f(pe + h * C + l[h]) : 0.f;
 #pragma unroll
       for (int k = 0; k < C; ++k) {   // an odd last pixel leaves half of its pair's words undefined: computed, not written
         const uint32_t w = px[k];
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(256) ce_nhwc_pair(size_t pixels, int vec, cons
             const __nv_bfloat16* old = dx + (i + h) * C;
 #pragma unroll
             for (int c = 0; c < C; ++c) v[h * C + c] += ld_f(old + c);
-            xl[h] += ld_f(old + l[h]);
+            if (l[h] < C) xl[h] += ld_f(old + l[h]);
           }
       }
       if (BWD) {
@@ -306,7 +308,8 @@ __global__ void __launch_bounds__(256) ce_nhwc_pair(size_t pixels, int vec, cons
           px[k] = *reinterpret_cast<const uint32_t*>(&g);
         }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) st_f(pe + h * C + l[h], xl[h]);
+        for (int h = 0; h < 2; ++h)
+          if (l[h] < C) st_f(pe + h * C + l[h], xl[h]);
       }
     }
     if (BWD) {
@@ -382,7 +385,7 @@ __global__ void __launch_bounds__(256) ce_nhwc_small(uint32_t C, size_t pixels, 
       }
       float z = 0.f;
       if (!BWD) {
-        const float vl = ld_f(px + l);
+        const float vl = l < C ? ld_f(px + l) : 0.f;
   #pragma unroll
         for (uint32_t c = 0; c < CM; ++c) z += expf(v[c] - m);
         loss[i] = (logf(z) + m) - vl;

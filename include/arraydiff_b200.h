@@ -235,6 +235,8 @@ int ad_softmax_nll_loss_bwd(uint32_t num_channels, uint32_t batch_size, const fl
  *   fwd: loss[n,t] = logsumexp_c(logits) - logits[label]   (fp32 [N][HW]); picked (optional) gets
  *        the flat element index of the selected logit, for exact label-index checks.
  *   bwd: dlogits[n,c,t] (+)= dloss[n,t] * (softmax_c - [c == label]);  accumulate != 0 adds.
+ * A label >= C is no class: logits[label] counts as 0 and [c == label] is 0 for every c, so that a pixel whose
+ * dloss is 0 leaves its gradient alone whatever its label.
  * C <= 1024.
  */
 int ad_softmax_ce_pixel_fwd(int32_t dtype, int32_t layout, uint32_t N, uint32_t C, uint32_t HW,

@@ -117,6 +117,56 @@ def test_softmax_ce_pixel(Cc, layout, dtype):
     assert H.max_rel(got, dlog_w) < (1e-5 if dtype == "f32" else 2e-2)
 
 
+# one class count per form of the kernel: NCHW in registers (8, 32 classes) and read again (more); NHWC a pixel or a pair of pixels
+# per thread (to 32), a warp's registers (two, four and eight classes per lane), a warp per pixel
+@pytest.mark.parametrize("accumulate", [0, 1])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("layout,Cc", [(abi.AD_NCHW, 5), (abi.AD_NCHW, 19), (abi.AD_NCHW, 40), (abi.AD_NHWC, 1), (abi.AD_NHWC, 2), (abi.AD_NHWC, 19),
+                                       (abi.AD_NHWC, 32), (abi.AD_NHWC, 40), (abi.AD_NHWC, 100), (abi.AD_NHWC, 200), (abi.AD_NHWC, 300)])
+def test_softmax_ce_pixel_labels_outside(layout, Cc, dtype, accumulate):
+    """Labels that are no class leave their pixel with logsumexp and dloss * softmax, and every other pixel alone; several
+    tiles of 512 pixels and an odd last one."""
+    import torch
+    N, HW = 1, 1301
+    logits = H.normal(60, (N, Cc, HW), 2.0)
+    base = H.normal(61, (N, Cc, HW))
+    if dtype == "bf16":
+        logits, base = orc.round_bf16(logits), orc.round_bf16(base)
+    g = H.rng(62)
+    label = g.integers(0, Cc, (N, HW)).astype(np.uint32)
+    outside = g.random((N, HW)) < 0.3
+    outside[0, [0, 510, 511, 512, 1023, HW - 1]] = True
+    bad = np.array([Cc, Cc + 1, Cc + 13, 255 if Cc < 255 else 1000, 65536, 0x7fffffff, 0xffffff9c, 0xffffffff], np.uint32)
+    label[outside] = g.choice(bad, int(outside.sum()))
+    dloss = H.uniform(63, (N, HW))
+    dloss[outside & (g.random((N, HW)) < 0.5)] = 0.0
+    x = logits.astype(np.float64)
+    m = x.max(1, keepdims=True)
+    e = np.exp(x - m)
+    z = e.sum(1, keepdims=True)
+    hit = np.arange(Cc)[None, :, None] == label[:, None, :]
+    loss_w = (np.log(z) + m)[:, 0] - (x * hit).sum(1)
+    dlog_w = dloss[:, None, :] * (e / z - hit) + (base if accumulate else 0.0)
+    lay = (lambda a: a) if layout == abi.AD_NCHW else (lambda a: np.ascontiguousarray(np.transpose(a, (0, 2, 1))))
+    put = H.dev if dtype == "f32" else H.dev_bf16
+    d, dlog = put(lay(logits)), put(lay(base))
+    dl = torch.from_numpy(label.view(np.int32)).cuda()
+    loss = torch.empty((N, HW), device="cuda")
+    L = abi.lib()
+    dt = abi.AD_F32 if dtype == "f32" else abi.AD_BF16
+    abi.check(L.ad_softmax_ce_pixel_fwd(dt, layout, N, Cc, HW, H.ptr(d), H.ptr(dl), H.ptr(loss), None, H.stream()))
+    ddl = H.dev(dloss)
+    abi.check(L.ad_softmax_ce_pixel_bwd(dt, layout, N, Cc, HW, H.ptr(d), H.ptr(dl), H.ptr(ddl), H.ptr(dlog), accumulate, H.stream()))
+    H.sync()
+    got = H.host(dlog)
+    got = got if layout == abi.AD_NCHW else np.transpose(got, (0, 2, 1))
+    assert np.abs(H.host(loss) - loss_w).max() < 2e-5 * max(1.0, np.abs(loss_w).max())
+    # one rounding of the result and of the fp32 sums: 2^-8 of the value in bf16
+    assert (np.abs(got - dlog_w) <= (1e-5 if dtype == "f32" else 2 ** -8) * np.abs(dlog_w) + 1e-5).all()
+    quiet = np.broadcast_to((outside & (dloss == 0))[:, None, :], got.shape)
+    assert np.array_equal(got[quiet], (base if accumulate else np.zeros_like(base))[quiet])
+
+
 def _views(arr_nchw, layout, dtype, pad=0):
     """Device tensor (optionally inside a zero halo-padded buffer) + Tensor4 view of the interior."""
     import torch
