@@ -162,9 +162,10 @@ __global__ void __launch_bounds__(kUpThreads) upsample_fwd_rows(UpRowP p) {
     bilin_src(u.y_row0 + oy, inv, u.in_rows_total, y0, y1, fy);
     const T* X = (const T*)u.x.base + plane_off(u.x, plane, per_n) + (long long)lo * p.Ci;
     const T *X0 = X + (y0 - u.x_row0) * u.x.sy, *X1 = X + (y1 - u.x_row0) * u.x.sy;
-    // one column of zeros past the last: the right edge blends it with weight 0 (an infinity there, times 0, would be NaN)
+    // one column of zeros past the last: the right edge blends it with weight 0 (an infinity there, times 0, would be NaN).  Only the
+    // chunk that holds the last column has room for it: a chunk that ends one before reads all of its row
     for (uint32_t i = threadIdx.x; i < cols; i += kUpThreads) L[r * pitch + i] = (1.f - fy) * ld_f(X0 + i) + fy * ld_f(X1 + i);
-    if (hi == u.XW)
+    if (xb == u.XW)
       for (uint32_t i = threadIdx.x; i < p.Ci; i += kUpThreads) L[r * pitch + cols + i] = 0.f;
   }
   int2* tab = (int2*)(L + (((size_t)p.rb * pitch + 1) & ~(size_t)1));   // per output column: where its left source column lies, weight of the right one

@@ -52,6 +52,24 @@ def test_upsample_rows(dtype, shape, scale):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("shape,scale", [((1, 256, 2, 273), 4), ((2, 256, 3, 290), 4), ((1, 1500, 3, 21), 1), ((1, 1500, 2, 31), 1)])
+def test_upsample_rows_last_chunk_of_one_column(dtype, shape, scale):
+    """Rows cut into chunks (of 17 columns, of 5) whose last has one column, so that the one before ends at the last but one: it has
+    all of its row in shared memory and the table of columns right behind (of fewer words than a column has channels)."""
+    import torch
+    N, Cc, Hh, W = shape
+    x = _q(H.normal(1, shape), dtype)
+    want = orc.upsample_bilinear_fwd(x, scale)
+    t = (H.dev if dtype == "f32" else H.dev_bf16)(orc.nchw_to_nhwc(x))
+    y = torch.empty((N, Hh * scale, W * scale, Cc), dtype=t.dtype, device="cuda")
+    vx, vy = H.view_nhwc(t), H.view_nhwc(y)
+    abi.check(abi.lib().ad_upsample_bilinear_fwd(C.byref(vx), C.byref(vy), scale, 0, Hh, 0, H.stream()))
+    H.sync()
+    # two blends of two values: a rounding of each, and bf16's own
+    assert H.max_rel(orc.nhwc_to_nchw(H.host(y)), want) < (1e-6 if dtype == "f32" else 8e-3)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
 @pytest.mark.parametrize("Cc,W,scale", [(19, 40, 8), (3, 300, 4), (1, 1100, 2), (31, 70, 4), (2, 33, 16), (64, 18, 8), (5, 300, 2),
                                         (36, 25, 8), (107, 21, 4)])   # 6 blocks of 4 columns and one of the last, 5 and one
