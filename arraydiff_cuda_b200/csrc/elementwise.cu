@@ -572,6 +572,15 @@ __global__ void __launch_bounds__(384) im2col_pipe_kernel(View x, uint32_t C, ui
   }
   if (threadIdx.x == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
+// The limit belongs to the function, so every call sets the most that its path takes: of two threads with calls of different
+// sizes, one would lower it between the other's setting and its launch.
+constexpr size_t kIm2colPipeMost = 96 * 1024, kIm2colRowMost = 100 * 1024;
+template <typename K>
+static bool im2col_limit(K kernel, size_t most) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
 template <typename T>
 static int launch_im2col_row(const View& v, const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t sh, uint32_t sw, uint32_t dh,
                              uint32_t dw, uint32_t P, uint32_t Q, __nv_bfloat16* out, uint32_t ldo, uint32_t rowlen, uint32_t qseg, size_t smem,
@@ -579,10 +588,7 @@ static int launch_im2col_row(const View& v, const ad_tensor4* x, uint32_t kh, ui
   const bool even = dw == 1 && ((sw * x->C) & 1u) == 0;   // and the row pitch has the parity of a row of taps
   auto kern = even ? im2col_row_kernel<T, true> : im2col_row_kernel<T, false>;
   const uint32_t pairs = ldo / 2, threads = pairs > 256 ? 256 : 384 / pairs * pairs > 384 ? 384 : (384 / pairs * pairs + 31) / 32 * 32;
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return AD_ERR_CUDA;
-  }
+  if (smem > 48 * 1024 && !im2col_limit(kern, kIm2colRowMost)) return AD_ERR_CUDA;
   launch(kern, x->N * P * ((Q + qseg - 1) / qseg), threads, smem, s, v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, out, ldo, rowlen, qseg);
   return AD_OK;
 }
@@ -601,14 +607,11 @@ extern "C" int ad_im2col(const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t
     const uint32_t pairs = ldo / 2, reach = (kw - 1) * dw + 1;
     if (x->dtype == AD_BF16 && x->sc == 1 && x->sx == (int64_t)x->C && !((uintptr_t)x->base & 15u) && x->sn >= 0 && x->sy >= 0 && pairs <= 384 &&
         (sw * x->C) % 2 == 0) {
-      // two stages of input rows and a tile of 48 KB at most, three or four blocks per SM
+      // two stages of input rows and a tile of 48 KB at most; as many blocks per SM as fit, four at most
       const uint32_t qs = std::max(1u, std::min(Q, 24576u / ldo)), len = (((qs - 1) * sw + reach) * x->C + 14) / 8 * 8;
       const size_t need = 2 * ((size_t)kh * len * 2 + 16) + (size_t)qs * ldo * 2, segs = (size_t)x->N * P * ((Q + qs - 1) / qs);
-      if (need <= 96 * 1024 && segs < (1ull << 31)) {
-        if (need > 48 * 1024 && cudaFuncSetAttribute(adk::im2col_pipe_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) != cudaSuccess) {
-          cudaGetLastError();
-          return AD_ERR_CUDA;
-        }
+      if (need <= adk::kIm2colPipeMost && segs < (1ull << 31)) {
+        if (need > 48 * 1024 && !adk::im2col_limit(adk::im2col_pipe_kernel, adk::kIm2colPipeMost)) return AD_ERR_CUDA;
         const uint32_t per_sm = std::min(4u, (uint32_t)(220 * 1024 / (need + 1024)));
         launch(adk::im2col_pipe_kernel, (unsigned)std::min<size_t>(segs, adk::kNumSMs * per_sm), 384 / pairs * pairs > 32 ? (384 / pairs * pairs + 31) / 32 * 32 : 32,
                need, adk::as_stream(stream), v, x->C, x->H, x->W, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo, len, qs, (uint32_t)segs);
@@ -620,7 +623,7 @@ extern "C" int ad_im2col(const ad_tensor4* x, uint32_t kh, uint32_t kw, uint32_t
     uint32_t rowlen = ((qseg - 1) * sw + (kw - 1) * dw + 1) * x->C;
     rowlen += (rowlen ^ (kw * x->C)) & 1u;
     const size_t smem = (((size_t)kh * rowlen * 2 + 15) & ~(size_t)15) + 16;   // a masked pair may read past the last element
-    if (smem <= 100 * 1024 && (size_t)x->N * P * Q < (1ull << 31) && (size_t)Q * (ldo / 8) < (1ull << 31)) {
+    if (smem <= adk::kIm2colRowMost && (size_t)x->N * P * Q < (1ull << 31) && (size_t)Q * (ldo / 8) < (1ull << 31)) {
       int st = AD_OK;
       AD_DISPATCH_DTYPE(x->dtype, (st = adk::launch_im2col_row<T>(v, x, kh, kw, sh, sw, dh, dw, P, Q, (__nv_bfloat16*)out_bf16, ldo,
                                                                   rowlen, qseg, smem, adk::as_stream(stream))));

@@ -431,10 +431,11 @@ static int launch_ce(int32_t layout, uint32_t N, uint32_t C, uint32_t HW, const 
       const int rc = launch_ce_pair<BWD>(C, pixels, s, vec, x, label, loss, picked, dloss, dx, accumulate);
       if (rc != AD_OK) return rc;
     } else {
-      const int smem = (int)(2 * 256 * C * sizeof(T));
+      const int smem = (int)(2 * 256 * C * sizeof(T)), most = (int)(2 * 256 * ((C + 3) / 4 * 4) * sizeof(T));
       bool ok = true;
       auto go = [&](auto kernel) {
-        if (smem > 48 * 1024) ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
+        // the limit belongs to the function: the most that it takes, whatever other threads' class counts
+        if (smem > 48 * 1024) ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
         if (ok) launch(kernel, grid_for((pixels + 255) / 256, 1, 6), 256, smem, s, C, pixels, vec, x, label, loss, picked, dloss, dx, accumulate);
       };
       switch ((C + 3) / 4) {

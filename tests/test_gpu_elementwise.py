@@ -523,6 +523,38 @@ def test_patch_matrix(Cc, Hh, W, k, stride, dil, ldo, lift):
     assert torch.count_nonzero(out[:-1, k * k * Cc:]) == 0 and (out[-1] == 7).all()
 
 
+# channels, width, filter, row pitch: more than 48 KB of shared memory each, of different sizes
+@pytest.mark.parametrize("dtype,forms", [("bf16", [(3, 600, 7, 192), (3, 1300, 3, 32)]), ("f32", [(60, 300, 3, 544), (40, 300, 3, 360)])])
+def test_patch_matrices_of_two_threads(dtype, forms):
+    """Calls of different sizes from two threads: neither lowers the shared memory that the other's kernel may ask for."""
+    import threading
+
+    import torch
+    L = abi.lib()
+    jobs, status = [], [[], []]
+    for Cc, W, k, ldo in forms:
+        x = torch.rand(1, k, W, Cc, device="cuda").to(torch.float32 if dtype == "f32" else torch.bfloat16)
+        Q = (W - k) // 2 + 1
+        jobs.append((x, H.view_nhwc(x), k, Q, ldo, torch.full((Q, ldo), 7.0, dtype=torch.bfloat16, device="cuda"), torch.cuda.Stream()))
+    H.sync()
+
+    def work(i):
+        x, vx, k, Q, ldo, out, st = jobs[i]
+        for _ in range(2000):
+            status[i].append(L.ad_im2col(C.byref(vx), k, k, 2, 2, 1, 1, 1, Q, out.data_ptr(), ldo, C.c_void_p(st.cuda_stream)))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    H.sync()
+    assert all(len(s) == 2000 and not any(s) for s in status)
+    for x, _, k, Q, ldo, out, _ in jobs:
+        want = torch.stack([x[0, r, s:s + 2 * Q - 1:2] for r in range(k) for s in range(k)], 1).reshape(Q, -1).bfloat16()
+        assert torch.equal(out[:, :want.shape[1]], want)
+
+
 @pytest.mark.parametrize("shape", [(2, 3, 5, 8), (1, 3, 4, 13), (3, 1, 7, 4), (2, 4, 3, 40), (1, 2, 6, 257)])
 @pytest.mark.parametrize("lift,gap", [(0, 0), (1, 0), (4, 4), (0, 5)])
 def test_planes_to_pixels(shape, lift, gap):
