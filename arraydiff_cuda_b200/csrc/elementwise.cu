@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(512) im2col_row_kernel(View x, uint32_t C, uin
   const uint32_t p = row % P, n = row / P, cols = kh * kw * C, nq = Q - q0 < qseg ? Q - q0 : qseg;
   const bool packed = x.sc == 1 && x.sx == (long long)C;
   const T* src = (const T*)x.base + n * x.sn + (long long)p * sh * x.sy + (long long)q0 * sw * x.sx;
-  const uint32_t left = W - q0 * sw;   // input columns from the segment's first on
+  const uint32_t left = q0 * sw < W ? W - q0 * sw : 0u;   // input columns from the segment's first on
   const uint32_t have = packed ? (left * C < rowlen ? left * C : rowlen) : 0u;
   // eight rows at a time, so that a thread's loads are in flight together
   for (uint32_t r0 = 0; r0 < kh; r0 += 8)
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(384) im2col_pipe_kernel(View x, uint32_t C, ui
   const uint32_t per_row = rowlen / 8, r0 = threadIdx.x / per_row, k0 = threadIdx.x - r0 * per_row;
   auto fetch = [&](const Place& t, bool any, uint32_t buf) {
     if (any) {
-      const uint32_t left = (W - t.q * qseg * sw) * C, have = left < rowlen ? left : rowlen;
+      const uint32_t x0 = t.q * qseg * sw, left = x0 < W ? (W - x0) * C : 0u, have = left < rowlen ? left : rowlen;   // none: a segment past the last column
       const long long base = first_of(t);
       __nv_bfloat16* rows = (__nv_bfloat16*)(im2col_smem + buf * rows_bytes);
       for (uint32_t i = threadIdx.x, r = r0, k = k0; i < kh * per_row; i += blockDim.x, r = i / per_row, k = i - r * per_row) {

@@ -523,6 +523,29 @@ def test_patch_matrix(Cc, Hh, W, k, stride, dil, ldo, lift):
     assert torch.count_nonzero(out[:-1, k * k * Cc:]) == 0 and (out[-1] == 7).all()
 
 
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("Cc,Hh,W,k,stride,ldo,Q", [
+    (3, 9, 20, 3, 2, 512, 150),    # segments of 48 pixels: the second starts past the last column
+    (3, 6, 10, 3, 2, 728, 70),           # of 33
+    (4, 7, 50, 2, 1, 16, 400),           # of 1536 and of 128 by the other form
+])
+def test_patch_matrix_past_the_last_column(Cc, Hh, W, k, stride, ldo, Q, dtype):
+    """Output rows of several segments, of which some lie past the input's last column altogether: zeros, and nothing is read there."""
+    import torch
+    N, P = 2, (Hh - k) // stride + 3
+    x = H.uniform(70, (N, Hh, W, Cc))
+    t = H.dev(x) if dtype == "f32" else H.dev_bf16(x)
+    out = torch.full((N * P * Q + 1, ldo), 7.0, dtype=torch.bfloat16, device="cuda")
+    vx = H.view_nhwc(t)
+    abi.check(abi.lib().ad_im2col(C.byref(vx), k, k, stride, stride, 1, 1, P, Q, out.data_ptr(), ldo, H.stream()))
+    H.sync()
+    pad = torch.zeros((N, (P - 1) * stride + k + Hh, (Q - 1) * stride + k + W, Cc), device="cuda", dtype=torch.bfloat16)
+    pad[:, :Hh, :W] = t
+    want = torch.stack([pad[:, r:r + (P - 1) * stride + 1:stride, s:s + (Q - 1) * stride + 1:stride] for r in range(k) for s in range(k)], 3)
+    assert torch.equal(out[:-1, :k * k * Cc], want.reshape(N * P * Q, k * k * Cc))
+    assert torch.count_nonzero(out[:-1, k * k * Cc:]) == 0 and (out[-1] == 7).all()
+
+
 # channels, width, filter, row pitch: more than 48 KB of shared memory each, of different sizes
 @pytest.mark.parametrize("dtype,forms", [("bf16", [(3, 600, 7, 192), (3, 1300, 3, 32)]), ("f32", [(60, 300, 3, 544), (40, 300, 3, 360)])])
 def test_patch_matrices_of_two_threads(dtype, forms):
