@@ -1070,7 +1070,7 @@ static int launch_apply(const BnApply& a, const ad_tensor4* x, bool vec, bool pl
   } else {
     const size_t total = (size_t)x->N * x->C * x->H * x->W;
     const unsigned long long hw = (unsigned long long)x->H * x->W, chunks = planes_vec ? (hw + kPlaneApplyVec - 1) / kPlaneApplyVec : (hw + kPlaneApply - 1) / kPlaneApply;
-    if (!a.c_fastest && hw < (1ull << 31) && (unsigned long long)x->N * x->C * chunks < (1ull << 31)) {
+    if (total && !a.c_fastest && hw < (1ull << 31) && (unsigned long long)x->N * x->C * chunks < (1ull << 31)) {
       const unsigned grid = (unsigned)(x->N * x->C * chunks);
       if (planes_vec) launch(bn_apply_planes<float, MODE, true>, grid, 256, 0, s, a, (uint32_t)chunks);
       else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply_planes<T, MODE, false>, grid, 256, 0, s, a, (uint32_t)chunks)));

@@ -289,6 +289,27 @@ def test_batch_norm_two_phase_matches_single_call_across_strips():
 
 @pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("N,Hh,W", [(0, 4, 4), (2, 0, 4), (2, 4, 0)])
+def test_batch_norm_two_phase_of_an_empty_strip(layout, dtype, N, Hh, W):
+    """A strip without pixels beside others: the others' statistics for it, nothing to write."""
+    import torch
+    Cc = 8
+    dt = torch.float32 if dtype == "f32" else torch.bfloat16
+    t = torch.full((2, Cc, 4, 4) if layout == abi.AD_NCHW else (2, 4, 4, Cc), 3.0, dtype=dt, device="cuda")
+    v = H.view_nchw(t) if layout == abi.AD_NCHW else H.view_nhwc(t)
+    v.N, v.H, v.W = N, Hh, W
+    L = abi.lib()
+    total = torch.cat([torch.full((Cc,), 40.0), torch.full((Cc,), 120.0)]).cuda()
+    g, b, mean, invstd = torch.ones(Cc, device="cuda"), torch.zeros(Cc, device="cuda"), torch.empty(Cc, device="cuda"), torch.empty(Cc, device="cuda")
+    abi.check(L.ad_bn_finalize_apply(C.byref(v), C.byref(v), H.ptr(total), C.c_double(20), H.ptr(g), H.ptr(b), H.ptr(mean), H.ptr(invstd), None, f32(1e-5), 1,
+                                     H.stream()))
+    H.sync()
+    assert torch.all(mean == 2.0) and torch.allclose(invstd, torch.full_like(invstd, 2.00001 ** -0.5), rtol=1e-6)
+    assert torch.all(t == 3.0)
+
+
+@pytest.mark.parametrize("layout", [abi.AD_NCHW, abi.AD_NHWC])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("Cc", [5, 16])
 def test_maxpool_3x3_s2_on_padded_input(layout, dtype, Cc):
     """The reference's pool sees the explicit zero pad cells (pad value 0, not -inf)."""
