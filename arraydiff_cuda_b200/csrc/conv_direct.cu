@@ -168,7 +168,7 @@ size_t f32_dgrad_scratch(const ad_conv2d_args* a, uint32_t P, uint32_t Q);
 // 10 - 19 us for the smallest calls too; but these sums of 9 terms and of channels are the more precise ones, 0.75e-7 against
 // 0.85 - 1.2e-7, and the calls stay here.)
 static bool direct_wins(const ConvG& g, int pass) {
-  if (const char* t = getenv("ARRAYDIFF_B200_F32_TILES")) return t[0] == '0';   // the parity tests: "1" tiled, "0" direct
+  if (const char* t = getenv("ARRAYDIFF_B200_F32_TILES")) return t[0] == '0';   // the parity tests: "1" tiled, "2" 3x3 kernels first (conv_f32.cu), "0" direct
   const double taps = (double)g.kh * g.kw, px = (double)g.N * g.P * g.Q, mmac = px * g.K * g.C * taps * 1e-6;
   const bool one = g.kh * g.kw == 1;
   auto most = [](double x, double y) { return x > y ? x : y; };

@@ -17,6 +17,7 @@
 // Measured on a B200 against one thread per output (the kernels of conv_direct.cu, which remain for geometries outside
 // f32_gemm_ok and for the smallest calls, direct_wins): figures at the launchers.
 #include <algorithm>
+#include <cstdlib>
 
 #include "conv_f32.cuh"
 
@@ -283,6 +284,12 @@ static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uin
   return launch_f32(conv_gemm_f32<LM, WM, WN, DGRAD>, dim3(tn * cs, tm, classes), T::threads, T::smem, cs, p, l, s);
 }
 
+// The parity tests: "2" sends every layer that the 3x3 kernels can serve to them (conv_direct.cu has the other values)
+static bool f32_k3_forced() {
+  const char* t = getenv("ARRAYDIFF_B200_F32_TILES");
+  return t && t[0] == '2';
+}
+
 // The 3x3 kernels own blocks of 4 x 2 pixels.  Where more than a fifth of them lies past the edges of the map (a third, if the
 // reduction is long), for 16 rows and fewer, and for long reductions into few tiles of 32 rows, which go to 8 CTAs at
 // most, the general tiles are as fast or faster: 17 x 42 x 13 x 5 -> 346 channels, two thirds used, 25 against 31 us;
@@ -291,7 +298,9 @@ static int launch_gemm_f32(const GemmF32& p, uint32_t npx, uint32_t classes, uin
 // instead of 24 and three quarters of a tile's rows and pixels have to be used: 137 -> 209, 2 x 14 x 34, 0.71, 33 against 39 us;
 // 156 -> 276, 4 x 12 x 21, 0.82, the other way, 47 -> 43.
 static bool f32_k3_gemm_wins(const GemmF32& p, bool dgrad) {
-  if (p.kh != 3 || p.kw != 3 || p.sh != p.sw || p.sh > (dgrad ? 1u : 2u) || (p.sh == 2 && (p.dh != 1 || p.dw != 1)) || p.M <= 16) return false;
+  if (p.kh != 3 || p.kw != 3 || p.sh != p.sw || p.sh > (dgrad ? 1u : 2u) || (p.sh == 2 && (p.dh != 1 || p.dw != 1))) return false;
+  if (f32_k3_forced()) return true;
+  if (p.M <= 16) return false;
   const unsigned long long used = (unsigned long long)p.OH * p.OW, blocks = f32_k3_blocks(p.OH, p.OW, p.dh, p.dw);
   if (p.M <= 32 && p.CR > 128 && p.NI * blocks < (p.sh == 2 ? 48 : 24) * 32) return false;
   if (p.sh == 2 && p.M > 32 && 4 * used * p.M < 3 * 8 * blocks * ((p.M + 63) / 64 * 64)) return false;
@@ -545,8 +554,10 @@ bool f32_gemm_ok(const ad_conv2d_args* a, uint32_t P, uint32_t Q, long long y_pi
 // alone is split into 128 CTAs at most: with more than four stages for each, the general kernel, which has more of them, is
 // faster (8 x 24 x 60 x 60 -> 32: 47 against 56 us).
 static bool f32_k3_wgrad_wins(const ad_conv2d_args* a, uint32_t P, uint32_t Q) {
-  if (a->kh != 3 || a->kw != 3 || a->stride_h != a->stride_w || a->stride_h > 2 || a->K <= 16 || a->C < 16) return false;
+  if (a->kh != 3 || a->kw != 3 || a->stride_h != a->stride_w || a->stride_h > 2) return false;
   if (a->stride_h == 2 && (a->dil_h != 1 || a->dil_w != 1)) return false;
+  if (f32_k3_forced()) return true;
+  if (a->K <= 16 || a->C < 16) return false;
   if (a->K <= 64 && a->C <= (a->K <= 32 ? 32u : 16u) && (unsigned long long)a->N * P * f32_k3_segments(Q, a->dil_w) > 4 * 4 * 128) return false;
   // under dilation a segment's pixels are dil apart: seven tenths of segments and tiles together (27 x 41 x 14 x 33 -> 57, dilation 4,
   // 0.37: 39 against 54 us; 29 x 26 x 16 x 58 -> 177, 0.68: 118 against 131)

@@ -189,15 +189,22 @@ K3_CASES = [
     (2, 20, 20, 21, 64, 2, 1, 2),  # 20 x 21 under dilation 2: maps of 10 x 11 and 10 x 10
     (1, 30, 16, 27, 24, 0, 1, 3),  # 10 x 21: 4, 3 and 3 rows
     (2, 18, 24, 32, 70, 4, 1, 4),  # 24 x 32
+    # dilations that the rules send to the 3x3 kernels by themselves, in all three passes and in two
+    (2, 64, 32, 32, 64, 2, 1, 2), (2, 64, 48, 48, 64, 3, 1, 3), (1, 64, 64, 64, 70, 4, 1, 4),
+    (1, 5, 9, 12, 7, 3, 1, 3),     # fewer channels than a tile has rows; 9 x 12 under dilation 3: maps of 3 x 4
+    (1, 20, 11, 3, 18, 4, 1, 4),   # rows of 3 under dilation 4: a map and a segment without pixels
 ]
 
 
+# "1": as the rules choose (small maps stay with the general tiles), "2": the 3x3 kernels in every pass that they can serve (all but
+# the data gradient of a stride)
+@pytest.mark.parametrize("tiles", ["1", "2"])
 @pytest.mark.parametrize("scratch", [True, False])
 @pytest.mark.parametrize("case", K3_CASES)
-def test_conv_f32_3x3(case, scratch, monkeypatch):
+def test_conv_f32_3x3(case, scratch, tiles, monkeypatch):
     """The 3x3 kernels at the edges of their tiles, blocks, segments and splits, with strides and dilations; infinities stay where they have a weight."""
     import torch
-    monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", "1")
+    monkeypatch.setenv("ARRAYDIFF_B200_F32_TILES", tiles)
     N, Cc, Hh, W, K, pd, s, d = case
     x, w, b = H.uniform(1, (N, Cc, Hh, W)), H.normal(2, (K, Cc, 3, 3), float(np.sqrt(2.0 / (9 * Cc)))), H.normal(3, (K,))
     y_w = orc.conv2d_fprop(x, w, b, (s, s), (d, d), (pd, pd), omp=True)
