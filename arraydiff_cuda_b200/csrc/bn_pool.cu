@@ -58,7 +58,8 @@ static bool planes_vec_ok(const ad_tensor4* t) {
          ((unsigned long long)t->H * t->W) % 4 == 0 && (unsigned long long)t->H * t->W < (1ull << 31);
 }
 
-// NCHW-like: block (256) per (channel, split); threads stride over (n, y, x), 4 pixels at a time where the planes allow it (VEC).
+// NCHW-like: block (256) per (channel, split); threads stride over (n, y, x); the backward sums take 4 pixels at a time where the
+// planes of x and dy allow it (VEC), the forward ones always one.
 // The forward statistics are summed in fp32, one pixel after the other, and beside that in double, which a split writes as two
 // more rows of floats, high and low parts; bn_finish takes the double ones where the two differ (bn_statistics).  The
 // conversions and double additions are a tenth of what the SM can do in the time of the loads.
@@ -553,7 +554,7 @@ static void launch_finish(const BnFin& f, int nsplit, int dual, const float* par
 }
 // Both stages of the statistics of x (MODE 0) or of the backward sums (MODE 1) into what `f` names
 template <int MODE>
-static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, float* partial, cudaStream_t s, bool vec) {
+static int launch_reduce(const BnRed& p, const ad_tensor4* x, const BnFin& f, float* partial, cudaStream_t s, bool vec = false) {   // vec: MODE 1
   const bool cfast = x->sc == 1 && x->C > 1;
   int nsplit, dual = 0;
   BnFin fin = f;
@@ -1084,7 +1085,7 @@ extern "C" int ad_bn_partial_stats(const ad_tensor4* x, float* sums, void* scrat
   if (!x || !x->base || !sums || !scratch) return AD_ERR_BAD_ARG;
   if (scratch_bytes < ad_bn_scratch_bytes(x->C)) return AD_ERR_SCRATCH;
   BnRed p{bview(x), bview(x), x->N, x->C, x->H, x->W, 0, nullptr, nullptr, nullptr, nullptr};
-  return launch_reduce<0>(p, x, BnFin{2, x->C, 1.0, 0.f, nullptr, nullptr, nullptr, sums, nullptr, nullptr, 0}, (float*)scratch, as_stream(stream), planes_vec_ok(x));
+  return launch_reduce<0>(p, x, BnFin{2, x->C, 1.0, 0.f, nullptr, nullptr, nullptr, sums, nullptr, nullptr, 0}, (float*)scratch, as_stream(stream));
 }
 
 extern "C" int ad_bn_finalize_apply(const ad_tensor4* x, const ad_tensor4* y, const float* sums, double count,
@@ -1110,7 +1111,7 @@ extern "C" int ad_bn_fwd_train(const ad_tensor4* x, const ad_tensor4* y, const f
   cudaStream_t s = as_stream(stream);
   BnRed p{bview(x), bview(x), x->N, x->C, x->H, x->W, 0, nullptr, nullptr, nullptr, nullptr};
   const double count = (double)x->N * x->H * x->W;
-  int st = launch_reduce<0>(p, x, BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, (float*)scratch, s, planes_vec_ok(x));
+  int st = launch_reduce<0>(p, x, BnFin{0, x->C, count, eps, save_mean, save_invstd, batch_var, nullptr, nullptr, nullptr, 0}, (float*)scratch, s);
   if (st != AD_OK) return st;
   BnApply a{bview(x), bview(x), bview(y), bview(y), x->N, x->C, x->H, x->W, y->sc == 1 && y->C > 1, relu, 0,
             gamma, beta, save_mean, save_invstd, nullptr, 1, count};

@@ -137,10 +137,11 @@ inline uint32_t f32_held(void (*k)(Params), int threads, int smem, uint32_t cs, 
   return l.held[i] - 1;
 }
 
-// 3x3, stride and dilation 1 (conv_f32_k3.cu)
+// 3x3 (conv_f32_k3.cu): forward of stride 1 under any dilation or of stride 2, data gradient of stride 1 under any dilation
 template <bool DGRAD> int f32_k3_gemm(const GemmF32& p, cudaStream_t s);
 // 1x1 without padding (conv_f32_k1.cu)
 template <bool DGRAD> int f32_k1_gemm(const GemmF32& p, cudaStream_t s);
+// filter and bias gradient, as the forward pass
 F32Split f32_k3_wgrad_split(uint32_t K, uint32_t C, uint32_t N, uint32_t P, uint32_t Q, uint32_t stride, uint32_t dil);
 int f32_k3_wgrad(const WgradF32& p, uint32_t cs, cudaStream_t s);
 

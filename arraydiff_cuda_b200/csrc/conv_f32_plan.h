@@ -62,9 +62,11 @@ inline uint32_t f32_k3_segments(uint32_t Q, uint32_t dw) { return ((Q + dw - 1) 
 // Filter gradient of the 3x3 kernels: CTAs of a cluster x slices of the grid that share a tile's `all` stages of pixels
 struct F32Split { uint32_t cs, slices; };
 // A stage takes 3.0 us alone, 4.8 beside one other, 7.0 beside two: the most CTAs that are resident together win, up to what
-// their start, and writing and adding the slices' `words` (the gradient's size), cost.  The constants are a fit to 1000 times of
-// 40 layers: the choice is on average 1.6 % above the fastest (7.6 % with the forward kernels' ones: 256 -> 256, 4 x 14 x 14
-// 52 -> 44 us, 191 -> 75, 3 x 71 x 10 68 -> 54).  The slices' scratch stays within 32 MB.
+// their start, and writing and adding the slices' `words` (the gradient's size), cost.  The constants are not these times (which
+// are 1.3 and 2.1 where the longest counts 3) but a fit to 1000 times of whole calls of 40 layers: the choice is on average 1.6 %
+// above the fastest (7.6 % with the forward kernels' ones: 256 -> 256, 4 x 14 x 14 52 -> 44 us, 191 -> 75, 3 x 71 x 10 68 -> 54).
+// The slices' scratch stays within 32 MB.  The clusters that are held at a time are those of a whole GPU, not asked of the device:
+// the size of the scratch, which follows from the split, can be asked for where there is none.
 inline F32Split f32_k3_split(unsigned long long tiles, unsigned long long all, unsigned long long words, uint32_t sms, uint32_t per_sm) {
   // clusters of 1, 2, 4, 8 CTAs at a time, two or three CTAs per SM
   static const unsigned held2[4] = {296, 148, 70, 33}, held3[4] = {444, 222, 104, 48};
