@@ -109,7 +109,7 @@ def test_bn_planes_mean_far_above_the_spread(shape, gap):
     (_, tx, vx), (_, tdy, vdy) = _put(x, gap, 0), _put(dy, gap, 0)
     (_, ty, vy), (_, td, vd) = (_put(np.zeros(shape, np.float32), gap, 0) for _ in range(2))
     g_, b_ = H.dev(gamma), H.dev(beta)
-    mean, invstd, var, dg, db = (torch.ones(Cc, device="cuda") for _ in range(5))
+    mean, invstd, var, dg, db = (torch.zeros(Cc, device="cuda") for _ in range(5))     # the sums are added to
     L = abi.lib()
     scratch = torch.full((L.ad_bn_scratch_bytes(Cc),), 255, dtype=torch.uint8, device="cuda")
     sp, sb = H.ptr(scratch), scratch.numel()
