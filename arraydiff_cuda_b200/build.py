@@ -12,7 +12,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libarraydiff_b200.so")
 SOURCES = ["elementwise.cu", "segcopy.cu", "softmax.cu", "bn_pool.cu", "sync.cu", "conv_direct.cu", "conv_f32.cu", "conv_f32_k1.cu", "conv_f32_k3.cu", "conv_tc.cu", "conv_tc_row.cu", "upsample.cu", "head.cu"]
-HEADERS = ["bias_grad.cuh", "common.cuh", "conv_f32.cuh", "conv_f32_plan.h", "overlap.h", "tc_common.cuh"]
+HEADERS = ["bias_grad.cuh", "common.cuh", "conv_f32.cuh", "conv_f32_plan.h", "conv_tc_plan.h", "overlap.h", "tc_common.cuh"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",

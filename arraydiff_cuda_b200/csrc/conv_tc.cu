@@ -26,6 +26,7 @@
 #include <algorithm>
 
 #include "bias_grad.cuh"
+#include "conv_tc_plan.h"
 #include "overlap.h"
 #include "tc_common.cuh"
 
@@ -1149,29 +1150,6 @@ static int launch_wgrad(const CUtensorMap& mdy, const CUtensorMap& mx, const WgP
                    attr_done, s, mdy, mx, p);
 }
 
-// Input channels per CTA of the general filter-gradient kernel.  (A 256-wide tile halves the L2 fetches of the dy
-// tile but leaves room for two pipeline stages only: measured 15 % slower on the 512 -> 512 layers.)
-static int wgrad_bn(uint32_t C) { return C > 64 ? 128 : 64; }
-
-// Splits of the pixel range: the count with the shortest time by rounds of the machine's CTAs (pairs) and by what the partial
-// gradients cost on their way out and back (a pixel tile of an item takes about 0.5 us, 2.5 MB).  Most often that is as
-// many as fill one round; a count that leaves the last round nearly empty costs most: 1024 -> 256 channels 1x1, 65,536 pixels, 19
-// splits (152 items, 74 pairs) 62 us, 9 splits 45; 512 -> 512 3x3 on 64 x 4 x 7 pixels 3 splits 44, one 34.
-static uint32_t wgrad_splits(uint32_t sp_tiles, uint32_t KO, uint32_t C, uint32_t taps) {
-  const uint32_t BN = (uint32_t)wgrad_bn(C), ktiles = (KO + 127) / 128;
-  const bool pair = BN == 128 && ktiles % 2 == 0;
-  const unsigned long long outer = (unsigned long long)taps * (pair ? ktiles / 2 : ktiles) * ((C + BN - 1) / BN), units = pair ? kNumSMs / 2 : kNumSMs;
-  const double part = (double)KO * taps * C * 8 / 2.5e6;
-  uint32_t best = 1;
-  double best_cost = 0;
-  for (uint32_t n = 1; n <= sp_tiles && n <= 64; ++n) {   // above 64 the reduction takes a third trip to the L2 (64 -> 256: 36 us, 74 splits 39)
-    const double cost = (double)((outer * n + units - 1) / units) * ((sp_tiles + n - 1) / n) + n * part;
-    if (n == 1 || cost < best_cost) { best = n; best_cost = cost; }
-    if (outer * n > 8 * units) break;
-  }
-  return best;
-}
-
 static size_t round_1k(size_t b) { return (b + 1023) / 1024 * 1024; }
 // Gradient channel counts the tensor-core kernels take as they are: the data gradient reduces over K in
 // 64-channel slabs, the filter gradient needs 16-byte pixel pitches of dy.  Other counts (a 19-class head)
@@ -1198,7 +1176,7 @@ size_t conv_tc_scratch_bytes(const ad_conv2d_args* a, int pass) {
     uint32_t TN, TH, TW;
     pick_tile3(a->N, g.P, g.Q, a->stride_h, a->stride_w, TN, TH, TW);
     const uint32_t sp = ((a->N + TN - 1) / TN) * ((g.P + TH - 1) / TH) * ((g.Q + TW - 1) / TW);
-    size_t general = (size_t)wgrad_splits(sp, Kp, a->C, a->kh * a->kw) * wcount * 4;
+    size_t general = (size_t)wgrad_splits(sp, Kp, a->C, a->kh * a->kw, kNumSMs) * wcount * 4;
     size_t row = conv_tc_row_wgrad_scratch(a->N, a->C, a->K, a->kh, a->kw, a->stride_h, a->stride_w, a->dil_h, a->dil_w, g.P, g.Q);
     const size_t part = std::max(general + bias_grad_bytes(pixels, a->K), row);
     size_t b = 1024 + part;
@@ -1393,7 +1371,7 @@ int conv_tc_wgrad(const ad_conv2d_args* a, int32_t* status, cudaStream_t s) {
   p.ktiles = (Kp + 127) / 128;
   p.ctiles = (a->C + BN - 1) / BN;
   const uint32_t sp_tiles = p.tiles_b * p.tiles_y * p.tiles_x;
-  p.splits = wgrad_splits(sp_tiles, Kp, a->C, p.kh * p.kw);
+  p.splits = wgrad_splits(sp_tiles, Kp, a->C, p.kh * p.kw, kNumSMs);
   p.status = status;
   p.partial = (float*)part_base;
   const size_t wcount_p = (size_t)Kp * a->kh * a->kw * a->C;
