@@ -2,6 +2,8 @@
 // layer.  Small, HBM- / latency-bound kernels: the head works on [batch][channels] vectors.
 //   average pool:  CudnnPool2DOp with kAveragePool (reference src/op.cc:3346-3633; zoo.cc:1843-1852)
 //   linear:        CublasLinearOp (reference src/op.cc:1199-1340: cublasSgemm + bias add)
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace adk {
@@ -302,17 +304,71 @@ __global__ void __launch_bounds__(256) linear_fwd_kernel(uint32_t B, uint32_t I,
     if (o < O && j < nb) st_f(y + (size_t)(b0 + j) * O + o, acc[0] + (bias ? bias[o] : 0.f));
   }
 }
-// dx[b][i] (+)= sum_o dy[b][o] * w[o][i]: 16 warps share the rows o of 128 columns and 8 images, every 16th each; their sums are
-// added in order.  The gradients of the 8 images lie in shared memory, 1024 rows at a time.
-constexpr uint32_t kDxWarps = 16, kDxMaxO = 1024;
-constexpr int kDxSmem = (kDxMaxO * kLinB + kDxWarps * 32 * 32) * 4;
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(kDxWarps * 32) linear_dx_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ dy,
+// The same with a warp per output, the 8 images as fp32 in shared memory (1024 features at a time): rows of bf16 that no 8-byte load
+// reaches
+constexpr uint32_t kFwdI = 1024;
+template <typename T>
+__global__ void __launch_bounds__(256) linear_fwd_staged_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
+                                                                const float* __restrict__ w, const float* __restrict__ bias, T* y) {
+  grid_dependency();
+  __shared__ float xs[kLinB][kFwdI];
+  const uint32_t o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  for (uint32_t b0 = blockIdx.y * kLinB; b0 < B; b0 += gridDim.y * kLinB) {
+    const uint32_t nb = B - b0 < kLinB ? B - b0 : kLinB;
+    float acc[kLinB];
+#pragma unroll
+    for (uint32_t j = 0; j < kLinB; ++j) acc[j] = 0.f;
+    for (uint32_t i0 = 0; i0 < I; i0 += kFwdI) {
+      const uint32_t ni = I - i0 < kFwdI ? I - i0 : kFwdI;
+      __syncthreads();
+      for (uint32_t j = 0; j < kLinB; ++j)
+        for (uint32_t i = threadIdx.x; i < ni; i += 256) xs[j][i] = j < nb ? ld_f(x + (size_t)(b0 + j) * I + i0 + i) : 0.f;
+      __syncthreads();
+      if (o < O) {
+        const float* wr = w + (size_t)o * I + i0;
+        uint32_t i = lane;
+        for (; i + 7 * 32 < ni; i += 8 * 32) {
+          float wv[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) wv[u] = wr[i + u * 32];
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (uint32_t j = 0; j < kLinB; ++j) acc[j] = fmaf(xs[j][i + u * 32], wv[u], acc[j]);
+        }
+        for (; i < ni; i += 32) {
+          const float wv = wr[i];
+#pragma unroll
+          for (uint32_t j = 0; j < kLinB; ++j) acc[j] = fmaf(xs[j][i], wv, acc[j]);
+        }
+      }
+    }
+    if (o < O) {
+#pragma unroll
+      for (uint32_t j = 0; j < kLinB; ++j) {
+        const float v = warp_sum(acc[j]);
+        if (lane == 0 && j < nb) st_f(y + (size_t)(b0 + j) * O + o, v + (bias ? bias[o] : 0.f));
+      }
+    }
+  }
+}
+// Single loads of bf16 features bound the kernel of four outputs per warp, which reads each image's once for every four outputs
+// (64 x 2046 -> 100 33 us with the images in shared memory, 66; 256 x 2046 -> 4096 482, 610); short rows and, up to 1023 features,
+// many outputs run it all the same (1024 x 65 -> 4096 390, 170; 1024 x 511 -> 4096 682, 587).
+static bool lin_fwd_staged(bool vec, size_t es, uint32_t B, uint32_t I, uint32_t O) {
+  return !vec && es == 2 && B > 1 && (I >= 1024 || (I >= 256 && O < 1000));
+}
+// dx[b][i] (+)= sum_o dy[b][o] * w[o][i]: W warps share the rows o of 128 columns and 8 images, every W-th each; their sums are
+// added in order.  The gradients of the 8 images lie in shared memory, 1024 rows at a time.  W is 16, but where few rows in many
+// blocks leave a warp with less to sum than the W sums of the others (lin_dx_warps).
+constexpr uint32_t kDxMaxO = 1024;
+template <typename T, bool VEC, uint32_t W>
+__global__ void __launch_bounds__(W * 32) linear_dx_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ dy,
                                                                   const float* __restrict__ w, T* dx, int accumulate) {
   grid_dependency();
   extern __shared__ __align__(16) float lin_sm[];
-  float* const g = lin_sm;                                         // [row][image]
-  float* const part = lin_sm + kDxMaxO * kLinB;                    // [warp][image, column of four][lane]
+  float* const part = lin_sm;                                      // [warp][image, column of four][lane]
+  float* const g = lin_sm + W * 32 * 32;                           // [row][image]
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = blockIdx.x * 128;
   for (uint32_t b0 = blockIdx.y * kLinB; b0 < B; b0 += gridDim.y * kLinB) {
     const uint32_t nb = B - b0 < kLinB ? B - b0 : kLinB;
@@ -326,10 +382,10 @@ __global__ void __launch_bounds__(kDxWarps * 32) linear_dx_kernel(uint32_t B, ui
       __syncthreads();
 #pragma unroll
       for (uint32_t j = 0; j < kLinB; ++j)
-        for (uint32_t o = threadIdx.x; o < no; o += kDxWarps * 32) g[o * kLinB + j] = j < nb ? ld_f(dy + (size_t)(b0 + j) * O + oc + o) : 0.f;
+        for (uint32_t o = threadIdx.x; o < no; o += W * 32) g[o * kLinB + j] = j < nb ? ld_f(dy + (size_t)(b0 + j) * O + oc + o) : 0.f;
       __syncthreads();
 #pragma unroll 8
-      for (uint32_t o = warp; o < no; o += kDxWarps) {
+      for (uint32_t o = warp; o < no; o += W) {
         float wv[4];
         lin_ld4<float, VEC>(w + (size_t)(oc + o) * I, c0, lane, I, true, wv);
         const float4 g0 = *(const float4*)(g + o * kLinB), g1 = *(const float4*)(g + o * kLinB + 4);
@@ -345,12 +401,12 @@ __global__ void __launch_bounds__(kDxWarps * 32) linear_dx_kernel(uint32_t B, ui
 #pragma unroll
       for (int e = 0; e < 4; ++e) part[(warp * 32 + j * 4 + e) * 32 + lane] = acc[j][e];
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < 32 * 32; t += kDxWarps * 32) {
+    for (uint32_t t = threadIdx.x; t < 32 * 32; t += W * 32) {
       const uint32_t j = t >> 7, e = (t >> 5) & 3, i = lin_col<VEC>(c0, t & 31, e);
       if (j >= nb || i >= I) continue;
       float v = 0.f;
 #pragma unroll
-      for (uint32_t q = 0; q < kDxWarps; ++q) v += part[q * 32 * 32 + t];
+      for (uint32_t q = 0; q < W; ++q) v += part[q * 32 * 32 + t];
       T* d = dx + (size_t)(b0 + j) * I + i;
       st_f(d, accumulate ? ld_f(d) + v : v);
     }
@@ -426,9 +482,57 @@ __global__ void __launch_bounds__(128) linear_dw_kernel(uint32_t B, uint32_t I, 
     if (db && blockIdx.x == 0 && threadIdx.x < no) db[o0 + threadIdx.x] = accumulate ? db[o0 + threadIdx.x] + accb : accb;
   }
 }
+// The same by a thread per column: rows that no 16-byte load reaches
+template <typename T>
+__global__ void __launch_bounds__(256) linear_dw_column_kernel(uint32_t B, uint32_t I, uint32_t O, const T* __restrict__ x,
+                                                               const T* __restrict__ dy, float* dw, float* db, int accumulate) {
+  grid_dependency();
+  __shared__ __align__(16) float g[64][8];
+  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+  for (uint32_t o0 = blockIdx.y * 8; o0 < O; o0 += gridDim.y * 8) {
+    const uint32_t no = O - o0 < 8 ? O - o0 : 8;
+    float acc[8], accb[8], old[8];
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+      acc[j] = accb[j] = 0.f;
+      old[j] = accumulate && j < no && i < I ? dw[(size_t)(o0 + j) * I + i] : 0.f;
+    }
+    for (uint32_t b0 = 0; b0 < B; b0 += 64) {
+      const uint32_t nb = B - b0 < 64 ? B - b0 : 64;
+      __syncthreads();
+      for (uint32_t t = threadIdx.x; t < nb * 8; t += 256) g[t >> 3][t & 7] = (t & 7) < no ? ld_f(dy + (size_t)(b0 + (t >> 3)) * O + o0 + (t & 7)) : 0.f;
+      __syncthreads();
+      if (i < I) {
+#pragma unroll 8
+        for (uint32_t b = 0; b < nb; ++b) {
+          const float xv = ld_f(x + (size_t)(b0 + b) * I + i);
+          const float4 g0 = *(const float4*)&g[b][0], g1 = *(const float4*)&g[b][4];
+          const float gv[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+#pragma unroll
+          for (uint32_t j = 0; j < 8; ++j) { acc[j] = fmaf(gv[j], xv, acc[j]); accb[j] += gv[j]; }
+        }
+      }
+    }
+    if (i < I) {
+#pragma unroll
+      for (uint32_t j = 0; j < 8; ++j)
+        if (j < no) {
+          dw[(size_t)(o0 + j) * I + i] = accumulate ? old[j] + acc[j] : acc[j];
+          if (db && i == 0) db[o0 + j] = accumulate ? db[o0 + j] + accb[j] : accb[j];
+        }
+    }
+  }
+}
 // rows of four elements per load: x and dx of `es` bytes each
 static bool lin_vec(uint32_t I, const void* w, const void* x, size_t es) {
   return I % 4 == 0 && ((uintptr_t)w & 15u) == 0 && ((uintptr_t)x & (4 * es - 1)) == 0;
+}
+// Filter gradient with a thread per column.  Four columns per thread leave a quarter of the warps, which without 16-byte loads wait
+// three times as long (1024 x 2046 -> 100 fp32 181 us by columns, 478; 64 x 511 -> 1000 bf16 16, 33), but for a few images and
+// many outputs, where the stores count (1 x 2046 -> 4096: 18, 14).  Of 64 features in bf16 half a warp has work: 1024 x 64 ->
+// 4096 135, 161.
+static bool lin_dw_by_columns(bool vec, size_t es, uint32_t B, uint32_t I, uint32_t O) {
+  return vec ? es == 2 && I <= 64 && O >= 2048 : I < 512 || B > (O < 512 ? 0u : O < 2048 ? 4u : 16u);
 }
 
 }  // namespace adk
@@ -473,26 +577,41 @@ extern "C" int ad_linear_fwd(int32_t dtype, uint32_t batch, uint32_t in_features
   if (!x || !w || !y) return AD_ERR_BAD_ARG;
   if ((size_t)batch * out_features >= (1ull << 31) || (size_t)batch * in_features >= (1ull << 31)) return AD_ERR_LIMIT;
   if (batch == 0 || out_features == 0) return AD_OK;
-  const dim3 grid((unsigned)(((size_t)out_features + 31) / 32), lin_groups(batch, kLinB));
-  AD_DISPATCH_DTYPE(dtype, (launch(lin_vec(in_features, w, x, sizeof(T)) ? linear_fwd_kernel<T, true> : linear_fwd_kernel<T, false>, grid, 256, 0,
-                                   as_stream(stream), batch, in_features, out_features, (const T*)x, w, bias, (T*)y)));
+  AD_DISPATCH_DTYPE(dtype, {
+    const bool vec = lin_vec(in_features, w, x, sizeof(T)), staged = lin_fwd_staged(vec, sizeof(T), batch, in_features, out_features);
+    const unsigned per = staged ? 8 : 32;
+    launch(staged ? linear_fwd_staged_kernel<T> : vec ? linear_fwd_kernel<T, true> : linear_fwd_kernel<T, false>,
+           dim3((unsigned)(((size_t)out_features + per - 1) / per), lin_groups(batch, kLinB)), 256, 0, as_stream(stream), batch, in_features, out_features,
+           (const T*)x, w, bias, (T*)y);
+  });
   count_launch();
   return launch_status();
 }
 
-template <typename T, bool VEC>
+// Warps that share a block's rows.  16 x 4 KB of sums for 128 rows and fewer cost more than their products where the blocks fill the
+// machine (fp32, 1024 x 8192 -> 10 207 us with 16 warps, 43 with 4, -> 100 323, 145 with 8); fewer blocks are one chain of rows each.
+static uint32_t lin_dx_warps(uint32_t B, uint32_t I, uint32_t O) {
+  if (O > 128 || (unsigned long long)((I + 127) / 128) * lin_groups(B, kLinB) <= kNumSMs) return 16;
+  return O > 32 ? 8 : 4;
+}
+template <typename T, bool VEC, uint32_t W>
 static int launch_linear_dx(uint32_t B, uint32_t I, uint32_t O, const T* dy, const float* w, T* dx, int accumulate, cudaStream_t s) {
+  if (lin_dx_warps(B, I, O) != W) {
+    if constexpr (W > 4) return launch_linear_dx<T, VEC, W / 2>(B, I, O, dy, w, dx, accumulate, s);
+  }
+  constexpr uint32_t most = (kDxMaxO * kLinB + W * 32 * 32) * 4;
   static unsigned attr_done = 0;       // one bit per device
   int dev = 0;
   cudaGetDevice(&dev);
   if (!(attr_done & (1u << (dev & 31)))) {
-    if (cudaFuncSetAttribute(linear_dx_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDxSmem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(linear_dx_kernel<T, VEC, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
       cudaGetLastError();
       return AD_ERR_CUDA;
     }
     attr_done |= 1u << (dev & 31);
   }
-  launch(linear_dx_kernel<T, VEC>, dim3((I + 127) / 128, lin_groups(B, kLinB)), kDxWarps * 32, kDxSmem, s, B, I, O, dy, w, dx, accumulate);
+  const uint32_t smem = (std::min(O, kDxMaxO) * kLinB + W * 32 * 32) * 4;
+  launch(linear_dx_kernel<T, VEC, W>, dim3((I + 127) / 128, lin_groups(B, kLinB)), W * 32, smem, s, B, I, O, dy, w, dx, accumulate);
   return AD_OK;
 }
 
@@ -507,15 +626,23 @@ extern "C" int ad_linear_bwd(int32_t dtype, uint32_t batch, uint32_t in_features
   cudaStream_t s = as_stream(stream);
   if (dx && in_features) {
     AD_DISPATCH_DTYPE(dtype, {
-      const int st = lin_vec(in_features, w, w, sizeof(T)) ? launch_linear_dx<T, true>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s)
-                                                           : launch_linear_dx<T, false>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s);
+      const int st = lin_vec(in_features, w, w, sizeof(T)) ? launch_linear_dx<T, true, 16>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s)
+                                                           : launch_linear_dx<T, false, 16>(batch, in_features, out_features, (const T*)dy, w, (T*)dx, accumulate_dx, s);
       if (st != AD_OK) return st;
     });
     count_launch();
   }
   if (dw && in_features && out_features) {
-    const dim3 grid((in_features + 511) / 512, lin_groups(out_features, 8));
-    AD_DISPATCH_DTYPE(dtype, (launch(lin_vec(in_features, dw, x, sizeof(T)) ? linear_dw_kernel<T, true> : linear_dw_kernel<T, false>, grid, 128, 0, s, batch, in_features, out_features, (const T*)x, (const T*)dy, dw, db, accumulate_dw)));
+    AD_DISPATCH_DTYPE(dtype, {
+      const bool vec = lin_vec(in_features, dw, x, sizeof(T));
+      const unsigned groups = lin_groups(out_features, 8);
+      if (lin_dw_by_columns(vec, sizeof(T), batch, in_features, out_features))
+        launch(linear_dw_column_kernel<T>, dim3((in_features + 255) / 256, groups), 256, 0, s, batch, in_features, out_features, (const T*)x, (const T*)dy, dw, db,
+               accumulate_dw);
+      else
+        launch(vec ? linear_dw_kernel<T, true> : linear_dw_kernel<T, false>, dim3((in_features + 511) / 512, groups), 128, 0, s, batch, in_features, out_features,
+               (const T*)x, (const T*)dy, dw, db, accumulate_dw);
+    });
     count_launch();
   }
   return launch_status();

@@ -228,6 +228,46 @@ def test_linear_groups(dtype, B, I, O):
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("lift", [0, 1])                # bases off by one element: no vectors
+@pytest.mark.parametrize("B,I,O", [
+    (9, 1030, 17), (2, 1024, 9), (2, 259, 999), (3, 255, 40),      # images in shared memory: past its 1024 features, at the ends of its range
+    (600, 510, 10), (593, 512, 32), (600, 510, 33), (600, 512, 128), (600, 512, 129),   # 4, 8 and 16 warps per block of the data gradient
+    (70, 257, 9), (65, 64, 2048), (16, 66, 2049), (17, 66, 2048), (4, 70, 513), (5, 70, 513),   # filter gradient by columns or by fours
+])
+def test_linear_forms(dtype, lift, B, I, O):
+    """Each form of the three kernels at the ends of the range that its rule gives it, against 64 bits."""
+    import torch
+    x, w, b, dy = _q(H.normal(8, (B, I)), dtype), H.normal(9, (O, I), 0.1), H.normal(10, (O,)), _q(H.normal(11, (B, O)), dtype)
+    x64, w64, dy64 = x.astype(np.float64), w.astype(np.float64), dy.astype(np.float64)
+    dt, td = FMT[dtype][0], torch.float32 if dtype == "f32" else torch.bfloat16
+
+    def put(a, t):
+        flat = torch.full((a.size + 4,), 7.0, dtype=t, device="cuda")
+        flat[lift:lift + a.size] = torch.from_numpy(np.ascontiguousarray(a)).cuda().to(t).reshape(-1)
+        return flat, flat[lift:lift + a.size].view(a.shape)
+
+    (_, tx), (_, tw), (_, tb), (_, tdy) = put(x, td), put(w, torch.float32), put(b, torch.float32), put(dy, td)
+    outs = [put(np.ones((B, O), np.float32), td), put(np.ones_like(x), td), put(np.ones_like(w), torch.float32), put(np.ones_like(b), torch.float32)]
+    (_, y), (_, gx), (_, gw), (_, gb) = outs
+    L = abi.lib()
+    eps = 2.0 ** -24
+    half = 0.0 if dtype == "f32" else 2.0 ** -8                    # the result's own rounding
+    # a sum of n products: chains of at most n / 32 roundings of partial sums, and the sums of the chains
+    far = lambda got, want, mag, n, half: np.all(np.abs(H.host(got) - want) <= (n / 32 + 40) * eps * mag + half * np.abs(want) + 1e-6)  # noqa: E731
+    abi.check(L.ad_linear_fwd(dt, B, I, O, H.ptr(tx), H.ptr(tw), H.ptr(tb), H.ptr(y), H.stream()))
+    for acc in (1, 0):
+        abi.check(L.ad_linear_bwd(dt, B, I, O, H.ptr(tx), H.ptr(tw), H.ptr(tdy), H.ptr(gx), H.ptr(gw), H.ptr(gb), acc, acc, H.stream()))
+        H.sync()
+        assert far(gx, acc + dy64 @ w64, acc + np.abs(dy64) @ np.abs(w64), O, half)
+        assert far(gw, acc + dy64.T @ x64, acc + np.abs(dy64).T @ np.abs(x64), 32 * B, 0.0)
+        assert far(gb, acc + dy64.sum(0), acc + np.abs(dy64).sum(0), 32 * B, 0.0)
+    assert far(y, x64 @ w64.T + b, np.abs(x64) @ np.abs(w64).T + np.abs(b), I, half)
+    for flat, t in outs:                                           # nothing beside the results is written
+        t.fill_(7.0)
+        assert torch.all(flat == 7.0)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("shape,k,s", [
     ((1, 8, 3, 3), (3, 3), (2, 2)), ((2, 16, 33, 35), (3, 3), (2, 2)), ((1, 24, 17, 16), (2, 2), (2, 2)), ((1, 72, 18, 31), (3, 3), (1, 1)),
     ((1, 40, 20, 21), (2, 5), (1, 3)), ((2, 8, 65, 66), (3, 3), (4, 4)), ((1, 8, 40, 70), (7, 9), (2, 2)), ((1, 8, 37, 37), (17, 2), (1, 1)),
