@@ -290,14 +290,18 @@ __global__ void __launch_bounds__(256) bn_apply(BnApply p) {
   }
 }
 // The same for views that are not channel-fastest: a block serves part of one (image, channel) plane, so that the channel's
-// constants are read once and a pixel's place costs one 32-bit division (VEC: none, 4 pixels per load).  Element by
-// element over the whole tensor (bn_apply, with 64-bit divisions and the sums divided by the count for each) the 34
-// normalisations of an 18-layer net on 4 x 224 x 224 took 527 us, so 205; with the sums 867 -> 372.
+// constants are read once and a pixel's place costs one 32-bit division (VEC: none, 4 pixels per load).  Element by element
+// over the whole tensor (bn_apply, with 64-bit divisions and the sums divided by the count for each) the 34 normalisations
+// of an 18-layer net on 4 x 224 x 224 took 527 us, so 205; with the sums 867 -> 372.
+// Small planes: several per block, 2^shift threads each.  Fixed statistics, us element by element, with a block per plane, so: 64 x
+// 2048 x 7 x 7 44, 239, 30; 64 x 1024 x 14 x 14 81, 75, 24; backward 97, 306, 73 and 196, 130, 60.
 constexpr uint32_t kPlaneApply = 1024, kPlaneApplyVec = 2048;   // pixels per block
 template <typename T, int MODE, bool VEC>
-__global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunks) {
+__global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunks, uint32_t shift) {
   grid_dependency();
-  const uint32_t plane = blockIdx.x / chunks, chunk = blockIdx.x - plane * chunks, n = plane / p.C, c = plane - n * p.C, hw = p.H * p.W;
+  const uint32_t lanes = 1u << shift, lane = threadIdx.x & (lanes - 1), unit = (blockIdx.x << (8 - shift)) + (threadIdx.x >> shift);
+  const uint32_t plane = unit / chunks, chunk = unit - plane * chunks, n = plane / p.C, c = plane - n * p.C, hw = p.H * p.W;
+  if (n >= p.N) return;
   const float mean = p.mean[c], invstd = p.invstd[c], gam = p.gamma[c], bet = p.beta[c];
   const float m1 = MODE ? p.partial[2 * p.C + c] : 0.f, m2 = MODE ? p.partial[3 * p.C + c] : 0.f, scale = gam * invstd;
   const T *xb = (const T*)p.x.base + n * p.x.sn + c * p.x.sc, *db = (const T*)p.dy.base + n * p.dy.sn + c * p.dy.sc;
@@ -317,10 +321,10 @@ __global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunk
     constexpr int U = kPlaneApplyVec / 1024;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     float4 xv[U], g[U], old[U];
-    const uint32_t i0 = chunk * kPlaneApplyVec + threadIdx.x * 4;
+    const uint32_t i0 = chunk * kPlaneApplyVec + lane * 4;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint32_t i = i0 + u * 1024;
+      const uint32_t i = i0 + u * lanes * 4;
       xv[u] = g[u] = old[u] = zero;
       if (i < hw) {
         xv[u] = *(const float4*)(xb + i);
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunk
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint32_t i = i0 + u * 1024;
+      const uint32_t i = i0 + u * lanes * 4;
       if (i < hw)
         *(float4*)(ob + i) = make_float4(value(xv[u].x, g[u].x, old[u].x), value(xv[u].y, g[u].y, old[u].y), value(xv[u].z, g[u].z, old[u].z),
                                          value(xv[u].w, g[u].w, old[u].w));
@@ -341,7 +345,7 @@ __global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunk
     long long at[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const uint32_t i = chunk * kPlaneApply + u * 256 + threadIdx.x, y = i / p.W, x = i - y * p.W;
+      const uint32_t i = chunk * kPlaneApply + u * lanes + lane, y = i / p.W, x = i - y * p.W;
       xv[u] = g[u] = old[u] = 0.f;
       at[u] = y * p.out.sy + x * p.out.sx;
       if (i < hw) {
@@ -352,7 +356,7 @@ __global__ void __launch_bounds__(256) bn_apply_planes(BnApply p, uint32_t chunk
     }
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (chunk * kPlaneApply + u * 256 + threadIdx.x < hw) st_f(ob + at[u], value(xv[u], g[u], old[u]));
+      if (chunk * kPlaneApply + u * lanes + lane < hw) st_f(ob + at[u], value(xv[u], g[u], old[u]));
   }
 }
 
@@ -1072,9 +1076,12 @@ static int launch_apply(const BnApply& a, const ad_tensor4* x, bool vec, bool pl
     const size_t total = (size_t)x->N * x->C * x->H * x->W;
     const unsigned long long hw = (unsigned long long)x->H * x->W, chunks = planes_vec ? (hw + kPlaneApplyVec - 1) / kPlaneApplyVec : (hw + kPlaneApply - 1) / kPlaneApply;
     if (total && !a.c_fastest && hw < (1ull << 31) && (unsigned long long)x->N * x->C * chunks < (1ull << 31)) {
-      const unsigned grid = (unsigned)(x->N * x->C * chunks);
-      if (planes_vec) launch(bn_apply_planes<float, MODE, true>, grid, 256, 0, s, a, (uint32_t)chunks);
-      else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply_planes<T, MODE, false>, grid, 256, 0, s, a, (uint32_t)chunks)));
+      // as many threads per plane as its pixels take, eight (VEC) or four each
+      uint32_t shift = 0;
+      while (shift < 8 && ((unsigned long long)(planes_vec ? kPlaneApplyVec : kPlaneApply) >> (8 - shift)) < hw) ++shift;
+      const unsigned grid = (unsigned)((x->N * x->C * chunks + (256u >> shift) - 1) >> (8 - shift));
+      if (planes_vec) launch(bn_apply_planes<float, MODE, true>, grid, 256, 0, s, a, (uint32_t)chunks, shift);
+      else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply_planes<T, MODE, false>, grid, 256, 0, s, a, (uint32_t)chunks, shift)));
     } else AD_DISPATCH_DTYPE(x->dtype, (launch(bn_apply<T, MODE>, grid_for(total, 256, 16), 256, 0, s, a)));
   }
   count_launch();

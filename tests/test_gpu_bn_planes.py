@@ -50,6 +50,7 @@ PLANES = [
     ((3, 4, 5, 7), 0, 0), ((2, 3, 31, 67), 0, 0), ((9, 2, 45, 47), 0, 0),
     ((2, 3, 20, 60), 4, 0), ((2, 3, 40, 31), 1, 0), ((3, 4, 6, 6), 0, 1), ((2, 3, 28, 76), 0, 2),
     ((33, 40, 1, 1), 0, 0), ((16, 130, 7, 7), 0, 0), ((8, 520, 2, 2), 0, 0), ((4, 6, 1, 3), 0, 0),
+    ((3, 130, 1, 5), 0, 0), ((2, 65, 16, 16), 0, 0), ((2, 65, 4, 65), 0, 0), ((5, 67, 16, 17), 0, 1), ((5, 67, 3, 43), 2, 0),   # several planes per block, a last block of fewer
 ]
 
 
